@@ -268,6 +268,10 @@ size_t sd_backward_scratch_bytes(const sd_shape *shape);
 int sd_forward(const sd_forward_args *args, void *stream);
 int sd_backward(const sd_backward_args *args, void *stream);
 int sd_decode_step(const sd_decode_args *args, void *stream);
+/* The same step from other states than the ones it writes: C_in / S_in are only read (NULL: zero state), args->C and
+ * args->S receive the updated ones.  What a functional caller otherwise pays two device copies for. */
+int sd_decode_step_from(const sd_decode_args *args, const float *C_in, const float *S_in, void *stream);
+
 
 /*
  * Predictor only: the sub-owner entry oja_residual(target, source, beta, log_decay, query,

@@ -227,7 +227,7 @@ class NormGateArgs(ctypes.Structure):
 
 EXPORTS = (
     "sd_saved_bytes", "sd_forward_scratch_bytes", "sd_backward_scratch_bytes",
-    "sd_forward", "sd_backward", "sd_decode_step", "sd_forward_launches",
+    "sd_forward", "sd_backward", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
     "sd_backward_launches", "sd_panel_info", "sd_status_string", "sd_version",
     "sd_chunk_tokens", "sd_forward_static", "sd_panel_kind", "sd_device_fault", "sd_device_fault_clear",
     "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step", "sd_add_rmsnorm", "sd_swiglu",
@@ -287,6 +287,8 @@ def _declare(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.sd_backward.argtypes = [ctypes.POINTER(BackwardArgs), ctypes.c_void_p]
     lib.sd_decode_step.restype = ctypes.c_int
     lib.sd_decode_step.argtypes = [ctypes.POINTER(DecodeArgs), ctypes.c_void_p]
+    lib.sd_decode_step_from.restype = ctypes.c_int
+    lib.sd_decode_step_from.argtypes = [ctypes.POINTER(DecodeArgs), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     lib.sd_forward_launches.restype = ctypes.c_int
     lib.sd_forward_launches.argtypes = [sp]
     lib.sd_backward_launches.restype = ctypes.c_int

@@ -308,8 +308,6 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_state_scan_tc, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<true>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<false>, DECODE_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<true>, DECODE_SMEM)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) {
         void* w = nullptr;
         if ((e = cudaGetSymbolAddress(&w, g_scan_fault_word)) != cudaSuccess) return e;
@@ -374,6 +372,28 @@ bool operands_ok(const sd_operand* ops, int n) {
     for (int i = 0; i < n; ++i)
         if (ops[i].ptr == nullptr) return false;
     return true;
+}
+
+template <bool MIXER, int NS, int WARPS>
+cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int streams, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(streams * NS));
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = NS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = NS > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS>, p, m);
+}
+template <bool MIXER>
+int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, cudaStream_t stream) {
+    const cudaError_t e = decode_split(streams) == 4 ? launch_decode_ns<MIXER, 4, 8>(p, m, streams, stream)
+                                                     : launch_decode_ns<MIXER, 1, 16>(p, m, streams, stream);
+    mark(stream);
+    return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }
 
 }  // namespace
@@ -1142,12 +1162,11 @@ int sd_pack_rows(const sd_pack_rows_args* a, void* stream_) {
     return launch_status();
 }
 
-int sd_decode_step(const sd_decode_args* a, void* stream_) {
+static int decode_impl(const sd_decode_args* a, const float* C_in, const float* S_in, void* stream_) {
     if (!a || !shape_ok(&a->shape) || a->shape.T != 1) return SD_ERR_INVALID_ARGUMENT;
     if (!shape_supported(&a->shape)) return SD_ERR_UNSUPPORTED_SHAPE;
     const sd_operand ops[] = {a->u, a->h, a->q, a->keys, a->values, a->erase_raw, a->write_raw, a->log_decay, a->gamma};
     if (!operands_ok(ops, 9) || !a->C || !a->S || !a->y) return SD_ERR_INVALID_ARGUMENT;
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
     DecodeParams p;
     p.g = make_geometry(a->shape);
     p.u = make_operand(a->u, 2);
@@ -1159,13 +1178,20 @@ int sd_decode_step(const sd_decode_args* a, void* stream_) {
     p.wr = make_operand(a->write_raw, 2);
     p.ld = make_operand(a->log_decay, 4);
     p.gam = make_operand(a->gamma, 4);
+    p.Cin = C_in;
+    p.Sin = S_in;
     p.C = a->C;
     p.S = a->S;
     p.y = a->y;
-    if (configure_kernels() != cudaSuccess) return SD_ERR_NO_DEVICE;
-    k_decode_step<false><<<a->shape.B * a->shape.H, DEC_THREADS, DECODE_SMEM, stream>>>(p, MixerDecode{});
-    mark(stream);
-    return launch_status();
+    return launch_decode<false>(p, MixerDecode{}, a->shape.B * a->shape.H, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+int sd_decode_step(const sd_decode_args* a, void* stream_) {
+    return a ? decode_impl(a, a->C, a->S, stream_) : SD_ERR_INVALID_ARGUMENT;
+}
+
+int sd_decode_step_from(const sd_decode_args* a, const float* C_in, const float* S_in, void* stream_) {
+    return decode_impl(a, C_in, S_in, stream_);
 }
 
 int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) {
@@ -1184,10 +1210,10 @@ int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) {
     p.wr = make_operand(a->write_raw, 2);
     p.q = p.k = p.v = p.u;       // unused by the fused instantiation
     p.ld = p.gam = p.u;
-    p.C = a->C;
-    p.S = a->S;
+    p.Cin = p.C = a->C;
+    p.Sin = p.S = a->S;
     p.y = a->y;
-    MixerDecode m;
+    MixerDecode m{};
     m.qkv = reinterpret_cast<const __nv_bfloat16*>(a->qkv);
     m.qkv_sb = a->qkv_stride_b;
     m.conv_w = a->conv_weight;
@@ -1221,9 +1247,9 @@ int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) {
         return SD_ERR_INVALID_ARGUMENT;
     }
     if (m.norm_w != nullptr && m.gate == nullptr && m.gate_w == nullptr) return SD_ERR_INVALID_ARGUMENT;
-    if (configure_kernels() != cudaSuccess) return SD_ERR_NO_DEVICE;
-    k_decode_step<true><<<a->shape.B * a->shape.H, DEC_THREADS, DECODE_SMEM, stream>>>(p, m);
-    return launch_status();
+    auto al8 = [](const void* q, long long stride) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0 && (stride & 3) == 0; };
+    m.hid_vec = al8(m.decay_hidden, m.dh_sb) && al8(m.gate_hidden, m.gh_sb);
+    return launch_decode<true>(p, m, a->shape.B * a->shape.H, stream);
 }
 
 }  // extern "C"
