@@ -20,6 +20,9 @@ LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200.so")
 # the profiling build: same sources with -DSD_DIAGNOSTICS (phase clock stamps, per-launch events);
 # only bench.py's per-kernel breakdown loads it
 DIAG_LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200_diag.so")
+# the host side of the entry points (checks, tensors, autograd node) as a Python extension over the C ABI
+HOST_PATH = os.path.join(_BUILD, "sd_host.so")
+HOST_SOURCE = os.path.join(_SRC, "sd_host.cpp")
 HEADER_PATH = os.path.join(_ROOT, "include", "solvedelta_b200.h")
 
 NVCC_FLAGS = [
@@ -70,7 +73,35 @@ def build(force: bool = False, verbose: bool = False) -> str:
     for cmd, proc in jobs:
         if proc.wait() != 0:
             raise subprocess.CalledProcessError(proc.returncode, cmd)
+    _build_host(force)
     return LIB_PATH
+
+
+def _build_host(force: bool) -> None:
+    """Compile csrc/sd_host.cpp against the installed torch; it is linked to the product library by a path relative
+    to itself."""
+    if not force and os.path.exists(HOST_PATH):
+        built = os.path.getmtime(HOST_PATH)
+        if all(os.path.getmtime(p) <= built for p in (HOST_SOURCE, HEADER_PATH)):
+            return
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cxx = shutil.which("g++")
+    if cxx is None:
+        raise RuntimeError("g++ not found: cannot build " + os.path.basename(HOST_PATH))
+    cuda = os.path.dirname(os.path.dirname(_nvcc() or "/usr/local/cuda/bin/nvcc"))
+    includes = [p for p in cpp_extension.include_paths() if os.path.isdir(p)] + [
+        os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=sd_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[a for p in includes for a in ("-isystem", p)], HOST_SOURCE, "-o", HOST_PATH,
+           "-L" + _BUILD, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+           "-L" + torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    subprocess.check_call(cmd)
 
 
 class Shape(ctypes.Structure):
@@ -272,6 +303,27 @@ def load() -> ctypes.CDLL:
             "solvedelta_b200.build()'` (needs nvcc); there is no fallback path")
     _lib = _declare(ctypes.CDLL(LIB_PATH))
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The host extension; raises like :func:`load` if it has not been built."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: run solvedelta_b200.build(); there is no fallback path")
+        import importlib.util
+
+        import torch  # noqa: F401  (its shared objects must be loaded first)
+
+        spec = importlib.util.spec_from_file_location("sd_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def _declare(lib: ctypes.CDLL) -> ctypes.CDLL:

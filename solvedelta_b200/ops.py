@@ -75,96 +75,6 @@ def _fill_operands(args, tensors):
     args.gamma = _gamma_operand(gam)
 
 
-def _mask_bytes(mask: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """bool [B,T] -> the same bytes as uint8 (a view, no copy when contiguous)."""
-    if mask is None:
-        return None
-    return mask.contiguous().view(torch.uint8)
-
-
-class _SolveDeltaFunction(torch.autograd.Function):
-    """forward(u,h,q,k,v,log_decay,erase_raw,write_raw,gamma[B,T,H],C0|None,S0|None,valid|None,reset|None)
-    -> (y, C_T, S_T); k,v,erase_raw,write_raw are the 4-D views without the edit axis; valid / reset
-    are uint8 [B,T] token masks applied inside the kernels."""
-
-    @staticmethod
-    def forward(ctx, u, h, q, k, v, log_decay, erase_raw, write_raw, gamma, C0, S0, valid=None, reset=None):
-        lib = _lib.load()
-        device = u.device
-        B, T, H, r = u.shape
-        V = v.shape[-1]
-        shape = _shape(u, V)
-        with torch.cuda.device(device):
-            y = torch.empty(B, T, H, V, dtype=torch.bfloat16, device=device)
-            C_T = torch.empty(B, H, r, r, dtype=torch.float32, device=device)
-            S_T = torch.empty(B, H, r, V, dtype=torch.float32, device=device)
-            saved = _buffer(lib.sd_saved_bytes(ctypes.byref(shape)), device)
-            scratch = _buffer(lib.sd_forward_scratch_bytes(ctypes.byref(shape)), device)
-            C0c = None if C0 is None else C0.contiguous()
-            S0c = None if S0 is None else S0.contiguous()
-            args = _lib.ForwardArgs()
-            args.shape = shape
-            _fill_operands(args, (u, h, q, k, v, log_decay, erase_raw, write_raw, gamma))
-            args.C0, args.S0 = _ptr(C0c), _ptr(S0c)
-            args.y, args.C_T, args.S_T = y.data_ptr(), C_T.data_ptr(), S_T.data_ptr()
-            args.saved, args.saved_bytes = saved.data_ptr(), saved.numel()
-            args.scratch, args.scratch_bytes = scratch.data_ptr(), scratch.numel()
-            args.valid_mask, args.reset_mask = _ptr(valid), _ptr(reset)
-            _lib.check(lib.sd_forward(ctypes.byref(args), _stream_ptr(device)))
-        ctx.set_materialize_grads(False)
-        ctx.has_state = (C0 is not None, S0 is not None)
-        ctx.masks = (valid, reset)
-        ctx.save_for_backward(u, h, q, k, v, log_decay, erase_raw, write_raw, gamma, saved)
-        return y, C_T, S_T
-
-    @staticmethod
-    def backward(ctx, dy, dC_T, dS_T):
-        lib = _lib.load()
-        u, h, q, k, v, log_decay, erase_raw, write_raw, gamma, saved = ctx.saved_tensors
-        device = u.device
-        B, T, H, r = u.shape
-        V = v.shape[-1]
-        shape = _shape(u, V)
-        with torch.cuda.device(device):
-            if dy is None:
-                dy = torch.zeros(B, T, H, V, dtype=torch.bfloat16, device=device)
-            elif dy.dtype != torch.bfloat16 or dy.stride(-1) != 1:
-                dy = dy.to(torch.bfloat16).contiguous()
-            dC_T = None if dC_T is None else dC_T.float().contiguous()
-            dS_T = None if dS_T is None else dS_T.float().contiguous()
-            bf = dict(dtype=torch.bfloat16, device=device)
-            du = torch.empty(B, T, H, r, **bf)
-            dh = torch.empty(B, T, H, r, **bf)
-            dq = torch.empty(B, T, H, r, **bf)
-            dk = torch.empty(B, T, H, r, **bf)
-            dv = torch.empty(B, T, H, V, **bf)
-            der = torch.empty(B, T, H, r, **bf)
-            dwr = torch.empty(B, T, H, V, **bf)
-            dld = torch.empty(B, T, H, r, dtype=torch.float32, device=device)
-            dgam = torch.empty(B, T, H, dtype=torch.float32, device=device)
-            dC0 = torch.empty(B, H, r, r, dtype=torch.float32, device=device)
-            dS0 = torch.empty(B, H, r, V, dtype=torch.float32, device=device)
-            scratch = _buffer(lib.sd_backward_scratch_bytes(ctypes.byref(shape)), device)
-            args = _lib.BackwardArgs()
-            args.shape = shape
-            _fill_operands(args, (u, h, q, k, v, log_decay, erase_raw, write_raw, gamma))
-            args.dy = _operand(dy)
-            args.dC_T, args.dS_T = _ptr(dC_T), _ptr(dS_T)
-            args.saved, args.saved_bytes = saved.data_ptr(), saved.numel()
-            args.scratch, args.scratch_bytes = scratch.data_ptr(), scratch.numel()
-            args.du, args.dh, args.dq = du.data_ptr(), dh.data_ptr(), dq.data_ptr()
-            args.dkeys, args.dvalues = dk.data_ptr(), dv.data_ptr()
-            args.derase_raw, args.dwrite_raw = der.data_ptr(), dwr.data_ptr()
-            args.dlog_decay, args.dgamma = dld.data_ptr(), dgam.data_ptr()
-            args.dC0, args.dS0 = dC0.data_ptr(), dS0.data_ptr()
-            valid, reset = ctx.masks
-            args.valid_mask, args.reset_mask = _ptr(valid), _ptr(reset)
-            _lib.check(lib.sd_backward(ctypes.byref(args), _stream_ptr(device)))
-        has_C0, has_S0 = ctx.has_state
-        return (du, dh, dq, dk, dv, dld, der, dwr, dgam,
-                dC0 if has_C0 else None, dS0 if has_S0 else None, None, None)
-
-
 class _OjaResidual(torch.autograd.Function):
     """forward(target, source, beta[B,T,H], log_decay, query, C0|None) -> (frame_action, update, C_T)."""
 
@@ -266,27 +176,6 @@ def oja_residual(target: torch.Tensor, source: torch.Tensor, beta: torch.Tensor,
     return action, update, (final if output_final_state else None)
 
 
-def _decode_step(u, h, q, k, v, log_decay, erase_raw, write_raw, gamma, C0, S0, inplace=False):
-    lib = _lib.load()
-    device = u.device
-    B, T, H, r = u.shape
-    V = v.shape[-1]
-    with torch.cuda.device(device):
-        # the kernel updates the cache in place; by default it works on copies, as upstream returns new tensors
-        keep = inplace and C0 is not None and S0 is not None and C0.is_contiguous() and S0.is_contiguous()
-        C = (torch.zeros(B, H, r, r, dtype=torch.float32, device=device) if C0 is None
-             else (C0.detach() if keep else C0.detach().clone(memory_format=torch.contiguous_format)))
-        S = (torch.zeros(B, H, r, V, dtype=torch.float32, device=device) if S0 is None
-             else (S0.detach() if keep else S0.detach().clone(memory_format=torch.contiguous_format)))
-        y = torch.empty(B, 1, H, V, dtype=torch.bfloat16, device=device)
-        args = _lib.DecodeArgs()
-        args.shape = _shape(u, V)
-        _fill_operands(args, (u, h, q, k, v, log_decay, erase_raw, write_raw, gamma))
-        args.C, args.S, args.y = C.data_ptr(), S.data_ptr(), y.data_ptr()
-        _lib.check(lib.sd_decode_step(ctypes.byref(args), _stream_ptr(device)))
-    return y, C, S
-
-
 def solvedelta_residual_frame_native(
     u: torch.Tensor,
     h: torch.Tensor,
@@ -312,74 +201,11 @@ def solvedelta_residual_frame_native(
     kernels with neutral tokens (the upstream path pads with zero tokens,
     residual_frame/operator.py:218-245, which is the same arithmetic).
     """
-    if u.ndim != 4:
-        raise ValueError("u must have shape [B,T,H,r]")
-    batch, length, heads, rank = u.shape
-    if h.shape != u.shape or q.shape != u.shape:
-        raise ValueError("h and q must match u")
-    if keys.shape != (batch, length, heads, 1, rank):
-        raise ValueError("Residual-Frame SolveDelta requires keys [B,T,H,1,r]")
-    if values.ndim != 5 or values.shape[:4] != (batch, length, heads, 1):
-        raise ValueError("values must have shape [B,T,H,1,d_v]")
-    value_dim = values.shape[-1]
-    if associative_log_decay.shape != (batch, length, heads, rank):
-        raise ValueError("associative_log_decay must have shape [B,T,H,r]")
-    if erase_raw.shape != keys.shape or write_raw.shape != values.shape:
-        raise ValueError("erase_raw/write_raw shapes must match keys/values")
-    if geometry_write.shape not in ((heads,), (1, heads), (batch, length, heads)):
-        raise ValueError("geometry_write must have shape [H], [1,H], or [B,T,H]")
-    if u.device.type != "cuda" or u.dtype != torch.bfloat16:
-        raise TypeError("the production Residual-Frame path requires BF16 CUDA operands")
-    if any(x.dtype != u.dtype for x in (h, q, keys, values, erase_raw, write_raw)):
-        raise TypeError("all public vector operands must be BF16")
-    if associative_log_decay.dtype != torch.float32:
-        raise TypeError("associative_log_decay must be FP32")
-    if geometry_write.dtype != torch.float32:
-        raise TypeError("geometry_write must be FP32")
-    if rank > 128 or value_dim > 128:
-        raise ValueError("the B200 kernels support head widths up to 128")
-    if any(x.stride(-1) != 1 for x in (u, h, q, keys, values, erase_raw, write_raw)):
-        raise ValueError("native vector operands require unit innermost stride")
-    if associative_log_decay.stride(-1) != 1:
-        associative_log_decay = associative_log_decay.contiguous()
-
-    predictor_initial = memory_initial = None
-    if initial_state is not None:
-        expected = ((batch, heads, rank, rank), (batch, heads, rank, value_dim))
-        if any(value.shape != exp for value, exp in zip(initial_state, expected)):
-            raise ValueError("initial_state shapes do not match the input geometry")
-        if any(value.dtype != torch.float32 for value in initial_state):
-            raise TypeError("all continuation states must be FP32")
-        predictor_initial, memory_initial = initial_state
-
-    if geometry_write.shape != (batch, length, heads):
-        geometry_write = geometry_write.reshape(1, 1, heads).expand(batch, length, heads)
-
-    k4, v4 = keys.squeeze(-2), values.squeeze(-2)
-    er4, wr4 = erase_raw.squeeze(-2), write_raw.squeeze(-2)
-
-    if length == 0:
-        output = values.new_zeros(batch, 0, heads, value_dim)
-        if not return_final_state:
-            return output, None
-        if initial_state is not None:
-            return output, initial_state
-        return output, solvedelta_zero_state(batch, heads, rank, value_dim, dtype=torch.float32,
-                                             device=u.device)
-
-    masked = _valid_mask is not None or _reset_mask is not None
-    if length == 1 and not torch.is_grad_enabled() and not masked:
-        # single-token recurrent inference (causallsso/ops/residual_frame/operator.py:198-216)
-        y, C, S = _decode_step(u, h, q, k4, v4, associative_log_decay, er4, wr4, geometry_write,
-                               predictor_initial, memory_initial, inplace=_inplace_state)
-        return y, (SolveDeltaState(C, S) if return_final_state else None)
-
-    y, C_T, S_T = _SolveDeltaFunction.apply(
-        u, h, q, k4, v4, associative_log_decay, er4, wr4, geometry_write,
-        predictor_initial, memory_initial, _mask_bytes(_valid_mask), _mask_bytes(_reset_mask))
-    if not return_final_state:
-        return y, None
-    return y, SolveDeltaState(predictor=C_T, S=S_T)
+    C0, S0 = (None, None) if initial_state is None else initial_state
+    y, C, S = _lib.host().residual_frame(
+        u, h, q, keys, values, associative_log_decay, erase_raw, write_raw, geometry_write, C0, S0,
+        return_final_state, _valid_mask, _reset_mask, _inplace_state)
+    return y, (SolveDeltaState(C, S) if return_final_state else None)
 
 
 def solvedelta_native(
@@ -403,19 +229,11 @@ def solvedelta_native(
     single-token no-grad step update the tensors of ``initial_state`` in place and return them, for a cache
     that owns its state; by default the step works on copies, as upstream returns new tensors.
     """
-    if u.device.type != "cuda" or u.dtype != torch.bfloat16:
-        raise TypeError("solvedelta_native requires BF16 CUDA activations")
-    if keys.ndim != 5 or keys.shape[-2] != 1:
-        raise ValueError("the current production path requires num_edits=1")
-    if erase_raw.shape != keys.shape or erase_raw.dtype != torch.bfloat16:
-        raise ValueError("erase_raw must be BF16 with the same shape as keys")
-    if write_raw.shape != values.shape or write_raw.dtype != torch.bfloat16:
-        raise ValueError("write_raw must be BF16 with the same shape as values")
-    if any(operand.stride(-1) != 1 for operand in (u, h, q, keys, values, erase_raw, write_raw)):
-        raise ValueError("native vector operands require unit innermost stride")
-    return solvedelta_residual_frame_native(
-        u, h, q, keys, values, associative_log_decay, erase_raw, write_raw, geometry_write,
-        initial_state=initial_state, return_final_state=return_final_state, _inplace_state=_inplace_state)
+    C0, S0 = (None, None) if initial_state is None else initial_state
+    y, C, S = _lib.host().dense(
+        u, h, q, keys, values, associative_log_decay, erase_raw, write_raw, geometry_write, C0, S0,
+        return_final_state, _inplace_state)
+    return y, (SolveDeltaState(C, S) if return_final_state else None)
 
 
 def solvedelta_segmented_native(
