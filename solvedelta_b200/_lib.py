@@ -22,7 +22,7 @@ LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200.so")
 DIAG_LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200_diag.so")
 # the host side of the entry points (checks, tensors, autograd node) as a Python extension over the C ABI
 HOST_PATH = os.path.join(_BUILD, "sd_host.so")
-HOST_SOURCE = os.path.join(_SRC, "sd_host.cpp")
+HOST_SOURCES = [os.path.join(_SRC, n) for n in ("sd_host.cpp", "sd_host_glue.cpp")]
 HEADER_PATH = os.path.join(_ROOT, "include", "solvedelta_b200.h")
 
 NVCC_FLAGS = [
@@ -78,11 +78,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 
 def _build_host(force: bool) -> None:
-    """Compile csrc/sd_host.cpp against the installed torch; it is linked to the product library by a path relative
-    to itself."""
+    """Compile the host sources against the installed torch; the extension is linked to the product library by a path
+    relative to itself."""
+    headers = (HEADER_PATH, os.path.join(_SRC, "sd_host.h"))
     if not force and os.path.exists(HOST_PATH):
         built = os.path.getmtime(HOST_PATH)
-        if all(os.path.getmtime(p) <= built for p in (HOST_SOURCE, HEADER_PATH)):
+        if all(os.path.getmtime(p) <= built for p in (*HOST_SOURCES, *headers)):
             return
     import sysconfig
 
@@ -95,13 +96,21 @@ def _build_host(force: bool) -> None:
     cuda = os.path.dirname(os.path.dirname(_nvcc() or "/usr/local/cuda/bin/nvcc"))
     includes = [p for p in cpp_extension.include_paths() if os.path.isdir(p)] + [
         os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    compile_ = [cxx, "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=sd_host",
+                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                *[a for p in includes for a in ("-isystem", p)], "-c"]
+    objects, jobs = [], []
+    for source in HOST_SOURCES:   # side by side: each takes most of a minute
+        objects.append(os.path.join(_BUILD, os.path.basename(source)[:-4] + ".o"))
+        cmd = [*compile_, source, "-o", objects[-1]]
+        jobs.append((cmd, subprocess.Popen(cmd)))
+    for cmd, proc in jobs:
+        if proc.wait() != 0:
+            raise subprocess.CalledProcessError(proc.returncode, cmd)
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=sd_host",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[a for p in includes for a in ("-isystem", p)], HOST_SOURCE, "-o", HOST_PATH,
-           "-L" + _BUILD, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
-           "-L" + torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
-    subprocess.check_call(cmd)
+    subprocess.check_call([cxx, "-shared", *objects, "-o", HOST_PATH,
+                           "-L" + _BUILD, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN",
+                           "-L" + torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
 
 
 class Shape(ctypes.Structure):

@@ -4,41 +4,9 @@
 // Why it is native: at T = 1 the kernel takes 7 us, and the same steps in Python (checks, nine ctypes operands, tensor
 // allocation, torch.autograd.Function) took 59 us a call forward-only and 300 us with the reverse pass, so short calls
 // were bound by the interpreter.
-#include <torch/extension.h>
-#include <torch/csrc/autograd/custom_function.h>
-
-#include <c10/cuda/CUDAGuard.h>
-#include <c10/cuda/CUDAStream.h>
-
-#include "../../include/solvedelta_b200.h"
-
-namespace py = pybind11;
-using at::Tensor;
-using OptTensor = std::optional<at::Tensor>;
-using torch::autograd::AutogradContext;
-using torch::autograd::variable_list;
+#include "sd_host.h"
 
 namespace {
-
-void check(int status) {
-    TORCH_CHECK(status == SD_OK, "solvedelta_b200: ", sd_status_string(status), " (status ", status, ")");
-}
-
-void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
-
-// [B,T,H,w] (any outer strides, unit inner stride) or [B,T,H] -> C operand
-sd_operand operand(const Tensor& t) { return sd_operand{t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
-
-float* f32(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
-const unsigned char* bytes(const Tensor& t) {
-    return t.defined() ? static_cast<const unsigned char*>(t.data_ptr()) : nullptr;
-}
-Tensor bf16_like(const Tensor& t, at::IntArrayRef shape) { return at::empty(shape, t.options().dtype(at::kBFloat16)); }
-Tensor f32_like(const Tensor& t, at::IntArrayRef shape) { return at::empty(shape, t.options().dtype(at::kFloat)); }
-Tensor workspace(const Tensor& t, size_t n) {
-    return at::empty({(int64_t)(n < 16 ? 16 : n)}, t.options().dtype(at::kByte));
-}
-Tensor given(const OptTensor& t) { return t.has_value() ? *t : Tensor(); }
 
 // The nine operands, k / v / gate logits without their edit axis, gamma as [B,T,H].
 struct Operands {
@@ -136,14 +104,6 @@ struct OperatorFunction : torch::autograd::Function<OperatorFunction> {
         return {du, dh, dq, dk, dv, dld, der, dwr, dgam, dC0, dS0, Tensor(), Tensor()};
     }
 };
-
-void value_error(bool bad, const char* text) {
-    if (bad) throw py::value_error(text);
-}
-void type_error(bool bad, const char* text) {
-    if (bad) throw py::type_error(text);
-}
-bool is_shape(const Tensor& t, at::IntArrayRef shape) { return t.sizes() == shape; }
 
 // bool [B,T] -> the same bytes, contiguous
 OptTensor mask_bytes(const OptTensor& m) { return m.has_value() ? OptTensor(m->contiguous()) : OptTensor(); }
@@ -246,4 +206,5 @@ py::tuple dense(const Tensor& u, const Tensor& h, const Tensor& q, const Tensor&
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("dense", &dense);
     m.def("residual_frame", &residual_frame);
+    register_glue(m);
 }

@@ -1,0 +1,741 @@
+// Host side of the mixer and block glue in C++: the autograd nodes of the glue kernels, and the mixer's sequence of
+// projections and glue around the operator.  A layer's forward and reverse pass is some sixty launches; in Python their
+// checks, ctypes blocks, autograd.Function and view objects cost 1.1 ms a layer forward + reverse and 0.3 ms for the
+// seven launches of a cached token, several times the device time of short sequences.
+#include "sd_host.h"
+
+namespace {
+
+Tensor bf16_contiguous(const Tensor& t) { return t.to(at::kBFloat16).contiguous(); }
+Tensor f32_contiguous(const Tensor& t) { return t.detach().to(at::kFloat).contiguous(); }
+
+void require_bf16_cuda(const char* name, const Tensor& t) {
+    if (!t.is_cuda() || t.scalar_type() != at::kBFloat16)
+        throw py::type_error(std::string(name) + " must be a BF16 CUDA tensor");
+}
+
+bool records_gradients(std::initializer_list<const Tensor*> tensors) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor* t : tensors)
+        if (t->defined() && t->requires_grad()) return true;
+    return false;
+}
+
+// FP32 copies of parameters that the inference kernels read in FP32, made again when a parameter has changed.
+struct Fp32Copies {
+    struct Entry {
+        const void* ptr = nullptr;
+        int64_t version = -1;
+        Tensor copy;
+    };
+    std::vector<Entry> entries;
+    Tensor get(size_t slot, const Tensor& t) {
+        if (t.scalar_type() == at::kFloat && t.is_contiguous()) return t.detach();
+        if (entries.size() <= slot) entries.resize(slot + 1);
+        Entry& e = entries[slot];
+        if (e.ptr != t.data_ptr() || e.version != (int64_t)t._version()) {
+            e.copy = f32_contiguous(t);
+            e.ptr = t.data_ptr();
+            e.version = (int64_t)t._version();
+        }
+        return e.copy;
+    }
+};
+
+// ---- depthwise causal conv (4 taps) + SiLU ------------------------------------------------------------------
+Tensor conv_forward(const Tensor& x, const Tensor& w32, const Tensor& init, Tensor fin, const Tensor& valid,
+                    const Tensor& reset) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor y = bf16_like(x, x.sizes());
+    sd_conv4_forward_args a{};
+    a.B = (int32_t)x.size(0); a.T = (int32_t)x.size(1); a.D = (int32_t)x.size(2);
+    a.x = x.data_ptr(); a.x_stride_b = x.stride(0); a.x_stride_t = x.stride(1);
+    a.weight = f32(w32);
+    a.initial_state = raw(init); a.y = y.data_ptr(); a.final_state = raw(fin);
+    a.valid_mask = bytes(valid); a.reset_mask = bytes(reset);
+    check(sd_conv4_silu_forward(&a, stream_of(x)));
+    return y;
+}
+
+struct ConvFunction : torch::autograd::Function<ConvFunction> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const OptTensor& init_in,
+                                 bool want_state, const OptTensor& valid, const OptTensor& reset) {
+        const Tensor w32 = f32_contiguous(weight);
+        const Tensor init = init_in.has_value() ? bf16_contiguous(init_in->detach()) : Tensor();
+        Tensor fin = want_state ? bf16_like(x, {x.size(0), x.size(2), 3}) : Tensor();
+        const Tensor y = conv_forward(x, w32, init, fin, given(valid), given(reset));
+        ctx->save_for_backward({x, w32, init, given(valid), given(reset)});
+        ctx->saved_data["dtype"] = (int64_t)weight.scalar_type();
+        ctx->set_materialize_grads(false);
+        if (!want_state) return {y};
+        ctx->mark_non_differentiable({fin});
+        return {y, fin};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        const Tensor &x = sv[0], &w32 = sv[1], &init = sv[2];
+        const auto dtype = (at::ScalarType)ctx->saved_data["dtype"].toInt();
+        const int64_t B = x.size(0), T = x.size(1), D = x.size(2);
+        const c10::cuda::CUDAGuard guard(x.device());
+        if (!grads[0].defined())
+            return {at::zeros_like(x), at::zeros({D, 4}, x.options().dtype(dtype)), Tensor(), Tensor(), Tensor(), Tensor()};
+        const Tensor dy = bf16_contiguous(grads[0]);
+        Tensor dx = bf16_like(x, x.sizes()), dw = f32_like(x, {D, 4});
+        Tensor dinit = init.defined() ? bf16_like(x, {B, D, 3}) : Tensor();
+        const Tensor scratch = workspace(x, sd_conv4_backward_scratch_bytes((int32_t)B, (int32_t)T, (int32_t)D));
+        sd_conv4_backward_args a{};
+        a.B = (int32_t)B; a.T = (int32_t)T; a.D = (int32_t)D;
+        a.x = x.data_ptr(); a.x_stride_b = x.stride(0); a.x_stride_t = x.stride(1);
+        a.weight = f32(w32); a.initial_state = raw(init);
+        a.dy = dy.data_ptr(); a.dx = dx.data_ptr(); a.dweight = f32(dw); a.dinitial_state = raw(dinit);
+        a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+        a.valid_mask = bytes(sv[3]); a.reset_mask = bytes(sv[4]);
+        check(sd_conv4_silu_backward(&a, stream_of(x)));
+        return {dx, dw.to(dtype), dinit, Tensor(), Tensor(), Tensor()};
+    }
+};
+
+OptTensor conv_mask(const char* name, const OptTensor& mask, const Tensor& x) {
+    if (!mask.has_value()) return std::nullopt;
+    if (mask->scalar_type() != at::kBool || !is_shape(*mask, {x.size(0), x.size(1)}))
+        throw py::value_error(std::string(name) + " must be bool [B,T]");
+    value_error(mask->device() != x.device(), "masks must share the activation device");
+    return mask->contiguous();
+}
+
+// (y, final state or undefined)
+std::pair<Tensor, Tensor> conv(const Tensor& x, const Tensor& weight, const OptTensor& init, bool want_state,
+                               const OptTensor& valid_in, const OptTensor& reset_in, bool inplace_state) {
+    require_bf16_cuda("x", x);
+    value_error(x.dim() != 3 || x.stride(-1) != 1, "x must be [B,T,D] with unit channel stride");
+    value_error(!is_shape(weight, {x.size(2), 4}), "conv weight must have shape [D,4]");
+    value_error(init.has_value() && !is_shape(*init, {x.size(0), x.size(2), 3}), "conv initial state must have shape [B,D,3]");
+    const OptTensor valid = conv_mask("valid_mask", valid_in, x), reset = conv_mask("reset_mask", reset_in, x);
+    if (x.size(1) == 0) {
+        Tensor fin;
+        if (want_state) fin = init.has_value() ? init->to(at::kBFloat16) : at::zeros({x.size(0), x.size(2), 3}, x.options());
+        return {at::zeros(x.sizes(), x.options()), fin};
+    }
+    const Tensor init_t = given(init);
+    if (!records_gradients({&x, &weight, &init_t})) {
+        // a cache that owns its state may have a single-token step update it in place: a thread reads the three
+        // entries of its channels before it writes them
+        const bool inplace = inplace_state && want_state && init.has_value() && x.size(1) == 1 &&
+                             !at::GradMode::is_enabled() && !valid.has_value() && !reset.has_value() &&
+                             init->scalar_type() == at::kBFloat16 && init->is_contiguous();
+        const Tensor state = init.has_value() ? bf16_contiguous(init->detach()) : Tensor();
+        Tensor fin = inplace ? state : want_state ? bf16_like(x, {x.size(0), x.size(2), 3}) : Tensor();
+        return {conv_forward(x.detach(), f32_contiguous(weight), state, fin, given(valid), given(reset)), fin};
+    }
+    const variable_list out = ConvFunction::apply(x, weight, init, want_state, valid, reset);
+    return {out[0], want_state ? out[1] : Tensor()};
+}
+
+py::tuple conv4_silu(const Tensor& x, const Tensor& weight, const OptTensor& init, bool want_state,
+                     const OptTensor& valid, const OptTensor& reset, bool inplace_state) {
+    const auto [y, fin] = conv(x, weight, init, want_state, valid, reset, inplace_state);
+    if (!fin.defined()) return py::make_tuple(y, py::none());
+    return py::make_tuple(y, fin);
+}
+
+// ---- decay gate ---------------------------------------------------------------------------------------------
+Tensor gate_forward(const Tensor& raw_in, const Tensor& A, const Tensor& b) {
+    const c10::cuda::CUDAGuard guard(raw_in.device());
+    const int64_t H = raw_in.size(-2), r = raw_in.size(-1);
+    Tensor out = f32_like(raw_in, raw_in.sizes());
+    sd_kda_gate_args a{};
+    a.rows = raw_in.numel() / (H * r); a.H = (int32_t)H; a.r = (int32_t)r;
+    a.raw = raw_in.data_ptr(); a.log_rate = f32(A); a.bias = f32(b); a.log_decay = f32(out);
+    check(sd_kda_gate_forward(&a, stream_of(raw_in)));
+    return out;
+}
+
+struct GateFunction : torch::autograd::Function<GateFunction> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& raw_in, const Tensor& log_rate, const Tensor& bias) {
+        const Tensor x = raw_in.contiguous(), A = f32_contiguous(log_rate), b = f32_contiguous(bias);
+        ctx->save_for_backward({x, A, b});
+        ctx->saved_data["rate_shape"] = log_rate.sizes().vec();
+        ctx->saved_data["bias_shape"] = bias.sizes().vec();
+        ctx->saved_data["rate_dtype"] = (int64_t)log_rate.scalar_type();
+        ctx->saved_data["bias_dtype"] = (int64_t)bias.scalar_type();
+        return gate_forward(x, A, b);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        const Tensor& x = sv[0];
+        const int64_t H = x.size(-2), r = x.size(-1), rows = x.numel() / (H * r);
+        const c10::cuda::CUDAGuard guard(x.device());
+        const Tensor dout = grads[0].to(at::kFloat).contiguous();
+        Tensor dx = at::empty_like(x), dA = f32_like(x, {H}), db = f32_like(x, {H, r});
+        const Tensor scratch = workspace(x, sd_kda_gate_backward_scratch_bytes(rows, (int32_t)H, (int32_t)r));
+        sd_kda_gate_args a{};
+        a.rows = rows; a.H = (int32_t)H; a.r = (int32_t)r;
+        a.raw = x.data_ptr(); a.log_rate = f32(sv[1]); a.bias = f32(sv[2]); a.dlog_decay = f32(dout);
+        a.draw = dx.data_ptr(); a.dlog_rate = f32(dA); a.dbias = f32(db);
+        a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+        check(sd_kda_gate_backward(&a, stream_of(x)));
+        return {dx, dA.reshape(ctx->saved_data["rate_shape"].toIntVector()).to((at::ScalarType)ctx->saved_data["rate_dtype"].toInt()),
+                db.reshape(ctx->saved_data["bias_shape"].toIntVector()).to((at::ScalarType)ctx->saved_data["bias_dtype"].toInt())};
+    }
+};
+
+Tensor kda_decay_gate(const Tensor& raw_in, const Tensor& log_rate, const Tensor& bias) {
+    require_bf16_cuda("raw", raw_in);
+    const int64_t H = raw_in.size(-2), r = raw_in.size(-1);
+    value_error(log_rate.numel() != H || bias.numel() != H * r, "log_rate must have H entries and bias H*r entries");
+    if (!records_gradients({&raw_in, &log_rate, &bias}))
+        return gate_forward(raw_in.detach().contiguous(), f32_contiguous(log_rate), f32_contiguous(bias));
+    return GateFunction::apply(raw_in, log_rate, bias);
+}
+
+// ---- sigmoid-gated RMSNorm, alone and in front of a projection ----------------------------------------------
+Tensor norm_gate_forward(const Tensor& x, const Tensor& gate, const Tensor& w, double eps) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor y = bf16_like(x, x.sizes());
+    sd_norm_gate_args a{};
+    a.V = (int32_t)x.size(-1); a.rows = x.numel() / a.V; a.eps = (float)eps;
+    a.x = x.data_ptr(); a.gate = gate.data_ptr(); a.weight = f32(w); a.y = y.data_ptr();
+    check(sd_norm_gate_forward(&a, stream_of(x)));
+    return y;
+}
+
+// (dx, dgate, dweight FP32)
+std::array<Tensor, 3> norm_gate_backward(const Tensor& x, const Tensor& gate, const Tensor& w, double eps, const Tensor& dy) {
+    Tensor dx = at::empty_like(x), dg = at::empty_like(gate), dw = f32_like(x, {x.size(-1)});
+    sd_norm_gate_args a{};
+    a.V = (int32_t)x.size(-1); a.rows = x.numel() / a.V; a.eps = (float)eps;
+    const Tensor scratch = workspace(x, sd_norm_gate_backward_scratch_bytes(a.rows, a.V));
+    a.x = x.data_ptr(); a.gate = gate.data_ptr(); a.weight = f32(w); a.dy = dy.data_ptr();
+    a.dx = dx.data_ptr(); a.dgate = dg.data_ptr(); a.dweight = f32(dw);
+    a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+    check(sd_norm_gate_backward(&a, stream_of(x)));
+    return {dx, dg, dw};
+}
+
+struct NormGateFunction : torch::autograd::Function<NormGateFunction> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& gate_in, const Tensor& weight, double eps) {
+        const Tensor x = x_in.contiguous(), gate = gate_in.contiguous(), w = f32_contiguous(weight);
+        ctx->save_for_backward({x, gate, w});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["dtype"] = (int64_t)weight.scalar_type();
+        return norm_gate_forward(x, gate, w, eps);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        const c10::cuda::CUDAGuard guard(sv[0].device());
+        const auto [dx, dg, dw] =
+            norm_gate_backward(sv[0], sv[1], sv[2], ctx->saved_data["eps"].toDouble(), bf16_contiguous(grads[0]));
+        return {dx, dg, dw.to((at::ScalarType)ctx->saved_data["dtype"].toInt()), Tensor()};
+    }
+};
+
+// Gated RMSNorm in front of a projection.  The normalised panel is not kept for the reverse pass: it is produced again
+// from x and gate there (one more pass of the norm kernel instead of a saved [..., H*D] BF16 tensor per layer).
+// causallsso/ops/norm_gate.py:46-159
+Tensor norm_linear_forward(const Tensor& x, const Tensor& gate, const Tensor& w, const Tensor& packed, const Tensor& bias, double eps) {
+    return at::linear(norm_gate_forward(x, gate, w, eps).flatten(-2), packed,
+                      bias.defined() ? OptTensor(bias.detach().to(at::kBFloat16)) : OptTensor());
+}
+// (dx, dgate, dweight of the norm FP32, dweight of the projection BF16, dbias FP32 or undefined)
+std::array<Tensor, 5> norm_linear_backward(const Tensor& x, const Tensor& gate, const Tensor& w, const Tensor& packed, bool bias,
+                                           double eps, const Tensor& dout_in) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Tensor dout = dout_in.to(at::kBFloat16).reshape({-1, dout_in.size(-1)});
+    Tensor dlinear;
+    {
+        const Tensor y = norm_gate_forward(x, gate, w, eps);   // regenerated, not saved
+        dlinear = at::mm(dout.t(), y.view({dout.size(0), -1}));
+    }
+    const auto [dx, dg, dw] = norm_gate_backward(x, gate, w, eps, at::mm(dout, packed).view(x.sizes()));
+    return {dx, dg, dw, dlinear, bias ? dout.to(at::kFloat).sum(0) : Tensor()};
+}
+
+struct NormGateLinearFunction : torch::autograd::Function<NormGateLinearFunction> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x_in, const Tensor& gate_in, const Tensor& norm_weight,
+                          const Tensor& weight, const OptTensor& bias, double eps) {
+        const Tensor x = x_in.contiguous(), gate = gate_in.contiguous(), w = f32_contiguous(norm_weight);
+        const Tensor packed = weight.detach().to(at::kBFloat16);
+        ctx->save_for_backward({x, gate, w, packed});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["norm_dtype"] = (int64_t)norm_weight.scalar_type();
+        ctx->saved_data["weight_dtype"] = (int64_t)weight.scalar_type();
+        ctx->saved_data["bias_dtype"] = bias.has_value() ? (int64_t)bias->scalar_type() : (int64_t)-1;
+        ctx->set_materialize_grads(false);
+        return norm_linear_forward(x, gate, w, packed, given(bias), eps);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+        const variable_list sv = ctx->get_saved_variables();
+        const int64_t bias_dtype = ctx->saved_data["bias_dtype"].toInt();
+        auto [dx, dg, dw, dlinear, dbias] = norm_linear_backward(sv[0], sv[1], sv[2], sv[3], bias_dtype >= 0,
+                                                                 ctx->saved_data["eps"].toDouble(), grads[0]);
+        if (dbias.defined()) dbias = dbias.to((at::ScalarType)bias_dtype);
+        return {dx, dg, dw.to((at::ScalarType)ctx->saved_data["norm_dtype"].toInt()),
+                dlinear.to((at::ScalarType)ctx->saved_data["weight_dtype"].toInt()), dbias, Tensor()};
+    }
+};
+
+void norm_gate_checks(const Tensor& x, const Tensor& gate, const Tensor& weight) {
+    require_bf16_cuda("x", x);
+    require_bf16_cuda("gate", gate);
+    value_error(x.sizes() != gate.sizes() || x.dim() < 2, "x and gate must have the same [...,H,D] shape");
+    value_error(!is_shape(weight, {x.size(-1)}), "weight must have shape [D]");
+}
+
+Tensor rms_norm_gated(const Tensor& x, const Tensor& gate, const Tensor& weight, double eps) {
+    norm_gate_checks(x, gate, weight);
+    if (!records_gradients({&x, &gate, &weight}))
+        return norm_gate_forward(x.detach().contiguous(), gate.detach().contiguous(), f32_contiguous(weight), eps);
+    return NormGateFunction::apply(x, gate, weight, eps);
+}
+
+Tensor rms_norm_gated_linear(const Tensor& x, const Tensor& gate, const Tensor& norm_weight, const Tensor& weight,
+                             const OptTensor& bias, double eps) {
+    norm_gate_checks(x, gate, norm_weight);
+    value_error(weight.dim() != 2 || weight.size(1) != x.size(-2) * x.size(-1), "the linear layer must take the flattened [H*D] rows");
+    const Tensor b = given(bias);
+    if (!records_gradients({&x, &gate, &norm_weight, &weight, &b}))
+        return norm_linear_forward(x.detach().contiguous(), gate.detach().contiguous(), f32_contiguous(norm_weight),
+                                   weight.detach().to(at::kBFloat16), b, eps);
+    return NormGateLinearFunction::apply(x, gate, norm_weight, weight, bias, eps);
+}
+
+// The two halves above for the node of rms_norm_gated_linear (mixer_ops.py), whose saved tensors callers can list.
+Tensor norm_linear_raw(const Tensor& x, const Tensor& gate, const Tensor& norm_weight, const Tensor& weight, const OptTensor& bias,
+                       double eps) {
+    norm_gate_checks(x, gate, norm_weight);
+    value_error(weight.dim() != 2 || weight.size(1) != x.size(-2) * x.size(-1), "the linear layer must take the flattened [H*D] rows");
+    return norm_linear_forward(x, gate, norm_weight, weight, given(bias), eps);
+}
+std::vector<OptTensor> norm_linear_raw_backward(const Tensor& x, const Tensor& gate, const Tensor& w, const Tensor& weight, bool bias,
+                                                double eps, const Tensor& dout) {
+    std::vector<OptTensor> out;
+    for (const Tensor& t : norm_linear_backward(x, gate, w, weight, bias, eps, dout)) out.push_back(optional(t));
+    return out;
+}
+
+// ---- residual add + RMSNorm ---------------------------------------------------------------------------------
+bool addnorm_reverse_ok(int64_t width) { return width > 0 && width % 256 == 0 && width <= 2048; }
+
+// (sum or undefined when delta is, normed)
+std::pair<Tensor, Tensor> addnorm_forward(const Tensor& x, const Tensor& delta, const Tensor& w, double eps) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor normed = at::empty_like(x), total = delta.defined() ? at::empty_like(x) : Tensor();
+    sd_add_rmsnorm_args a{};
+    a.D = (int32_t)x.size(-1); a.rows = x.numel() / a.D; a.eps = (float)eps;
+    a.x = x.data_ptr(); a.delta = raw(delta); a.weight = f32(w); a.sum = raw(total); a.normed = normed.data_ptr();
+    check(sd_add_rmsnorm(&a, stream_of(x)));
+    return {total, normed};
+}
+
+// (x + delta, RMSNorm(x + delta) * weight) with one reverse kernel: the cotangents of both outputs become the single
+// gradient that x and delta share, plus the weight gradient.  Only the sum is saved.  Without delta the sum is x itself
+// and only the norm is returned.
+struct AddNormFunction : torch::autograd::Function<AddNormFunction> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x_in, const OptTensor& delta_in, const Tensor& weight,
+                                 double eps) {
+        const Tensor x = x_in.contiguous(), delta = delta_in.has_value() ? delta_in->contiguous() : Tensor();
+        const Tensor w = f32_contiguous(weight);
+        const auto [total, normed] = addnorm_forward(x, delta, w, eps);
+        ctx->save_for_backward({delta.defined() ? total : x, w});
+        ctx->saved_data["eps"] = eps;
+        ctx->saved_data["delta"] = delta.defined();
+        ctx->saved_data["dtype"] = (int64_t)weight.scalar_type();
+        ctx->set_materialize_grads(false);
+        if (!delta.defined()) return {normed};
+        return {total, normed};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list sv = ctx->get_saved_variables();
+        const Tensor &total = sv[0], &w = sv[1];
+        const bool has_delta = ctx->saved_data["delta"].toBool();
+        const Tensor dtotal = has_delta ? grads[0] : Tensor(), dnormed = grads.back();
+        if (!dnormed.defined()) return {dtotal, has_delta ? dtotal : Tensor(), Tensor(), Tensor()};
+        const c10::cuda::CUDAGuard guard(total.device());
+        const Tensor dn = bf16_contiguous(dnormed), dt = dtotal.defined() ? bf16_contiguous(dtotal) : Tensor();
+        Tensor dx = at::empty_like(total), dw = f32_like(total, {total.size(-1)});
+        sd_add_rmsnorm_backward_args a{};
+        a.D = (int32_t)total.size(-1); a.rows = total.numel() / a.D; a.eps = (float)ctx->saved_data["eps"].toDouble();
+        const Tensor scratch = workspace(total, sd_add_rmsnorm_backward_scratch_bytes(a.rows, a.D));
+        a.sum = total.data_ptr(); a.weight = f32(w); a.dsum = raw(dt); a.dnormed = dn.data_ptr(); a.dx = dx.data_ptr();
+        a.dweight = f32(dw); a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+        check(sd_add_rmsnorm_backward(&a, stream_of(total)));
+        return {dx, has_delta ? dx : Tensor(), dw.to((at::ScalarType)ctx->saved_data["dtype"].toInt()), Tensor()};
+    }
+};
+
+py::tuple add_rmsnorm(const Tensor& x, const OptTensor& delta_in, const Tensor& weight, double eps) {
+    require_bf16_cuda("x", x);
+    const Tensor delta = given(delta_in);
+    if (delta.defined()) {
+        require_bf16_cuda("delta", delta);
+        value_error(x.sizes() != delta.sizes(), "x and delta must share a shape [...,D]");
+    }
+    value_error(!is_shape(weight, {x.size(-1)}), "weight must be [D]");
+    const bool reverse_ok = addnorm_reverse_ok(x.size(-1));
+    if (records_gradients({&x, &weight, &delta})) {
+        value_error(!reverse_ok, "the reverse pass takes rows of 256, 512, ..., 2048 channels");
+        const variable_list out = AddNormFunction::apply(x, delta_in, weight, eps);
+        return delta.defined() ? py::make_tuple(out[0], out[1]) : py::make_tuple(x, out[0]);
+    }
+    value_error(weight.scalar_type() != at::kFloat, "weight must be FP32 [D]");
+    value_error(!delta.defined() && !reverse_ok, "the norm alone takes rows of 256, 512, ..., 2048 channels");
+    const auto [total, normed] = addnorm_forward(x.detach().contiguous(), delta.defined() ? delta.detach().contiguous() : delta,
+                                                 weight.detach().contiguous(), eps);
+    return py::make_tuple(delta.defined() ? total : x, normed);
+}
+
+// ---- gated MLP ----------------------------------------------------------------------------------------------
+Tensor swiglu_forward(const Tensor& gv) {
+    const c10::cuda::CUDAGuard guard(gv.device());
+    std::vector<int64_t> shape = gv.sizes().vec();
+    shape.back() /= 2;
+    Tensor out = bf16_like(gv, shape);
+    sd_swiglu_args a{};
+    a.I = (int32_t)shape.back(); a.rows = out.numel() / a.I; a.gate_value = gv.data_ptr(); a.out = out.data_ptr();
+    check(sd_swiglu(&a, stream_of(gv)));
+    return out;
+}
+
+struct SwigluFunction : torch::autograd::Function<SwigluFunction> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& gate_value) {
+        const Tensor gv = gate_value.contiguous();
+        ctx->save_for_backward({gv});
+        return swiglu_forward(gv);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const Tensor gv = ctx->get_saved_variables()[0];
+        const c10::cuda::CUDAGuard guard(gv.device());
+        const Tensor dout = bf16_contiguous(grads[0]);
+        Tensor dgv = at::empty_like(gv);
+        sd_swiglu_args a{};
+        a.I = (int32_t)(gv.size(-1) / 2); a.rows = gv.numel() / (2 * a.I);
+        a.gate_value = gv.data_ptr(); a.dout = dout.data_ptr(); a.dgate_value = dgv.data_ptr();
+        check(sd_swiglu_backward(&a, stream_of(gv)));
+        return {dgv};
+    }
+};
+
+Tensor swiglu(const Tensor& gate_value) {
+    require_bf16_cuda("gate_value", gate_value);
+    value_error(gate_value.size(-1) % 2 != 0, "the last axis must hold gate and value halves");
+    if (records_gradients({&gate_value})) return SwigluFunction::apply(gate_value);
+    return swiglu_forward(gate_value.detach().contiguous());
+}
+
+constexpr int64_t GEMV_MAX_ROWS = 4;
+bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+
+// The projection of a cached single-token step in the one-warp-per-column kernel, or undefined when the call is not one
+// it takes.
+Tensor small_projection(const Tensor& x, const Tensor& weight, const Tensor& bias, bool with_swiglu) {
+    if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || weight.scalar_type() != at::kBFloat16 || weight.dim() != 2) return {};
+    const int64_t K = x.size(-1), N = weight.size(0);
+    const int64_t rows = K > 0 ? x.numel() / K : 0;
+    if (rows < 1 || rows > GEMV_MAX_ROWS || x.stride(-1) != 1 || records_gradients({&x, &weight})) return {};
+    if (weight.size(1) != K || !weight.is_contiguous() || weight.device() != x.device() || K % 8 != 0 ||
+        (bias.defined() && (bias.scalar_type() != at::kBFloat16 || !bias.is_contiguous())))
+        return {};
+    const Tensor x2 = x.reshape({rows, K});   // a view for the layouts a decode step produces
+    const int64_t stride = rows > 1 ? x2.stride(0) : K;
+    if (stride % 8 != 0 || !aligned16(x2) || !aligned16(weight) || (with_swiglu && N % 2 != 0)) return {};
+    const c10::cuda::CUDAGuard guard(x.device());
+    std::vector<int64_t> shape = x.sizes().vec();
+    shape.back() = with_swiglu ? N / 2 : N;
+    Tensor out = bf16_like(x, shape);
+    sd_gemv_args a{};
+    a.M = (int32_t)rows; a.N = (int32_t)N; a.K = (int32_t)K; a.swiglu = with_swiglu ? 1 : 0;
+    a.x = x2.data_ptr(); a.x_stride = stride; a.weight = weight.data_ptr(); a.bias = raw(bias);
+    a.y = out.data_ptr(); a.y_stride = shape.back();
+    check(sd_gemv(&a, stream_of(x)));
+    return out;
+}
+
+std::optional<Tensor> small_linear(const Tensor& x, const Tensor& weight, const OptTensor& bias, bool with_swiglu) {
+    return optional(small_projection(x, weight, given(bias), with_swiglu));
+}
+
+// x W^T (+ b) in the activation's type: the small kernel for a few rows, else the library product
+Tensor projection(const Tensor& x, const Tensor& weight_in, const OptTensor& bias_in) {
+    const Tensor weight = weight_in.to(x.scalar_type()), bias = bias_in.has_value() ? bias_in->to(x.scalar_type()) : Tensor();
+    const Tensor small = small_projection(x, weight, bias, false);
+    if (small.defined()) return small;
+    if (!bias.defined()) return at::linear(x, weight);
+    // one GEMM with the bias in its epilogue: on a strided slice of the projection row at::linear would run the product
+    // and a separate element-wise add
+    std::vector<int64_t> shape = x.sizes().vec();
+    shape.back() = weight.size(0);
+    return at::addmm(bias, x.reshape({-1, x.size(-1)}), weight.t()).view(shape);
+}
+
+Tensor gated_mlp(const Tensor& x, const Tensor& up, const OptTensor& up_bias, const Tensor& down, const OptTensor& down_bias) {
+    // a cached single-token step: projection + activation in one launch, then the second projection
+    Tensor act = small_projection(x, up, given(up_bias), true);
+    if (!act.defined()) act = swiglu(at::linear(x, up, up_bias));   // activation and product in one kernel
+    const Tensor out = small_projection(act, down, given(down_bias), false);
+    return out.defined() ? out : at::linear(act, down, down_bias);
+}
+
+// ---- slices of the fused projection row ---------------------------------------------------------------------
+// One BF16 row-shaped tensor holding `pieces` side by side (undefined: zeros), or undefined when the layout is not one
+// the kernel takes.
+Tensor pack(const variable_list& pieces, at::IntArrayRef widths, at::IntArrayRef row_shape, at::TensorOptions options) {
+    const int64_t P = row_shape.back();
+    if (!options.device().is_cuda() || widths.size() > SD_PACK_MAX_PIECES || P % 8 != 0) return {};
+    sd_pack_rows_args a{};
+    variable_list held(pieces.size());
+    for (size_t k = 0; k < widths.size(); ++k) {
+        if (widths[k] % 8 != 0 || (pieces[k].defined() && pieces[k].scalar_type() != at::kBFloat16)) return {};
+        if (pieces[k].defined()) held[k] = pieces[k].contiguous();
+        a.piece[k].src = raw(held[k]);
+        a.piece[k].width = (int32_t)widths[k];
+    }
+    const c10::cuda::CUDAGuard guard(options.device());
+    Tensor out = at::empty(row_shape, options.dtype(at::kBFloat16));
+    a.rows = out.numel() / P; a.pieces = (int32_t)widths.size(); a.row_width = (int32_t)P; a.dst = out.data_ptr();
+    check(sd_pack_rows(&a, stream_of(out)));
+    return out;
+}
+
+std::optional<Tensor> pack_rows(const std::vector<OptTensor>& pieces, const std::vector<int64_t>& widths,
+                                const std::vector<int64_t>& row_shape, const at::Device& device) {
+    variable_list list;
+    for (const OptTensor& p : pieces) list.push_back(given(p));
+    return optional(pack(list, widths, row_shape, at::TensorOptions().device(device)));
+}
+
+// Slices of the fused projection row as views (no copy), with a reverse pass that writes every slice gradient once into
+// one row-shaped buffer.  Plain slicing would make autograd allocate and add one zero-filled full row per slice (ten
+// rows of 7488 columns per token for the mixer).
+variable_list row_slices(const Tensor& row, at::IntArrayRef sizes) {
+    variable_list pieces;
+    int64_t start = 0;
+    for (const int64_t size : sizes) {
+        pieces.push_back(row.narrow(-1, start, size));
+        start += size;
+    }
+    return pieces;
+}
+
+struct SplitRowFunction : torch::autograd::Function<SplitRowFunction> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& row, std::vector<int64_t> sizes) {
+        ctx->saved_data["sizes"] = sizes;
+        ctx->saved_data["shape"] = row.sizes().vec();
+        ctx->saved_data["dtype"] = (int64_t)row.scalar_type();
+        ctx->saved_data["device"] = row.device();
+        ctx->set_materialize_grads(false);
+        return row_slices(row, sizes);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const std::vector<int64_t> sizes = ctx->saved_data["sizes"].toIntVector(), shape = ctx->saved_data["shape"].toIntVector();
+        const auto options = at::TensorOptions().device(ctx->saved_data["device"].toDevice())
+                                 .dtype((at::ScalarType)ctx->saved_data["dtype"].toInt());
+        bool any = false;
+        for (const Tensor& g : grads) any = any || g.defined();
+        if (!any) return {Tensor(), Tensor()};
+        if (options.dtype() == at::kBFloat16) {
+            const Tensor packed = pack(grads, sizes, shape, options);   // one kernel for the whole row
+            if (packed.defined()) return {packed, Tensor()};
+        }
+        Tensor drow = at::empty(shape, options);
+        int64_t start = 0;
+        for (size_t k = 0; k < sizes.size(); ++k) {
+            Tensor target = drow.narrow(-1, start, sizes[k]);
+            if (grads[k].defined()) target.copy_(grads[k]); else target.zero_();
+            start += sizes[k];
+        }
+        if (start < shape.back()) drow.narrow(-1, start, shape.back() - start).zero_();   // padding of the projection
+        return {drow, Tensor()};
+    }
+};
+
+// ---- the mixer around the operator --------------------------------------------------------------------------
+struct MixerShape {
+    int64_t heads, width, value_width;
+    // q | k | v stay one slice when they go through the conv, which reads it in place
+    std::vector<int64_t> sizes(bool conv) const {
+        const int64_t hr = heads * width, hv = heads * value_width;
+        if (conv) return {2 * hr + hv, hr, hr, hr, hv, heads, value_width, value_width};
+        return {hr, hr, hv, hr, hr, hr, hv, heads, value_width, value_width};
+    }
+};
+
+// From the hidden rows to the operator's operands: fused projection, conv4 + SiLU, decay gate, geometry rate, output
+// gate.  Returns (u, h, q, keys, values, log_decay, erase_raw, write_raw, geometry_write, output_gate, conv state |
+// None).  causallsso/model.py:321-394
+py::tuple mixer_front(const Tensor& x, int64_t heads, int64_t width, int64_t value_width, const Tensor& in_weight,
+                      const OptTensor& in_bias, const OptTensor& conv_weight, const OptTensor& conv_state,
+                      const OptTensor& valid, const OptTensor& reset, bool want_state, bool inplace_state,
+                      const Tensor& decay_weight, const Tensor& gate_weight, const OptTensor& gate_bias,
+                      const Tensor& log_rate, const Tensor& decay_bias, const Tensor& geometry_bias, bool geometry_enabled,
+                      bool decay_enabled) {
+    const MixerShape shape{heads, width, value_width};
+    const bool with_conv = conv_weight.has_value();
+    const std::vector<int64_t> sizes = shape.sizes(with_conv);
+    const Tensor row = projection(x, in_weight, in_bias);   // [B,T,P], slices stay views
+    const variable_list piece = records_gradients({&row}) ? SplitRowFunction::apply(row, sizes) : row_slices(row, sizes);
+    const auto view = [&](const Tensor& t, int64_t w) { return t.unflatten(-1, {heads, w}); };
+    Tensor q, k, v, fin;
+    size_t at = 1;
+    if (with_conv) {
+        const auto [qkv, state] = conv(piece[0], *conv_weight, conv_state, want_state, valid, reset, inplace_state);
+        fin = state;
+        const variable_list parts = qkv.split_with_sizes({heads * width, heads * width, heads * value_width}, -1);
+        q = parts[0]; k = parts[1]; v = parts[2];
+    } else {
+        q = at::silu(piece[0]); k = at::silu(piece[1]); v = at::silu(piece[2]);
+        at = 3;
+    }
+    const Tensor decay_raw = view(projection(piece[at + 5], decay_weight, std::nullopt), width);
+    const Tensor output_gate = view(projection(piece[at + 6], gate_weight, gate_bias), value_width);
+    Tensor log_decay = kda_decay_gate(decay_raw, log_rate, decay_bias);
+    Tensor geometry = at::sigmoid(piece[at + 4].to(at::kFloat) + geometry_bias.to(at::kFloat).view({1, 1, heads}));
+    if (!geometry_enabled) geometry = at::zeros_like(geometry);
+    if (!decay_enabled) log_decay = at::zeros_like(log_decay);
+    return py::make_tuple(view(piece[at], width), view(piece[at + 1], width), view(q, width), view(k, width).unsqueeze(-2),
+                          view(v, value_width).unsqueeze(-2), log_decay, view(piece[at + 2], width).unsqueeze(-2),
+                          view(piece[at + 3], value_width).unsqueeze(-2), geometry, output_gate,
+                          fin.defined() ? py::cast(fin) : py::none());
+}
+
+// One cached token between the fused projection row and the output projection, in one launch; argument meanings as in
+// mixer_decode_step (mixer_ops.py).
+struct DecodeToken {
+    Tensor u, h, erase, write, qkv, conv_weight, conv_state, decay_raw, log_rate, decay_bias, geometry_raw, geometry_bias;
+    Tensor predictor, memory, output_gate, norm_weight;
+    Tensor decay_hidden, decay_weight, gate_hidden, gate_weight, gate_bias;   // the fused gate projections, or undefined
+    double eps;
+};
+
+Tensor decode_launch(const DecodeToken& t) {
+    const int64_t B = t.u.size(0), H = t.u.size(2), r = t.u.size(3), V = t.write.size(-1), D = 2 * H * r + H * V;
+    value_error(t.u.size(1) != 1, "mixer_decode_step takes exactly one token");
+    const bool fused = t.decay_weight.defined();
+    for (const auto& [name, x] : {std::pair<const char*, const Tensor&>{"u", t.u}, {"h", t.h}, {"erase_raw", t.erase},
+                                  {"write_raw", t.write}, {"qkv", t.qkv}, {"geometry_raw", t.geometry_raw}, {"conv_state", t.conv_state}})
+        require_bf16_cuda(name, x);
+    if (!fused) require_bf16_cuda("decay_raw", t.decay_raw);
+    for (const auto& [name, x] : {std::pair<const char*, const Tensor&>{"conv_weight", t.conv_weight}, {"log_rate", t.log_rate},
+                                  {"decay_bias", t.decay_bias}, {"geometry_bias", t.geometry_bias},
+                                  {"predictor", t.predictor}, {"memory", t.memory}})
+        if (x.scalar_type() != at::kFloat || !x.is_contiguous()) throw py::type_error(std::string(name) + " must be contiguous FP32");
+    value_error(!is_shape(t.qkv, {B, 1, D}) || !is_shape(t.conv_state, {B, D, 3}) || !t.conv_state.is_contiguous(),
+                "qkv must be [B,1,D] and conv_state contiguous [B,D,3] with D = 2*H*r + H*V");
+    value_error(t.qkv.stride(-1) != 1 || t.geometry_raw.stride(-1) != 1 || (t.decay_raw.defined() && t.decay_raw.stride(-1) != 1),
+                "row operands require unit innermost stride");
+    const c10::cuda::CUDAGuard guard(t.u.device());
+    Tensor y = bf16_like(t.u, {B, 1, H, V});
+    sd_mixer_decode_args a{};
+    a.shape = sd_shape{(int32_t)B, 1, (int32_t)H, (int32_t)r, (int32_t)V};
+    a.u = operand(t.u); a.h = operand(t.h); a.erase_raw = operand(t.erase); a.write_raw = operand(t.write);
+    a.qkv = t.qkv.data_ptr(); a.qkv_stride_b = t.qkv.stride(0);
+    a.conv_weight = f32(t.conv_weight); a.conv_state = t.conv_state.data_ptr();
+    const Tensor decay = t.decay_raw.defined() ? t.decay_raw.contiguous().view({B, H * r}) : Tensor();
+    if (decay.defined()) {
+        a.decay_raw = decay.data_ptr();
+        a.decay_stride_b = decay.stride(0);
+    }
+    a.log_rate = f32(t.log_rate); a.decay_bias = f32(t.decay_bias);
+    a.geometry_raw = t.geometry_raw.data_ptr(); a.geometry_stride_b = t.geometry_raw.stride(0);
+    a.geometry_bias = f32(t.geometry_bias);
+    a.C = f32(t.predictor); a.S = f32(t.memory); a.y = y.data_ptr();
+    if (fused) {
+        const int64_t G = t.decay_hidden.size(-1);
+        for (const auto& [name, x] : {std::pair<const char*, const Tensor&>{"decay_hidden", t.decay_hidden}, {"decay_proj.weight", t.decay_weight},
+                                      {"gate_hidden", t.gate_hidden}, {"output_gate_proj.weight", t.gate_weight}})
+            require_bf16_cuda(name, x);
+        value_error(!is_shape(t.decay_weight, {H * r, G}) || !is_shape(t.gate_weight, {H * V, G}) || !t.decay_weight.is_contiguous() ||
+                        !t.gate_weight.is_contiguous() || G % 8 != 0 || G > 128 || !t.norm_weight.defined(),
+                    "fused gate projections: weights [H*r,G] / [H*V,G] contiguous, G a multiple of 8, at most 128, and the fused norm");
+        a.gate_rank = (int32_t)G;
+        a.decay_hidden = t.decay_hidden.data_ptr(); a.decay_hidden_stride_b = t.decay_hidden.stride(0);
+        a.gate_hidden = t.gate_hidden.data_ptr(); a.gate_hidden_stride_b = t.gate_hidden.stride(0);
+        a.decay_proj_weight = t.decay_weight.data_ptr(); a.gate_proj_weight = t.gate_weight.data_ptr();
+        a.gate_proj_bias = raw(t.gate_bias);
+    }
+    if (t.norm_weight.defined()) {
+        value_error(!fused && (!t.output_gate.defined() || t.output_gate.scalar_type() != at::kBFloat16 || !t.output_gate.is_contiguous()),
+                    "the fused norm needs a contiguous BF16 output_gate [B,1,H,V]");
+        type_error(t.norm_weight.scalar_type() != at::kFloat || !is_shape(t.norm_weight, {V}), "norm_weight must be FP32 [V]");
+        a.norm_weight = f32(t.norm_weight); a.norm_eps = (float)t.eps;
+        if (t.output_gate.defined()) {
+            a.output_gate = t.output_gate.data_ptr();
+            a.output_gate_stride_b = H * V;
+        }
+    }
+    check(sd_mixer_decode_step(&a, stream_of(t.u)));
+    return y;
+}
+
+Tensor mixer_decode_step(const Tensor& u, const Tensor& h, const Tensor& erase, const Tensor& write, const Tensor& qkv,
+                         const Tensor& conv_weight, const Tensor& conv_state, const OptTensor& decay_raw, const Tensor& log_rate,
+                         const Tensor& decay_bias, const Tensor& geometry_raw, const Tensor& geometry_bias, const Tensor& predictor,
+                         const Tensor& memory, const OptTensor& output_gate, const OptTensor& norm_weight, double eps,
+                         const OptTensor& decay_hidden, const OptTensor& decay_weight, const OptTensor& gate_hidden,
+                         const OptTensor& gate_weight, const OptTensor& gate_bias) {
+    const at::NoGradGuard no_grad;
+    return decode_launch(DecodeToken{u, h, erase, write, qkv, conv_weight, conv_state, given(decay_raw), log_rate, decay_bias,
+                                     geometry_raw, geometry_bias, predictor, memory, given(output_gate), given(norm_weight),
+                                     given(decay_hidden), given(decay_weight), given(gate_hidden), given(gate_weight),
+                                     given(gate_bias), eps});
+}
+
+// The whole mixer for one cached token without gradients: fused projection, decode launch (conv window and operator
+// states advanced in place), output projection.
+Tensor mixer_decode(Fp32Copies& copies, const Tensor& x, int64_t heads, int64_t width, int64_t value_width, const Tensor& in_weight,
+                    const OptTensor& in_bias, const Tensor& conv_weight, const Tensor& conv_state, const Tensor& decay_weight,
+                    const Tensor& gate_weight, const OptTensor& gate_bias, const Tensor& log_rate, const Tensor& decay_bias,
+                    const Tensor& geometry_bias, const Tensor& predictor, const Tensor& memory, const Tensor& norm_weight, double eps,
+                    const Tensor& out_weight, const OptTensor& out_bias) {
+    const MixerShape shape{heads, width, value_width};
+    const int64_t B = x.size(0);
+    const Tensor row = projection(x, in_weight, in_bias);
+    const variable_list piece = row_slices(row, shape.sizes(true));
+    const auto view = [&](const Tensor& t, int64_t w) { return t.unflatten(-1, {heads, w}); };
+    DecodeToken t;
+    t.u = view(piece[1], width); t.h = view(piece[2], width);
+    t.erase = view(piece[3], width); t.write = view(piece[4], value_width);
+    t.qkv = piece[0];
+    t.conv_weight = copies.get(0, conv_weight); t.conv_state = conv_state;
+    t.log_rate = copies.get(1, log_rate); t.decay_bias = copies.get(2, decay_bias);
+    t.geometry_raw = piece[5]; t.geometry_bias = copies.get(3, geometry_bias);
+    t.predictor = predictor; t.memory = memory;
+    t.norm_weight = copies.get(4, norm_weight); t.eps = eps;
+    const Tensor gb = given(gate_bias);
+    if (decay_weight.scalar_type() == at::kBFloat16 && gate_weight.scalar_type() == at::kBFloat16 && decay_weight.is_contiguous() &&
+        gate_weight.is_contiguous() && (!gb.defined() || gb.scalar_type() == at::kBFloat16) && decay_weight.size(1) % 16 == 0 &&
+        decay_weight.size(1) <= 128 && aligned16(decay_weight) && aligned16(gate_weight)) {
+        // the two small projections in front of the gates run inside the kernel too
+        t.decay_hidden = piece[6]; t.decay_weight = decay_weight;
+        t.gate_hidden = piece[7]; t.gate_weight = gate_weight; t.gate_bias = gb;
+    } else {
+        t.decay_raw = view(projection(piece[6], decay_weight, std::nullopt), width);
+        t.output_gate = view(projection(piece[7], gate_weight, gate_bias), value_width);
+    }
+    return projection(decode_launch(t).view({B, 1, heads * value_width}), out_weight, out_bias);
+}
+
+}  // namespace
+
+void register_glue(py::module_& m) {
+    // holds nothing that a copy or a pickle of its module has to carry
+    py::class_<Fp32Copies>(m, "Fp32Copies")
+        .def(py::init<>())
+        .def("get", &Fp32Copies::get)
+        .def("__deepcopy__", [](const Fp32Copies&, py::dict) { return Fp32Copies(); })
+        .def(py::pickle([](const Fp32Copies&) { return py::tuple(); }, [](py::tuple) { return Fp32Copies(); }));
+    m.def("conv4_silu", &conv4_silu);
+    m.def("kda_decay_gate", &kda_decay_gate);
+    m.def("rms_norm_gated", &rms_norm_gated);
+    m.def("rms_norm_gated_linear", &rms_norm_gated_linear);
+    m.def("norm_linear_forward", &norm_linear_raw);
+    m.def("norm_linear_backward", &norm_linear_raw_backward);
+    m.def("add_rmsnorm", &add_rmsnorm);
+    m.def("swiglu", &swiglu);
+    m.def("small_linear", &small_linear);
+    m.def("gated_mlp", &gated_mlp);
+    m.def("pack_rows", &pack_rows);
+    m.def("mixer_front", &mixer_front);
+    m.def("mixer_decode_step", &mixer_decode_step);
+    m.def("mixer_decode", &mixer_decode);
+}

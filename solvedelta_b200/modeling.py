@@ -24,7 +24,7 @@ from transformers.modeling_outputs import BaseModelOutputWithPast, CausalLMOutpu
 from . import _lib
 from .config import SolveDeltaConfig
 from .ops import SolveDeltaState
-from .mixer_ops import add_rmsnorm, add_rmsnorm_reverse_supported, small_linear, swiglu
+from .mixer_ops import add_rmsnorm, add_rmsnorm_reverse_supported, gated_mlp
 from .model import SolveDelta, SolveDeltaLayerState
 
 FP32_PARAMETERS = ("geometry_write_bias", "associative_log_rate", "associative_decay_bias")
@@ -130,12 +130,8 @@ class SolveDeltaMLP(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if self.hidden_act == "swish" and x.is_cuda and x.dtype == torch.bfloat16:
-            # a cached single-token step: projection + activation in one launch, then the second projection
-            act = small_linear(x, self.gate_up_proj.weight, self.gate_up_proj.bias, swiglu=True)
-            if act is None:
-                act = swiglu(self.gate_up_proj(x))   # activation and product in one kernel
-            out = small_linear(act, self.down_proj.weight, self.down_proj.bias)
-            return out if out is not None else self.down_proj(act)
+            up, down = self.gate_up_proj, self.down_proj
+            return gated_mlp(x, up.weight, up.bias, down.weight, down.bias)
         gate, value = self.gate_up_proj(x).chunk(2, dim=-1)
         if self.hidden_act == "swish":
             activated = F.silu(gate)
@@ -211,14 +207,10 @@ def _fp32_weight(norm: nn.Module) -> torch.Tensor:
     weight = norm.weight
     if torch.is_grad_enabled() and weight.requires_grad:
         return weight
-    if weight.dtype == torch.float32 and weight.is_contiguous():
-        return weight.detach()
-    key = (weight.data_ptr(), weight._version)
-    hit = norm.__dict__.get("_fp32_weight_copy")
-    if hit is None or hit[0] != key:
-        hit = (key, weight.detach().float().contiguous())
-        norm.__dict__["_fp32_weight_copy"] = hit
-    return hit[1]
+    copies = norm.__dict__.get("_fp32_weight_copy")
+    if copies is None:
+        copies = norm.__dict__["_fp32_weight_copy"] = _lib.host().Fp32Copies()
+    return copies.get(0, weight)
 
 
 class SolveDeltaBlock(nn.Module):
