@@ -193,6 +193,34 @@ typedef struct {
 int sd_gemv(const sd_gemv_args *args, void *stream);
 
 /*
+ * The same projection for up to SD_TOKEN_MAX_ROWS rows, with the block's residual add and RMSNorm in front of it:
+ * when norm_weight is given (M <= 8, K <= 2048) the rows of the product are RMSNorm(x + delta) * norm_weight, rounded
+ * as sd_add_rmsnorm rounds them, and sum receives x + delta (with delta == NULL: RMSNorm(x), sum unused).
+ * chained != 0: the launch may start while the kernel before it in the stream still runs and reads its weights
+ * meanwhile; x, delta and what that kernel wrote are read after it has finished.  The weights, and the states of
+ * sd_mixer_decode_step_chained, must then not be written by the kernel directly before.
+ * SD_ERR_UNSUPPORTED_SHAPE: more rows, rows that do not fit shared memory (about 200 KB in all), K or x_stride no
+ * multiple of 8, pointers off 16-byte boundaries.
+ */
+#define SD_TOKEN_MAX_ROWS 32
+typedef struct {
+    int32_t M, N, K;
+    int32_t swiglu;
+    const void *x;                     /* BF16 [M][K], rows x_stride elements apart */
+    int64_t x_stride;
+    const void *weight;                /* BF16 [N][K] contiguous */
+    const void *bias;                  /* BF16 [N] or NULL */
+    void *y;                           /* out BF16, rows y_stride elements apart */
+    int64_t y_stride;
+    const void *delta;                 /* BF16 [M][K], rows x_stride elements apart, or NULL */
+    const float *norm_weight;          /* [K] or NULL */
+    float norm_eps;
+    int32_t chained;
+    void *sum;                         /* out BF16 [M][K] contiguous */
+} sd_token_linear_args;
+int sd_token_linear(const sd_token_linear_args *args, void *stream);
+
+/*
  * Cross entropy over BF16 logits, the owner behind fuse_cross_entropy upstream
  * (FusedCrossEntropyLoss, causallsso/modeling_solvedelta.py:469-470).  Forward: per row the log-sum-exp
  * and -log softmax(label), 0 for rows whose label is ignore_index.  Backward: d logits =
@@ -258,6 +286,8 @@ typedef struct {
 } sd_mixer_decode_args;
 
 int sd_mixer_decode_step(const sd_mixer_decode_args *args, void *stream);
+/* The same launch chained to the one before it in the stream (see sd_token_linear). */
+int sd_mixer_decode_step_chained(const sd_mixer_decode_args *args, void *stream);
 
 /* Bytes of the buffer sd_forward fills for sd_backward. */
 size_t sd_saved_bytes(const sd_shape *shape);

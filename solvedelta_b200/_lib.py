@@ -187,6 +187,14 @@ class GemvArgs(ctypes.Structure):
                 ("bias", ctypes.c_void_p), ("y", ctypes.c_void_p), ("y_stride", ctypes.c_int64)]
 
 
+class TokenLinearArgs(ctypes.Structure):
+    _fields_ = [("M", ctypes.c_int32), ("N", ctypes.c_int32), ("K", ctypes.c_int32), ("swiglu", ctypes.c_int32),
+                ("x", ctypes.c_void_p), ("x_stride", ctypes.c_int64), ("weight", ctypes.c_void_p),
+                ("bias", ctypes.c_void_p), ("y", ctypes.c_void_p), ("y_stride", ctypes.c_int64),
+                ("delta", ctypes.c_void_p), ("norm_weight", ctypes.c_void_p), ("norm_eps", ctypes.c_float),
+                ("chained", ctypes.c_int32), ("sum", ctypes.c_void_p)]
+
+
 class CrossEntropyArgs(ctypes.Structure):
     _fields_ = [("rows", ctypes.c_int64), ("V", ctypes.c_int32), ("logits", ctypes.c_void_p),
                 ("labels", ctypes.c_void_p), ("ignore_index", ctypes.c_int64), ("lse", ctypes.c_void_p),
@@ -270,7 +278,8 @@ EXPORTS = (
     "sd_forward", "sd_backward", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
     "sd_backward_launches", "sd_panel_info", "sd_status_string", "sd_version",
     "sd_chunk_tokens", "sd_forward_static", "sd_panel_kind", "sd_device_fault", "sd_device_fault_clear",
-    "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step", "sd_add_rmsnorm", "sd_swiglu",
+    "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step",
+    "sd_mixer_decode_step_chained", "sd_token_linear", "sd_add_rmsnorm", "sd_swiglu",
     "sd_add_rmsnorm_backward_scratch_bytes", "sd_add_rmsnorm_backward", "sd_swiglu_backward", "sd_pack_rows",
     "sd_cross_entropy_forward", "sd_cross_entropy_backward", "sd_gemv",
     "sd_conv4_backward_scratch_bytes", "sd_conv4_silu_forward", "sd_conv4_silu_backward",
@@ -366,7 +375,8 @@ def _declare(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.sd_add_rmsnorm_backward_scratch_bytes.restype = ctypes.c_size_t
     lib.sd_add_rmsnorm_backward_scratch_bytes.argtypes = [ctypes.c_int64, ctypes.c_int32]
     for name, struct in (("sd_predictor_forward", PredictorForwardArgs), ("sd_predictor_backward", PredictorBackwardArgs),
-                         ("sd_mixer_decode_step", MixerDecodeArgs), ("sd_add_rmsnorm", AddRmsnormArgs),
+                         ("sd_mixer_decode_step", MixerDecodeArgs),
+                         ("sd_mixer_decode_step_chained", MixerDecodeArgs), ("sd_token_linear", TokenLinearArgs), ("sd_add_rmsnorm", AddRmsnormArgs),
                          ("sd_swiglu", SwigluArgs), ("sd_swiglu_backward", SwigluArgs),
                          ("sd_add_rmsnorm_backward", AddRmsnormBackwardArgs), ("sd_pack_rows", PackRowsArgs),
                          ("sd_cross_entropy_forward", CrossEntropyArgs), ("sd_cross_entropy_backward", CrossEntropyArgs),

@@ -14,6 +14,7 @@
 #include "sd_scan.cuh"
 #include "sd_scan_tc.cuh"
 #include "sd_output_tc.cuh"
+#include "sd_token.cuh"
 
 namespace {
 
@@ -308,6 +309,16 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_state_scan_tc, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<true>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 2, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 1, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 2, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 1, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<1, 2, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 1, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 2, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<4, 1, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<4, 2, 0>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) {
         void* w = nullptr;
         if ((e = cudaGetSymbolAddress(&w, g_scan_fault_word)) != cudaSuccess) return e;
@@ -374,24 +385,67 @@ bool operands_ok(const sd_operand* ops, int n) {
     return true;
 }
 
+// A launch whose kernel may start while the one before it in the stream still runs (it waits for it itself).
+cudaLaunchAttribute chained_launch() {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    return at;
+}
+
+template <int RG, int CG, int NORM>
+cudaError_t launch_token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) {
+    const int outs = p.swiglu ? p.N / 2 : p.N, width = p.swiglu ? 8 : 8 * CG, tiles = (outs + width - 1) / width;
+    const size_t smem = token_smem(p.M, p.K, NORM > 0);
+    const int resident = 148 * (RG <= 2 && smem <= TOKEN_SMEM_MAX / 2 ? 2 : 1);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(tiles < resident ? tiles : resident));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at = chained_launch();
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_token_linear<RG, CG, NORM>, p);
+}
+template <int CG>
+cudaError_t dispatch_token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) {
+    if (p.norm_w != nullptr)
+        return p.K <= 1024 ? launch_token_linear<1, CG, 4>(p, chained, stream) : launch_token_linear<1, CG, 8>(p, chained, stream);
+    if (p.M <= 8) return launch_token_linear<1, CG, 0>(p, chained, stream);
+    if (p.M <= 16) return launch_token_linear<2, CG, 0>(p, chained, stream);
+    return launch_token_linear<4, CG, 0>(p, chained, stream);
+}
+int token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) {
+    // 16 columns a tile while that gives every SM one, else 8
+    const cudaError_t e = p.swiglu || p.N >= 16 * 148 ? dispatch_token_linear<2>(p, chained, stream)
+                                                      : dispatch_token_linear<1>(p, chained, stream);
+    return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
+}
+
 template <bool MIXER, int NS, int WARPS>
-cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int streams, cudaStream_t stream) {
+cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(streams * NS));
     cfg.blockDim = dim3(WARPS * 32);
     cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = NS;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (chained) at[n++] = chained_launch();
+    if (NS > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = NS;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = NS > 1 ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS>, p, m);
 }
 template <bool MIXER>
-int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, cudaStream_t stream) {
-    const cudaError_t e = decode_split(streams) == 4 ? launch_decode_ns<MIXER, 4, 8>(p, m, streams, stream)
-                                                     : launch_decode_ns<MIXER, 1, 16>(p, m, streams, stream);
+int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
+    const cudaError_t e = decode_split(streams) == 4 ? launch_decode_ns<MIXER, 4, 8>(p, m, streams, chained, stream)
+                                                     : launch_decode_ns<MIXER, 1, 16>(p, m, streams, chained, stream);
     mark(stream);
     return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }
@@ -1123,18 +1177,36 @@ int sd_cross_entropy_backward(const sd_cross_entropy_args* a, void* stream_) {
 
 int sd_gemv(const sd_gemv_args* a, void* stream_) {
     if (!a || a->M <= 0 || a->N <= 0 || a->K <= 0 || !a->x || !a->weight || !a->y) return SD_ERR_INVALID_ARGUMENT;
-    if (a->M > GEMV_MAX_ROWS || a->K % 8 != 0 || a->x_stride % 8 != 0 || (a->swiglu && a->N % 2 != 0) ||
-        ((reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->weight)) & 15) != 0)
+    if (a->M > 4) return SD_ERR_UNSUPPORTED_SHAPE;
+    sd_token_linear_args t{};
+    t.M = a->M; t.N = a->N; t.K = a->K; t.swiglu = a->swiglu;
+    t.x = a->x; t.x_stride = a->x_stride; t.weight = a->weight; t.bias = a->bias; t.y = a->y; t.y_stride = a->y_stride;
+    return sd_token_linear(&t, stream_);
+}
+
+int sd_token_linear(const sd_token_linear_args* a, void* stream_) {
+    if (!a || a->M <= 0 || a->N <= 0 || a->K <= 0 || !a->x || !a->weight || !a->y) return SD_ERR_INVALID_ARGUMENT;
+    auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    if (a->M > TOKEN_MAX_ROWS || a->K % 8 != 0 || a->x_stride % 8 != 0 || (a->swiglu && a->N % 2 != 0) || !al(a->x) ||
+        !al(a->weight))
         return SD_ERR_UNSUPPORTED_SHAPE;
-    GemvParams p{};
+    if (a->norm_weight != nullptr) {
+        if (a->delta != nullptr && a->sum == nullptr) return SD_ERR_INVALID_ARGUMENT;
+        if (a->M > TOKEN_NORM_MAX_ROWS || a->K > TOKEN_NORM_MAX_K || !al(a->norm_weight) || !al(a->delta) || !al(a->sum))
+            return SD_ERR_UNSUPPORTED_SHAPE;
+    }
+    if (token_smem(a->M, a->K, a->norm_weight != nullptr) > TOKEN_SMEM_MAX) return SD_ERR_UNSUPPORTED_SHAPE;
+    if (configure_kernels() != cudaSuccess) return SD_ERR_NO_DEVICE;
+    TokenLinearParams p{};
     p.M = a->M; p.N = a->N; p.K = a->K; p.swiglu = a->swiglu ? 1 : 0;
     p.x = reinterpret_cast<const __nv_bfloat16*>(a->x); p.x_stride = a->x_stride;
     p.W = reinterpret_cast<const __nv_bfloat16*>(a->weight);
     p.bias = reinterpret_cast<const __nv_bfloat16*>(a->bias);
     p.y = reinterpret_cast<__nv_bfloat16*>(a->y); p.y_stride = a->y_stride;
-    const int outs = p.swiglu ? p.N / 2 : p.N;
-    k_gemv<<<(unsigned)((outs + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(p);
-    return launch_status();
+    p.delta = a->norm_weight ? reinterpret_cast<const __nv_bfloat16*>(a->delta) : nullptr;
+    p.norm_w = a->norm_weight; p.eps = a->norm_eps;
+    p.sum = reinterpret_cast<__nv_bfloat16*>(a->sum);
+    return token_linear(p, a->chained != 0, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 int sd_pack_rows(const sd_pack_rows_args* a, void* stream_) {
@@ -1183,7 +1255,7 @@ static int decode_impl(const sd_decode_args* a, const float* C_in, const float* 
     p.C = a->C;
     p.S = a->S;
     p.y = a->y;
-    return launch_decode<false>(p, MixerDecode{}, a->shape.B * a->shape.H, reinterpret_cast<cudaStream_t>(stream_));
+    return launch_decode<false>(p, MixerDecode{}, a->shape.B * a->shape.H, false, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 int sd_decode_step(const sd_decode_args* a, void* stream_) {
@@ -1194,7 +1266,7 @@ int sd_decode_step_from(const sd_decode_args* a, const float* C_in, const float*
     return decode_impl(a, C_in, S_in, stream_);
 }
 
-int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) {
+static int mixer_decode_impl(const sd_mixer_decode_args* a, bool chained, void* stream_) {
     if (!a || !shape_ok(&a->shape) || a->shape.T != 1) return SD_ERR_INVALID_ARGUMENT;
     if (!shape_supported(&a->shape)) return SD_ERR_UNSUPPORTED_SHAPE;
     const sd_operand ops[] = {a->u, a->h, a->erase_raw, a->write_raw};
@@ -1249,7 +1321,10 @@ int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) {
     if (m.norm_w != nullptr && m.gate == nullptr && m.gate_w == nullptr) return SD_ERR_INVALID_ARGUMENT;
     auto al8 = [](const void* q, long long stride) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0 && (stride & 3) == 0; };
     m.hid_vec = al8(m.decay_hidden, m.dh_sb) && al8(m.gate_hidden, m.gh_sb);
-    return launch_decode<true>(p, m, a->shape.B * a->shape.H, stream);
+    return launch_decode<true>(p, m, a->shape.B * a->shape.H, chained, stream);
 }
+
+int sd_mixer_decode_step(const sd_mixer_decode_args* a, void* stream_) { return mixer_decode_impl(a, false, stream_); }
+int sd_mixer_decode_step_chained(const sd_mixer_decode_args* a, void* stream_) { return mixer_decode_impl(a, true, stream_); }
 
 }  // extern "C"

@@ -20,6 +20,7 @@
 #include "sd_bf16.cuh"
 #include "sd_common.cuh"
 #include "sd_mixer.cuh"
+#include "sd_token.cuh"
 
 namespace sd {
 
@@ -134,19 +135,27 @@ __device__ __forceinline__ float dec_channel(const float (&x)[4], int a) {
     return __shfl_sync(0xffffffffu, v, a >> 2);
 }
 
-// One conv channel of the token: output rounded to BF16 as the separate conv kernel stores it; `next`: the advanced
-// window.
-__device__ __forceinline__ float dec_conv(const MixerDecode& m, int b, int D, int chn, __nv_bfloat16 (&next)[3]) {
-    const __nv_bfloat16* st = m.conv_state + ((long long)b * D + chn) * 3;
-    const __nv_bfloat16 b0 = st[0], b1 = st[1], b2 = st[2], b3 = m.qkv[(long long)b * m.qkv_sb + chn];
-    const float4 w = *reinterpret_cast<const float4*>(m.conv_w + (long long)chn * 4);
-    const float z = w.x * __bfloat162float(b0) + w.y * __bfloat162float(b1) + w.z * __bfloat162float(b2) +
-                    w.w * __bfloat162float(b3);
-    next[0] = b1;
-    next[1] = b2;
-    next[2] = b3;
-    return __bfloat162float(__float2bfloat16_rn(silu_f(z)));
-}
+// One conv channel of the token: its carried window and taps, then the output, rounded to BF16 as the separate conv
+// kernel stores it.
+struct DecConv {
+    __nv_bfloat16 window[3];   // oldest first; after `step` the advanced one
+    float4 taps;
+    __device__ __forceinline__ void load(const MixerDecode& m, int b, int D, int chn) {
+        const __nv_bfloat16* st = m.conv_state + ((long long)b * D + chn) * 3;
+        window[0] = st[0];
+        window[1] = st[1];
+        window[2] = st[2];
+        taps = *reinterpret_cast<const float4*>(m.conv_w + (long long)chn * 4);
+    }
+    __device__ __forceinline__ float step(__nv_bfloat16 now) {
+        const float z = taps.x * __bfloat162float(window[0]) + taps.y * __bfloat162float(window[1]) +
+                        taps.z * __bfloat162float(window[2]) + taps.w * __bfloat162float(now);
+        window[0] = window[1];
+        window[1] = window[2];
+        window[2] = now;
+        return __bfloat162float(__float2bfloat16_rn(silu_f(z)));
+    }
+};
 
 __device__ __forceinline__ void dec_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -218,32 +227,41 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
     const int D = 2 * p.g.H * r + p.g.H * V;
     const int live_v = V - c0 < 4 ? (V - c0 < 0 ? 0 : V - c0) : 4;
     const bool fused_proj = MIXER && mix.decay_w != nullptr;
-    __nv_bfloat16 next[CONV_PER][3];
-    const float ha = my_row < r ? __bfloat162float(row_bf16(p.h, ch, 0)[my_row]) : 0.f;
-    if (MIXER) {
-        // conv channels, one a thread: every CTA needs all of q and k for the norms
-        auto channel = [&](int t, int& dst) {   // t -> (slot in s_conv, channel) of q | k | v; -1: none
-            const int part = t / DP, c = t - part * DP;
-            dst = t;
-            if (part > 2 || c >= (part == 2 ? V : r)) return -1;
-            return part == 2 ? 2 * p.g.H * r + hh * V + c : part * p.g.H * r + hh * r + c;
-        };
+    // conv channels, one a thread: every CTA needs all of q and k for the norms
+    DecConv conv[CONV_PER];
+    auto channel = [&](int t) {   // slot t of q | k | v in s_conv -> conv channel, -1: none
+        const int part = t / DP, c = t - part * DP;
+        if (part > 2 || c >= (part == 2 ? V : r)) return -1;
+        return part == 2 ? 2 * p.g.H * r + hh * V + c : part * p.g.H * r + hh * r + c;
+    };
+    uint2 wd[MIXER ? RW : 1], wgt[MIXER ? RW : 1];
+    if constexpr (MIXER) {
+        // what the projection before this launch does not write is requested ahead of the wait for it: conv windows and
+        // taps, and this CTA's rows of the two small projections (one row per warp and load)
 #pragma unroll
         for (int n = 0; n < CONV_PER; ++n) {
-            int dst;
-            const int chn = channel(tid + n * THREADS, dst);
-            if (dst < 3 * DP) s_conv[dst] = chn >= 0 ? dec_conv(mix, b, D, chn, next[n]) : 0.f;
+            const int chn = channel(tid + n * THREADS);
+            if (chn >= 0) conv[n].load(mix, b, D, chn);
         }
-        if (fused_proj) {   // the two small projections, this CTA's rows of each: one row per warp and load
-            uint2 wd[RW], wgt[RW];
-            const bool lg = c0 < mix.G;   // G is a multiple of 16
+        const bool lg = fused_proj && c0 < mix.G;   // G is a multiple of 16
 #pragma unroll
-            for (int j = 0; j < RW; ++j) {
-                const int a = row0 + j;
-                wd[j] = wgt[j] = make_uint2(0u, 0u);
-                if (lg && a < r) wd[j] = *reinterpret_cast<const uint2*>(mix.decay_w + (long long)(hh * r + a) * mix.G + c0);
-                if (lg && a < V) wgt[j] = *reinterpret_cast<const uint2*>(mix.gate_w + (long long)(hh * V + a) * mix.G + c0);
-            }
+        for (int j = 0; j < RW; ++j) {
+            const int a = row0 + j;
+            wd[j] = wgt[j] = make_uint2(0u, 0u);
+            if (lg && a < r) wd[j] = *reinterpret_cast<const uint2*>(mix.decay_w + (long long)(hh * r + a) * mix.G + c0);
+            if (lg && a < V) wgt[j] = *reinterpret_cast<const uint2*>(mix.gate_w + (long long)(hh * V + a) * mix.G + c0);
+        }
+        chain_wait();
+        chain_release();
+    }
+    const float ha = my_row < r ? __bfloat162float(row_bf16(p.h, ch, 0)[my_row]) : 0.f;
+    if constexpr (MIXER) {
+#pragma unroll
+        for (int n = 0; n < CONV_PER; ++n) {
+            const int dst = tid + n * THREADS, chn = channel(dst);
+            if (dst < 3 * DP) s_conv[dst] = chn >= 0 ? conv[n].step(mix.qkv[(long long)b * mix.qkv_sb + chn]) : 0.f;
+        }
+        if (fused_proj) {   // the two small projections
             float hdf[4], hgf[4], dd[RW], gg[RW];
             dec_bf4(mix.decay_hidden + (long long)b * mix.dh_sb, c0, mix.G, mix.hid_vec, hdf);
             dec_bf4(mix.gate_hidden + (long long)b * mix.gh_sb, c0, mix.G, mix.hid_vec, hgf);
@@ -498,13 +516,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
         if (MIXER) {   // advance the conv windows: every thread of the cluster has read them before the exchange
 #pragma unroll
             for (int n = 0; n < CONV_PER; ++n) {
-                const int t = tid + n * THREADS, pt = t / DP, c = t - pt * DP;
-                if (pt < 3 && c < (pt == 2 ? V : r)) {
-                    const int chn = pt == 2 ? 2 * p.g.H * r + hh * V + c : pt * p.g.H * r + hh * r + c;
+                const int chn = channel(tid + n * THREADS);
+                if (chn >= 0) {
                     __nv_bfloat16* st = mix.conv_state + ((long long)b * D + chn) * 3;
-                    st[0] = next[n][0];
-                    st[1] = next[n][1];
-                    st[2] = next[n][2];
+                    st[0] = conv[n].window[0];
+                    st[1] = conv[n].window[1];
+                    st[2] = conv[n].window[2];
                 }
             }
         }

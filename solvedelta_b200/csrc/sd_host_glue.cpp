@@ -715,6 +715,206 @@ Tensor mixer_decode(Fp32Copies& copies, const Tensor& x, int64_t heads, int64_t 
     return projection(decode_launch(t).view({B, 1, heads * value_width}), out_weight, out_bias);
 }
 
+// ---- a cached token through the whole stack ------------------------------------------------------------------
+// The blocks and the final norm of a model for one cached token without gradients, as one call: five chained launches a
+// layer on pointers into one workspace (seven past eight rows, where the norms are launches of their own).  The
+// parameters are held as the module's own tensors; what is watched says when the module has changed under it (see
+// token_stack.py).
+struct TokenLayer {
+    Tensor mixer_norm, mlp_norm;
+    Tensor in_weight, in_bias, conv_weight, decay_weight, gate_weight, gate_bias, log_rate, decay_bias, geometry_bias;
+    Tensor out_norm, out_weight, out_bias, up_weight, down_weight;
+    double mixer_eps, mlp_eps, out_eps;
+    int64_t heads, width, value_width;
+    Fp32Copies copies;
+};
+
+struct TokenStack {
+    std::vector<TokenLayer> layers;
+    Tensor norm;
+    double norm_eps = 0;
+    Fp32Copies copies;
+    std::vector<std::tuple<py::dict, py::object, py::object>> same;   // dict[key] is value
+    std::vector<std::pair<py::dict, py::object>> absent;              // key not in dict
+    std::vector<py::dict> empty;                                      // hooks
+
+    bool unchanged() const {
+        for (const auto& [d, k, v] : same)
+            if (PyDict_GetItemWithError(d.ptr(), k.ptr()) != v.ptr()) return false;
+        for (const auto& [d, k] : absent)
+            if (PyDict_Contains(d.ptr(), k.ptr()) != 0) return false;
+        for (const auto& d : empty)
+            if (PyDict_Size(d.ptr()) != 0) return false;
+        return true;
+    }
+
+    void add_layer(const Tensor& mixer_norm, double mixer_eps, const Tensor& mlp_norm, double mlp_eps, int64_t heads, int64_t width,
+                   int64_t value_width, const Tensor& in_weight, const OptTensor& in_bias, const Tensor& conv_weight,
+                   const Tensor& decay_weight, const Tensor& gate_weight, const OptTensor& gate_bias, const Tensor& log_rate,
+                   const Tensor& decay_bias, const Tensor& geometry_bias, const Tensor& out_norm, double out_eps,
+                   const Tensor& out_weight, const OptTensor& out_bias, const Tensor& up_weight, const Tensor& down_weight) {
+        layers.push_back(TokenLayer{mixer_norm, mlp_norm, in_weight, given(in_bias), conv_weight, decay_weight, gate_weight,
+                                    given(gate_bias), log_rate, decay_bias, geometry_bias, out_norm, out_weight, given(out_bias),
+                                    up_weight, down_weight, mixer_eps, mlp_eps, out_eps, heads, width, value_width, {}});
+    }
+
+    static bool bf16_dense(const Tensor& t, const Tensor& like) {
+        return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.device() == like.device() && aligned16(t);
+    }
+    static bool layer_ok(const TokenLayer& l, const Tensor& x) {
+        const int64_t D = x.size(-1), H = l.heads, r = l.width, V = l.value_width;
+        for (const Tensor* t : {&l.in_weight, &l.decay_weight, &l.gate_weight, &l.out_weight, &l.up_weight, &l.down_weight})
+            if (!bf16_dense(*t, x)) return false;
+        for (const Tensor* t : {&l.in_bias, &l.gate_bias, &l.out_bias})
+            if (t->defined() && !bf16_dense(*t, x)) return false;
+        const int64_t inner = l.up_weight.size(0) / 2;
+        return l.in_weight.size(1) == D && l.in_weight.size(0) % 8 == 0 && is_shape(l.out_weight, {D, H * V}) && l.up_weight.size(1) == D &&
+               is_shape(l.down_weight, {D, inner}) && l.up_weight.size(0) % 16 == 0 && (H * V) % 8 == 0 && (H * r) % 8 == 0 &&
+               is_shape(l.decay_weight, {H * r, V}) && is_shape(l.gate_weight, {H * V, V}) && V % 16 == 0 && V <= 128 && r <= 128 &&
+               l.conv_weight.size(0) == 2 * H * r + H * V && fits_smem(x.size(0), inner) && fits_smem(x.size(0), H * V);
+    }
+    static bool fits_smem(int64_t rows, int64_t width) { return rows * (width + 96) * 2 <= 200 * 1024; }
+
+    // hidden [B,1,D] and the cache's per-layer dicts -> the normalised hidden rows [B,1,D], or with `head` [vocabulary, D]
+    // the logits; None when this is not a call the launches take (nothing has been touched then)
+    std::optional<Tensor> step(const Tensor& x, const py::list& states, const OptTensor& head) {
+        const int64_t B = x.size(0), D = x.size(2);
+        if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || !x.is_contiguous() || x.size(1) != 1 || B < 1 || B > SD_TOKEN_MAX_ROWS ||
+            D % 8 != 0 || D > 2048 || !aligned16(x) || !fits_smem(B, D) || states.size() != layers.size() ||
+            (head.has_value() && (!bf16_dense(*head, x) || head->size(1) != D)))
+            return std::nullopt;
+        struct State { Tensor C, S, conv; };
+        std::vector<State> state;
+        state.reserve(layers.size());
+        // interned once and never released: a static Python object must not outlive the interpreter
+        static PyObject* const recurrent_key = PyUnicode_InternFromString("recurrent_state");
+        static PyObject* const conv_key = PyUnicode_InternFromString("conv_state");
+        size_t row_max = 0, y_max = 0, act_max = 0;
+        for (size_t i = 0; i < layers.size(); ++i) {
+            const TokenLayer& l = layers[i];
+            const py::object entry = states[i];
+            if (!layer_ok(l, x) || !PyDict_Check(entry.ptr())) return std::nullopt;
+            PyObject* pair = PyDict_GetItemWithError(entry.ptr(), recurrent_key);
+            PyObject* conv_obj = PyDict_GetItemWithError(entry.ptr(), conv_key);
+            if (pair == nullptr || conv_obj == nullptr || !PyTuple_Check(pair) || PyTuple_GET_SIZE(pair) != 2) return std::nullopt;
+            PyObject *c = PyTuple_GET_ITEM(pair, 0), *s = PyTuple_GET_ITEM(pair, 1);
+            if (!THPVariable_Check(c) || !THPVariable_Check(s) || !THPVariable_Check(conv_obj)) return std::nullopt;
+            State st{THPVariable_Unpack(c), THPVariable_Unpack(s), THPVariable_Unpack(conv_obj)};
+            const int64_t H = l.heads, r = l.width, V = l.value_width;
+            if (!is_shape(st.C, {B, H, r, r}) || !is_shape(st.S, {B, H, r, V}) || !is_shape(st.conv, {B, 2 * H * r + H * V, 3})) return std::nullopt;
+            for (const Tensor* t : {&st.C, &st.S, &st.conv})
+                if (!t->is_contiguous() || t->device() != x.device() || t->scalar_type() != (t == &st.conv ? at::kBFloat16 : at::kFloat))
+                    return std::nullopt;
+            state.push_back(std::move(st));
+            row_max = std::max(row_max, (size_t)l.in_weight.size(0));
+            y_max = std::max(y_max, (size_t)(H * V));
+            act_max = std::max(act_max, (size_t)(l.up_weight.size(0) / 2));
+        }
+        const c10::cuda::CUDAGuard guard(x.device());
+        void* stream = stream_of(x);
+        const auto piece = [&](size_t width) { return (width * (size_t)B * 2 + 255) & ~size_t(255); };
+        const size_t row_b = piece(row_max), y_b = piece(y_max), act_b = piece(act_max), d_b = piece((size_t)D);
+        const Tensor work = workspace(x, row_b + y_b + act_b + 5 * d_b);
+        char* base = static_cast<char*>(work.data_ptr());
+        char *row = base, *y = row + row_b, *act = y + y_b, *mixed = act + act_b, *mlp = mixed + d_b, *normed = mlp + d_b;
+        char* sums[2] = {normed + d_b, normed + 2 * d_b};
+        int next = 0;
+        const void* residual = x.data_ptr();
+        const void* delta = nullptr;
+        bool chained = false;   // nothing of this call is in flight: the first launch follows the stream in full
+        const bool fuse_norm = B <= 8;
+        const auto linear = [&](const void* in, int64_t K, const Tensor& weight, const void* bias, void* out, bool with_swiglu,
+                                const float* norm_w, double eps) {
+            if (B > 16 && !with_swiglu && weight.size(0) >= 16 * 148) {
+                // wide products of more than 16 rows: the library's tiles read a row of x once for many columns
+                // (32 rows x 32000 x 1024: 14 us against 32)
+                const auto options = x.options();
+                const Tensor in_t = at::from_blob(const_cast<void*>(in), {B, K}, options);
+                Tensor out_t = at::from_blob(out, {B, weight.size(0)}, options);
+                if (bias != nullptr)
+                    at::addmm_out(out_t, at::from_blob(const_cast<void*>(bias), {weight.size(0)}, options), in_t, weight.t());
+                else
+                    at::mm_out(out_t, in_t, weight.t());
+                chained = false;
+                return;
+            }
+            sd_token_linear_args a{};
+            a.M = (int32_t)B; a.N = (int32_t)weight.size(0); a.K = (int32_t)K; a.swiglu = with_swiglu;
+            a.x = in; a.x_stride = K; a.weight = weight.data_ptr(); a.bias = bias;
+            a.y = out; a.y_stride = with_swiglu ? weight.size(0) / 2 : weight.size(0);
+            a.chained = chained;
+            chained = true;
+            if (norm_w != nullptr) {
+                a.norm_weight = norm_w; a.norm_eps = (float)eps; a.delta = delta;
+                if (delta != nullptr) a.sum = sums[next];
+            }
+            check(sd_token_linear(&a, stream));
+        };
+        const auto advance = [&] {   // the sum that a norm has just stored is the residual stream from here on
+            if (delta == nullptr) return;
+            residual = sums[next];
+            next ^= 1;
+        };
+        const auto norm_rows = [&](const float* norm_w, double eps, void* out) {
+            sd_add_rmsnorm_args a{};
+            a.rows = B; a.D = (int32_t)D; a.eps = (float)eps;
+            a.x = residual; a.delta = delta; a.weight = norm_w; a.sum = delta != nullptr ? sums[next] : nullptr; a.normed = out;
+            check(sd_add_rmsnorm(&a, stream));
+            chained = false;   // a plain launch: the next one follows it in full
+            advance();
+        };
+        // projection of the normalised residual stream
+        const auto norm_linear = [&](const float* norm_w, double eps, const Tensor& weight, const void* bias, void* out, bool with_swiglu) {
+            if (fuse_norm) {
+                linear(residual, D, weight, bias, out, with_swiglu, norm_w, eps);
+                advance();
+            } else {
+                norm_rows(norm_w, eps, normed);
+                linear(normed, D, weight, bias, out, with_swiglu, nullptr, 0);
+            }
+        };
+        if (!fuse_norm && (D % 256 != 0)) return std::nullopt;   // the norm alone takes whole groups of 256 channels
+        for (size_t i = 0; i < layers.size(); ++i) {
+            TokenLayer& l = layers[i];
+            State& st = state[i];
+            const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0);
+            norm_linear(f32(l.copies.get(0, l.mixer_norm)), l.mixer_eps, l.in_weight, raw(l.in_bias), row, false);
+            sd_mixer_decode_args a{};
+            a.shape = sd_shape{(int32_t)B, 1, (int32_t)H, (int32_t)r, (int32_t)V};
+            const auto at_col = [&](int64_t c) { return row + 2 * c; };
+            const int64_t qkv = 2 * H * r + H * V, geom = qkv + 3 * H * r + H * V;
+            a.u = sd_operand{at_col(qkv), P, P, r};
+            a.h = sd_operand{at_col(qkv + H * r), P, P, r};
+            a.erase_raw = sd_operand{at_col(qkv + 2 * H * r), P, P, r};
+            a.write_raw = sd_operand{at_col(qkv + 3 * H * r), P, P, V};
+            a.qkv = row; a.qkv_stride_b = P;
+            a.conv_weight = f32(l.copies.get(1, l.conv_weight)); a.conv_state = st.conv.data_ptr();
+            a.log_rate = f32(l.copies.get(2, l.log_rate)); a.decay_bias = f32(l.copies.get(3, l.decay_bias));
+            a.geometry_raw = at_col(geom); a.geometry_stride_b = P; a.geometry_bias = f32(l.copies.get(4, l.geometry_bias));
+            a.C = f32(st.C); a.S = f32(st.S); a.y = y;
+            a.norm_weight = f32(l.copies.get(5, l.out_norm)); a.norm_eps = (float)l.out_eps;
+            a.gate_rank = (int32_t)V;
+            a.decay_hidden = at_col(geom + H); a.decay_hidden_stride_b = P;
+            a.gate_hidden = at_col(geom + H + V); a.gate_hidden_stride_b = P;
+            a.decay_proj_weight = l.decay_weight.data_ptr(); a.gate_proj_weight = l.gate_weight.data_ptr();
+            a.gate_proj_bias = raw(l.gate_bias);
+            check(sd_mixer_decode_step_chained(&a, stream));
+            linear(y, H * V, l.out_weight, raw(l.out_bias), mixed, false, nullptr, 0);
+            delta = mixed;
+            norm_linear(f32(l.copies.get(6, l.mlp_norm)), l.mlp_eps, l.up_weight, nullptr, act, true);
+            linear(act, l.up_weight.size(0) / 2, l.down_weight, nullptr, mlp, false, nullptr, 0);
+            delta = mlp;
+        }
+        const Tensor norm_w = copies.get(0, norm);
+        Tensor out = bf16_like(x, {B, 1, head.has_value() ? head->size(0) : D});
+        if (head.has_value())
+            norm_linear(f32(norm_w), norm_eps, *head, nullptr, out.data_ptr(), false);
+        else
+            norm_rows(f32(norm_w), norm_eps, out.data_ptr());
+        return out;
+    }
+};
+
 }  // namespace
 
 void register_glue(py::module_& m) {
@@ -724,6 +924,19 @@ void register_glue(py::module_& m) {
         .def("get", &Fp32Copies::get)
         .def("__deepcopy__", [](const Fp32Copies&, py::dict) { return Fp32Copies(); })
         .def(py::pickle([](const Fp32Copies&) { return py::tuple(); }, [](py::tuple) { return Fp32Copies(); }));
+    py::class_<TokenStack>(m, "TokenStack")
+        .def(py::init([](const Tensor& norm, double eps) {
+            TokenStack t;
+            t.norm = norm;
+            t.norm_eps = eps;
+            return t;
+        }))
+        .def("add_layer", &TokenStack::add_layer)
+        .def("watch_same", [](TokenStack& t, py::dict d, py::object k, py::object v) { t.same.emplace_back(d, k, v); })
+        .def("watch_absent", [](TokenStack& t, py::dict d, py::object k) { t.absent.emplace_back(d, k); })
+        .def("watch_empty", [](TokenStack& t, py::dict d) { t.empty.push_back(d); })
+        .def("unchanged", &TokenStack::unchanged)
+        .def("step", &TokenStack::step);
     m.def("conv4_silu", &conv4_silu);
     m.def("kda_decay_gate", &kda_decay_gate);
     m.def("rms_norm_gated", &rms_norm_gated);

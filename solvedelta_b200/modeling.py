@@ -26,6 +26,7 @@ from .config import SolveDeltaConfig
 from .ops import SolveDeltaState
 from .mixer_ops import add_rmsnorm, add_rmsnorm_reverse_supported, gated_mlp
 from .model import SolveDelta, SolveDeltaLayerState
+from .token_stack import token_stack
 
 FP32_PARAMETERS = ("geometry_write_bias", "associative_log_rate", "associative_decay_bias")
 
@@ -307,6 +308,19 @@ class SolveDeltaModel(SolveDeltaPreTrainedModel):
     def set_input_embeddings(self, value):
         self.embeddings = value
 
+    def _cached_token(self, hidden_states: torch.Tensor, cache: SolveDeltaCache,
+                      head: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+        """One token per row on a filled cache, without gradients: all blocks and the final norm (with ``head``: and
+        the logits) in one native call that updates the cache's tensors in place.  None when that call does not
+        apply; nothing has been touched then."""
+        if hidden_states.shape[1] != 1 or torch.is_grad_enabled() or len(cache.states) != len(self.layers):
+            return None
+        stack = token_stack(self, SolveDeltaBlock, SolveDeltaCacheAdapter, SolveDeltaMLP)
+        token = None if stack is None else stack.step(hidden_states, cache.states, head)
+        if token is not None:
+            cache._seen_tokens += 1
+        return token
+
     def forward(self, input_ids: Optional[torch.Tensor] = None, attention_mask: Optional[torch.Tensor] = None,
                 inputs_embeds: Optional[torch.Tensor] = None,
                 past_key_values: Union[SolveDeltaCache, Sequence[Dict[str, Any]], None] = None,
@@ -323,6 +337,10 @@ class SolveDeltaModel(SolveDeltaPreTrainedModel):
             past_key_values = SolveDeltaCache.from_legacy_cache(past_key_values)
         elif not use_cache:
             past_key_values = None
+        if use_cache and attention_mask is None and not output_hidden_states and not kwargs:
+            token = self._cached_token(hidden_states, past_key_values)
+            if token is not None:
+                return BaseModelOutputWithPast(last_hidden_state=token, past_key_values=past_key_values)
         cu_seqlens = kwargs.get("cu_seqlens")
         if cu_seqlens is not None and "solvedelta_reset_mask" not in kwargs:
             kwargs["solvedelta_reset_mask"] = segment_reset_mask(hidden_states, cu_seqlens)
@@ -380,6 +398,23 @@ class SolveDeltaForCausalLM(SolveDeltaPreTrainedModel, GenerationMixin):
             parameter.data = parameter.data.to(torch.float32 if keep else torch.bfloat16)
         return self
 
+    def _plain_head(self) -> bool:
+        """The head is a bare projection and nothing is hooked to it or to the inner model."""
+        head, inner = self.lm_head, self.model
+        return (type(head) is nn.Linear and head.bias is None and type(inner) is SolveDeltaModel
+                and not (head._forward_hooks or head._forward_pre_hooks or inner._forward_hooks
+                         or inner._forward_pre_hooks)
+                and "forward" not in head.__dict__ and "forward" not in inner.__dict__)
+
+    def _cached_token_logits(self, input_ids, cache: SolveDeltaCache, use_cache: Optional[bool]) -> Optional[torch.Tensor]:
+        """Logits of one token per row on a filled cache (``SolveDeltaModel._cached_token`` with the head), or None."""
+        inner = self.model
+        if use_cache is None:
+            use_cache = inner.config.use_cache if not inner.training else False
+        if not use_cache or input_ids is None or input_ids.ndim != 2 or input_ids.shape[1] != 1 or torch.is_grad_enabled():
+            return None
+        return inner._cached_token(inner.embeddings(input_ids), cache, self.lm_head.weight)
+
     @classmethod
     def _supports_default_dynamic_cache(cls) -> bool:
         return False   # the recurrent cache comes out of the prefill; generate() must not build a key/value cache
@@ -399,6 +434,11 @@ class SolveDeltaForCausalLM(SolveDeltaPreTrainedModel, GenerationMixin):
                 labels: Optional[torch.Tensor] = None, use_cache: Optional[bool] = None,
                 output_hidden_states: bool = False, logits_to_keep: Optional[int] = 0,
                 **kwargs) -> CausalLMOutputWithPast:
+        if (isinstance(past_key_values, SolveDeltaCache) and labels is None and attention_mask is None
+                and inputs_embeds is None and not output_hidden_states and not kwargs and self._plain_head()):
+            logits = self._cached_token_logits(input_ids, past_key_values, use_cache)
+            if logits is not None:
+                return CausalLMOutputWithPast(logits=logits, past_key_values=past_key_values)
         outputs = self.model(input_ids=input_ids, attention_mask=attention_mask, inputs_embeds=inputs_embeds,
                              past_key_values=past_key_values, use_cache=use_cache,
                              output_hidden_states=output_hidden_states, **kwargs)

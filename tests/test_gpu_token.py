@@ -1,0 +1,60 @@
+"""The projections of a cached token at the edges of their tiles, and the native token stack against the module path."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from solvedelta_b200 import SolveDeltaConfig, SolveDeltaForCausalLM, _lib
+from tests.helpers import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K,norm,delta,swiglu", [
+    (1, 24, 8, False, False, False), (7, 2376, 264, True, True, False), (8, 2368, 2048, True, False, False),
+    (9, 40, 2816, False, False, False), (16, 2384, 1000, False, False, False), (17, 8, 72, False, False, True),
+    (32, 112, 1024, False, False, True), (3, 48, 1024, True, True, True)])
+def test_token_linear(M, N, K, norm, delta, swiglu):
+    gen = torch.Generator().manual_seed(M * N + K)
+    bf = lambda *s: torch.randn(*s, generator=gen).to(torch.bfloat16).cuda()
+    x, d, w, b = bf(M, K), bf(M, K), bf(N, K) / K ** 0.5, bf(N)
+    nw = (1 + 0.2 * torch.randn(K, generator=gen)).cuda()
+    y = torch.full((M, N // 2 if swiglu else N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    total = torch.empty_like(x)
+    a = _lib.TokenLinearArgs(M, N, K, int(swiglu), x.data_ptr(), K, w.data_ptr(), b.data_ptr(), y.data_ptr(), y.shape[1],
+                             d.data_ptr() if delta else None, nw.data_ptr() if norm else None, 1e-6, 1, total.data_ptr())
+    _lib.check(_lib.load().sd_token_linear(ctypes.byref(a),
+                                           ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    rows = x
+    if delta:
+        rows = x + d
+        assert torch.equal(total, rows)
+    rows = rows.float()
+    if norm:
+        rows = (rows * torch.rsqrt(rows.pow(2).mean(-1, keepdim=True) + 1e-6) * nw).to(torch.bfloat16).float()
+    want = rows @ w.float().t() + b.float()
+    if swiglu:
+        gate, value = want.to(torch.bfloat16).float().chunk(2, -1)
+        want = F.silu(gate) * value
+    assert rel_l2(y.float().cpu().numpy(), want.cpu().numpy()) <= 4e-3
+
+
+@pytest.mark.parametrize("B", [1, 8, 9, 20])
+def test_token_stack_equals_the_module_path(B):
+    torch.manual_seed(5)
+    model = SolveDeltaForCausalLM(SolveDeltaConfig(hidden_size=256, num_heads=4, head_k_dim=64, head_v_dim=64,
+                                                   num_hidden_layers=2, vocab_size=320)).prepare("cuda").eval()
+    ids = torch.randint(0, 320, (B, 70), device="cuda")
+    seen = []
+    for hooked in (False, True):
+        handle = model.model.layers[1].mlp.register_forward_hook(lambda *a: None) if hooked else None
+        with torch.no_grad():
+            cache = model(input_ids=ids[:, :66], use_cache=True).past_key_values
+            logits = [model(input_ids=ids[:, t:t + 1], past_key_values=cache, use_cache=True).logits for t in range(66, 70)]
+        assert cache.get_seq_length() == 70
+        seen.append((torch.cat(logits, 1), cache[1]["recurrent_state"][1].clone(), cache[1]["conv_state"].clone()))
+        if handle is not None:
+            handle.remove()
+    for got, want in zip(*seen):
+        assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
