@@ -120,8 +120,6 @@ long long* g_dbg = nullptr;  // set by sd_debug_timeline (profiling build only)
 // sd_device_fault reads it back, sd_device_fault_clear resets it.
 __device__ int g_scan_fault_word = 0;
 int* g_scan_fault_ptr[64] = {};
-// Tensor map of a [chunks][CL][DP] FP32 panel array for the scan's tiled load: dimensions (4 elements,
-// CL rows, DP/4 K-chunks, chunks) with byte strides (row pitch, 16, panel size), box = one whole panel.
 // cuTensorMapEncodeTiled is a driver function; it is reached through the runtime so that the library
 // links against the runtime alone.
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -138,20 +136,8 @@ TensorMapEncodeFn tensor_map_encoder() {
     }
     return encode;
 }
-bool make_panel_map(CUtensorMap* map, const float* panels, long long chunks) {
-    const TensorMapEncodeFn encode = tensor_map_encoder();
-    if (encode == nullptr) return false;
-    const cuuint64_t dims[4] = {4, (cuuint64_t)CL, (cuuint64_t)(DP / 4), (cuuint64_t)chunks};
-    const cuuint64_t strides[3] = {(cuuint64_t)DP * 4, 16, (cuuint64_t)CL * DP * 4};
-    const cuuint32_t box[4] = {4, (cuuint32_t)CL, (cuuint32_t)(DP / 4), 1};
-    const cuuint32_t elem[4] = {1, 1, 1, 1};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(panels), dims, strides, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// The same panel array as rows of DP columns: dimensions (DP, CL, chunks), box (`cols`, CL, 1).
-bool make_row_map(CUtensorMap* map, const float* panels, long long chunks, int cols) {
+// Tensor map of a [chunks][CL][DP] FP32 panel array: dimensions (DP, CL, chunks), box (`cols`, CL, 1).
+bool make_row_map(CUtensorMap* map, const float* panels, long long chunks, int cols, CUtensorMapSwizzle swizzle) {
     const TensorMapEncodeFn encode = tensor_map_encoder();
     if (encode == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)DP, (cuuint64_t)CL, (cuuint64_t)chunks};
@@ -159,7 +145,7 @@ bool make_row_map(CUtensorMap* map, const float* panels, long long chunks, int c
     const cuuint32_t box[3] = {(cuuint32_t)cols, (cuuint32_t)CL, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(panels), dims, strides, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -227,8 +213,9 @@ bool scan_maps(const ScanParams& sp, long long chunks, const ScanMaps** out) {
     next = (next + 1) % SLOTS;
     m.q = nullptr;
     m.chunks = 0;
-    if (!make_panel_map(&m.qmap, sp.Q, chunks) || !make_row_map(&m.rmap, sp.R, chunks, DP) ||
-        !make_row_map(&m.pmap, sp.P, chunks, SCAN_NS))
+    if (!make_row_map(&m.qmap, sp.Q, chunks, 32, CU_TENSOR_MAP_SWIZZLE_128B) ||
+        !make_row_map(&m.rmap, sp.R, chunks, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B) ||
+        !make_row_map(&m.pmap, sp.P, chunks, SCAN_NS, CU_TENSOR_MAP_SWIZZLE_NONE))
         return false;
     m.q = sp.Q; m.r = sp.R; m.p = sp.P; m.chunks = chunks;
     *out = &m;
@@ -275,11 +262,16 @@ inline void set_dbg(Geometry&, int, int) {}
 inline long long* scan_dbg(int) { return nullptr; }
 #endif
 
-bool launch_scan_tc(const ScanParams& sp, long long chunks, dim3 grid, cudaStream_t stream, long long* dbg) {
+bool launch_scan_tc(ScanParams sp, int streams, cudaStream_t stream, long long* dbg) {
     const ScanMaps* m = nullptr;
-    if (!scan_maps(sp, chunks, &m)) return false;
-    k_state_scan_tc<<<grid, TC_THREADS, SCAN_TC_SMEM_BYTES, stream>>>(sp, m->qmap, m->rmap, m->pmap, scan_fault_ptr(),
-                                                                      dbg);
+    if (!scan_maps(sp, (long long)streams * sp.NC, &m)) return false;
+    if (sp.segs > 1) {
+        k_state_scan_tc<true><<<streams * (sp.segs - 1) * 4, TC_THREADS, SCAN_TC_SMEM_BYTES, stream>>>(
+            sp, m->qmap, m->rmap, m->pmap, scan_fault_ptr(), nullptr);
+        k_scan_combine<<<streams * (DP / COMBINE_COLS), COMBINE_THREADS, 0, stream>>>(sp.seg_state, sp.segs);
+    }
+    k_state_scan_tc<false><<<streams * sp.segs * (DP / SCAN_NS), TC_THREADS, SCAN_TC_SMEM_BYTES, stream>>>(
+        sp, m->qmap, m->rmap, m->pmap, scan_fault_ptr(), dbg);
     return true;
 }
 
@@ -306,7 +298,8 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_primal_exterior_fwd<true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_state_scan_tc, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_state_scan_tc<false>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<true>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
@@ -579,7 +572,6 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
 
     const int chunks = (int)total_chunks(s);
     const int streams = s->B * s->H;
-    const dim3 scan_grid((DP / SCAN_NS) * streams);
     const Operand fwd_ops[] = {p.u, p.h, p.q, p.k, p.v, p.er, p.wr, p.ld};
     const bool fast = all_fast(fwd_ops, 8, *s);
     const bool masked = a->valid_mask != nullptr || a->reset_mask != nullptr;
@@ -596,8 +588,8 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         sp.lam = p.Lam; sp.X = p.Delta; sp.ck = p.CtCk; sp.Xb = nullptr;
         sp.ckb = bpanel_at(kSaved, s, a->saved, "CtCkB");
         sp.init = a->C0; sp.fin = a->C_T;
-        sp.NC = p.g.NC; sp.reverse = 0; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
-        if (!launch_scan_tc(sp, total_chunks(s), scan_grid, stream, scan_dbg(1))) return SD_ERR_LAUNCH_FAILED;
+        sp.NC = p.g.NC; sp.segs = 1; sp.seg_len = p.g.NC; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
+        if (!launch_scan_tc(sp, streams, stream, scan_dbg(1))) return SD_ERR_LAUNCH_FAILED;
         mark(stream);
     }
     set_dbg(p.g, 2, chunks);
@@ -612,8 +604,8 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         sp.P = p.Ud; sp.Q = p.Wd; sp.R = p.Dt;
         sp.lam = p.Lam; sp.X = nullptr; sp.ck = nullptr; sp.Xb = p.Zt; sp.ckb = p.SCk;
         sp.init = a->S0; sp.fin = a->S_T;
-        sp.NC = p.g.NC; sp.reverse = 0; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
-        if (!launch_scan_tc(sp, total_chunks(s), scan_grid, stream, scan_dbg(3))) return SD_ERR_LAUNCH_FAILED;
+        sp.NC = p.g.NC; sp.segs = 1; sp.seg_len = p.g.NC; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
+        if (!launch_scan_tc(sp, streams, stream, scan_dbg(3))) return SD_ERR_LAUNCH_FAILED;
         mark(stream);
     }
     set_dbg(p.g, 4, chunks);

@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
             const float4 ge = *reinterpret_cast<const float4*>(s_ge + I * DP + c4);
             const float4 gl = *reinterpret_cast<const float4*>(GL + c4);
             *reinterpret_cast<float4*>(gUbar + i * DP + c4) =
-                make_float4(un.x * __expf(gl.x - ge.x), un.y * __expf(gl.y - ge.y), un.z * __expf(gl.z - ge.z),
-                            un.w * __expf(gl.w - ge.w));
+                make_float4(round_tf32(un.x * __expf(gl.x - ge.x)), round_tf32(un.y * __expf(gl.y - ge.y)),
+                            round_tf32(un.z * __expf(gl.z - ge.z)), round_tf32(un.w * __expf(gl.w - ge.w)));
         }
     }
     __syncthreads();
@@ -494,7 +494,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
             store8_smem(s_er, i, c0, ern);
             store8_smem(s_ag, i, c0, ag);
             store8_smem(s_z, i, c0, z);
-            store8_panel(gDt, i, c0, dt);
+            {   // an operand of the state scan, like Ubar, Qc and Wd: rounded to TF32 here
+                float rt[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) rt[e] = round_tf32(dt[e]);
+                store8_panel(gDt, i, c0, rt);
+            }
             store8_bpanel(gXg, i, c0, xg);
             store8_bpanel(bpanel_ptr(p.Ag, ch.gi), i, c0, ag);
             store8_bpanel(bpanel_ptr(p.Xr, ch.gi), i, c0, xr);

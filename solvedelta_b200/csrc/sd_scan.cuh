@@ -33,7 +33,8 @@ struct ScanParams {
     const float* init; // nullable: true-dimension state [S][rows][cols] (or transposed)
     float* fin;        // nullable
     int NC;            // chunks per stream
-    int reverse;       // walk chunks last to first
+    int segs, seg_len; // segments a stream is cut into, and their chunks (the last one may be shorter)
+    float* seg_state;  // [streams][segs - 1][2][DP][DP]: end states and transfer matrices, then entry states (segs > 1)
     int transposed_io; // init/fin hold the transpose (predictor state C[a][c])
     int nrows, ncols;  // true dims of the carried St: rows (<= DP), cols (<= DP)
 };

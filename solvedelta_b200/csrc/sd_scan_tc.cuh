@@ -1,37 +1,30 @@
 // The forward chunk-state scan on the fifth-generation tensor cores (tcgen05).
 //
-// Same recurrence, ScanParams and launch grid as k_state_scan:
-//     X  = P + Q * St ;  checkpoint St ;  St = diag(lam) St + R^T X
-// A CTA carries a [DP][NS] column slice of one stream's state.  The slice
-// lives in tensor memory as the accumulator of the update contraction (lane =
-// state row p, column = slice column c); the step's X is a second
-// accumulator, held transposed (lane = slice column, column = token):
-//     X^T[c][tok] = sum_p St[p][c] * Q[tok][p]       M=128 (64 used) N=64 K=128
-//     St [p][c]  += sum_t R[tok][p] * X[tok][c]      M=128           N=64 K=64
-// All four operands are K-major in shared memory, in the unswizzled canonical
-// layout of 8 x 16-byte core matrices (the first contraction's M is padded to
-// 128: rows 64..127 of its A operand alias whatever follows in shared memory
-// and only feed accumulator lanes nobody reads).  Q [tok][p] arrives by ONE
-// tiled TMA load per chunk (cp.async.bulk.tensor.4d, completion counted on an
-// mbarrier): the tensor map lists the 16-byte K-chunk as a dimension of its own,
-// so the panel lands as [K-chunk][row][4 elements], which is the canonical layout.  X^T is written by the thread that holds the row after
-// tcgen05.ld, four consecutive tokens to a 16-byte chunk.  The state, held by
-// rows, is written element by element into the transposed operand, with the
-// K-chunk pitch padded to 144 bytes so that a warp's 32 rows hit 32 banks.
-// R [tok][p], whose contraction index is the slow one in global memory, is
-// landed as it lies by a tiled TMA load (with the CTA's slice of P) and turned
-// through registers: a thread reads columns of it, one lane per column, and
-// writes each as 16-byte chunks of one operand row (the warps without X^T
-// rows do this, two columns per thread).  The decay
-// diag(lam) is one scalar per thread, applied on the way back into tensor
-// memory; checkpoints and X go to global memory from the same registers.
-// Operands are rounded to TF32 (round to nearest) before the tensor core,
-// which would truncate, sees them: the state, X and R in registers here, Q by
-// the kernels that write the Q panels.
+//     X  = P + Q St ;  checkpoint St ;  St = diag(lam) St + R^T X
+// for every chunk of a stream in order.  A CTA carries a 64-column slice of one stream's state, transposed, in tensor
+// memory (lane = slice column c, column = state row p), and both contractions take their A operand from tensor memory:
+//     X^T[c][tok] = sum_p St^T[c][p] Q[tok][p]      A = rounded state,  B = Q as it lies (K-major)
+//     St^T[c][p] += sum_t X^T[c][tok] R[tok][p]     A = rounded X,      B = R as it lies (MN-major)
+// (M = 128 of which 64 lanes are used), so neither the state nor X passes through shared memory and no panel is
+// transposed.  Q and R land as tiles of 128-byte rows by TMA: Q with the 128-byte swizzle, R with its 32-byte-atom form,
+// the one an MN-major TF32 operand takes.  The roles are split over the warps: one thread issues the loads two chunks
+// ahead, one issues the contractions, and the 256 threads that own lanes 0..63 (32 state and 16 X columns each) round,
+// decay, add P and store; mbarriers connect them, so no step has a CTA-wide barrier.  Checkpoints are stored behind the
+// first contraction and X behind the second one.
 //
-// Every mbarrier wait is bounded: a wait that runs out raises the fault word
-// the host reads back, the thread stops waiting for the rest of the launch,
-// and the kernel still walks to its end and frees its tensor memory.
+// What bounds it: the chain of two contractions per chunk with their hand-overs.
+//
+// Segments.  With few streams the chain is long and most SMs are idle.  The recurrence is affine in St, so the chunks of
+// a stream may be cut into segments: a first pass (TRANSFER) walks all segments but the last at once and gives each
+// one's end state from zero and its transfer matrix (the end states from the identity's columns with P left out);
+// k_scan_combine chains them in FP32 into the segments' entry states; the second pass is the scan itself with all
+// segments at once.
+//
+// Operands are rounded to TF32 (round to nearest) before the tensor core, which would truncate, sees them: the state and
+// X in registers here, Q and R by the kernels that write those panels.
+//
+// Every mbarrier wait is bounded: a wait that runs out raises the fault word the host reads back, the thread stops
+// waiting for the rest of the launch, and the kernel still walks to its end and frees its tensor memory.
 #pragma once
 #include <cuda.h>   // CUtensorMap (types only: the encoder is reached through the runtime's driver entry point)
 
@@ -39,27 +32,7 @@
 
 namespace sd {
 
-constexpr int TC_PARTS = 2;               // warps per lane quarter: each takes 64/TC_PARTS columns (or tokens)
-constexpr int TC_N = 64 / TC_PARTS;        // columns of the state slice, or tokens of X^T, per thread
-constexpr int TC_THREADS = 128 * TC_PARTS; // lane quarter = warp % 4, part = warp / 4
-constexpr int TC_TMEM_COLS = 128;         // 64 state-slice columns + 64 X^T columns
-constexpr int TC_X_COL = SCAN_NS;         // first tensor-memory column of X^T
-constexpr unsigned TC_CORE = 128;         // bytes of one 8 x 16-byte core matrix
-constexpr unsigned TC_Q_LBO = CL * 16;               // Q landed by TMA: K-chunk pitch (all 64 rows of one 16-byte chunk)
-constexpr unsigned TC_Q_SBO = 8 * 16;                // ... and the pitch of its 8-row groups
-constexpr unsigned TC_KT_SBO = (CL / 4) * TC_CORE;  // K = tokens (X, R): bytes between 8-row groups
-constexpr unsigned TC_PANEL_BYTES = CL * DP * 4;    // one [CL][DP] or [DP][CL] operand
-constexpr unsigned TC_S_LBO = TC_CORE + 16;         // padded K-chunk pitch of the transposed state operand
-constexpr unsigned TC_S_SBO = (DP / 4) * TC_S_LBO;  // its bytes between 8-row groups
-constexpr unsigned TC_S_BYTES = (SCAN_NS / 8) * TC_S_SBO;   // the 64 rows that are written
-constexpr unsigned TC_X_BYTES = SCAN_NS * CL * 4;
-// Q ring, state operand, X operand, R operand.  The padded A operand of the first contraction reaches
-// 2 * TC_S_BYTES past the start of the state operand, which must stay inside this allocation.
-constexpr size_t SCAN_TC_OPERAND_BYTES = size_t(2) * TC_PANEL_BYTES + TC_S_BYTES + TC_X_BYTES + TC_PANEL_BYTES;
-constexpr unsigned TC_RAW_P_BYTES = CL * SCAN_NS * 4;   // the P slice as it lies, [CL][NS]
-// ... followed by R as it lies ([CL][DP]) and the P slice, both landed by TMA one step ahead
-constexpr size_t SCAN_TC_SMEM_BYTES = SCAN_TC_OPERAND_BYTES + TC_PANEL_BYTES + TC_RAW_P_BYTES;
-static_assert(2 * TC_S_BYTES <= TC_S_BYTES + TC_X_BYTES + TC_PANEL_BYTES, "padded operand rows leave the allocation");
+constexpr unsigned TC_R_SBO = 512;          // bytes between the 4-row groups of an MN-major TF32 tile
 constexpr int TC_WAIT_LIMIT = 1 << 20;    // polls of one mbarrier before the wait is given up
 
 __device__ __forceinline__ unsigned tc_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -72,14 +45,6 @@ __device__ __forceinline__ unsigned long long tc_desc(unsigned addr, unsigned lb
 // Instruction descriptor: FP32 accumulator, TF32 operands, both K-major, M = 128.
 __device__ __forceinline__ unsigned tc_idesc(int n) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(n >> 3) << 17) | ((128u >> 4) << 24);
-}
-__device__ __forceinline__ void tc_mma(unsigned d_tmem, unsigned long long da, unsigned long long db, unsigned idesc,
-                                       unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
 }
 __device__ __forceinline__ void tc_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -157,311 +122,316 @@ __device__ __forceinline__ void tc_st(unsigned taddr, const float* r) {
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// One full 32-byte sector per thread (256-bit store; the address is 32-byte aligned).
-__device__ __forceinline__ void tc_store32(void* g, const unsigned (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(g), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                 : "memory");
-}
-
 __device__ __forceinline__ float tc_round(float x) { return __uint_as_float(f2tf32(x)); }
 
-// One tiled TMA load lands the [CL][DP] panel Q of chunk `chunk` as a K-major unswizzled operand:
-// the map's dimensions are (4 elements, CL rows, DP/4 K-chunks, chunks), so shared memory receives
-// [K-chunk][row][4 elements].  Completion is counted in bytes on `bar`.
-__device__ __forceinline__ void tc_load_q(unsigned char* sm, const CUtensorMap* map, int chunk, unsigned bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(TC_PANEL_BYTES) : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-            tc_smem(sm)),
-        "l"(reinterpret_cast<unsigned long long>(map)), "r"(0), "r"(0), "r"(0), "r"(chunk), "r"(bar)
-        : "memory");
-}
-
-// Row-major tiled loads (map dimensions: DP columns, CL rows, chunks): all of R, and the CTA's
-// NS-column slice of P, both counted on `bar`.
-__device__ __forceinline__ void tc_load_rp(unsigned char* sR_raw, unsigned char* sP_raw, const CUtensorMap* rmap,
-                                           const CUtensorMap* pmap, int chunk, int col0, unsigned bar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                 "r"(TC_PANEL_BYTES + TC_RAW_P_BYTES)
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            tc_smem(sR_raw)),
-        "l"(reinterpret_cast<unsigned long long>(rmap)), "r"(0), "r"(0), "r"(chunk), "r"(bar)
-        : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            tc_smem(sP_raw)),
-        "l"(reinterpret_cast<unsigned long long>(pmap)), "r"(col0), "r"(0), "r"(chunk), "r"(bar)
-        : "memory");
+// `N` rows of one column per thread as BF16, rows DP apart: neighbouring lanes swap halves of a row pair, so that each
+// store moves two columns.
+template <int N>
+__device__ __forceinline__ void tc_store_pairs(bf16* rows, int c, int lane, const float (&v)[N]) {
+    const bool odd = lane & 1;
+    bf16* dst = rows + (c & ~1) + (odd ? DP : 0);
+#pragma unroll
+    for (int j = 0; j < N; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        const __nv_bfloat162 w = odd ? __floats2bfloat162_rn(other, v[j + 1]) : __floats2bfloat162_rn(v[j], other);
+        *reinterpret_cast<__nv_bfloat162*>(dst + j * DP) = w;
+    }
 }
 
 // Profiling build only: thread 0 of the first CTA records the SM clock at the phase boundaries of its ninth step.
 #ifdef SD_DIAGNOSTICS
 #define TC_STAMP(k)                                                                              \
     do {                                                                                         \
-        if (dbg != nullptr && blockIdx.x == 0 && tid == 0 && step == 8)                          \
+        if (dbg != nullptr && blockIdx.x == 0 && tid == 0 && n == 8)                          \
             dbg[k] = clock64();                                                                  \
     } while (0)
 #else
 #define TC_STAMP(k) do { } while (0)
 #endif
 
-__global__ void __launch_bounds__(TC_THREADS, 1) k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap,
-                                                                  const __grid_constant__ CUtensorMap rmap,
-                                                                  const __grid_constant__ CUtensorMap pmap, int* fault,
-                                                                  long long* dbg) {
-    extern __shared__ __align__(128) unsigned char tsm[];
-    unsigned char* sQ = tsm;                          // [2] B of the first contraction (rows = tokens, K = state rows)
-    unsigned char* sS = sQ + 2 * TC_PANEL_BYTES;      // A of the first: slice^T        (rows = slice columns, K = state rows)
-    unsigned char* sX = sS + TC_S_BYTES;              // B of the second: X^T           (rows = slice columns, K = tokens)
-    unsigned char* sR = sX + TC_X_BYTES;              // A of the second: R^T           (rows = state rows, K = tokens)
-    unsigned char* sRraw = tsm + SCAN_TC_OPERAND_BYTES;   // R as it lies, [CL][DP]
-    unsigned char* sPraw = sRraw + TC_PANEL_BYTES;        // the P slice as it lies, [CL][NS]
-    __shared__ __align__(8) unsigned long long bars[6];   // two contractions, two Q slots, R/P landed, R/P taken
+// The kernel's shared memory: a two-slot ring of the chunk's operands, every tile on a 1024-byte boundary.
+constexpr int TC_THREADS = 512;
+constexpr int TC_WORKERS = 256;            // threads that own tensor-memory lanes 0..63 (lane quarters 0 and 1)
+constexpr int TC_SCOLS = DP / 4;           // state columns (rows p of St) per worker thread
+constexpr int TC_XCOLS = CL / 4;           // tokens of X per worker thread
+constexpr unsigned TC_PANEL_BYTES = CL * DP * 4;        // Q or R: four boxes of 32 channels
+constexpr unsigned TC_BOX_BYTES = CL * 32 * 4;          // [64 tokens][32 channels], 128-byte rows
+constexpr unsigned TC_P_BYTES = CL * SCAN_NS * 4;       // the CTA's columns of P, as they lie
+constexpr unsigned TC_LAM_BYTES = DP * 4;
+constexpr unsigned TC_SLOT_BYTES = 2 * TC_PANEL_BYTES + TC_P_BYTES;
+constexpr size_t SCAN_TC_SMEM_BYTES = 2 * size_t(TC_SLOT_BYTES) + 2 * TC_LAM_BYTES + 1024;   // + room to align
+// tensor-memory columns: the state, its rounded copy (operand), X, its rounded copy
+constexpr unsigned TC_S_COL = 0, TC_SA_COL = 128, TC_X_COL = 256, TC_XA_COL = 320, TC_TMEM_COLS = 512;
+
+// D[128][N] (+)= A[128][8] B[8][N] with A in tensor memory (lane = row, column = contraction index)
+__device__ __forceinline__ void tc_mma_ta(unsigned d_tmem, unsigned a_tmem, unsigned long long db, unsigned idesc,
+                                          unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_load_box(unsigned char* sm, const CUtensorMap* map, int col, int chunk, unsigned bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            tc_smem(sm)),
+        "l"(reinterpret_cast<unsigned long long>(map)), "r"(col), "r"(0), "r"(chunk), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tc_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// TRANSFER: the pass that prepares a segmented scan (see ScanParams::segs): the CTA's slice starts from zero (the first
+// segment: from the given state), or from a column block of the identity with P left out, and only its last state is
+// stored.
+template <bool TRANSFER>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap rmap,
+                const __grid_constant__ CUtensorMap pmap, int* fault, long long* dbg) {
+    extern __shared__ __align__(16) unsigned char tsm_raw[];
+    unsigned char* tsm = tsm_raw + ((1024u - (tc_smem(tsm_raw) & 1023u)) & 1023u);
+    float* s_lam = reinterpret_cast<float*>(tsm + 2 * TC_SLOT_BYTES);   // [2][DP]
+    __shared__ __align__(8) unsigned long long bars[8];
     __shared__ unsigned s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quarter = warp & 3, part = warp >> 2;
 
-    // grid.x = stream * (DP / NS) + column slice (the x dimension has no 65535 limit)
-    const int col0 = (blockIdx.x % (DP / SCAN_NS)) * SCAN_NS;
-    const int s = blockIdx.x / (DP / SCAN_NS);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, part = warp >> 2;
-    // This thread's tensor-memory lane: state row p for the state accumulator and for the R column
-    // it turns; slice column c for the X^T accumulator (lanes 0..63 only).
-    const int row = quarter * 32 + lane;
-    const bool has_x = quarter < 2;
-    const long long base = (long long)s * p.NC;
+    // grid: (stream, segment, column slice); the transfer pass has no last segment and four slices
+    int block = blockIdx.x;
+    const int slices = TRANSFER ? 4 : DP / SCAN_NS, nseg = TRANSFER ? p.segs - 1 : p.segs;
+    const int slice = block % slices;
+    block /= slices;
+    const int seg = block % nseg, s = block / nseg;
+    const bool identity = TRANSFER && slice >= 2;
+    if (identity && seg == 0) return;   // the first segment starts from a known state
+    const int col0 = (slice & 1) * SCAN_NS;
+    const int first = seg * p.seg_len, steps = p.NC - first < p.seg_len ? p.NC - first : p.seg_len;
+    const long long base = (long long)s * p.NC + first;
 
+    const unsigned full0 = tc_smem(&bars[0]), free0 = tc_smem(&bars[2]), bar_a = tc_smem(&bars[4]), bar_x = tc_smem(&bars[5]);
+    const unsigned bar1 = tc_smem(&bars[6]), bar2 = tc_smem(&bars[7]);
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[0])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[1])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[2])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[3])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[4])));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&bars[5])), "r"(TC_THREADS));
+        for (int i = 0; i < 8; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&bars[i])), "r"(i == 4 || i == 5 ? TC_WORKERS : 1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&s_tmem)),
-                     "r"(TC_TMEM_COLS));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&s_tmem)), "r"(TC_TMEM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-    }
-    auto chunk_at = [&](int step) { return base + (p.reverse ? (p.NC - 1 - step) : step); };
-    // thread 0 alone moves Q: one tiled load per chunk into the two-slot ring
-    auto issue = [&](int step) {
-        if (tid == 0 && step < p.NC)
-            tc_load_q(sQ + (step & 1) * TC_PANEL_BYTES, &qmap, (int)chunk_at(step), tc_smem(&bars[2 + (step & 1)]));
-    };
-
-    // this thread's part of the slice: state row `row`, slice columns [TC_N*part, TC_N*part+TC_N)
-    float st[TC_N];
-    const int c0 = part * TC_N;
-#pragma unroll
-    for (int j = 0; j < TC_N; ++j) {
-        float v = 0.f;
-        int cc = col0 + c0 + j;
-        if (p.init != nullptr && row < p.nrows && cc < p.ncols) {
-            const float* src = p.init + (long long)s * p.nrows * p.ncols;
-            v = p.transposed_io ? src[(long long)cc * p.nrows + row] : src[(long long)row * p.ncols + cc];
-        }
-        st[j] = v;
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const unsigned tbase = s_tmem;
-    const unsigned t_state = tbase + ((unsigned)(quarter * 32) << 16) + c0;
-    const unsigned t_x = tbase + ((unsigned)(quarter * 32) << 16) + TC_X_COL + part * TC_N;
-    const unsigned bar1 = tc_smem(&bars[0]), bar2 = tc_smem(&bars[1]);
-    const unsigned idesc = tc_idesc(SCAN_NS);   // N = 64 for both: tokens, then slice columns
-    const unsigned own_row = (row >> 3) * TC_KT_SBO + (row & 7) * 16;                 // this thread's row of sR (and sX)
-    const unsigned own_col = (row >> 2) * TC_S_LBO + (row & 3) * 4;                   // its K position in the state operand
     bool alive = true;   // cleared by the first wait that runs out
-    issue(0);
-    auto issue_rp = [&](int step) {   // single slot: called once every thread is past its reads of the previous one
-        if (tid == 0 && step < p.NC)
-            tc_load_rp(sRraw, sPraw, &rmap, &pmap, (int)chunk_at(step), col0, tc_smem(&bars[4]));
+    auto wait = [&](unsigned bar, int parity, int code) {
+        if (alive && !tc_wait(bar, parity)) {
+            alive = false;
+            atomicExch(fault, code);
+        }
     };
-    issue_rp(0);
 
-    for (int step = 0; step < p.NC; ++step) {
-        const long long gi = chunk_at(step);
-        const int b = step & 1;
-        TC_STAMP(0);
-        // next step's Q: its ring slot was last read by the first contraction of the previous step, which every
-        // thread has seen complete, so the load gets a whole step to land
-        issue(step + 1);
-        const float lam = p.lam[gi * DP + row];
-        // the slice, transposed and rounded, as this step's A operand
+    if (warp == 2) {   // ---- loads: one elected thread, two chunks ahead
+        if (lane == 0) {
+            for (int n = 0; n < steps; ++n) {
+                const int b = n & 1;
+                if (n >= 2) wait(free0 + 8 * b, ((n >> 1) - 1) & 1, 5);
+                unsigned char* slot = tsm + b * TC_SLOT_BYTES;
+                const unsigned bar = full0 + 8 * b;
+                const int chunk = (int)(base + n);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"(2 * TC_PANEL_BYTES + (identity ? 0u : TC_P_BYTES) + TC_LAM_BYTES)
+                             : "memory");
 #pragma unroll
-        for (int j = 0; j < TC_N; ++j) {
-            const int c = c0 + j;
-            *reinterpret_cast<float*>(sS + (c >> 3) * TC_S_SBO + (c & 7) * 16 + own_col) = tc_round(st[j]);
-        }
-        if (alive && !tc_wait(tc_smem(&bars[2 + b]), (step >> 1) & 1)) {   // this step's Q has landed
-            alive = false;
-            atomicExch(fault, 3);
-        }
-        tc_fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const unsigned aS = tc_smem(sS), bQ = tc_smem(sQ + b * TC_PANEL_BYTES);
+                for (int i = 0; i < 4; ++i) tc_load_box(slot + i * TC_BOX_BYTES, &qmap, 32 * i, chunk, bar);
 #pragma unroll
-            for (int ks = 0; ks < DP / 8; ++ks)
-                tc_mma(tbase + TC_X_COL, tc_desc(aS + ks * 2 * TC_S_LBO, TC_S_LBO, TC_S_SBO),
-                       tc_desc(bQ + ks * 2 * TC_Q_LBO, TC_Q_LBO, TC_Q_SBO), idesc, ks > 0);
-            tc_commit(bar1);
-        }
-        __syncwarp();
-        TC_STAMP(1);
-        // behind the first contraction: this thread's R (and P) values, checkpoints, decay
-        // The warps that own X^T rows (lane quarters 0 and 1) take their P values and later run the X
-        // epilogue; the other two quarters turn R, for two state rows each (their own and the one 64
-        // below).  Both read the panels as TMA landed them: rows of consecutive columns, one lane each.
-        if (alive && !tc_wait(tc_smem(&bars[4]), step & 1)) {
-            alive = false;
-            atomicExch(fault, 4);
-        }
-        float rv[TC_N], rv2[TC_N], pv[TC_N];
-        if (has_x) {
-            const float* ps = reinterpret_cast<const float*>(sPraw) + (part * TC_N) * SCAN_NS + row;
-#pragma unroll
-            for (int j = 0; j < TC_N; ++j) pv[j] = ps[j * SCAN_NS];
-        } else {
-            const float* rs = reinterpret_cast<const float*>(sRraw) + (part * TC_N) * DP + row;
-#pragma unroll
-            for (int j = 0; j < TC_N; ++j) rv[j] = rs[j * DP];
-#pragma unroll
-            for (int j = 0; j < TC_N; ++j) rv2[j] = rs[j * DP - 64];
-        }
-        // every thread reports that it holds its values; thread 0 then refills the slot for the next step
-        // right away instead of after the second barrier (the load gets most of a step to land)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem(&bars[5])) : "memory");
-        if (tid == 0) {
-            if (alive && !tc_wait(tc_smem(&bars[5]), step & 1)) {
-                alive = false;
-                atomicExch(fault, 5);
+                for (int i = 0; i < 4; ++i) tc_load_box(slot + TC_PANEL_BYTES + i * TC_BOX_BYTES, &rmap, 32 * i, chunk, bar);
+                if (!identity) tc_load_box(slot + 2 * TC_PANEL_BYTES, &pmap, col0, chunk, bar);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 tc_smem(s_lam + b * DP)),
+                             "l"(p.lam + (long long)chunk * DP), "r"(TC_LAM_BYTES), "r"(bar)
+                             : "memory");
             }
-            issue_rp(step + 1);
         }
         __syncwarp();
-        TC_STAMP(2);
-        if (p.ckb != nullptr) {
-            bf16* ck = p.ckb + gi * (long long)(DP * DP) + row * DP + col0 + c0;
+    } else if (warp == 3) {   // ---- contractions: one elected thread
+        if (lane == 0) {
+            const unsigned id1 = tc_idesc(CL), id2 = tc_idesc(DP) | (1u << 16);   // second one: B is MN-major
+            for (int n = 0; n < steps; ++n) {
+                const int b = n & 1;
+                const unsigned sq = tc_smem(tsm + b * TC_SLOT_BYTES), sr = sq + TC_PANEL_BYTES;
+                wait(full0 + 8 * b, (n >> 1) & 1, 3);
+                wait(bar_a, n & 1, 8);
+                tc_fence_after();
 #pragma unroll
-            for (int j16 = 0; j16 < TC_N / 16; ++j16) {
-                unsigned w[8];
+                for (int k = 0; k < DP / 8; ++k)   // X^T = S^T Q^T
+                    tc_mma_ta(tbase + TC_X_COL, tbase + TC_SA_COL + 8 * k,
+                              tc_desc(sq + (k / 4) * TC_BOX_BYTES + (k % 4) * 32, 16, 1024) | (2ull << 61), id1, k > 0);
+                tc_commit(bar1);
+                wait(bar_x, n & 1, 9);
+                tc_fence_after();
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(st[16 * j16 + 2 * e], st[16 * j16 + 2 * e + 1]);
-                    w[e] = *reinterpret_cast<unsigned*>(&h2);
+                for (int k = 0; k < CL / 8; ++k)   // S^T += X^T R
+                    tc_mma_ta(tbase + TC_S_COL, tbase + TC_XA_COL + 8 * k, tc_desc(sr + k * 1024, TC_BOX_BYTES, TC_R_SBO) | (1ull << 61),
+                              id2, 1u);
+                tc_commit(bar2);
+                tc_commit(free0 + 8 * b);
+            }
+        }
+        __syncwarp();
+    } else if (quarter < 2) {   // ---- workers: lane = state column c
+        const int c = col0 + quarter * 32 + lane, p0 = part * TC_SCOLS, x0 = part * TC_XCOLS;
+        const unsigned t_lane = tbase + ((unsigned)(quarter * 32) << 16);
+        float st[TC_SCOLS];
+#pragma unroll
+        for (int j = 0; j < TC_SCOLS; ++j) {
+            float v = 0.f;
+            if (identity) {
+                v = p0 + j == c ? 1.f : 0.f;
+            } else if (seg > 0) {
+                if (!TRANSFER) v = p.seg_state[((long long)(s * (p.segs - 1) + seg - 1) * 2 * DP + p0 + j) * DP + c];
+            } else if (p.init != nullptr && p0 + j < p.nrows && c < p.ncols) {
+                const float* src = p.init + (long long)s * p.nrows * p.ncols;
+                v = p.transposed_io ? src[(long long)c * p.nrows + p0 + j] : src[(long long)(p0 + j) * p.ncols + c];
+            }
+            st[j] = v;
+        }
+        for (int n = 0; n < steps; ++n) {
+            const int b = n & 1;
+            const long long gi = base + n;
+            TC_STAMP(0);
+            if (n > 0) {
+                wait(bar2, (n - 1) & 1, 2);
+                tc_fence_after();
+                tc_ld<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+                tc_wait_ld();
+            }
+            TC_STAMP(1);
+            {   // operand of the first contraction
+                float r[TC_SCOLS];
+#pragma unroll
+                for (int j = 0; j < TC_SCOLS; ++j) r[j] = tc_round(st[j]);
+                tc_st<TC_SCOLS>(t_lane + TC_SA_COL + p0, r);
+                tc_wait_st();
+                tc_fence_before();
+                tc_arrive(bar_a);
+            }
+            TC_STAMP(2);
+            if (!TRANSFER) {   // checkpoints, behind the first contraction: 32 lanes = 32 consecutive columns
+                if (p.ck != nullptr) {
+                    float* ck = state_ptr(p.ck, gi) + p0 * DP + c;
+#pragma unroll
+                    for (int j = 0; j < TC_SCOLS; ++j) __stcs(ck + j * DP, st[j]);
                 }
-                tc_store32(ck + 16 * j16, w);
+                if (p.ckb != nullptr) tc_store_pairs<TC_SCOLS>(p.ckb + gi * (long long)(DP * DP) + p0 * DP, c, lane, st);
             }
-        }
-        if (p.ck != nullptr) {
-            float* ck = state_ptr(p.ck, gi) + row * DP + col0 + c0;
+            TC_STAMP(3);
+            wait(full0 + 8 * b, (n >> 1) & 1, 4);   // decay and P of this chunk
 #pragma unroll
-            for (int j8 = 0; j8 < TC_N / 8; ++j8) {
-                unsigned w[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(st[8 * j8 + e]);
-                tc_store32(ck + 8 * j8, w);
+            for (int j = 0; j < TC_SCOLS; j += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(s_lam + b * DP + p0 + j);
+                st[j] *= l.x;
+                st[j + 1] *= l.y;
+                st[j + 2] *= l.z;
+                st[j + 3] *= l.w;
             }
-        }
+            tc_st<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+            float pv[TC_XCOLS], x[TC_XCOLS];
+            if (!identity) {
+                const float* ps = reinterpret_cast<const float*>(tsm + b * TC_SLOT_BYTES + 2 * TC_PANEL_BYTES) + x0 * SCAN_NS + quarter * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < TC_N; ++j) st[j] *= lam;
-        TC_STAMP(3);
-        tc_st<TC_N>(t_state, st);
-        tc_wait_st();
-        TC_STAMP(4);
-        // R^T as the second contraction's A operand (the previous step's second contraction has completed)
-        if (!has_x) {
-#pragma unroll
-            for (int j4 = 0; j4 < TC_N / 4; ++j4) {
-                float4 v = make_float4(tc_round(rv[4 * j4]), tc_round(rv[4 * j4 + 1]), tc_round(rv[4 * j4 + 2]),
-                                       tc_round(rv[4 * j4 + 3]));
-                *reinterpret_cast<float4*>(sR + own_row + (part * (TC_N / 4) + j4) * TC_CORE) = v;
-                float4 w = make_float4(tc_round(rv2[4 * j4]), tc_round(rv2[4 * j4 + 1]), tc_round(rv2[4 * j4 + 2]),
-                                       tc_round(rv2[4 * j4 + 3]));
-                *reinterpret_cast<float4*>(sR + own_row - 8 * TC_KT_SBO + (part * (TC_N / 4) + j4) * TC_CORE) = w;
+                for (int j = 0; j < TC_XCOLS; ++j) pv[j] = ps[j * SCAN_NS];
             }
-        }
-
-        TC_STAMP(5);
-        if (alive && !tc_wait(bar1, step & 1)) {
-            alive = false;
-            atomicExch(fault, 1);
-        }
-        tc_fence_after();
-        TC_STAMP(6);
-        if (has_x) {   // warp-uniform: lanes 0..63 of the X^T accumulator
-            float x[TC_N];
-            tc_ld<TC_N>(t_x, x);
-            tc_wait_ld();
-#pragma unroll
-            for (int j = 0; j < TC_N; ++j) x[j] += pv[j];
-            if (p.Xb != nullptr) {
-                bf16* xb = bpanel_ptr(p.Xb, gi) + (part * TC_N) * DP + col0 + row;
-#pragma unroll
-                for (int j = 0; j < TC_N; ++j) xb[j * DP] = __float2bfloat16_rn(x[j]);
-            } else {
-                float* xg = panel_ptr(p.X, gi) + (part * TC_N) * DP + col0 + row;
-#pragma unroll
-                for (int j = 0; j < TC_N; ++j) __stcg(xg + j * DP, x[j]);
-            }
-#pragma unroll
-            for (int j4 = 0; j4 < TC_N / 4; ++j4) {
-                float4 v = make_float4(tc_round(x[4 * j4]), tc_round(x[4 * j4 + 1]), tc_round(x[4 * j4 + 2]),
-                                       tc_round(x[4 * j4 + 3]));
-                *reinterpret_cast<float4*>(sX + own_row + (part * (TC_N / 4) + j4) * TC_CORE) = v;
-            }
-        }
-        tc_fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
+            tc_wait_st();
+            TC_STAMP(4);
+            wait(bar1, n & 1, 1);
             tc_fence_after();
-            const unsigned aR = tc_smem(sR), bX = tc_smem(sX);
+            TC_STAMP(5);
+            tc_ld<TC_XCOLS>(t_lane + TC_X_COL + x0, x);
+            tc_wait_ld();
+            {
+                float r[TC_XCOLS];
 #pragma unroll
-            for (int ks = 0; ks < CL / 8; ++ks)
-                tc_mma(tbase, tc_desc(aR + ks * 2 * TC_CORE, TC_CORE, TC_KT_SBO),
-                       tc_desc(bX + ks * 2 * TC_CORE, TC_CORE, TC_KT_SBO), idesc, 1u);
-            tc_commit(bar2);
-        }
-        __syncwarp();
-        TC_STAMP(7);
-        TC_STAMP(8);
-        if (alive && !tc_wait(bar2, step & 1)) {
-            alive = false;
-            atomicExch(fault, 2);
-        }
-        tc_fence_after();
-        tc_ld<TC_N>(t_state, st);
-        tc_wait_ld();
-        TC_STAMP(9);
-    }
-
-    if (p.fin != nullptr) {
-        float* dst = p.fin + (long long)s * p.nrows * p.ncols;
-#pragma unroll
-        for (int j = 0; j < TC_N; ++j) {
-            int cc = col0 + c0 + j;
-            if (row < p.nrows && cc < p.ncols) {
-                if (p.transposed_io)
-                    dst[(long long)cc * p.nrows + row] = st[j];
-                else
-                    dst[(long long)row * p.ncols + cc] = st[j];
+                for (int j = 0; j < TC_XCOLS; ++j) {
+                    if (!identity) x[j] += pv[j];
+                    r[j] = tc_round(x[j]);
+                }
+                tc_st<TC_XCOLS>(t_lane + TC_XA_COL + x0, r);
+                tc_wait_st();
+                tc_fence_before();
+                tc_arrive(bar_x);
             }
+            TC_STAMP(6);
+            if (!TRANSFER) {   // behind the second contraction
+                if (p.Xb != nullptr) {
+                    tc_store_pairs<TC_XCOLS>(bpanel_ptr(p.Xb, gi) + x0 * DP, c, lane, x);
+                } else {
+                    float* xg = panel_ptr(p.X, gi) + x0 * DP + c;
+#pragma unroll
+                    for (int j = 0; j < TC_XCOLS; ++j) xg[j * DP] = x[j];
+                }
+            }
+            TC_STAMP(7);
+        }
+        wait(bar2, (steps - 1) & 1, 2);
+        tc_fence_after();
+        tc_ld<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+        tc_wait_ld();
+        if (TRANSFER) {
+            float* dst = p.seg_state + ((long long)((s * (p.segs - 1) + seg) * 2 + (identity ? 1 : 0)) * DP + p0) * DP + c;
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; ++j) dst[j * DP] = st[j];
+        } else if (p.fin != nullptr && seg == p.segs - 1 && c < p.ncols) {
+            float* dst = p.fin + (long long)s * p.nrows * p.ncols;
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; ++j)
+                if (p0 + j < p.nrows)
+                    dst[p.transposed_io ? (long long)c * p.nrows + p0 + j : (long long)(p0 + j) * p.ncols + c] = st[j];
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TC_TMEM_COLS));
+}
+
+// Entry states of the segments of a segmented scan: E_g = local_g + transfer_g E_{g-1}, written over local_g, where
+// (local, transfer) are the pairs the transfer pass stored.  FP32 throughout.  One CTA per stream and 16 columns: they
+// never exchange data.
+constexpr int COMBINE_COLS = 16, COMBINE_THREADS = 256;
+__global__ void __launch_bounds__(COMBINE_THREADS) k_scan_combine(float* seg_state, int segs) {
+    __shared__ __align__(16) float s_e[DP][COMBINE_COLS];
+    const int col0 = (blockIdx.x % (DP / COMBINE_COLS)) * COMBINE_COLS, s = blockIdx.x / (DP / COMBINE_COLS);
+    const int row = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * 8;
+    for (int g = 0; g < segs - 1; ++g) {
+        float* local = seg_state + (long long)(s * (segs - 1) + g) * 2 * DP * DP;
+        float acc[8];
+        {
+            const float4 a = *reinterpret_cast<const float4*>(local + row * DP + col0 + c0);
+            const float4 b = *reinterpret_cast<const float4*>(local + row * DP + col0 + c0 + 4);
+            acc[0] = a.x; acc[1] = a.y; acc[2] = a.z; acc[3] = a.w;
+            acc[4] = b.x; acc[5] = b.y; acc[6] = b.z; acc[7] = b.w;
+        }
+        if (g > 0) {
+            const float* t = local + DP * DP + row * DP;
+#pragma unroll 8
+            for (int k = 0; k < DP; k += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(t + k);
+                const float wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] = fmaf(wv[i], s_e[k + i][c0 + e], acc[e]);
+            }
+            *reinterpret_cast<float4*>(local + row * DP + col0 + c0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+            *reinterpret_cast<float4*>(local + row * DP + col0 + c0 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s_e[row][c0 + e] = acc[e];
+        __syncthreads();
+    }
 }
 
 }  // namespace sd
