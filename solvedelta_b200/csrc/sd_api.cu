@@ -1,7 +1,6 @@
 // C ABI of the SolveDelta chunked recurrence for B200 (sm_100a).
 // Declarations and the upstream interfaces they replace: include/solvedelta_b200.h
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 
 #include "../../include/solvedelta_b200.h"
@@ -11,7 +10,6 @@
 #include "sd_decode.cuh"
 #include "sd_forward.cuh"
 #include "sd_mixer.cuh"
-#include "sd_scan.cuh"
 #include "sd_scan_tc.cuh"
 #include "sd_output_tc.cuh"
 #include "sd_token.cuh"
@@ -222,6 +220,34 @@ bool scan_maps(const ScanParams& sp, long long chunks, const ScanMaps** out) {
     return true;
 }
 
+struct ScanBMaps {
+    const void *q, *r, *r2, *x2, *p;
+    long long chunks;
+    CUtensorMap qmap, rmap, r2map, x2map, pmap;
+};
+bool scan_b_maps(const ScanParamsB& sp, long long chunks, const ScanBMaps** out) {
+    constexpr int SLOTS = 4;
+    thread_local ScanBMaps cache[SLOTS] = {};
+    thread_local int next = 0;
+    for (int i = 0; i < SLOTS; ++i)
+        if (cache[i].q == sp.Q && cache[i].r == sp.R && cache[i].r2 == sp.R2 && cache[i].x2 == sp.X2 && cache[i].p == sp.P &&
+            cache[i].chunks == chunks && chunks != 0) {
+            *out = &cache[i];
+            return true;
+        }
+    ScanBMaps& m = cache[next];
+    next = (next + 1) % SLOTS;
+    m.q = nullptr;
+    m.chunks = 0;
+    if (!make_bpanel_map(&m.qmap, sp.Q, chunks, CL, DP) || !make_bpanel_map(&m.rmap, sp.R, chunks, CL, DP) ||
+        !make_bpanel_map(&m.r2map, sp.R2, chunks, CL, DP) || !make_bpanel_map(&m.x2map, sp.X2, chunks, CL, DP) ||
+        !make_bpanel_map(&m.pmap, sp.P, chunks, CL, DP))
+        return false;
+    m.q = sp.Q; m.r = sp.R; m.r2 = sp.R2; m.x2 = sp.X2; m.p = sp.P; m.chunks = chunks;
+    *out = &m;
+    return true;
+}
+
 int* scan_fault_ptr() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -262,16 +288,87 @@ inline void set_dbg(Geometry&, int, int) {}
 inline long long* scan_dbg(int) { return nullptr; }
 #endif
 
-bool launch_scan_tc(ScanParams sp, int streams, cudaStream_t stream, long long* dbg) {
+// A launch whose kernel may start while the one before it in the stream still runs (it waits for it itself).
+cudaLaunchAttribute chained_launch() {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    return at;
+}
+
+// Launches a kernel of the operator's sequence, chained to the one before it unless it is the first of a call.
+template <class... Params, class... Args>
+void launch(void (*kernel)(Params...), long long grid, int threads, size_t smem, bool chained, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at = chained_launch();
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+// How many segments to cut a scan into: the number with the least time by a model of what the launches were measured to
+// take (us): 6.5 + steps x step for a scan or transfer pass while its CTAs fit the 148 SMs, a multiple of the steps past
+// that, and 6 + 2.3 per product for the chaining in between.  A cut that gains less than a tenth is not made.  It is not
+// made up to 64 chunks either: the rule depends on the number of streams, and a shard of a batch's streams is to give the
+// bits of the whole batch at training lengths.  Past 24 streams the SMs are busy and nothing is cut.
+constexpr float FWD_STEP_US = 2.2f, FWD_TRANSFER_US = 1.8f, BWD_STEP_US = 1.42f, BWD_TRANSFER_US = 1.18f;
+int scan_segments(int streams, int NC, float step, float transfer_step) {
+    constexpr int SMS = 148, MIN_CHUNKS = 64;
+    if (NC <= MIN_CHUNKS) return 1;
+    const auto waves = [](int ctas) { return (ctas + SMS - 1) / SMS; };
+    const float whole = 6.5f + waves(2 * streams) * NC * step;
+    float best = 0.9f * whole;
+    int segs = 1;
+    for (int g = 2; g <= NC && 2 * streams * (g - 1) <= 2 * SMS; ++g) {
+        const int len = (NC + g - 1) / g;
+        const float t = 13.f + len * (waves(streams * (4 * g - 6)) * transfer_step + waves(2 * streams * g) * step) + 6.f +
+                        2.3f * (g - 2) * waves(streams * (DP / COMBINE_COLS));
+        if (t < best) {
+            best = t;
+            segs = g;
+        }
+    }
+    return segs;
+}
+// Cuts a scan into segments; `room`: scratch that is free while it runs, for the segment states.
+template <class P>
+void set_segments(P& sp, int streams, float step, float transfer_step, void* room, size_t room_bytes) {
+    sp.segs = scan_segments(streams, sp.NC, step, transfer_step);
+    while (sp.segs > 1 && size_t(streams) * (sp.segs - 1) * 2 * DP * DP * 4 > room_bytes) --sp.segs;
+    sp.seg_len = (sp.NC + sp.segs - 1) / sp.segs;
+    sp.segs = (sp.NC + sp.seg_len - 1) / sp.seg_len;   // no empty segment
+    sp.seg_state = static_cast<float*>(room);
+}
+bool launch_scan_tc(ScanParams sp, int streams, void* room, size_t room_bytes, cudaStream_t stream, long long* dbg) {
     const ScanMaps* m = nullptr;
     if (!scan_maps(sp, (long long)streams * sp.NC, &m)) return false;
+    set_segments(sp, streams, FWD_STEP_US, FWD_TRANSFER_US, room, room_bytes);
     if (sp.segs > 1) {
-        k_state_scan_tc<true><<<streams * (sp.segs - 1) * 4, TC_THREADS, SCAN_TC_SMEM_BYTES, stream>>>(
-            sp, m->qmap, m->rmap, m->pmap, scan_fault_ptr(), nullptr);
-        k_scan_combine<<<streams * (DP / COMBINE_COLS), COMBINE_THREADS, 0, stream>>>(sp.seg_state, sp.segs);
+        launch(k_state_scan_tc<true>, streams * (sp.segs - 1) * 4, TC_THREADS, SCAN_TC_SMEM_BYTES, true, stream, sp,
+               m->qmap, m->rmap, m->pmap, scan_fault_ptr(), nullptr);
+        launch(k_scan_combine, streams * (DP / COMBINE_COLS), COMBINE_THREADS, COMBINE_SMEM, true, stream,
+               sp.seg_state, sp.segs);
     }
-    k_state_scan_tc<false><<<streams * sp.segs * (DP / SCAN_NS), TC_THREADS, SCAN_TC_SMEM_BYTES, stream>>>(
-        sp, m->qmap, m->rmap, m->pmap, scan_fault_ptr(), dbg);
+    launch(k_state_scan_tc<false>, streams * sp.segs * (DP / SCAN_NS), TC_THREADS, SCAN_TC_SMEM_BYTES, true, stream, sp,
+               m->qmap, m->rmap, m->pmap, scan_fault_ptr(), dbg);
+    return true;
+}
+bool launch_scan_b(ScanParamsB sp, int streams, void* room, size_t room_bytes, cudaStream_t stream) {
+    const ScanBMaps* m = nullptr;
+    if (!scan_b_maps(sp, (long long)streams * sp.NC, &m)) return false;
+    set_segments(sp, streams, BWD_STEP_US, BWD_TRANSFER_US, room, room_bytes);
+    if (sp.segs > 1) {
+        launch(k_state_scan_b<true>, streams * (sp.segs - 1) * 4, TC_THREADS, SCAN_TB_SMEM_BYTES, true, stream, sp,
+               m->qmap, m->rmap, m->r2map, m->x2map, m->pmap, scan_fault_ptr());
+        launch(k_scan_combine, streams * (DP / COMBINE_COLS), COMBINE_THREADS, COMBINE_SMEM, true, stream,
+               sp.seg_state, sp.segs);
+    }
+    launch(k_state_scan_b<false>, streams * sp.segs * (DP / SCAN_NS), TC_THREADS, SCAN_TB_SMEM_BYTES, true, stream, sp,
+               m->qmap, m->rmap, m->r2map, m->x2map, m->pmap, scan_fault_ptr());
     return true;
 }
 
@@ -317,7 +414,9 @@ cudaError_t configure_kernels() {
         if ((e = cudaGetSymbolAddress(&w, g_scan_fault_word)) != cudaSuccess) return e;
         g_scan_fault_ptr[dev] = static_cast<int*>(w);
     }
-    if ((e = allow_smem(k_state_scan_b, SCAN_B_SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_state_scan_b<false>, SCAN_TB_SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_state_scan_b<true>, SCAN_TB_SMEM_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_scan_combine, COMBINE_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_exterior_prep_bwd<true, false>, EXT_PREP_BWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_exterior_prep_bwd<false, false>, EXT_PREP_BWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_exterior_prep_bwd<true, true>, EXT_PREP_BWD_SMEM)) != cudaSuccess) return e;
@@ -364,26 +463,18 @@ const char* const kLaunchNames[] = {
 int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_LAUNCH_FAILED; }
 
 // One chunk kernel, instantiated for (vector-aligned operands?, token masks present?).
-#define SD_LAUNCH_CHUNK(kernel, smem)                                                          \
-    do {                                                                                       \
-        if (fast && !masked) kernel<true, false><<<chunks, NTHREADS, smem, stream>>>(p);       \
-        else if (fast) kernel<true, true><<<chunks, NTHREADS, smem, stream>>>(p);              \
-        else if (!masked) kernel<false, false><<<chunks, NTHREADS, smem, stream>>>(p);         \
-        else kernel<false, true><<<chunks, NTHREADS, smem, stream>>>(p);                       \
+#define SD_LAUNCH_CHUNK(kernel, smem, chained)                                                          \
+    do {                                                                                                \
+        if (fast && !masked) launch(kernel<true, false>, chunks, NTHREADS, smem, chained, stream, p);   \
+        else if (fast) launch(kernel<true, true>, chunks, NTHREADS, smem, chained, stream, p);          \
+        else if (!masked) launch(kernel<false, false>, chunks, NTHREADS, smem, chained, stream, p);     \
+        else launch(kernel<false, true>, chunks, NTHREADS, smem, chained, stream, p);                   \
     } while (0)
 
 bool operands_ok(const sd_operand* ops, int n) {
     for (int i = 0; i < n; ++i)
         if (ops[i].ptr == nullptr) return false;
     return true;
-}
-
-// A launch whose kernel may start while the one before it in the stream still runs (it waits for it itself).
-cudaLaunchAttribute chained_launch() {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    return at;
 }
 
 template <int RG, int CG, int NORM>
@@ -481,8 +572,15 @@ int sd_panel_kind(const sd_shape* shape, int which, const char* name) {
     return found ? kind : SD_ERR_INVALID_ARGUMENT;
 }
 
-int sd_forward_launches(const sd_shape* shape) { return shape_ok(shape) ? 5 : 0; }
-int sd_backward_launches(const sd_shape* shape) { return shape_ok(shape) ? 6 : 0; }
+// a scan that is cut into segments is three launches
+int sd_forward_launches(const sd_shape* shape) {
+    if (!shape_ok(shape)) return 0;
+    return 5 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, FWD_STEP_US, FWD_TRANSFER_US) > 1 ? 4 : 0);
+}
+int sd_backward_launches(const sd_shape* shape) {
+    if (!shape_ok(shape)) return 0;
+    return 6 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, BWD_STEP_US, BWD_TRANSFER_US) > 1 ? 4 : 0);
+}
 int sd_chunk_tokens(void) { return CL; }
 int sd_version(void) { return 1; }
 
@@ -576,11 +674,15 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     const bool fast = all_fast(fwd_ops, 8, *s);
     const bool masked = a->valid_mask != nullptr || a->reset_mask != nullptr;
 
+    // the segment states of a scan live in the panels of the other one: Wd, Ud, Dt (and Upd, Qc, Ubar) are neighbours in
+    // the scratch, not yet written when the C scan runs (already read when the S scan runs)
+    const size_t panel_bytes = kind_bytes(0) * (size_t)chunks;
+
     set_dbg(p.g, 0, chunks);
     if (po)   // the predictor-only instantiations: general operand layout, mask-aware (null masks are legal)
         k_prep_fwd<false, true, true><<<chunks, NTHREADS, PREP_FWD_SMEM, stream>>>(p);
     else
-        SD_LAUNCH_CHUNK(k_prep_fwd, PREP_FWD_SMEM);
+        SD_LAUNCH_CHUNK(k_prep_fwd, PREP_FWD_SMEM, false);
     mark(stream);
     {
         ScanParams sp{};
@@ -588,8 +690,8 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         sp.lam = p.Lam; sp.X = p.Delta; sp.ck = p.CtCk; sp.Xb = nullptr;
         sp.ckb = bpanel_at(kSaved, s, a->saved, "CtCkB");
         sp.init = a->C0; sp.fin = a->C_T;
-        sp.NC = p.g.NC; sp.segs = 1; sp.seg_len = p.g.NC; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
-        if (!launch_scan_tc(sp, streams, stream, scan_dbg(1))) return SD_ERR_LAUNCH_FAILED;
+        sp.NC = p.g.NC; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
+        if (!launch_scan_tc(sp, streams, p.Wd, 3 * panel_bytes, stream, scan_dbg(1))) return SD_ERR_LAUNCH_FAILED;
         mark(stream);
     }
     set_dbg(p.g, 2, chunks);
@@ -597,15 +699,15 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         k_primal_exterior_fwd<false, true, true><<<chunks, NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p);
         return launch_status();   // the kernel stops after its primal half
     }
-    SD_LAUNCH_CHUNK(k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
+    SD_LAUNCH_CHUNK(k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM, true);
     mark(stream);
     {
         ScanParams sp{};
         sp.P = p.Ud; sp.Q = p.Wd; sp.R = p.Dt;
         sp.lam = p.Lam; sp.X = nullptr; sp.ck = nullptr; sp.Xb = p.Zt; sp.ckb = p.SCk;
         sp.init = a->S0; sp.fin = a->S_T;
-        sp.NC = p.g.NC; sp.segs = 1; sp.seg_len = p.g.NC; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
-        if (!launch_scan_tc(sp, streams, stream, scan_dbg(3))) return SD_ERR_LAUNCH_FAILED;
+        sp.NC = p.g.NC; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
+        if (!launch_scan_tc(sp, streams, p.Upd, 3 * panel_bytes, stream, scan_dbg(3))) return SD_ERR_LAUNCH_FAILED;
         mark(stream);
     }
     set_dbg(p.g, 4, chunks);
@@ -615,11 +717,11 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         int* fault = scan_fault_ptr();
         if (fault == nullptr || !output_maps(p, total_chunks(s), &m)) return SD_ERR_LAUNCH_FAILED;
         if (masked)
-            k_output_fwd_tc<true><<<chunks, OUT_TC_THREADS, OUTPUT_TC_SMEM, stream>>>(p, m->xg_map, m->aqd_map,
-                                                                                    m->s_map, m->zt_map, fault);
+            launch(k_output_fwd_tc<true>, chunks, OUT_TC_THREADS, OUTPUT_TC_SMEM, true, stream, p, m->xg_map, m->aqd_map,
+                   m->s_map, m->zt_map, fault);
         else
-            k_output_fwd_tc<false><<<chunks, OUT_TC_THREADS, OUTPUT_TC_SMEM, stream>>>(p, m->xg_map, m->aqd_map,
-                                                                                     m->s_map, m->zt_map, fault);
+            launch(k_output_fwd_tc<false>, chunks, OUT_TC_THREADS, OUTPUT_TC_SMEM, true, stream, p, m->xg_map, m->aqd_map,
+                   m->s_map, m->zt_map, fault);
     }
     mark(stream);
     return launch_status();
@@ -689,7 +791,8 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
 
     const int chunks = (int)total_chunks(s);
     const int streams = s->B * s->H;
-    const dim3 scan_grid((DP / SCAN_NS) * streams);
+    // segment states: the dS scan's in duPart .. Xext (neighbours, not yet written), the dC scan's in Pp .. dR (already read)
+    const size_t bpanel_bytes = kind_bytes(4) * (size_t)chunks;
     const Operand bwd_ops[] = {p.u, p.h, p.q, p.k, p.v, p.er, p.wr, p.ld, p.dy};
     const bool fast = all_fast(bwd_ops, 9, *s);
     const bool masked = a->valid_mask != nullptr || a->reset_mask != nullptr;
@@ -713,41 +816,41 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
             k_predictor_seed_bwd<false><<<chunks, NTHREADS, 0, stream>>>(p, dact, dupd, act);
     } else {
     set_dbg(p.g, 5, chunks);
-    SD_LAUNCH_CHUNK(k_exterior_prep_bwd, EXT_PREP_BWD_SMEM);
+    SD_LAUNCH_CHUNK(k_exterior_prep_bwd, EXT_PREP_BWD_SMEM, false);
     mark(stream);
     {
         ScanParamsB sp{};
         sp.P = p.Pp; sp.Q = p.Qp; sp.R = p.Ag; sp.R2 = p.Xg; sp.X2 = p.Dyf;
         sp.lam = p.Lam; sp.X = p.dR; sp.ck = p.dSeCk;
         sp.init = a->dS_T; sp.fin = a->dS0;
-        sp.NC = p.g.NC; sp.reverse = 1; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
-        k_state_scan_b<<<scan_grid, SCAN_THREADS, SCAN_B_SMEM_BYTES, stream>>>(sp);
+        sp.NC = p.g.NC; sp.transposed_io = 0; sp.nrows = s->r; sp.ncols = s->V;
+        if (!launch_scan_b(sp, streams, p.duPart, 6 * bpanel_bytes, stream)) return SD_ERR_LAUNCH_FAILED;
     mark(stream);
     }
     set_dbg(p.g, 7, chunks);
-    SD_LAUNCH_CHUNK(k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM);
+    SD_LAUNCH_CHUNK(k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM, true);
     mark(stream);
     }
     set_dbg(p.g, 8, chunks);
     if (po)
         k_primal_bwd<false, true, true><<<chunks, NTHREADS, PRIMAL_BWD_SMEM, stream>>>(p);
     else
-        SD_LAUNCH_CHUNK(k_primal_bwd, PRIMAL_BWD_SMEM);
+        SD_LAUNCH_CHUNK(k_primal_bwd, PRIMAL_BWD_SMEM, true);
     mark(stream);
     {
         ScanParamsB sp{};
         sp.P = p.Ppp; sp.Q = p.Qpp; sp.R = p.Rneg; sp.R2 = p.DG; sp.X2 = p.Khat;
         sp.lam = p.Lam; sp.X = p.dRr; sp.ck = p.dCeCk;
         sp.init = a->dC_T; sp.fin = a->dC0;
-        sp.NC = p.g.NC; sp.reverse = 1; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
-        k_state_scan_b<<<scan_grid, SCAN_THREADS, SCAN_B_SMEM_BYTES, stream>>>(sp);
+        sp.NC = p.g.NC; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
+        if (!launch_scan_b(sp, streams, p.Pp, 4 * bpanel_bytes, stream)) return SD_ERR_LAUNCH_FAILED;
     mark(stream);
     }
     set_dbg(p.g, 10, chunks);
     if (po)
         k_predictor_close_bwd<false, true, true><<<chunks, NTHREADS, PRED_CLOSE_BWD_SMEM, stream>>>(p);
     else
-        SD_LAUNCH_CHUNK(k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM);
+        SD_LAUNCH_CHUNK(k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM, true);
     mark(stream);
     return launch_status();
 }

@@ -99,6 +99,8 @@ constexpr size_t EXT_PREP_BWD_SMEM = 2 * BSLOT_BYTES + BMAT_BYTES + MAT_BYTES;
 // 61 KB of shared memory and few registers: two CTAs share an SM
 template <bool FAST, bool MASKED>
 __global__ void __launch_bounds__(NTHREADS, 2) k_exterior_prep_bwd(BwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -284,6 +286,8 @@ __device__ __forceinline__ void epi_scale_store_bsm(float (&acc)[NTW][4], int r0
 
 template <bool FAST, bool MASKED>
 __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -463,6 +467,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
 // and zeros for what only the exterior contributes (dkPart: d - k^ has no direct k^ term; duPart, Xext, SdS).
 template <bool MASKED>
 __global__ void __launch_bounds__(NTHREADS) k_predictor_seed_bwd(BwdParams p, Operand dact, Operand dupd, Operand act) {
+    chain_wait();
+    chain_release();
     const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const int r = p.g.r;
     const int lr = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
@@ -508,6 +514,8 @@ constexpr size_t PRIMAL_BWD_SMEM = 7 * BSLOT_BYTES + BSTATE_BYTES + 2 * BMAT_BYT
 
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -779,6 +787,8 @@ static_assert(3 * size_t(CL) * LDP * 4 >= 2 * BSTATE_BYTES, "closure panels over
 
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -135,6 +135,12 @@ __device__ __forceinline__ const float* state_ptr(const float* base, long long g
     return base + gi * (long long)(DP * DP);
 }
 
+// Programmatic dependent launch.  A kernel of this library lets its dependents start only after its own wait has
+// returned, so when one of them runs, everything before its predecessor is complete: what it may read ahead of its wait
+// is weights and data that was written two launches ago or earlier.  Both are no-ops in a launch without the attribute.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 1 / (1 + exp(-x)) with the fast reciprocal (2 ulp): exp(-x) = inf gives exactly 0.
 __device__ __forceinline__ float sigmoidf_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
 

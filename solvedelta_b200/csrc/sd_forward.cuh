@@ -116,6 +116,8 @@ static_assert(2 * (PREP_FWD_SMEM + 1024) <= 228 * 1024, "two CTAs of the predict
 
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) float smem[];
@@ -304,6 +306,8 @@ __device__ __forceinline__ void async_state_cols_f32(float* sm, const float* st,
 
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p) {
+    chain_wait();
+    chain_release();
     int ph = 0;
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) float smem[];

@@ -74,7 +74,6 @@ k_output_fwd_tc(FwdParams p, const __grid_constant__ CUtensorMap xg_map, const _
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(sZt + OUT_ZT_BYTES);
     unsigned* s_tmem = reinterpret_cast<unsigned*>(bars + 2);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const int V = p.g.V;
     int ph = 0;
     SD_PHASE(p.g, ph);
@@ -91,6 +90,9 @@ k_output_fwd_tc(FwdParams p, const __grid_constant__ CUtensorMap xg_map, const _
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_wait();   // the set-up above overlaps the end of the scan before
+    chain_release();
+    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const unsigned tbase = *s_tmem;
     const unsigned bar_load = tc_smem(&bars[0]), bar_mma = tc_smem(&bars[1]);
     SD_PHASE(p.g, ph);

@@ -1,7 +1,9 @@
-// The forward chunk-state scan on the fifth-generation tensor cores (tcgen05).
+// The serial chunk-state scans on the fifth-generation tensor cores (tcgen05): C and S forward, dS and dC in reverse (at
+// the end of this file).
 //
 //     X  = P + Q St ;  checkpoint St ;  St = diag(lam) St + R^T X
-// for every chunk of a stream in order.  A CTA carries a 64-column slice of one stream's state, transposed, in tensor
+// for every chunk of a stream in order (the predictor state is carried transposed, St[c][a] = C[a][c], so that both C and
+// S decay by rows; column slices never exchange data).  A CTA carries a 64-column slice of one stream's state, transposed, in tensor
 // memory (lane = slice column c, column = state row p), and both contractions take their A operand from tensor memory:
 //     X^T[c][tok] = sum_p St^T[c][p] Q[tok][p]      A = rounded state,  B = Q as it lies (K-major)
 //     St^T[c][p] += sum_t X^T[c][tok] R[tok][p]     A = rounded X,      B = R as it lies (MN-major)
@@ -28,9 +30,31 @@
 #pragma once
 #include <cuda.h>   // CUtensorMap (types only: the encoder is reached through the runtime's driver entry point)
 
-#include "sd_scan.cuh"
+#include "sd_bf16.cuh"
+#include "sd_common.cuh"
 
 namespace sd {
+
+constexpr int SCAN_NS = 64;   // state columns per CTA (2 CTAs per stream)
+
+struct ScanParams {
+    const float* P;    // [chunks][CL][DP]
+    const float* Q;
+    const float* R;
+    const float* lam;  // [chunks][DP]
+    float* X;          // out [chunks][CL][DP]            (FP32; or null when Xb is set)
+    float* ck;         // out [chunks][DP][DP] state before the chunk's update (or null when ckb is set)
+    bf16* Xb;          // BF16 alternatives for consumers that only feed BF16 contractions
+    bf16* ckb;
+    const float* init; // nullable: true-dimension state [S][rows][cols] (or transposed)
+    float* fin;        // nullable
+    int NC;            // chunks per stream
+    int segs, seg_len; // segments a stream is cut into, and their chunks (the last one may be shorter)
+    float* seg_state;  // [streams][segs - 1][2][DP][DP]: end states and transfer matrices, then entry states (segs > 1)
+    int transposed_io; // init/fin hold the transpose (predictor state C[a][c])
+    int nrows, ncols;  // true dims of the carried St: rows (<= DP), cols (<= DP)
+};
+
 
 constexpr unsigned TC_R_SBO = 512;          // bytes between the 4-row groups of an MN-major TF32 tile
 constexpr int TC_WAIT_LIMIT = 1 << 20;    // polls of one mbarrier before the wait is given up
@@ -183,6 +207,43 @@ __device__ __forceinline__ void tc_arrive(unsigned bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// Rows p0.. of column c of a stream's carried state, from and to the caller's [rows][cols] (or transposed) layout.  The
+// transposed layout holds a thread's rows side by side: 16-byte accesses when every row starts on such a boundary.
+__device__ __forceinline__ void tc_init_state(const float* init, int s, int nrows, int ncols, int transposed, int p0, int c,
+                                              float (&st)[TC_SCOLS]) {
+#pragma unroll
+    for (int j = 0; j < TC_SCOLS; ++j) st[j] = 0.f;
+    if (init == nullptr || c >= ncols) return;
+    const float* src = init + (long long)s * nrows * ncols;
+    if (transposed && (nrows & 3) == 0 && (reinterpret_cast<uintptr_t>(init) & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < TC_SCOLS; j += 4)
+            if (p0 + j < nrows) {
+                const float4 v = *reinterpret_cast<const float4*>(src + (long long)c * nrows + p0 + j);
+                st[j] = v.x; st[j + 1] = v.y; st[j + 2] = v.z; st[j + 3] = v.w;
+            }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < TC_SCOLS; ++j)
+        if (p0 + j < nrows) st[j] = transposed ? src[(long long)c * nrows + p0 + j] : src[(long long)(p0 + j) * ncols + c];
+}
+__device__ __forceinline__ void tc_final_state(float* fin, int s, int nrows, int ncols, int transposed, int p0, int c,
+                                               const float (&st)[TC_SCOLS]) {
+    if (fin == nullptr || c >= ncols) return;
+    float* dst = fin + (long long)s * nrows * ncols;
+    if (transposed && (nrows & 3) == 0 && (reinterpret_cast<uintptr_t>(fin) & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < TC_SCOLS; j += 4)
+            if (p0 + j < nrows)
+                *reinterpret_cast<float4*>(dst + (long long)c * nrows + p0 + j) = make_float4(st[j], st[j + 1], st[j + 2], st[j + 3]);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < TC_SCOLS; ++j)
+        if (p0 + j < nrows) dst[transposed ? (long long)c * nrows + p0 + j : (long long)(p0 + j) * ncols + c] = st[j];
+}
+
 // TRANSFER: the pass that prepares a segmented scan (see ScanParams::segs): the CTA's slice starts from zero (the first
 // segment: from the given state), or from a column block of the identity with P left out, and only its last state is
 // stored.
@@ -223,6 +284,8 @@ k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap, const __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    chain_wait();   // the set-up above overlaps the end of the kernel before
+    chain_release();
     const unsigned tbase = s_tmem;
     bool alive = true;   // cleared by the first wait that runs out
     auto wait = [&](unsigned bar, int parity, int code) {
@@ -284,18 +347,15 @@ k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap, const __
         const int c = col0 + quarter * 32 + lane, p0 = part * TC_SCOLS, x0 = part * TC_XCOLS;
         const unsigned t_lane = tbase + ((unsigned)(quarter * 32) << 16);
         float st[TC_SCOLS];
+if (identity) {
 #pragma unroll
-        for (int j = 0; j < TC_SCOLS; ++j) {
-            float v = 0.f;
-            if (identity) {
-                v = p0 + j == c ? 1.f : 0.f;
-            } else if (seg > 0) {
-                if (!TRANSFER) v = p.seg_state[((long long)(s * (p.segs - 1) + seg - 1) * 2 * DP + p0 + j) * DP + c];
-            } else if (p.init != nullptr && p0 + j < p.nrows && c < p.ncols) {
-                const float* src = p.init + (long long)s * p.nrows * p.ncols;
-                v = p.transposed_io ? src[(long long)c * p.nrows + p0 + j] : src[(long long)(p0 + j) * p.ncols + c];
-            }
-            st[j] = v;
+            for (int j = 0; j < TC_SCOLS; ++j) st[j] = p0 + j == c ? 1.f : 0.f;
+        } else if (seg > 0) {
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; ++j)
+                st[j] = TRANSFER ? 0.f : p.seg_state[((long long)(s * (p.segs - 1) + seg - 1) * 2 * DP + p0 + j) * DP + c];
+        } else {
+            tc_init_state(p.init, s, p.nrows, p.ncols, p.transposed_io, p0, c, st);
         }
         for (int n = 0; n < steps; ++n) {
             const int b = n & 1;
@@ -382,12 +442,259 @@ k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap, const __
             float* dst = p.seg_state + ((long long)((s * (p.segs - 1) + seg) * 2 + (identity ? 1 : 0)) * DP + p0) * DP + c;
 #pragma unroll
             for (int j = 0; j < TC_SCOLS; ++j) dst[j * DP] = st[j];
-        } else if (p.fin != nullptr && seg == p.segs - 1 && c < p.ncols) {
-            float* dst = p.fin + (long long)s * p.nrows * p.ncols;
+        } else if (seg == p.segs - 1) {
+            tc_final_state(p.fin, s, p.nrows, p.ncols, p.transposed_io, p0, c, st);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TC_TMEM_COLS));
+}
+
+// ---------------------------------------------------------------------------
+// The two reverse scans (dS and dC), chunks last to first:
+//     X = P + Q St ;  checkpoint St ;  St = diag(lam) St + R^T X + R2^T X2
+// Same structure with BF16 panels and kind::f16 contractions (gradient tolerances admit BF16 operands; the state itself
+// stays FP32).  All panels land with the 128-byte swizzle as tiles of 64 channels; X2, whose columns are the M side, is
+// an MN-major A operand in shared memory (rows 64..127 of it alias what follows and feed lanes nobody reads).  The X2
+// term does not wait for X: it is issued behind the first contraction as soon as the decayed state is back.
+struct ScanParamsB {
+    const bf16 *P, *Q, *R, *R2, *X2;   // [chunks][CL][DP]
+    const float* lam;                  // [chunks][DP]
+    bf16* X;                           // out [chunks][CL][DP]
+    bf16* ck;                          // out [chunks][DP][DP]
+    const float* init;
+    float* fin;
+    int NC;
+    int segs, seg_len;                 // as in ScanParams; segment 0 holds the last chunks
+    float* seg_state;
+    int transposed_io, nrows, ncols;
+};
+
+constexpr unsigned TB_TILE_BYTES = CL * 64 * 2;         // [64 tokens][64 channels]
+constexpr unsigned TB_Q = 0, TB_R = 2 * TB_TILE_BYTES, TB_R2 = 4 * TB_TILE_BYTES, TB_X2 = 6 * TB_TILE_BYTES, TB_P = 7 * TB_TILE_BYTES;
+constexpr unsigned TB_SLOT_BYTES = 8 * TB_TILE_BYTES;   // X2 and P: the CTA's 64 columns
+constexpr size_t SCAN_TB_SMEM_BYTES = 2 * size_t(TB_SLOT_BYTES) + 2 * TC_LAM_BYTES + 1024;
+constexpr unsigned TB_SA_COL = 128, TB_X_COL = 192, TB_XA_COL = 256;   // BF16 operands: two elements a column
+
+__device__ __forceinline__ void tb_mma_ta(unsigned d_tmem, unsigned a_tmem, unsigned long long db, unsigned idesc,
+                                          unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tb_mma_ss(unsigned d_tmem, unsigned long long da, unsigned long long db, unsigned idesc,
+                                          unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// N values as N / 2 packed tensor-memory columns
+template <int N>
+__device__ __forceinline__ void tb_st_packed(unsigned taddr, const float (&v)[N]) {
+    float w[N / 2];
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        w[j] = __uint_as_float(*reinterpret_cast<const unsigned*>(&h));
+    }
+    if constexpr (N == 16) {
+        const unsigned* u = reinterpret_cast<const unsigned*>(w);
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};" ::"r"(u[0]), "r"(u[1]),
+                     "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(taddr)
+                     : "memory");
+    } else {
+        tc_st<N / 2>(taddr, w);
+    }
+}
+
+template <bool TRANSFER>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+k_state_scan_b(ScanParamsB p, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap rmap,
+               const __grid_constant__ CUtensorMap r2map, const __grid_constant__ CUtensorMap x2map,
+               const __grid_constant__ CUtensorMap pmap, int* fault) {
+    extern __shared__ __align__(16) unsigned char tsm_raw[];
+    unsigned char* tsm = tsm_raw + ((1024u - (tc_smem(tsm_raw) & 1023u)) & 1023u);
+    float* s_lam = reinterpret_cast<float*>(tsm + 2 * TB_SLOT_BYTES);   // [2][DP]
+    __shared__ __align__(8) unsigned long long bars[9];
+    __shared__ unsigned s_tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quarter = warp & 3, part = warp >> 2;
+
+    int block = blockIdx.x;
+    const int slices = TRANSFER ? 4 : DP / SCAN_NS, nseg = TRANSFER ? p.segs - 1 : p.segs;
+    const int slice = block % slices;
+    block /= slices;
+    const int seg = block % nseg, s = block / nseg;
+    const bool identity = TRANSFER && slice >= 2;
+    if (identity && seg == 0) return;
+    const int col0 = (slice & 1) * SCAN_NS;
+    const int first = seg * p.seg_len, steps = p.NC - first < p.seg_len ? p.NC - first : p.seg_len;
+    const long long last = (long long)s * p.NC + p.NC - 1 - first;   // chunk of step n: last - n
+
+    const unsigned full0 = tc_smem(&bars[0]), free0 = tc_smem(&bars[2]), bar_a = tc_smem(&bars[4]), bar_x = tc_smem(&bars[5]);
+    const unsigned bar1 = tc_smem(&bars[6]), bar2 = tc_smem(&bars[7]), bar_s = tc_smem(&bars[8]);
+    if (tid == 0) {
+        for (int i = 0; i < 9; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem(&bars[i])),
+                         "r"(i == 4 || i == 5 || i == 8 ? TC_WORKERS : 1));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&s_tmem)), "r"(TC_TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    chain_wait();   // the set-up above overlaps the end of the kernel before
+    chain_release();
+    const unsigned tbase = s_tmem;
+    bool alive = true;
+    auto wait = [&](unsigned bar, int parity, int code) {
+        if (alive && !tc_wait(bar, parity)) {
+            alive = false;
+            atomicExch(fault, code);
+        }
+    };
+
+    if (warp == 2) {   // ---- loads
+        if (lane == 0) {
+            for (int n = 0; n < steps; ++n) {
+                const int b = n & 1;
+                if (n >= 2) wait(free0 + 8 * b, ((n >> 1) - 1) & 1, 5);
+                unsigned char* slot = tsm + b * TB_SLOT_BYTES;
+                const unsigned bar = full0 + 8 * b;
+                const int chunk = (int)(last - n);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"((identity ? 4u : 8u) * TB_TILE_BYTES + TC_LAM_BYTES)
+                             : "memory");
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    tc_load_box(slot + TB_Q + i * TB_TILE_BYTES, &qmap, 64 * i, chunk, bar);
+                    tc_load_box(slot + TB_R + i * TB_TILE_BYTES, &rmap, 64 * i, chunk, bar);
+                    if (!identity) tc_load_box(slot + TB_R2 + i * TB_TILE_BYTES, &r2map, 64 * i, chunk, bar);
+                }
+                if (!identity) {
+                    tc_load_box(slot + TB_X2, &x2map, col0, chunk, bar);
+                    tc_load_box(slot + TB_P, &pmap, col0, chunk, bar);
+                }
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 tc_smem(s_lam + b * DP)),
+                             "l"(p.lam + (long long)chunk * DP), "r"(TC_LAM_BYTES), "r"(bar)
+                             : "memory");
+            }
+        }
+        __syncwarp();
+    } else if (warp == 3) {   // ---- contractions
+        if (lane == 0) {
+            // FP32 accumulator, BF16 operands, M = 128; K-major unless a major bit (15: A, 16: B) says otherwise
+            const auto idesc = [](int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((128u >> 4) << 24); };
+            const auto desc = [](unsigned addr, unsigned lbo) { return tc_desc(addr, lbo, 1024) | (2ull << 61); };
+            const unsigned id1 = idesc(CL), id2 = idesc(DP) | (1u << 16), id3 = id2 | (1u << 15);
+            for (int n = 0; n < steps; ++n) {
+                const int b = n & 1;
+                const unsigned slot = tc_smem(tsm + b * TB_SLOT_BYTES);
+                wait(full0 + 8 * b, (n >> 1) & 1, 3);
+                wait(bar_a, n & 1, 8);
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < DP / 16; ++k)   // X^T = S^T Q^T
+                    tb_mma_ta(tbase + TB_X_COL, tbase + TB_SA_COL + 8 * k, desc(slot + TB_Q + (k / 4) * TB_TILE_BYTES + (k % 4) * 32, 16), id1, k > 0);
+                tc_commit(bar1);
+                wait(bar_s, n & 1, 10);
+                tc_fence_after();
+                if (!identity) {
+#pragma unroll
+                    for (int k = 0; k < CL / 16; ++k)   // S^T += X2^T R2
+                        tb_mma_ss(tbase + TC_S_COL, desc(slot + TB_X2 + k * 2048, TB_TILE_BYTES), desc(slot + TB_R2 + k * 2048, TB_TILE_BYTES), id3, 1u);
+                }
+                wait(bar_x, n & 1, 9);
+                tc_fence_after();
+#pragma unroll
+                for (int k = 0; k < CL / 16; ++k)   // S^T += X^T R
+                    tb_mma_ta(tbase + TC_S_COL, tbase + TB_XA_COL + 8 * k, desc(slot + TB_R + k * 2048, TB_TILE_BYTES), id2, 1u);
+                tc_commit(bar2);
+                tc_commit(free0 + 8 * b);
+            }
+        }
+        __syncwarp();
+    } else if (quarter < 2) {   // ---- workers: lane = state column c
+        const int cl = quarter * 32 + lane, c = col0 + cl, p0 = part * TC_SCOLS, x0 = part * TC_XCOLS;
+        const unsigned t_lane = tbase + ((unsigned)(quarter * 32) << 16);
+        float st[TC_SCOLS];
+        if (identity) {
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; ++j) st[j] = p0 + j == c ? 1.f : 0.f;
+        } else if (seg > 0) {
 #pragma unroll
             for (int j = 0; j < TC_SCOLS; ++j)
-                if (p0 + j < p.nrows)
-                    dst[p.transposed_io ? (long long)c * p.nrows + p0 + j : (long long)(p0 + j) * p.ncols + c] = st[j];
+                st[j] = TRANSFER ? 0.f : p.seg_state[((long long)(s * (p.segs - 1) + seg - 1) * 2 * DP + p0 + j) * DP + c];
+        } else {
+            tc_init_state(p.init, s, p.nrows, p.ncols, p.transposed_io, p0, c, st);
+        }
+        for (int n = 0; n < steps; ++n) {
+            const int b = n & 1;
+            const long long gi = last - n;
+            if (n > 0) {
+                wait(bar2, (n - 1) & 1, 2);
+                tc_fence_after();
+                tc_ld<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+                tc_wait_ld();
+            }
+            tb_st_packed<TC_SCOLS>(t_lane + TB_SA_COL + p0 / 2, st);
+            tc_wait_st();
+            tc_fence_before();
+            tc_arrive(bar_a);
+            if (!TRANSFER) tc_store_pairs<TC_SCOLS>(p.ck + gi * (long long)(DP * DP) + p0 * DP, c, lane, st);
+            wait(full0 + 8 * b, (n >> 1) & 1, 4);
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; j += 4) {
+                const float4 l = *reinterpret_cast<const float4*>(s_lam + b * DP + p0 + j);
+                st[j] *= l.x;
+                st[j + 1] *= l.y;
+                st[j + 2] *= l.z;
+                st[j + 3] *= l.w;
+            }
+            tc_st<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+            tc_wait_st();
+            tc_fence_before();
+            tc_arrive(bar_s);
+            float x[TC_XCOLS], pv[TC_XCOLS];
+            if (!identity) {   // P as TMA landed it: 16-byte piece (c / 8) of a row sits at piece (c / 8) ^ (row % 8)
+                const unsigned char* ps = tsm + b * TB_SLOT_BYTES + TB_P + x0 * 128;
+#pragma unroll
+                for (int j = 0; j < TC_XCOLS; ++j)
+                    pv[j] = __bfloat162float(*reinterpret_cast<const bf16*>(ps + j * 128 + ((((cl >> 3) ^ (j & 7)) << 4) | ((cl & 7) << 1))));
+            }
+            wait(bar1, n & 1, 1);
+            tc_fence_after();
+            tc_ld<TC_XCOLS>(t_lane + TB_X_COL + x0, x);
+            tc_wait_ld();
+            if (!identity) {
+#pragma unroll
+                for (int j = 0; j < TC_XCOLS; ++j) x[j] += pv[j];
+            }
+            tb_st_packed<TC_XCOLS>(t_lane + TB_XA_COL + x0 / 2, x);
+            tc_wait_st();
+            tc_fence_before();
+            tc_arrive(bar_x);
+            if (!TRANSFER) tc_store_pairs<TC_XCOLS>(bpanel_ptr(p.X, gi) + x0 * DP, c, lane, x);
+        }
+        wait(bar2, (steps - 1) & 1, 2);
+        tc_fence_after();
+        tc_ld<TC_SCOLS>(t_lane + TC_S_COL + p0, st);
+        tc_wait_ld();
+        if (TRANSFER) {
+            float* dst = p.seg_state + ((long long)((s * (p.segs - 1) + seg) * 2 + (identity ? 1 : 0)) * DP + p0) * DP + c;
+#pragma unroll
+            for (int j = 0; j < TC_SCOLS; ++j) dst[j * DP] = st[j];
+        } else if (seg == p.segs - 1) {
+            tc_final_state(p.fin, s, p.nrows, p.ncols, p.transposed_io, p0, c, st);
         }
     }
     tc_fence_before();
@@ -397,39 +704,55 @@ k_state_scan_tc(ScanParams p, const __grid_constant__ CUtensorMap qmap, const __
 }
 
 // Entry states of the segments of a segmented scan: E_g = local_g + transfer_g E_{g-1}, written over local_g, where
-// (local, transfer) are the pairs the transfer pass stored.  FP32 throughout.  One CTA per stream and 16 columns: they
-// never exchange data.
-constexpr int COMBINE_COLS = 16, COMBINE_THREADS = 256;
+// (local, transfer) are the pairs the transfer pass stored.  FP32 throughout.  One CTA per stream and 8 columns (they
+// never exchange data); the next transfer matrix streams into shared memory while the current one is multiplied, since
+// the chain over segments would otherwise wait for memory at every link (5.8 us a segment against 1).
+constexpr int COMBINE_COLS = 8, COMBINE_THREADS = 256, COMBINE_PITCH = DP + 4;
+constexpr size_t COMBINE_SMEM = size_t(2) * DP * COMBINE_PITCH * 4 + DP * COMBINE_COLS * 4;
 __global__ void __launch_bounds__(COMBINE_THREADS) k_scan_combine(float* seg_state, int segs) {
-    __shared__ __align__(16) float s_e[DP][COMBINE_COLS];
+    chain_wait();
+    chain_release();
+    extern __shared__ __align__(16) float csm[];
+    float* s_t = csm;                                   // [2][DP][COMBINE_PITCH]
+    float* s_e = csm + 2 * DP * COMBINE_PITCH;          // [DP][COMBINE_COLS]
     const int col0 = (blockIdx.x % (DP / COMBINE_COLS)) * COMBINE_COLS, s = blockIdx.x / (DP / COMBINE_COLS);
-    const int row = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * 8;
-    for (int g = 0; g < segs - 1; ++g) {
-        float* local = seg_state + (long long)(s * (segs - 1) + g) * 2 * DP * DP;
-        float acc[8];
-        {
-            const float4 a = *reinterpret_cast<const float4*>(local + row * DP + col0 + c0);
-            const float4 b = *reinterpret_cast<const float4*>(local + row * DP + col0 + c0 + 4);
-            acc[0] = a.x; acc[1] = a.y; acc[2] = a.z; acc[3] = a.w;
-            acc[4] = b.x; acc[5] = b.y; acc[6] = b.z; acc[7] = b.w;
+    const int row = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * 4;
+    float* base = seg_state + (long long)s * (segs - 1) * 2 * DP * DP;
+    auto issue = [&](int g) {
+        if (g > 0 && g < segs - 1) {
+            const float* t = base + ((long long)g * 2 + 1) * DP * DP;
+            float* dst = s_t + (g & 1) * DP * COMBINE_PITCH;
+            for (int idx = threadIdx.x; idx < DP * (DP / 4); idx += COMBINE_THREADS)
+                cp16(dst + (idx >> 5) * COMBINE_PITCH + (idx & 31) * 4, t + idx * 4);
         }
+        cp_commit();
+    };
+    issue(1);
+    for (int g = 0; g < segs - 1; ++g) {
+        float* local = base + (long long)g * 2 * DP * DP + row * DP + col0 + c0;
+        float4 acc = *reinterpret_cast<const float4*>(local);
         if (g > 0) {
-            const float* t = local + DP * DP + row * DP;
+            issue(g + 1);
+            cp_wait<1>();
+            __syncthreads();
+            const float* t = s_t + (g & 1) * DP * COMBINE_PITCH + row * COMBINE_PITCH;
 #pragma unroll 8
             for (int k = 0; k < DP; k += 4) {
                 const float4 w = *reinterpret_cast<const float4*>(t + k);
                 const float wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[e] = fmaf(wv[i], s_e[k + i][c0 + e], acc[e]);
+                for (int i = 0; i < 4; ++i) {
+                    const float4 e = *reinterpret_cast<const float4*>(s_e + (k + i) * COMBINE_COLS + c0);
+                    acc.x = fmaf(wv[i], e.x, acc.x);
+                    acc.y = fmaf(wv[i], e.y, acc.y);
+                    acc.z = fmaf(wv[i], e.z, acc.z);
+                    acc.w = fmaf(wv[i], e.w, acc.w);
+                }
             }
-            *reinterpret_cast<float4*>(local + row * DP + col0 + c0) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            *reinterpret_cast<float4*>(local + row * DP + col0 + c0 + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+            *reinterpret_cast<float4*>(local) = acc;
         }
         __syncthreads();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) s_e[row][c0 + e] = acc[e];
+        *reinterpret_cast<float4*>(s_e + row * COMBINE_COLS + c0) = acc;
         __syncthreads();
     }
 }

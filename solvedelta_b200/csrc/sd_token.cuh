@@ -19,12 +19,6 @@
 
 namespace sd {
 
-// Programmatic dependent launch.  A kernel of this library lets its dependents start only after its own wait has
-// returned, so when one of them runs, everything before its predecessor is complete: what it may read ahead of its wait
-// is weights and data that was written two launches ago or earlier.  Both are no-ops in a launch without the attribute.
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // A 16-byte load of data the kernel before may have written: coherent, and kept where it stands.
 __device__ __forceinline__ uint4 load16_live(const __nv_bfloat16* p) {
     uint4 r;
