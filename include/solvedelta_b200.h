@@ -297,6 +297,10 @@ size_t sd_backward_scratch_bytes(const sd_shape *shape);
 /* `stream` is a cudaStream_t passed as void* (NULL = legacy default stream). */
 int sd_forward(const sd_forward_args *args, void *stream);
 int sd_backward(const sd_backward_args *args, void *stream);
+/* sd_forward for a call that no reverse pass follows: the panels only sd_backward reads are not stored, `saved` is a
+ * workspace of sd_inference_bytes. */
+size_t sd_inference_bytes(const sd_shape *shape);
+int sd_forward_inference(const sd_forward_args *args, void *stream);
 int sd_decode_step(const sd_decode_args *args, void *stream);
 /* The same step from other states than the ones it writes: C_in / S_in are only read (NULL: zero state), args->C and
  * args->S receive the updated ones.  What a functional caller otherwise pays two device copies for. */

@@ -275,7 +275,7 @@ class NormGateArgs(ctypes.Structure):
 
 EXPORTS = (
     "sd_saved_bytes", "sd_forward_scratch_bytes", "sd_backward_scratch_bytes",
-    "sd_forward", "sd_backward", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
+    "sd_forward", "sd_forward_inference", "sd_inference_bytes", "sd_backward", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
     "sd_backward_launches", "sd_panel_info", "sd_status_string", "sd_version",
     "sd_chunk_tokens", "sd_forward_static", "sd_panel_kind", "sd_device_fault", "sd_device_fault_clear",
     "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step",
@@ -346,11 +346,13 @@ def host():
 
 def _declare(lib: ctypes.CDLL) -> ctypes.CDLL:
     sp = ctypes.POINTER(Shape)
-    for name in ("sd_saved_bytes", "sd_forward_scratch_bytes", "sd_backward_scratch_bytes"):
+    for name in ("sd_saved_bytes", "sd_inference_bytes", "sd_forward_scratch_bytes", "sd_backward_scratch_bytes"):
         getattr(lib, name).restype = ctypes.c_size_t
         getattr(lib, name).argtypes = [sp]
     lib.sd_forward.restype = ctypes.c_int
     lib.sd_forward.argtypes = [ctypes.POINTER(ForwardArgs), ctypes.c_void_p]
+    lib.sd_forward_inference.restype = ctypes.c_int
+    lib.sd_forward_inference.argtypes = [ctypes.POINTER(ForwardArgs), ctypes.c_void_p]
     lib.sd_forward_static.restype = ctypes.c_int
     lib.sd_forward_static.argtypes = [ctypes.POINTER(ForwardArgs), ctypes.c_void_p]
     lib.sd_backward.restype = ctypes.c_int

@@ -29,6 +29,8 @@ const PanelDesc kSaved[] = {{"Lam", 3}, {"G", 0}, {"Delta", 0}, {"Dprim", 0}, {"
                             {"N", 1}, {"Aed", 1}, {"Aqd", 5},
                             // BF16 source panels of the exterior, written once by the forward pass
                             {"Xg", 4}, {"Ag", 4}, {"Xr", 4}, {"Er", 4}, {"Dcol", 4}, {"DtB", 4}, {"Chi", 4}, {"Ee", 4}};
+// what a call without gradients keeps of it: the panels that later forward kernels read
+const PanelDesc kInfer[] = {{"Lam", 3}, {"G", 0}, {"Delta", 0}, {"Zt", 4}, {"CtCk", 2}, {"SCk", 6}, {"Aqd", 5}, {"Xg", 4}};
 const PanelDesc kFwd[] = {{"Upd", 0}, {"Qc", 0}, {"Ubar", 0}, {"Wd", 0}, {"Ud", 0}, {"Dt", 0}};
 const PanelDesc kBwd[] = {{"Pp", 4},     {"Qp", 4},     {"Dyf", 4},    {"dR", 4},     {"dSeCk", 6},
                           {"SdS", 3},    {"duPart", 4}, {"dkPart", 4}, {"dGPart", 4}, {"dDelta", 4}, {"DG", 4},
@@ -542,6 +544,10 @@ size_t sd_saved_bytes(const sd_shape* shape) {
     if (!shape_ok(shape) || !shape_supported(shape)) return 0;
     return layout_bytes(kSaved, shape);
 }
+size_t sd_inference_bytes(const sd_shape* shape) {
+    if (!shape_ok(shape) || !shape_supported(shape)) return 0;
+    return layout_bytes(kInfer, shape);
+}
 size_t sd_forward_scratch_bytes(const sd_shape* shape) {
     if (!shape_ok(shape) || !shape_supported(shape)) return 0;
     return layout_bytes(kFwd, shape);
@@ -606,20 +612,22 @@ struct PredictorOnly {
     void *action, *update;                        // forward outputs, BF16 [B,T,H,r] contiguous
     const void *d_action, *d_update, *action_in;  // reverse inputs, same layout (the cotangents may be null)
 };
-int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po);
+int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po, bool keep = true);
 int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly* po);
 }  // namespace
 
 int sd_forward(const sd_forward_args* a, void* stream_) { return forward_impl(a, stream_, nullptr); }
+int sd_forward_inference(const sd_forward_args* a, void* stream_) { return forward_impl(a, stream_, nullptr, false); }
 int sd_backward(const sd_backward_args* a, void* stream_) { return backward_impl(a, stream_, nullptr); }
 
 namespace {
-int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po) {
+int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po, bool keep) {
     if (!a || !shape_ok(&a->shape)) return SD_ERR_INVALID_ARGUMENT;
     if (!shape_supported(&a->shape)) return SD_ERR_UNSUPPORTED_SHAPE;
     const sd_operand ops[] = {a->u, a->h, a->q, a->keys, a->values, a->erase_raw, a->write_raw, a->log_decay, a->gamma};
     if (!operands_ok(ops, 9) || !a->y || !a->saved || !a->scratch) return SD_ERR_INVALID_ARGUMENT;
-    if (a->saved_bytes < sd_saved_bytes(&a->shape) || a->scratch_bytes < sd_forward_scratch_bytes(&a->shape))
+    if (a->saved_bytes < (keep ? sd_saved_bytes(&a->shape) : sd_inference_bytes(&a->shape)) ||
+        a->scratch_bytes < sd_forward_scratch_bytes(&a->shape))
         return SD_ERR_BUFFER_TOO_SMALL;
     if ((reinterpret_cast<uintptr_t>(a->saved) & 15) || (reinterpret_cast<uintptr_t>(a->scratch) & 15))
         return SD_ERR_INVALID_ARGUMENT;
@@ -646,24 +654,16 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     p.Wd = panel_at(kFwd, s, a->scratch, "Wd");
     p.Ud = panel_at(kFwd, s, a->scratch, "Ud");
     p.Dt = panel_at(kFwd, s, a->scratch, "Dt");
-    p.Xg = bpanel_at(kSaved, s, a->saved, "Xg");
-    p.Ag = bpanel_at(kSaved, s, a->saved, "Ag");
-    p.Xr = bpanel_at(kSaved, s, a->saved, "Xr");
-    p.Er = bpanel_at(kSaved, s, a->saved, "Er");
-    p.Dcol = bpanel_at(kSaved, s, a->saved, "Dcol");
-    p.DtB = bpanel_at(kSaved, s, a->saved, "DtB");
-    p.Chi = bpanel_at(kSaved, s, a->saved, "Chi");
-    p.Ee = bpanel_at(kSaved, s, a->saved, "Ee");
-    p.Aqd = bpanel_at(kSaved, s, a->saved, "Aqd");
-    p.Npair = panel_at(kSaved, s, a->saved, "N");
-    p.Aed = panel_at(kSaved, s, a->saved, "Aed");
-    p.Lam = panel_at(kSaved, s, a->saved, "Lam");
-    p.Gp = panel_at(kSaved, s, a->saved, "G");
-    p.Delta = panel_at(kSaved, s, a->saved, "Delta");
-    p.Dprim = panel_at(kSaved, s, a->saved, "Dprim");
-    p.Zt = bpanel_at(kSaved, s, a->saved, "Zt");
-    p.CtCk = panel_at(kSaved, s, a->saved, "CtCk");
-    p.SCk = bpanel_at(kSaved, s, a->saved, "SCk");
+    const auto fp32 = [&](const char* name) {   // null where a call without gradients has no such panel
+        return keep ? panel_at(kSaved, s, a->saved, name) : panel_at(kInfer, s, a->saved, name);
+    };
+    const auto half = [&](const char* name) { return reinterpret_cast<bf16*>(fp32(name)); };
+    p.Xg = half("Xg"); p.Aqd = half("Aqd");
+    p.Ag = half("Ag"); p.Xr = half("Xr"); p.Er = half("Er"); p.Dcol = half("Dcol"); p.DtB = half("DtB");
+    p.Chi = half("Chi"); p.Ee = half("Ee");
+    p.Npair = fp32("N"); p.Aed = fp32("Aed"); p.Dprim = fp32("Dprim");
+    p.Lam = fp32("Lam"); p.Gp = fp32("G"); p.Delta = fp32("Delta"); p.CtCk = fp32("CtCk");
+    p.Zt = half("Zt"); p.SCk = half("SCk");
     p.y = a->y;
     p.action = po ? po->action : nullptr;
     p.update = po ? po->update : nullptr;
@@ -688,7 +688,7 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         ScanParams sp{};
         sp.P = p.Upd; sp.Q = p.Qc; sp.R = p.Ubar;
         sp.lam = p.Lam; sp.X = p.Delta; sp.ck = p.CtCk; sp.Xb = nullptr;
-        sp.ckb = bpanel_at(kSaved, s, a->saved, "CtCkB");
+        sp.ckb = half("CtCkB");
         sp.init = a->C0; sp.fin = a->C_T;
         sp.NC = p.g.NC; sp.transposed_io = 1; sp.nrows = s->r; sp.ncols = s->r;
         if (!launch_scan_tc(sp, streams, p.Wd, 3 * panel_bytes, stream, scan_dbg(1))) return SD_ERR_LAUNCH_FAILED;

@@ -186,7 +186,7 @@ constexpr size_t BSTATE_BYTES = size_t(DP) * LDB * 2;  // a whole state in BF16
 // After that every warp owns 16 of the 256 right-hand-side columns for the whole
 // solve and never waits for another warp: per block it subtracts the coupling with the
 // blocks already solved and applies the inverted diagonal block, both on the tensor
-// cores (TF32; split-TF32 "3x" coupling when SPLIT).  The identity part of the
+// cores (TF32).  The identity part of the
 // inverse is added from the FP32 registers, so only the correction (T_II^-1 - I) r
 // sees TF32 operand rounding.
 struct PanelF32 {
@@ -218,7 +218,7 @@ struct PanelBF16 {
     }
 };
 
-template <bool UPPER, bool SPLIT, class Panel>
+template <bool UPPER, class Panel>
 __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) {
     static_assert(NTHREADS == 2 * DP * 2, "16 warps of 16 right-hand-side columns each");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -291,23 +291,13 @@ __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) 
             for (int kk = kbeg; kk < kend; kk += 8) {
                 float af[4] = {Mr[(r0 + g) * LDA + kk + t], Mr[(r0 + g + 8) * LDA + kk + t],
                                Mr[(r0 + g) * LDA + kk + t + 4], Mr[(r0 + g + 8) * LDA + kk + t + 4]};
-                uint32_t ah[4], al[4];
+                uint32_t ah[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    ah[e] = f2tf32(af[e]);
-                    if (SPLIT) al[e] = f2tf32(af[e] - __uint_as_float(ah[e]));
-                }
+                for (int e = 0; e < 4; ++e) ah[e] = mma_tf32_bits(af[e]);
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    float b0 = P.get(kk + t, n0 + nt * 8 + g), b1 = P.get(kk + t + 4, n0 + nt * 8 + g);
-                    uint32_t bh0 = f2tf32(b0), bh1 = f2tf32(b1);
-                    if (SPLIT) {
-                        uint32_t bl0 = f2tf32(b0 - __uint_as_float(bh0)), bl1 = f2tf32(b1 - __uint_as_float(bh1));
-                        mma_tf32(acc[nt], al[0], al[1], al[2], al[3], bh0, bh1);
-                        mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], bl0, bl1);
-                    }
-                    mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], bh0, bh1);
-                }
+                for (int nt = 0; nt < 2; ++nt)
+                    mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], mma_tf32_bits(P.get(kk + t, n0 + nt * 8 + g)),
+                             mma_tf32_bits(P.get(kk + t + 4, n0 + nt * 8 + g)));
             }
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
@@ -325,14 +315,14 @@ __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) 
             acc_zero<2>(acc);
 #pragma unroll
             for (int kk = 0; kk < 16; kk += 8) {
-                const uint32_t a0 = f2tf32(Mr[(r0 + g) * LDA + r0 + kk + t]);
-                const uint32_t a1 = f2tf32(Mr[(r0 + g + 8) * LDA + r0 + kk + t]);
-                const uint32_t a2 = f2tf32(Mr[(r0 + g) * LDA + r0 + kk + t + 4]);
-                const uint32_t a3 = f2tf32(Mr[(r0 + g + 8) * LDA + r0 + kk + t + 4]);
+                const uint32_t a0 = mma_tf32_bits(Mr[(r0 + g) * LDA + r0 + kk + t]);
+                const uint32_t a1 = mma_tf32_bits(Mr[(r0 + g + 8) * LDA + r0 + kk + t]);
+                const uint32_t a2 = mma_tf32_bits(Mr[(r0 + g) * LDA + r0 + kk + t + 4]);
+                const uint32_t a3 = mma_tf32_bits(Mr[(r0 + g + 8) * LDA + r0 + kk + t + 4]);
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
-                    const uint32_t b0 = f2tf32(P.get(r0 + kk + t, n0 + nt * 8 + g));
-                    const uint32_t b1 = f2tf32(P.get(r0 + kk + t + 4, n0 + nt * 8 + g));
+                    const uint32_t b0 = mma_tf32_bits(P.get(r0 + kk + t, n0 + nt * 8 + g));
+                    const uint32_t b1 = mma_tf32_bits(P.get(r0 + kk + t + 4, n0 + nt * 8 + g));
                     mma_tf32(acc[nt], a0, a1, a2, a3, b0, b1);
                 }
             }

@@ -306,6 +306,9 @@ __device__ __forceinline__ uint32_t f2tf32(float x) {
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(x));
     return y;
 }
+// The same rounding for an operand of mma.sync alone, which reads the upper 19 bits: half a unit added, nothing masked
+// (one integer add; the conversion instruction has a quarter of its rate, and operands are rounded at every use).
+__device__ __forceinline__ uint32_t mma_tf32_bits(float x) { return __float_as_uint(x) + 0x1000u; }
 __device__ __forceinline__ float round_tf32(float x) { return __uint_as_float(f2tf32(x)); }
 // a [CL][DP] shared panel to global memory, rounded to TF32 on the way
 __device__ __forceinline__ void s2g_panel_tf32(float* g, const float* sm) {
@@ -340,14 +343,14 @@ __device__ __forceinline__ void warp_mma(float (&acc)[NTW][4], int r0, int n0, i
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll 2
     for (int kk = kbeg; kk < kend; kk += 8) {
-        uint32_t a0 = f2tf32(fa(r0 + g, kk + t));
-        uint32_t a1 = f2tf32(fa(r0 + g + 8, kk + t));
-        uint32_t a2 = f2tf32(fa(r0 + g, kk + t + 4));
-        uint32_t a3 = f2tf32(fa(r0 + g + 8, kk + t + 4));
+        uint32_t a0 = mma_tf32_bits(fa(r0 + g, kk + t));
+        uint32_t a1 = mma_tf32_bits(fa(r0 + g + 8, kk + t));
+        uint32_t a2 = mma_tf32_bits(fa(r0 + g, kk + t + 4));
+        uint32_t a3 = mma_tf32_bits(fa(r0 + g + 8, kk + t + 4));
 #pragma unroll
         for (int nt = 0; nt < NTW; ++nt) {
-            uint32_t b0 = f2tf32(fb(kk + t, n0 + nt * 8 + g));
-            uint32_t b1 = f2tf32(fb(kk + t + 4, n0 + nt * 8 + g));
+            uint32_t b0 = mma_tf32_bits(fb(kk + t, n0 + nt * 8 + g));
+            uint32_t b1 = mma_tf32_bits(fb(kk + t + 4, n0 + nt * 8 + g));
             mma_tf32(acc[nt], a0, a1, a2, a3, b0, b1);
         }
     }

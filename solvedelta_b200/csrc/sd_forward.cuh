@@ -19,8 +19,10 @@ struct FwdParams {
     // that it does not evaluate the sources a second time: -e exp(G), chi rowG, -e rowG, d col, d exp(GL-G),
     // and (only for chunks with a block on the direct path) chi and -e themselves
     bf16 *Ag, *Xr, *Er, *Dcol, *DtB, *Chi, *Ee;
-    // kept for backward
-    float *Lam, *Gp, *Delta, *Dprim, *CtCk;
+    float *Lam, *Gp, *Delta, *CtCk;
+    // only read by the reverse pass (with Ag .. Ee above): null in a call without gradients, which then stores 0.18 of
+    // the 0.95 MB a chunk task moves less
+    float *Dprim;
     float *Npair, *Aed;  // pair matrices N = Lm / gamma and Aed, [CL][CL]
     bf16 *Zt, *SCk;  // only BF16 contractions read these
     void* y;
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
     __syncthreads();
     // Lm = gamma stril(N), N[i][j] = sum_c u^_ic u^_jc exp(E_ic - G_jc); N itself is kept for backward.
     // Diagonal blocks that are not fast: direct evaluation, while u^ and G are still in the slots.
-    float* gN = mat_ptr(p.Npair, ch.gi);
+    float* gN = p.Npair != nullptr ? mat_ptr(p.Npair, ch.gi) : nullptr;
     {
         const int lr = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
 #pragma unroll 1
@@ -191,7 +193,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
                                    [&](int j, float (&G)[8]) { load8_smem(s_A, j, c0, G); }, out);
             const int j = (i & ~(BT - 1)) + (threadIdx.x & 15);
             s_lm[i * LDA + j] = s_gam[i] * out[0];
-            gN[i * CL + j] = out[0];
+            if (gN != nullptr) gN[i * CL + j] = out[0];
         }
     }
     {   // centred operands in place: every thread first reads what it needs of both slots, then all write
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
                            [&](int i, int j, float v0, float v1) {
                                float gm = s_gam[i];
                                *reinterpret_cast<float2*>(s_lm + i * LDA + j) = make_float2(gm * v0, gm * v1);
-                               *reinterpret_cast<float2*>(gN + i * CL + j) = make_float2(v0, v1);
+                               if (gN != nullptr) *reinterpret_cast<float2*>(gN + i * CL + j) = make_float2(v0, v1);
                            });
     {   // Ubar = u^ exp(GL - G) = (column-centred u^) exp(GL - Gend), before slot B is reused
         float* gUbar = panel_ptr(p.Ubar, ch.gi);
@@ -261,7 +263,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
     }
     __syncthreads();
     SD_PHASE(p.g, ph);
-    trisolve_blocked<false, false>(s_lm, 1.f, PanelF32{s_B, s_A});
+    trisolve_blocked<false>(s_lm, 1.f, PanelF32{s_B, s_A});
     SD_PHASE(p.g, ph);
     float* gUpd = panel_ptr(p.Upd, ch.gi);
     float* gQc = panel_ptr(p.Qc, ch.gi);
@@ -399,7 +401,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     }
     SD_PHASE(p.g, ph);
     __syncthreads();   // every warp has read k^ as an operand: d takes its place for the exterior half below
-    float* gd = panel_ptr(p.Dprim, ch.gi);
+    const bool keep = p.Dprim != nullptr;   // kernel-uniform: a reverse pass will follow
+    float* gd = keep ? panel_ptr(p.Dprim, ch.gi) : nullptr;
     const int ref = fast ? r0 + BT - 1 : r0 - 1;   // row whose prefix the accumulated sum is referenced to
     warp_epi<NT128>(acc, r0, n0, [&](int i, int j, float v0, float v1) {
         float2 kh = *reinterpret_cast<const float2*>(s_kh + i * LDP + j);
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
         if (!fast) dg = *reinterpret_cast<const float2*>(s_dl + i * LDP + j);
         const float2 act = make_float2(__expf(G.x - Gp.x) * v0 + dg.x, __expf(G.y - Gp.y) * v1 + dg.y);
         const float2 d = make_float2(kh.x + act.x, kh.y + act.y);
-        *reinterpret_cast<float2*>(gd + i * DP + j) = d;
+        if (keep) *reinterpret_cast<float2*>(gd + i * DP + j) = d;
         *reinterpret_cast<float2*>(s_kh + i * LDP + j) = PRED ? act : d;
     });
     __syncthreads();
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     float* s_z = s_st1;     // z          -> Ud
     float* s_aed = s_aqk;
     bf16* gAqd = bmat_ptr(p.Aqd, ch.gi);
-    float* gAed = mat_ptr(p.Aed, ch.gi);
+    float* gAed = keep ? mat_ptr(p.Aed, ch.gi) : nullptr;
     // with no block left to the direct evaluation nobody needs d itself: each row is centred as it is read
     const bool all_fast = block_is_fast(s_fastw, 0) && block_is_fast(s_fastw, 1) && block_is_fast(s_fastw, 2) &&
                           block_is_fast(s_fastw, 3);
@@ -505,18 +508,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
                 store8_panel(gDt, i, c0, rt);
             }
             store8_bpanel(gXg, i, c0, xg);
-            store8_bpanel(bpanel_ptr(p.Ag, ch.gi), i, c0, ag);
-            store8_bpanel(bpanel_ptr(p.Xr, ch.gi), i, c0, xr);
-            store8_bpanel(bpanel_ptr(p.Er, ch.gi), i, c0, ern);
-            store8_bpanel(bpanel_ptr(p.DtB, ch.gi), i, c0, dt);
+            if (keep) {
+                store8_bpanel(bpanel_ptr(p.Ag, ch.gi), i, c0, ag);
+                store8_bpanel(bpanel_ptr(p.Xr, ch.gi), i, c0, xr);
+                store8_bpanel(bpanel_ptr(p.Er, ch.gi), i, c0, ern);
+                store8_bpanel(bpanel_ptr(p.DtB, ch.gi), i, c0, dt);
+            }
             if (all_fast) {
                 float Ge[8], dc[8];
                 load8_smem(s_G, i0 + BT - 1, c0, Ge);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) dc[e] = d[e] * __expf(Ge[e] - G[e]);
                 store8_smem(s_d, i, c0, dc);
-                store8_bpanel(bpanel_ptr(p.Dcol, ch.gi), i, c0, dc);
-            } else {
+                if (keep) store8_bpanel(bpanel_ptr(p.Dcol, ch.gi), i, c0, dc);
+            } else if (keep) {
                 store8_bpanel(bpanel_ptr(p.Chi, ch.gi), i, c0, a[0]);
                 store8_bpanel(bpanel_ptr(p.Ee, ch.gi), i, c0, a[1]);
             }
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
                                         [&](int j, float (&Gj)[8]) { load8_smem(s_G, j, c0, Gj); }, out);
                 gAqd[i * CL + i0 + l16] = __float2bfloat16_rn(out[0]);
                 s_aed[i * LDA + i0 + l16] = (i0 + l16 < i) ? out[1] : 0.f;
-                gAed[i * CL + i0 + l16] = (i0 + l16 < i) ? out[1] : 0.f;
+                if (keep) gAed[i * CL + i0 + l16] = (i0 + l16 < i) ? out[1] : 0.f;
             }
         }
     }
@@ -543,9 +548,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
             d.x *= __expf(Ge.x - G.x); d.y *= __expf(Ge.y - G.y);
             d.z *= __expf(Ge.z - G.z); d.w *= __expf(Ge.w - G.w);
             *reinterpret_cast<float4*>(s_d + j * LDP + c4) = d;
-            bf16* gDc = bpanel_ptr(p.Dcol, ch.gi) + j * DP + c4;
-            *reinterpret_cast<__nv_bfloat162*>(gDc) = __floats2bfloat162_rn(d.x, d.y);
-            *reinterpret_cast<__nv_bfloat162*>(gDc + 2) = __floats2bfloat162_rn(d.z, d.w);
+            if (keep) {
+                bf16* gDc = bpanel_ptr(p.Dcol, ch.gi) + j * DP + c4;
+                *reinterpret_cast<__nv_bfloat162*>(gDc) = __floats2bfloat162_rn(d.x, d.y);
+                *reinterpret_cast<__nv_bfloat162*>(gDc + 2) = __floats2bfloat162_rn(d.z, d.w);
+            }
         }
         __syncthreads();
     }
@@ -559,12 +566,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
         pair_blocks_tf32<true>(s_M, s_ibeta, s_fastw, [&](int i, int k) { return s_er[i * LDP + k]; }, fc,
                                [&](int i, int j, float v0, float v1) {
                                    *reinterpret_cast<float2*>(s_aed + i * LDA + j) = make_float2(v0, v1);
-                                   *reinterpret_cast<float2*>(gAed + i * CL + j) = make_float2(v0, v1);
+                                   if (keep) *reinterpret_cast<float2*>(gAed + i * CL + j) = make_float2(v0, v1);
                                });
     }
     __syncthreads();
     SD_PHASE(p.g, ph);
-    trisolve_blocked<false, false>(s_aed, -1.f, PanelF32{s_ag, s_z});
+    trisolve_blocked<false>(s_aed, -1.f, PanelF32{s_ag, s_z});
     SD_PHASE(p.g, ph);
     s2g_panel_tf32(panel_ptr(p.Wd, ch.gi), s_ag);   // a contraction operand of the state scan
     s2g_panel(panel_ptr(p.Ud, ch.gi), s_z);

@@ -28,9 +28,9 @@ struct ForwardResult {
     Tensor y, C_T, S_T, saved;
 };
 
-// `states`: whether the final states are wanted.
+// `states`: whether the final states are wanted; `keep`: whether the reverse pass's panels are.
 ForwardResult forward_launch(const Operands& x, const Tensor& C0, const Tensor& S0, const Tensor& valid,
-                             const Tensor& reset, bool states) {
+                             const Tensor& reset, bool states, bool keep) {
     const sd_shape s = x.shape();
     ForwardResult out;
     out.y = bf16_like(x.u, {s.B, s.T, s.H, s.V});
@@ -38,7 +38,7 @@ ForwardResult forward_launch(const Operands& x, const Tensor& C0, const Tensor& 
         out.C_T = f32_like(x.u, {s.B, s.H, s.r, s.r});
         out.S_T = f32_like(x.u, {s.B, s.H, s.r, s.V});
     }
-    out.saved = workspace(x.u, sd_saved_bytes(&s));
+    out.saved = workspace(x.u, keep ? sd_saved_bytes(&s) : sd_inference_bytes(&s));
     const Tensor scratch = workspace(x.u, sd_forward_scratch_bytes(&s));
     sd_forward_args a{};
     x.fill(a);
@@ -47,7 +47,7 @@ ForwardResult forward_launch(const Operands& x, const Tensor& C0, const Tensor& 
     a.saved = out.saved.data_ptr(); a.saved_bytes = (size_t)out.saved.numel();
     a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
     a.valid_mask = bytes(valid); a.reset_mask = bytes(reset);
-    check(sd_forward(&a, stream_of(x.u)));
+    check(keep ? sd_forward(&a, stream_of(x.u)) : sd_forward_inference(&a, stream_of(x.u)));
     return out;
 }
 
@@ -58,9 +58,10 @@ struct OperatorFunction : torch::autograd::Function<OperatorFunction> {
                                  const OptTensor& valid_in, const OptTensor& reset_in) {
         const c10::cuda::CUDAGuard guard(u.device());
         const Tensor C0 = given(C0_in), S0 = given(S0_in), valid = given(valid_in), reset = given(reset_in);
-        const Operands x{u, h, q, k, v, ld, er, wr, gam};
+        // k, v and the gate logits come and go with their edit axis: dropping it out here would record a view node each
+        const Operands x{u, h, q, k.squeeze(-2), v.squeeze(-2), ld, er.squeeze(-2), wr.squeeze(-2), gam};
         const ForwardResult r = forward_launch(x, C0.defined() ? C0.contiguous() : C0,
-                                               S0.defined() ? S0.contiguous() : S0, valid, reset, true);
+                                               S0.defined() ? S0.contiguous() : S0, valid, reset, true, true);
         ctx->set_materialize_grads(false);
         ctx->saved_data["C0"] = C0.defined();
         ctx->saved_data["S0"] = S0.defined();
@@ -70,7 +71,7 @@ struct OperatorFunction : torch::autograd::Function<OperatorFunction> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list sv = ctx->get_saved_variables();
-        const Operands x{sv[0], sv[1], sv[2], sv[3], sv[4], sv[5], sv[6], sv[7], sv[8]};
+        const Operands x{sv[0], sv[1], sv[2], sv[3].squeeze(-2), sv[4].squeeze(-2), sv[5], sv[6].squeeze(-2), sv[7].squeeze(-2), sv[8]};
         const Tensor &saved = sv[9], &valid = sv[10], &reset = sv[11];
         const sd_shape s = x.shape();
         const c10::cuda::CUDAGuard guard(x.u.device());
@@ -83,8 +84,8 @@ struct OperatorFunction : torch::autograd::Function<OperatorFunction> {
         if (dS.defined()) dS = dS.to(at::kFloat).contiguous();
         const int64_t B = s.B, T = s.T, H = s.H, r = s.r, V = s.V;
         Tensor du = bf16_like(x.u, {B, T, H, r}), dh = bf16_like(x.u, {B, T, H, r}), dq = bf16_like(x.u, {B, T, H, r});
-        Tensor dk = bf16_like(x.u, {B, T, H, r}), dv = bf16_like(x.u, {B, T, H, V}), der = bf16_like(x.u, {B, T, H, r});
-        Tensor dwr = bf16_like(x.u, {B, T, H, V}), dld = f32_like(x.u, {B, T, H, r}), dgam = f32_like(x.u, {B, T, H});
+        Tensor dk = bf16_like(x.u, {B, T, H, 1, r}), dv = bf16_like(x.u, {B, T, H, 1, V}), der = bf16_like(x.u, {B, T, H, 1, r});
+        Tensor dwr = bf16_like(x.u, {B, T, H, 1, V}), dld = f32_like(x.u, {B, T, H, r}), dgam = f32_like(x.u, {B, T, H});
         const bool want_C = ctx->saved_data["C0"].toBool(), want_S = ctx->saved_data["S0"].toBool();
         Tensor dC0 = want_C ? f32_like(x.u, {B, H, r, r}) : Tensor(), dS0 = want_S ? f32_like(x.u, {B, H, r, V}) : Tensor();
         const Tensor scratch = workspace(x.u, sd_backward_scratch_bytes(&s));
@@ -153,14 +154,14 @@ py::tuple residual_frame(const Tensor& u, const Tensor& h, const Tensor& q, cons
         if (C0.defined()) return py::make_tuple(y, C0, S0);
         return py::make_tuple(y, at::zeros({B, H, r, r}, ld_in.options()), at::zeros({B, H, r, V}, ld_in.options()));
     }
-    x.u = u; x.h = h; x.q = q;
-    x.k = keys.squeeze(-2); x.v = values.squeeze(-2);
-    x.er = erase.squeeze(-2); x.wr = write.squeeze(-2);
     Tensor y, C_T, S_T;
     if (!at::GradMode::is_enabled()) {
         // inference: no autograd node, and at T = 1 the single-token recurrent step
         // (causallsso/ops/residual_frame/operator.py:198-216)
         const c10::cuda::CUDAGuard guard(u.device());
+        x.u = u; x.h = h; x.q = q;
+        x.k = keys.squeeze(-2); x.v = values.squeeze(-2);
+        x.er = erase.squeeze(-2); x.wr = write.squeeze(-2);
         const Tensor Cin = C0.defined() ? C0.contiguous() : C0, Sin = S0.defined() ? S0.contiguous() : S0;
         if (T == 1 && !masked) {
             // the updated states are new tensors, as upstream returns them, unless the caller's cache owns its state
@@ -173,11 +174,11 @@ py::tuple residual_frame(const Tensor& u, const Tensor& h, const Tensor& q, cons
             a.C = f32(C_T); a.S = f32(S_T); a.y = y.data_ptr();
             check(sd_decode_step_from(&a, f32(Cin), f32(Sin), stream_of(u)));
         } else {
-            const ForwardResult f = forward_launch(x, Cin, Sin, given(mask_bytes(valid_in)), given(mask_bytes(reset_in)), want_state);
+            const ForwardResult f = forward_launch(x, Cin, Sin, given(mask_bytes(valid_in)), given(mask_bytes(reset_in)), want_state, false);
             y = f.y; C_T = f.C_T; S_T = f.S_T;
         }
     } else {
-        const variable_list out = OperatorFunction::apply(x.u, x.h, x.q, x.k, x.v, x.ld, x.er, x.wr, x.gam, C0_in, S0_in,
+        const variable_list out = OperatorFunction::apply(u, h, q, keys, values, x.ld, erase, write, x.gam, C0_in, S0_in,
                                                           mask_bytes(valid_in), mask_bytes(reset_in));
         y = out[0]; C_T = out[1]; S_T = out[2];
     }
