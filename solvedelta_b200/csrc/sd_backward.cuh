@@ -48,6 +48,24 @@ __device__ __forceinline__ void norm_vjp8(const float (&dxh)[8], const float (&x
     for (int e = 0; e < 8; ++e) dx[e] = (dxh[e] - dot * xh[e]) * rstd;
 }
 
+// Two neighbouring channels j (even), j + 1 of a BF16 row; zeros past the width and where the row is not `ok`.
+template <bool FAST>
+__device__ __forceinline__ float2 load2_bf16(const __nv_bfloat16* row, int j, int width, bool ok) {
+    if (FAST) return ok && j < width ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + j)) : make_float2(0.f, 0.f);
+    return make_float2(ok && j < width ? __bfloat162float(row[j]) : 0.f, ok && j + 1 < width ? __bfloat162float(row[j + 1]) : 0.f);
+}
+// ... of a contiguous output row; a row that is not `ok` gets zeros
+template <bool FAST>
+__device__ __forceinline__ void store2_bf16(__nv_bfloat16* row, int j, int width, bool ok, const float (&v)[2]) {
+    const __nv_bfloat162 w = __floats2bfloat162_rn(ok ? v[0] : 0.f, ok ? v[1] : 0.f);
+    if (FAST) {
+        if (j < width) *reinterpret_cast<__nv_bfloat162*>(row + j) = w;
+    } else {
+        if (j < width) row[j] = w.x;
+        if (j + 1 < width) row[j + 1] = w.y;
+    }
+}
+
 // shared BF16 panel -> dense BF16 global panel
 __device__ __forceinline__ void s2g_bpanel(bf16* g, const bf16* sm) {
     for (int idx = threadIdx.x; idx < CL * (DP / 8); idx += NTHREADS) {
@@ -156,16 +174,15 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_exterior_prep_bwd(BwdParams p) 
 // d chi, -d e, the decay part of d d (all final), dDt and dR are read from the
 // shared BF16 panels the contractions of the same CTA just produced.
 template <bool FAST, class CH>
-__device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& ch, const bf16* sA1,
+__device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& ch, const float* sG, const bf16* sA1,
                                                  const bf16* sA2, const bf16* sPY, const bf16* sdDt,
                                                  const bf16* sdR) {
     const int r = p.g.r, V = p.g.V;
     const int lr = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
     const float* gDelta = panel_ptr(p.Delta, ch.gi);
     const float* gd = panel_ptr(p.Dprim, ch.gi);
-    const float* gG = panel_ptr(p.Gp, ch.gi);
     float GL[8];
-    load8_panel(gG, CL - 1, c0, GL);
+    load8_smem(sG, CL - 1, c0, GL);
 #pragma unroll 1
     for (int pp = 0; pp < ROW_PASSES; ++pp) {
         const int i = lr + ROWS_PER_PASS * pp;
@@ -173,7 +190,7 @@ __device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& c
         float dd[8], xext[8];
         {
             float G[8], d[8], py[8], ddt[8], dg_[8];
-            load8_panel(gG, i, c0, G);
+            load8_smem(sG, i, c0, G);
             load8_panel(gd, i, c0, d);
             load8_bsm(sPY, i, c0, py);
             load8_bsm(sdDt, i, c0, ddt);
@@ -273,7 +290,8 @@ __device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& c
 // The four results stay in shared memory (over operands that are no longer
 // needed) and the per-token reverse of the sources runs on them in the same CTA.
 constexpr size_t EXT_PAIR_BWD_SMEM =
-    6 * BSLOT_BYTES + 2 * BSTATE_BYTES + 2 * BMAT_BYTES + (NBLK * DP + 16) * sizeof(float);
+    6 * BSLOT_BYTES + 2 * BSTATE_BYTES + 2 * BMAT_BYTES + (NBLK * DP + 16 + CL * LDP) * sizeof(float);
+static_assert(EXT_PAIR_BWD_SMEM <= 227 * 1024, "fits the shared memory of one CTA");
 
 // acc rows (i = r0+g, r0+g+8) x columns scaled by exp(x_i - ref) with x, ref rows of the prefix panel
 template <int NTW, class FX>
@@ -303,6 +321,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     bf16* b_daed = b_daqd + BMAT_ELEMS;
     float* s_beta = reinterpret_cast<float*>(b_daed + BMAT_ELEMS);
     int* s_fastw = reinterpret_cast<int*>(s_beta + NBLK * DP);
+    float* s_G = reinterpret_cast<float*>(s_fastw + 16);   // [CL][LDP] prefix: every epilogue and the row pass use it
     const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const float* gG = panel_ptr(p.Gp, ch.gi);
     auto fG = [&](int i, int c) { return gG[i * DP + c]; };
@@ -311,6 +330,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     async_bpanel(b_dr, bpanel_ptr(p.dR, ch.gi));
     async_bpanel(b_zt, bpanel_ptr(p.Zt, ch.gi));
     cp_commit();
+    async_panel_f32(s_G, gG);
     async_bpanel(b_dc, bpanel_ptr(p.Dcol, ch.gi));
     async_bstate(b_S, bstate_ptr(p.SCk, ch.gi));
     cp_commit();
@@ -362,17 +382,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     // exp(G_i - G_ref) for the accumulator element pair (i, j), (i, j + 1); ref < 0: the chunk start
     auto row_factor = [&](int i, int j) {
         const int ref = fast ? r0 + BT - 1 : r0 - 1;
-        const float2 G = *reinterpret_cast<const float2*>(gG + i * DP + j);
+        const float2 G = *reinterpret_cast<const float2*>(s_G + i * LDP + j);
         float2 Gp = make_float2(0.f, 0.f);
-        if (ref >= 0) Gp = *reinterpret_cast<const float2*>(gG + ref * DP + j);
+        if (ref >= 0) Gp = *reinterpret_cast<const float2*>(s_G + ref * LDP + j);
         return make_float2(__expf(G.x - Gp.x), __expf(G.y - Gp.y));
     };
     // exp(G_ref - G_j) for rows of block J = I of the anti-causal result
     auto col_factor = [&](int i, int j) {
         const int ref = fast ? r0 - 1 : r0 + BT - 1;
-        const float2 G = *reinterpret_cast<const float2*>(gG + i * DP + j);
+        const float2 G = *reinterpret_cast<const float2*>(s_G + i * LDP + j);
         float2 Ge = make_float2(0.f, 0.f);
-        if (ref >= 0) Ge = *reinterpret_cast<const float2*>(gG + ref * DP + j);
+        if (ref >= 0) Ge = *reinterpret_cast<const float2*>(s_G + ref * LDP + j);
         return make_float2(__expf(Ge.x - G.x), __expf(Ge.y - G.y));
     };
     {
@@ -454,7 +474,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     }
     __syncthreads();
     SD_PHASE(p.g, ph);
-    sources_bwd_rows<FAST>(p, ch, b_dy, b_dc, b_xr, b_er, b_dr);
+    sources_bwd_rows<FAST>(p, ch, s_G, b_dy, b_dc, b_xr, b_er, b_dr);
     SD_PHASE(p.g, ph);
 }
 
@@ -690,11 +710,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
             float2 pb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gkp + ib * DP + j));
             acc[nt][0] += pa.x; acc[nt][1] += pa.y;
             acc[nt][2] += pb.x; acc[nt][3] += pb.y;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                kha[nt][e] = (ch.ok(ia) && j + e < r) ? __bfloat162float(ka[j + e]) * rka : 0.f;
-                khb[nt][e] = (ch.ok(ib) && j + e < r) ? __bfloat162float(kb[j + e]) * rkb : 0.f;
-            }
+            const float2 fa = load2_bf16<FAST>(ka, j, r, ch.ok(ia)), fb = load2_bf16<FAST>(kb, j, r, ch.ok(ib));
+            kha[nt][0] = fa.x * rka; kha[nt][1] = fa.y * rka;
+            khb[nt][0] = fb.x * rkb; khb[nt][1] = fb.y * rkb;
             dota = fmaf(acc[nt][0], kha[nt][0], fmaf(acc[nt][1], kha[nt][1], dota));
             dotb = fmaf(acc[nt][2], khb[nt][0], fmaf(acc[nt][3], khb[nt][1], dotb));
         }
@@ -717,16 +735,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
 #pragma unroll
         for (int nt = 0; nt < NT128; ++nt) {
             const int j = n0 + nt * 8 + 2 * t;
+            float va[2], vb[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                if (j + e < r) {
-                    // rows that came in as unit vectors get the gradient of the row itself (no projection)
-                    const float va = PRED ? acc[nt][e] : (acc[nt][e] - dota * kha[nt][e]) * rka;
-                    const float vb = PRED ? acc[nt][2 + e] : (acc[nt][2 + e] - dotb * khb[nt][e]) * rkb;
-                    if (ia < ch.nvalid) rowa[j + e] = __float2bfloat16_rn(ch.ok(ia) ? va : 0.f);
-                    if (ib < ch.nvalid) rowb[j + e] = __float2bfloat16_rn(ch.ok(ib) ? vb : 0.f);
-                }
+                // rows that came in as unit vectors get the gradient of the row itself (no projection)
+                va[e] = PRED ? acc[nt][e] : (acc[nt][e] - dota * kha[nt][e]) * rka;
+                vb[e] = PRED ? acc[nt][2 + e] : (acc[nt][2 + e] - dotb * khb[nt][e]) * rkb;
             }
+            if (ia < ch.nvalid) store2_bf16<FAST>(rowa, j, r, ch.ok(ia), va);
+            if (ib < ch.nvalid) store2_bf16<FAST>(rowb, j, r, ch.ok(ib), vb);
         }
     }
     // every contraction that reads b_dl (Delta) is done: reuse it for dDelta_loc
@@ -905,13 +922,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
             __nv_bfloat162 da = *reinterpret_cast<const __nv_bfloat162*>(b_dr + ia * LDB + j);
             __nv_bfloat162 db = *reinterpret_cast<const __nv_bfloat162*>(b_dr + ib * LDB + j);
             float2 fa = __bfloat1622float2(da), fb = __bfloat1622float2(db);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                float h_a = (ch.ok(ia) && j + e < r) ? __bfloat162float(ha[j + e]) : 0.f;
-                float h_b = (ch.ok(ib) && j + e < r) ? __bfloat162float(hb[j + e]) : 0.f;
-                suma = fmaf(e ? fa.y : fa.x, h_a - acc[nt][e], suma);
-                sumb = fmaf(e ? fb.y : fb.x, h_b - acc[nt][2 + e], sumb);
-            }
+            const float2 h_a = load2_bf16<FAST>(ha, j, r, ch.ok(ia)), h_b = load2_bf16<FAST>(hb, j, r, ch.ok(ib));
+            suma = fmaf(fa.y, h_a.y - acc[nt][1], fmaf(fa.x, h_a.x - acc[nt][0], suma));
+            sumb = fmaf(fb.y, h_b.y - acc[nt][3], fmaf(fb.x, h_b.x - acc[nt][2], sumb));
         }
         suma += __shfl_xor_sync(0xffffffffu, suma, 1);
         suma += __shfl_xor_sync(0xffffffffu, suma, 2);

@@ -289,15 +289,14 @@ __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) 
             acc_zero<2>(acc);
 #pragma unroll
             for (int kk = kbeg; kk < kend; kk += 8) {
-                float af[4] = {Mr[(r0 + g) * LDA + kk + t], Mr[(r0 + g + 8) * LDA + kk + t],
-                               Mr[(r0 + g) * LDA + kk + t + 4], Mr[(r0 + g + 8) * LDA + kk + t + 4]};
-                uint32_t ah[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) ah[e] = mma_tf32_bits(af[e]);
+                // permuted contraction index, as in warp_mma_pairs
+                const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
+                const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
+                const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
-                    mma_tf32(acc[nt], ah[0], ah[1], ah[2], ah[3], mma_tf32_bits(P.get(kk + t, n0 + nt * 8 + g)),
-                             mma_tf32_bits(P.get(kk + t + 4, n0 + nt * 8 + g)));
+                    mma_tf32(acc[nt], a0, a1, a2, a3, mma_tf32_bits(P.get(kk + 2 * t, n0 + nt * 8 + g)),
+                             mma_tf32_bits(P.get(kk + 2 * t + 1, n0 + nt * 8 + g)));
             }
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
@@ -315,14 +314,13 @@ __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) 
             acc_zero<2>(acc);
 #pragma unroll
             for (int kk = 0; kk < 16; kk += 8) {
-                const uint32_t a0 = mma_tf32_bits(Mr[(r0 + g) * LDA + r0 + kk + t]);
-                const uint32_t a1 = mma_tf32_bits(Mr[(r0 + g + 8) * LDA + r0 + kk + t]);
-                const uint32_t a2 = mma_tf32_bits(Mr[(r0 + g) * LDA + r0 + kk + t + 4]);
-                const uint32_t a3 = mma_tf32_bits(Mr[(r0 + g + 8) * LDA + r0 + kk + t + 4]);
+                const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + r0 + kk + 2 * t);
+                const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + r0 + kk + 2 * t);
+                const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
-                    const uint32_t b0 = mma_tf32_bits(P.get(r0 + kk + t, n0 + nt * 8 + g));
-                    const uint32_t b1 = mma_tf32_bits(P.get(r0 + kk + t + 4, n0 + nt * 8 + g));
+                    const uint32_t b0 = mma_tf32_bits(P.get(r0 + kk + 2 * t, n0 + nt * 8 + g));
+                    const uint32_t b1 = mma_tf32_bits(P.get(r0 + kk + 2 * t + 1, n0 + nt * 8 + g));
                     mma_tf32(acc[nt], a0, a1, a2, a3, b0, b1);
                 }
             }

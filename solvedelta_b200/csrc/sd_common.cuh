@@ -15,7 +15,9 @@ namespace sd {
 constexpr int CL = 64;        // tokens per chunk
 constexpr int DP = 128;       // padded channel width
 constexpr int LDP = DP + 4;   // shared-memory row pitch of a panel
-constexpr int LDA = CL + 4;   // row pitch of a CL x CL matrix
+// Row pitch of a CL x CL FP32 matrix: 8 off a multiple of 32, so that a half-warp's 8-byte operand reads (rows g, columns
+// 2 t and 2 t + 1 of a contraction step) fall into distinct banks
+constexpr int LDA = CL + 8;
 constexpr int LDH = CL + 4;   // row pitch of a [DP][CL] half state (transposed read)
 constexpr int NTHREADS = 512;            // threads of a chunk CTA (16 warps)
 constexpr int ROWS_PER_PASS = NTHREADS / 16;  // token rows covered by one row-wise pass
@@ -151,6 +153,23 @@ __device__ __forceinline__ float row_sum16(float v) {
     v += __shfl_xor_sync(0xffffffffu, v, 2);
     v += __shfl_xor_sync(0xffffffffu, v, 1);
     return v;
+}
+
+// Eight consecutive channels of a shared FP32 row (16-byte aligned), lane l of 16 holding channels 8 l ..: lanes 4..7 and
+// 12..15 move their halves in the other order, so that the eight lanes of a phase touch 32 different banks (32-byte
+// steps alone would give every access two).
+__device__ __forceinline__ void load8_row(const float* row, float (&x)[8]) {
+    const int sw = (threadIdx.x >> 2) & 1;
+    const float4 a = *reinterpret_cast<const float4*>(row + 4 * sw), b = *reinterpret_cast<const float4*>(row + 4 - 4 * sw);
+    x[0] = sw ? b.x : a.x; x[1] = sw ? b.y : a.y; x[2] = sw ? b.z : a.z; x[3] = sw ? b.w : a.w;
+    x[4] = sw ? a.x : b.x; x[5] = sw ? a.y : b.y; x[6] = sw ? a.z : b.z; x[7] = sw ? a.w : b.w;
+}
+__device__ __forceinline__ void store8_row(float* row, const float (&x)[8]) {
+    const int sw = (threadIdx.x >> 2) & 1;
+    *reinterpret_cast<float4*>(row + 4 * sw) =
+        make_float4(sw ? x[4] : x[0], sw ? x[5] : x[1], sw ? x[6] : x[2], sw ? x[7] : x[3]);
+    *reinterpret_cast<float4*>(row + 4 - 4 * sw) =
+        make_float4(sw ? x[0] : x[4], sw ? x[1] : x[5], sw ? x[2] : x[6], sw ? x[3] : x[7]);
 }
 
 // ---- strided BF16 / FP32 row access --------------------------------------
@@ -356,6 +375,23 @@ __device__ __forceinline__ void warp_mma(float (&acc)[NTW][4], int r0, int n0, i
     }
 }
 
+// The same for an A with 8-byte operand reads, fa2(i, k) = A(i, k) and A(i, k + 1), k even, and a B that is read down its
+// rows: the contraction index is permuted (operand slots t and t + 4 are k = 2 t and 2 t + 1), which also takes a
+// step's rows of B two at a time and so, at a row pitch of 4 mod 32, to distinct banks.
+template <int NTW, class FA, class FB>
+__device__ __forceinline__ void warp_mma_pairs(float (&acc)[NTW][4], int r0, int n0, int kbeg, int kend, FA fa2, FB fb) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 2
+    for (int kk = kbeg; kk < kend; kk += 8) {
+        const float2 lo = fa2(r0 + g, kk + 2 * t), hi = fa2(r0 + g + 8, kk + 2 * t);
+        const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
+#pragma unroll
+        for (int nt = 0; nt < NTW; ++nt)
+            mma_tf32(acc[nt], a0, a1, a2, a3, mma_tf32_bits(fb(kk + 2 * t, n0 + nt * 8 + g)),
+                     mma_tf32_bits(fb(kk + 2 * t + 1, n0 + nt * 8 + g)));
+    }
+}
+
 // fe(i, j, v0, v1): element (i, j) = v0 and (i, j + 1) = v1, j even.
 template <int NTW, class FE>
 __device__ __forceinline__ void warp_epi(float (&acc)[NTW][4], int r0, int n0, FE fe) {
@@ -410,7 +446,8 @@ __device__ __forceinline__ void load_norm_panel(const Operand& op, const CH& ch,
         ss = row_sum16(ss);
         float rs = UNIT ? 1.f : rsqrtf(ss + 1e-24f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sm[i * LDP + c0 + e] = x[e] * rs;
+        for (int e = 0; e < 8; ++e) x[e] *= rs;
+        store8_row(sm + i * LDP + c0, x);
         if (rstd != nullptr && (threadIdx.x & 15) == 0) rstd[i] = rs;
     }
 }
@@ -423,8 +460,7 @@ __device__ __forceinline__ void load_raw_panel(const Operand& op, const CH& ch, 
         int i = lr + ROWS_PER_PASS * p;
         float x[8];
         load8_bf16<FAST>(row_bf16(op, ch, i), c0, width, op.vec, ch.ok(i), x);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sm[i * LDP + c0 + e] = x[e];
+        store8_row(sm + i * LDP + c0, x);
     }
 }
 
@@ -436,8 +472,7 @@ __device__ __forceinline__ void load_f32_panel(const Operand& op, const CH& ch, 
         int i = lr + ROWS_PER_PASS * p;
         float x[8];
         load8_f32<FAST>(row_f32(op, ch, i), c0, width, op.vec, ch.ok(i), x);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sm[i * LDP + c0 + e] = x[e];
+        store8_row(sm + i * LDP + c0, x);
     }
 }
 

@@ -94,14 +94,10 @@ __device__ __forceinline__ void store8_panel(float* panel, int i, int c0, const 
     *reinterpret_cast<float4*>(panel + i * DP + c0 + 4) = make_float4(x[4], x[5], x[6], x[7]);
 }
 __device__ __forceinline__ void load8_smem(const float* sm, int i, int c0, float (&x)[8]) {
-    float4 a = *reinterpret_cast<const float4*>(sm + i * LDP + c0);
-    float4 b = *reinterpret_cast<const float4*>(sm + i * LDP + c0 + 4);
-    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+    load8_row(sm + i * LDP + c0, x);
 }
 __device__ __forceinline__ void store8_smem(float* sm, int i, int c0, const float (&x)[8]) {
-    *reinterpret_cast<float4*>(sm + i * LDP + c0) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(sm + i * LDP + c0 + 4) = make_float4(x[4], x[5], x[6], x[7]);
+    store8_row(sm + i * LDP + c0, x);
 }
 
 // ---------------------------------------------------------------------------
@@ -289,7 +285,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
 //   Aqd[i][j] = sum_c chi_ic d_jc exp(G_ic - G_jc) (j <= i),  Aed likewise with -e (j < i)
 // in block-centred form, and the solved panels Wd = (I-Aed)^-1 ag, Ud = (I-Aed)^-1 Z
 // for the S scan (ag = -e exp(G), referenced to the chunk start like the scan itself).
-constexpr size_t PRIMAL_EXT_FWD_SMEM = 6 * SLOT_BYTES + MAT_BYTES + (NBLK * DP + 3 * DP + NBLK * DP + 16) * sizeof(float);
+constexpr int PANEL_FLOATS = CL * LDP;   // a panel; the half states need a whole slot
+constexpr size_t PRIMAL_EXT_FWD_SMEM = 4 * PANEL_FLOATS * sizeof(float) + 2 * SLOT_BYTES + MAT_BYTES + (NBLK * DP + 3 * DP + NBLK * DP + 16) * sizeof(float);
 static_assert(PRIMAL_EXT_FWD_SMEM <= 227 * 1024, "fits the shared memory of one CTA");
 
 
@@ -314,10 +311,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     SD_PHASE(p.g, ph);
     extern __shared__ __align__(16) float smem[];
     float* s_kh = smem;
-    float* s_un = s_kh + SLOT_FLOATS;
-    float* s_G = s_un + SLOT_FLOATS;
-    float* s_dl = s_G + SLOT_FLOATS;
-    float* s_st0 = s_dl + SLOT_FLOATS;
+    float* s_un = s_kh + PANEL_FLOATS;
+    float* s_G = s_un + PANEL_FLOATS;
+    float* s_dl = s_G + PANEL_FLOATS;
+    float* s_st0 = s_dl + PANEL_FLOATS;
     float* s_st1 = s_st0 + SLOT_FLOATS;
     float* s_aqk = s_st1 + SLOT_FLOATS;   // Aqk, later Aed
     float* s_beta = s_aqk + MAT_FLOATS;
@@ -396,8 +393,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     const bool fast = block_is_fast(s_fastw, r0 / BT);
     for (int J = 0; J * BT < r0 + (fast ? BT : 0); ++J) {
         scale_acc<NT128>(acc, s_beta + J * DP, n0);
-        warp_mma<NT128>(acc, r0, n0, J * BT, J * BT + BT, [&](int i, int k) { return s_aqk[i * LDA + k]; },
-                    [&](int k, int n) { return s_un[k * LDP + n]; });
+        warp_mma_pairs<NT128>(acc, r0, n0, J * BT, J * BT + BT,
+                              [&](int i, int k) { return *reinterpret_cast<const float2*>(s_aqk + i * LDA + k); },
+                              [&](int k, int n) { return s_un[k * LDP + n]; });
     }
     SD_PHASE(p.g, ph);
     __syncthreads();   // every warp has read k^ as an operand: d takes its place for the exterior half below
