@@ -401,6 +401,10 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<true>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<false, 1, 8, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<false, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<true, 1, 8, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<true, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 2, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 1, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
@@ -509,11 +513,12 @@ int token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) 
     return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }
 
-template <bool MIXER, int NS, int WARPS>
+template <bool MIXER, int NS, int WARPS, bool FULL>
 cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(streams * NS));
     cfg.blockDim = dim3(WARPS * 32);
+    cfg.dynamicSmemBytes = NS == 1 ? DECODE_STATE_BYTES : 0;
     cfg.stream = stream;
     cudaLaunchAttribute at[2];
     int n = 0;
@@ -526,12 +531,22 @@ cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int st
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS>, p, m);
+    return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS, FULL>, p, m);
 }
 template <bool MIXER>
 int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
-    const cudaError_t e = decode_split(streams) == 4 ? launch_decode_ns<MIXER, 4, 8>(p, m, streams, chained, stream)
-                                                     : launch_decode_ns<MIXER, 1, 16>(p, m, streams, chained, stream);
+    if (configure_kernels() != cudaSuccess) return SD_ERR_NO_DEVICE;
+    const uintptr_t states = reinterpret_cast<uintptr_t>(p.Cin) | reinterpret_cast<uintptr_t>(p.C) |
+                             reinterpret_cast<uintptr_t>(p.Sin) | reinterpret_cast<uintptr_t>(p.S);
+    // a full head with every row aligned: constant strides and no bounds (the operands q, k, v, ld of the mixer's step
+    // are not read)
+    const bool full = p.g.r == DP && p.g.V == DP && p.Cin != nullptr && p.Sin != nullptr && (states & 15) == 0 &&
+                      p.u.vec && p.er.vec && p.wr.vec && (MIXER || (p.q.vec && p.k.vec && p.v.vec && p.ld.vec));
+    const bool split = decode_split(streams) == 4;
+    const cudaError_t e = full ? (split ? launch_decode_ns<MIXER, 4, 8, true>(p, m, streams, chained, stream)
+                                        : launch_decode_ns<MIXER, 1, 8, true>(p, m, streams, chained, stream))
+                               : (split ? launch_decode_ns<MIXER, 4, 8, false>(p, m, streams, chained, stream)
+                                        : launch_decode_ns<MIXER, 1, 8, false>(p, m, streams, chained, stream));
     mark(stream);
     return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }

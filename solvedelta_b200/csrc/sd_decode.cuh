@@ -6,6 +6,7 @@
 // loads are in flight and how few times the threads of a stream wait for one another.  A stream is a cluster of NS
 // CTAs of 256 threads, each of which owns DP / NS rows of C and of S and holds them in REGISTERS for the whole step
 // (thread = 4 columns of RW rows): no shared-memory copy of a state, every load issued before anything is waited for.
+// With many streams NS is 1, and S waits in shared memory, each thread's elements in slots of its own (decode_split).
 // The recurrence is arranged so that ONE exchange between the CTAs is enough.  With b = sigmoid(erase) k^,
 //   delta_a = gamma (h_a - C_a . u^)                  needs row a of C only,
 //   Cnew^T k^ = alpha (C^T k^) + u^ (delta . k^)      so its column sums run over the OLD C,
@@ -177,12 +178,16 @@ __device__ __forceinline__ float2 dec_ld_remote2(unsigned a) {
     return v;
 }
 
-template <bool MIXER, int NS, int WARPS>
+// FULL: r = V = 128, every row aligned for the wide accesses, both states given.  Bounds and strides are then constants:
+// the row loops are loads at immediate offsets, without a predicate or an address each, which is a third of the step
+// (one CTA per stream: 55 -> 41 us at 768 streams; clusters of four: 6.6 -> 4.4 us at 8 streams).
+template <bool MIXER, int NS, int WARPS, bool FULL>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(DecodeParams p, MixerDecode mix) {
     constexpr int THREADS = WARPS * 32;
     constexpr int ROWS = DP / NS;            // state rows of this CTA
     constexpr int RW = ROWS / WARPS;         // ... of a warp
     constexpr int LPR = 32 / RW;             // lanes that hold a row's scalars after warp_sum_rows
+    constexpr bool SSH = NS == 1;            // S in shared memory (each thread its own slots), not in registers
     constexpr int CONV_PER = (3 * DP + THREADS - 1) / THREADS;
     static_assert(RW >= 1 && THREADS >= 2 * DP, "at least one row per warp, one thread per two columns");
     __shared__ __align__(16) float s_part[WARPS][4][DP];       // per-warp column sums: C^T k^, S^T(alpha b | delta | q^)
@@ -197,7 +202,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
     int rank = 0;
     if (NS > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int s = blockIdx.x / NS, b = s / p.g.H, hh = s - b * p.g.H;
-    const int r = p.g.r, V = p.g.V, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r = FULL ? DP : p.g.r, V = FULL ? DP : p.g.V, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int c0 = lane * 4, row0 = rank * ROWS + warp * RW;
     const int my_row = row0 + lane / LPR;    // the row whose scalars this lane works out
     Chunk ch;
@@ -205,27 +210,46 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
     ch.vm = 0ull; ch.rm = 0ull;
 
     // this warp's rows of both states, requested before anything else
-    const bool vecC = (r & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.Cin) | reinterpret_cast<uintptr_t>(p.C)) & 15) == 0;
-    const bool vecS = (V & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.Sin) | reinterpret_cast<uintptr_t>(p.S)) & 15) == 0;
-    float4 Cv[RW], Sv[RW];
+    const bool vecC = FULL || ((r & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.Cin) | reinterpret_cast<uintptr_t>(p.C)) & 15) == 0);
+    const bool vecS = FULL || ((V & 3) == 0 && ((reinterpret_cast<uintptr_t>(p.Sin) | reinterpret_cast<uintptr_t>(p.S)) & 15) == 0);
+    float4 Cv[RW], Sv[SSH ? 1 : RW];
 #pragma unroll
     for (int j = 0; j < RW; ++j) {
         const int a = row0 + j;
         Cv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a < r && p.Cin != nullptr) Cv[j] = dec_load4(p.Cin + ((long long)s * r + a) * r, c0, r, vecC);
+        if (FULL || (a < r && p.Cin != nullptr)) Cv[j] = dec_load4(p.Cin + ((long long)s * r + a) * r, c0, r, vecC);
     }
+    extern __shared__ __align__(16) float4 s_state[];   // SSH: [RW][THREADS]
+    if constexpr (SSH) {   // a thread reads only what it copied: no barrier
 #pragma unroll
-    for (int j = 0; j < RW; ++j) {
-        const int a = row0 + j;
-        Sv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a < r && p.Sin != nullptr) Sv[j] = dec_load4(p.Sin + ((long long)s * r + a) * V, c0, V, vecS);
+        for (int j = 0; j < RW; ++j) {
+            const int a = row0 + j;
+            const bool live = FULL || (a < r && c0 < V && p.Sin != nullptr);
+            const float* row = p.Sin + ((long long)s * r + a) * V;
+            if (vecS)
+                cp16_zfill(s_state + j * THREADS + tid, live ? row + c0 : p.S, live);
+            else
+                s_state[j * THREADS + tid] = live ? dec_load4(row, c0, V, false) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        cp_commit();
+    } else {
+#pragma unroll
+        for (int j = 0; j < RW; ++j) {
+            const int a = row0 + j;
+            Sv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (FULL || (a < r && p.Sin != nullptr)) Sv[j] = dec_load4(p.Sin + ((long long)s * r + a) * V, c0, V, vecS);
+        }
     }
+    auto state_s = [&](int j) {
+        if constexpr (SSH) return s_state[j * THREADS + tid];
+        else return Sv[j];
+    };
 
     // the token's rows, four channels a lane
     const bool v4r = (r & 3) == 0, v4v = (V & 3) == 0;
     float u[4], k[4], q[4], bq[4], al[4] = {1.f, 1.f, 1.f, 1.f}, vv[4], wg[4], gamma, own_alpha = 1.f;
     const int D = 2 * p.g.H * r + p.g.H * V;
-    const int live_v = V - c0 < 4 ? (V - c0 < 0 ? 0 : V - c0) : 4;
+    const int live_v = FULL ? 4 : V - c0 < 4 ? (V - c0 < 0 ? 0 : V - c0) : 4;
     const bool fused_proj = MIXER && mix.decay_w != nullptr;
     // conv channels, one a thread: every CTA needs all of q and k for the norms
     DecConv conv[CONV_PER];
@@ -234,7 +258,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
         if (part > 2 || c >= (part == 2 ? V : r)) return -1;
         return part == 2 ? 2 * p.g.H * r + hh * V + c : part * p.g.H * r + hh * r + c;
     };
-    uint2 wd[MIXER ? RW : 1], wgt[MIXER ? RW : 1];
+    uint2 wd[MIXER ? RW : 1], wgt[MIXER ? RW : 1];   // SSH: wgt after the first product, for want of registers
     if constexpr (MIXER) {
         // what the projection before this launch does not write is requested ahead of the wait for it: conv windows and
         // taps, and this CTA's rows of the two small projections (one row per warp and load)
@@ -248,13 +272,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
         for (int j = 0; j < RW; ++j) {
             const int a = row0 + j;
             wd[j] = wgt[j] = make_uint2(0u, 0u);
-            if (lg && a < r) wd[j] = *reinterpret_cast<const uint2*>(mix.decay_w + (long long)(hh * r + a) * mix.G + c0);
-            if (lg && a < V) wgt[j] = *reinterpret_cast<const uint2*>(mix.gate_w + (long long)(hh * V + a) * mix.G + c0);
+            if (lg && (FULL || a < r)) wd[j] = *reinterpret_cast<const uint2*>(mix.decay_w + (long long)(hh * r + a) * mix.G + c0);
+            if (!SSH && lg && (FULL || a < V)) wgt[j] = *reinterpret_cast<const uint2*>(mix.gate_w + (long long)(hh * V + a) * mix.G + c0);
         }
         chain_wait();
         chain_release();
     }
-    const float ha = my_row < r ? __bfloat162float(row_bf16(p.h, ch, 0)[my_row]) : 0.f;
+    const float ha = FULL || my_row < r ? __bfloat162float(row_bf16(p.h, ch, 0)[my_row]) : 0.f;
     if constexpr (MIXER) {
 #pragma unroll
         for (int n = 0; n < CONV_PER; ++n) {
@@ -271,12 +295,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
                 return a.x * x[0] + a.y * x[1] + c.x * x[2] + c.y * x[3];
             };
 #pragma unroll
+            for (int j = 0; j < RW; ++j) dd[j] = dot4(wd[j], hdf);
+            const float draw = warp_sum_rows<RW>(dd);
+#pragma unroll
             for (int j = 0; j < RW; ++j) {
-                dd[j] = dot4(wd[j], hdf);
-                gg[j] = dot4(wgt[j], hgf);
+                const int a = row0 + j;
+                if (SSH && c0 < mix.G && (FULL || a < V)) wgt[j] = *reinterpret_cast<const uint2*>(mix.gate_w + (long long)(hh * V + a) * mix.G + c0);
             }
-            const float draw = warp_sum_rows<RW>(dd), graw = warp_sum_rows<RW>(gg);
-            if (my_row < r) {
+#pragma unroll
+            for (int j = 0; j < RW; ++j) gg[j] = dot4(wgt[j], hgf);
+            const float graw = warp_sum_rows<RW>(gg);
+            if (FULL || my_row < r) {
                 const float z = __bfloat162float(__float2bfloat16_rn(draw)) + mix.decay_bias[hh * r + my_row];
                 own_alpha = __expf(-__expf(mix.log_rate[hh]) * softplus_fast(z));
             }
@@ -297,16 +326,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
         const float graw = __bfloat162float(mix.geom_raw[(long long)b * mix.geom_sb + hh]) + mix.geom_bias[hh];
         gamma = 1.f / (1.f + __expf(-graw));
     } else {
-        dec_bf4(row_bf16(p.k, ch, 0), c0, r, p.k.vec && v4r, k);
-        dec_bf4(row_bf16(p.q, ch, 0), c0, r, p.q.vec && v4r, q);
-        dec_bf4(row_bf16(p.v, ch, 0), c0, V, p.v.vec && v4v, vv);
-        const float4 l4 = dec_load4(row_f32(p.ld, ch, 0), c0, r, p.ld.vec && v4r);
+        dec_bf4(row_bf16(p.k, ch, 0), c0, r, FULL || (p.k.vec && v4r), k);
+        dec_bf4(row_bf16(p.q, ch, 0), c0, r, FULL || (p.q.vec && v4r), q);
+        dec_bf4(row_bf16(p.v, ch, 0), c0, V, FULL || (p.v.vec && v4v), vv);
+        const float4 l4 = dec_load4(row_f32(p.ld, ch, 0), c0, r, FULL || (p.ld.vec && v4r));
         al[0] = __expf(l4.x); al[1] = __expf(l4.y); al[2] = __expf(l4.z); al[3] = __expf(l4.w);
         gamma = *row_f32(p.gam, ch, 0);
     }
-    dec_bf4(row_bf16(p.u, ch, 0), c0, r, p.u.vec && v4r, u);
-    dec_bf4(row_bf16(p.er, ch, 0), c0, r, p.er.vec && v4r, bq);
-    dec_bf4(row_bf16(p.wr, ch, 0), c0, V, p.wr.vec && v4v, wg);
+    dec_bf4(row_bf16(p.u, ch, 0), c0, r, FULL || (p.u.vec && v4r), u);
+    dec_bf4(row_bf16(p.er, ch, 0), c0, r, FULL || (p.er.vec && v4r), bq);
+    dec_bf4(row_bf16(p.wr, ch, 0), c0, V, FULL || (p.wr.vec && v4v), wg);
     if constexpr (MIXER) {
         __syncthreads();
         const float4 q4 = *reinterpret_cast<const float4*>(s_conv + c0), k4 = *reinterpret_cast<const float4*>(s_conv + DP + c0);
@@ -344,7 +373,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
 #pragma unroll
         for (int j = 0; j < RW; ++j) dots[j] = Cv[j].x * u[0] + Cv[j].y * u[1] + Cv[j].z * u[2] + Cv[j].w * u[3];
         const float cu = warp_sum_rows<RW>(dots);
-        delta = my_row < r ? gamma * (ha - cu) : 0.f;
+        delta = FULL || my_row < r ? gamma * (ha - cu) : 0.f;
         // the per-channel values of that row sit in lane row / 4
         const int src = my_row >> 2, el = my_row & 3;
         auto at_row = [&](const float (&x)[4]) {
@@ -374,6 +403,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
         }
     }
     __syncwarp();
+    if constexpr (SSH) cp_wait<0>();
     {
         float part[4][4];
 #pragma unroll
@@ -382,8 +412,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
             for (int e = 0; e < 4; ++e) part[n][e] = 0.f;
 #pragma unroll
         for (int j = 0; j < RW; ++j) {
-            const float4 f = s_row[warp][j];
-            const float cv[4] = {Cv[j].x, Cv[j].y, Cv[j].z, Cv[j].w}, sv[4] = {Sv[j].x, Sv[j].y, Sv[j].z, Sv[j].w};
+            const float4 f = s_row[warp][j], sj = state_s(j);
+            const float cv[4] = {Cv[j].x, Cv[j].y, Cv[j].z, Cv[j].w}, sv[4] = {sj.x, sj.y, sj.z, sj.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 part[0][e] = fmaf(cv[e], f.x, part[0][e]);
@@ -483,11 +513,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
     for (int j = 0; j < RW; ++j) {
         const int a = row0 + j;
         const float da = dec_channel(d, a), dl = s_own[0][warp * RW + j], aa = s_own[1][warp * RW + j];
-        if (a < r) {
+        if (FULL || a < r) {
             const float4 cn = make_float4(fmaf(Cv[j].x, al[0], dl * u[0]), fmaf(Cv[j].y, al[1], dl * u[1]),
                                           fmaf(Cv[j].z, al[2], dl * u[2]), fmaf(Cv[j].w, al[3], dl * u[3]));
-            const float4 sn = make_float4(fmaf(aa, Sv[j].x, da * w[0]), fmaf(aa, Sv[j].y, da * w[1]),
-                                          fmaf(aa, Sv[j].z, da * w[2]), fmaf(aa, Sv[j].w, da * w[3]));
+            const float4 sj = state_s(j);
+            const float4 sn = make_float4(fmaf(aa, sj.x, da * w[0]), fmaf(aa, sj.y, da * w[1]),
+                                          fmaf(aa, sj.z, da * w[2]), fmaf(aa, sj.w, da * w[3]));
             dec_store4(p.C + ((long long)s * r + a) * r, c0, r, vecC, cn);
             dec_store4(p.S + ((long long)s * r + a) * V, c0, V, vecS, sn);
         }
@@ -530,9 +561,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
 }
 
 // CTAs per stream.  While a cluster of four per stream fits the device at two CTAs per SM (4 x 74 = 2 x 148) the
-// spread shortens every phase: 6.6 us a step at 8 streams, 8.2 us at 64, against 8.7 and 9.5 us with one CTA of 16
-// warps per stream.  Past that the redundant per-token work of the cluster costs more than it hides: 15.3 against
-// 10.2 us at 128 streams, 87 against 62 us at 768 (3.2 TB/s).
+// spread shortens every phase: 4.4 us a step at 8 streams and 6.1 us at 64.  Past that the redundant per-token work of
+// the cluster costs more than it hides, and a stream is one CTA of eight warps, two to an SM so that one's loads run
+// under the other's arithmetic: S then waits in shared memory, since the registers of eight warps hold one state only.
+// 7.9 us at 128 streams, 41 us at 768 (4.9 TB/s); one CTA of sixteen warps with both states in registers, one to an
+// SM: 10.2 and 62 us; the same walking over the streams with the next states on their way: 69 us; the next CTA's
+// states prefetched into L2: no gain.
 inline int decode_split(int streams) { return streams <= 74 ? 4 : 1; }
+constexpr size_t DECODE_STATE_BYTES = size_t(DP) * DP * sizeof(float);   // dynamic shared memory of the one-CTA form
 
 }  // namespace sd

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import solvedelta_oracle as orc
-from solvedelta_b200 import SolveDeltaState, solvedelta_native
+from solvedelta_b200 import SolveDelta, SolveDeltaConfig, SolveDeltaState, solvedelta_native
 from tests.gpu_harness import make_inputs, oracle_args, oracle_state
 from tests.helpers import max_rel
 
@@ -31,3 +31,26 @@ def test_decode_step_launch_shapes(B, H, r, V, with_state, inplace):
         assert (fin.S.data_ptr() == state.S.data_ptr()) == inplace
         if not inplace:
             np.testing.assert_array_equal(state.S.cpu().numpy(), cpu["S0"].numpy())
+
+
+@pytest.mark.parametrize("width", [64, 128])
+def test_mixer_step_does_not_depend_on_the_number_of_streams(width):
+    # 76 streams: one CTA each; 38: clusters of four
+    torch.manual_seed(11)
+    layer = SolveDelta(SolveDeltaConfig(hidden_size=256, num_heads=2, head_k_dim=width, head_v_dim=width))
+    layer = layer.cuda().to(torch.bfloat16)
+    for name in ("geometry_write_bias", "associative_log_rate", "associative_decay_bias"):
+        getattr(layer, name).data = getattr(layer, name).data.float()
+    x = torch.randn(38, 71, 256, device="cuda", dtype=torch.bfloat16)
+
+    def steps(rows):
+        with torch.no_grad():
+            _, state = layer(rows[:, :66], return_final_state=True)
+            outs = []
+            for t in range(66, 71):
+                y, state = layer(rows[:, t:t + 1], initial_state=state, return_final_state=True)
+                outs.append(y)
+            return torch.cat(outs, 1)
+
+    whole, halves = steps(x), torch.cat([steps(x[:19]), steps(x[19:])])
+    assert max_rel(whole.float().cpu().numpy(), halves.float().cpu().numpy()) <= 1.6e-2
