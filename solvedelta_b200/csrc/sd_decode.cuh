@@ -560,14 +560,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
     if (NS > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// CTAs per stream.  While a cluster of four per stream fits the device at two CTAs per SM (4 x 74 = 2 x 148) the
-// spread shortens every phase: 4.4 us a step at 8 streams and 6.1 us at 64.  Past that the redundant per-token work of
+// CTAs per stream.  While a cluster of four per stream fits the device at two CTAs per SM (64 clusters do, 72 do not) the
+// spread shortens every phase: 4.4 us a step at 8 streams and 6.0 us at 64, but 9.3 at 72.  Past that the redundant work of
 // the cluster costs more than it hides, and a stream is one CTA of eight warps, two to an SM so that one's loads run
 // under the other's arithmetic: S then waits in shared memory, since the registers of eight warps hold one state only.
 // 7.9 us at 128 streams, 41 us at 768 (4.9 TB/s); one CTA of sixteen warps with both states in registers, one to an
 // SM: 10.2 and 62 us; the same walking over the streams with the next states on their way: 69 us; the next CTA's
 // states prefetched into L2: no gain.
-inline int decode_split(int streams) { return streams <= 74 ? 4 : 1; }
+inline int decode_split(int streams) { return streams <= 64 ? 4 : 1; }
 constexpr size_t DECODE_STATE_BYTES = size_t(DP) * DP * sizeof(float);   // dynamic shared memory of the one-CTA form
 
 }  // namespace sd

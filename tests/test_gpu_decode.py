@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,H,r,V,with_state,inplace", [
-    (37, 2, 128, 128, True, False), (25, 3, 128, 128, True, False),   # 74 and 75 streams: the two launch shapes
+    (32, 2, 128, 128, True, False), (13, 5, 128, 128, True, False),   # 64 and 65 streams: the two launch shapes
     (1, 1, 7, 13, True, True), (76, 1, 7, 13, True, False),           # rows that are no multiple of four
     (1, 2, 128, 36, False, False), (80, 1, 20, 128, False, False)])
 def test_decode_step_launch_shapes(B, H, r, V, with_state, inplace):
