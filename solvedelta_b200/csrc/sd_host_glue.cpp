@@ -761,7 +761,7 @@ struct TokenStack {
     static bool bf16_dense(const Tensor& t, const Tensor& like) {
         return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.device() == like.device() && aligned16(t);
     }
-    static bool layer_ok(const TokenLayer& l, const Tensor& x) {
+    static bool weights_ok(const TokenLayer& l, const Tensor& x) {
         const int64_t D = x.size(-1), H = l.heads, r = l.width, V = l.value_width;
         for (const Tensor* t : {&l.in_weight, &l.decay_weight, &l.gate_weight, &l.out_weight, &l.up_weight, &l.down_weight})
             if (!bf16_dense(*t, x)) return false;
@@ -771,7 +771,10 @@ struct TokenStack {
         return l.in_weight.size(1) == D && l.in_weight.size(0) % 8 == 0 && is_shape(l.out_weight, {D, H * V}) && l.up_weight.size(1) == D &&
                is_shape(l.down_weight, {D, inner}) && l.up_weight.size(0) % 16 == 0 && (H * V) % 8 == 0 && (H * r) % 8 == 0 &&
                is_shape(l.decay_weight, {H * r, V}) && is_shape(l.gate_weight, {H * V, V}) && V % 16 == 0 && V <= 128 && r <= 128 &&
-               l.conv_weight.size(0) == 2 * H * r + H * V && fits_smem(x.size(0), inner) && fits_smem(x.size(0), H * V);
+               l.conv_weight.size(0) == 2 * H * r + H * V;
+    }
+    static bool layer_ok(const TokenLayer& l, const Tensor& x) {
+        return weights_ok(l, x) && fits_smem(x.size(0), l.up_weight.size(0) / 2) && fits_smem(x.size(0), l.heads * l.value_width);
     }
     static bool fits_smem(int64_t rows, int64_t width) { return rows * (width + 96) * 2 <= 200 * 1024; }
 
@@ -913,6 +916,129 @@ struct TokenStack {
             norm_rows(f32(norm_w), norm_eps, out.data_ptr());
         return out;
     }
+
+    // A prompt [B,T,D] through the stack without gradients, from empty states: the launches of the module path, in its
+    // order, on pointers into one workspace.  Module calls, views and small tensors cost the host about 270 us a layer,
+    // which is more than the device needs below some two thousand tokens.  Returns the normalised hidden rows and, per
+    // layer, (C, S, conv window) when they are wanted; None when this is not a call it takes.
+    py::object prompt(const Tensor& x, bool want_states) {
+        if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || !x.is_contiguous() || x.dim() != 3 || x.size(0) < 1 || x.size(1) < 2)
+            return py::none();
+        const int64_t B = x.size(0), T = x.size(1), D = x.size(2), R = B * T;
+        if (R <= SD_TOKEN_MAX_ROWS || !addnorm_reverse_ok(D) || !aligned16(x)) return py::none();
+        struct Plan { sd_shape shape; size_t saved, scratch; };
+        std::vector<Plan> plan;
+        const auto up256 = [](size_t n) { return (n + 255) & ~size_t(255); };
+        const auto bf16_rows = [&](int64_t width) { return up256((size_t)R * (size_t)width * 2); };
+        // the mixer's buffers and the MLP's are never alive together
+        size_t area = 0;
+        for (const TokenLayer& l : layers) {
+            if (!weights_ok(l, x)) return py::none();
+            const int64_t H = l.heads, r = l.width, V = l.value_width;
+            const sd_shape sh{(int32_t)B, (int32_t)T, (int32_t)H, (int32_t)r, (int32_t)V};
+            const Plan pl{sh, up256(sd_inference_bytes(&sh)), up256(sd_forward_scratch_bytes(&sh))};
+            const size_t mixer = bf16_rows(l.in_weight.size(0)) + bf16_rows(2 * H * r + H * V) + 3 * bf16_rows(H * r) + bf16_rows(2 * H) +
+                                 3 * bf16_rows(H * V) + pl.saved + pl.scratch;
+            area = std::max({area, mixer, bf16_rows(l.up_weight.size(0)) + bf16_rows(l.up_weight.size(0) / 2)});
+            plan.push_back(pl);
+        }
+        const c10::cuda::CUDAGuard guard(x.device());
+        void* stream = stream_of(x);
+        const size_t d_b = bf16_rows(D);
+        const Tensor work = workspace(x, area + 5 * d_b);
+        char* const base = static_cast<char*>(work.data_ptr());
+        char *mixed = base + area, *mlp = mixed + d_b, *normed = mlp + d_b;
+        char* sums[2] = {normed + d_b, normed + 2 * d_b};
+        const auto bf16 = x.options(), fp32 = x.options().dtype(at::kFloat);
+        const auto matrix = [&](const void* p, int64_t cols, int64_t pitch) {
+            return at::from_blob(const_cast<void*>(p), {R, cols}, {pitch, 1}, bf16);
+        };
+        const auto linear = [&](const void* in, int64_t pitch, const Tensor& weight, const Tensor& bias, void* out) {
+            Tensor out_t = matrix(out, weight.size(0), weight.size(0));
+            if (bias.defined())
+                at::addmm_out(out_t, bias, matrix(in, weight.size(1), pitch), weight.t());
+            else
+                at::mm_out(out_t, matrix(in, weight.size(1), pitch), weight.t());
+        };
+        int next = 0;
+        const void* residual = x.data_ptr();
+        const void* delta = nullptr;
+        const auto norm_rows = [&](const Tensor& w, double eps, void* out) {
+            sd_add_rmsnorm_args a{};
+            a.rows = R; a.D = (int32_t)D; a.eps = (float)eps;
+            a.x = residual; a.delta = delta; a.weight = f32(w); a.sum = delta != nullptr ? sums[next] : nullptr; a.normed = out;
+            check(sd_add_rmsnorm(&a, stream));
+            if (delta == nullptr) return;
+            residual = sums[next];
+            next ^= 1;
+        };
+        py::list states;
+        for (size_t i = 0; i < layers.size(); ++i) {
+            TokenLayer& l = layers[i];
+            const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0), Dc = 2 * H * r + H * V;
+            char* at = base;
+            const auto take = [&](size_t bytes) { char* p = at; at += bytes; return p; };
+            char *row = take(bf16_rows(P)), *qkv = take(bf16_rows(Dc)), *decay_raw = take(bf16_rows(H * r));
+            char *log_decay = take(2 * bf16_rows(H * r)), *geometry = take(bf16_rows(2 * H)), *gate = take(bf16_rows(H * V));
+            char *y = take(bf16_rows(H * V)), *y_normed = take(bf16_rows(H * V)), *saved = take(plan[i].saved), *scratch = take(plan[i].scratch);
+            norm_rows(l.copies.get(0, l.mixer_norm), l.mixer_eps, normed);
+            linear(normed, D, l.in_weight, l.in_bias, row);
+            Tensor C, S, window;
+            if (want_states) {
+                C = f32_like(x, {B, H, r, r});
+                S = f32_like(x, {B, H, r, V});
+                window = bf16_like(x, {B, Dc, 3});
+            }
+            sd_conv4_forward_args c{};
+            c.B = (int32_t)B; c.T = (int32_t)T; c.D = (int32_t)Dc;
+            c.x = row; c.x_stride_b = T * P; c.x_stride_t = P;
+            c.weight = f32(l.copies.get(1, l.conv_weight)); c.y = qkv; c.final_state = raw(window);
+            check(sd_conv4_silu_forward(&c, stream));
+            const auto at_col = [&](int64_t col) { return row + 2 * col; };
+            const int64_t geom = Dc + 3 * H * r + H * V;
+            linear(at_col(geom + H), P, l.decay_weight, Tensor(), decay_raw);
+            linear(at_col(geom + H + V), P, l.gate_weight, l.gate_bias, gate);
+            sd_kda_gate_args k{};
+            k.rows = R; k.H = (int32_t)H; k.r = (int32_t)r;
+            k.raw = decay_raw; k.log_rate = f32(l.copies.get(2, l.log_rate)); k.bias = f32(l.copies.get(3, l.decay_bias));
+            k.log_decay = reinterpret_cast<float*>(log_decay);
+            check(sd_kda_gate_forward(&k, stream));
+            Tensor rate = at::from_blob(geometry, {R, H}, fp32);
+            at::add_out(rate, matrix(at_col(geom), H, P), l.copies.get(4, l.geometry_bias));
+            at::sigmoid_(rate);
+            sd_forward_args a{};
+            a.shape = plan[i].shape;
+            const auto row_operand = [&](int64_t col, int64_t w) { return sd_operand{at_col(col), T * P, P, w}; };
+            const auto conv_operand = [&](int64_t col, int64_t w) { return sd_operand{qkv + 2 * col, T * Dc, Dc, w}; };
+            a.u = row_operand(Dc, r); a.h = row_operand(Dc + H * r, r);
+            a.erase_raw = row_operand(Dc + 2 * H * r, r); a.write_raw = row_operand(Dc + 3 * H * r, V);
+            a.q = conv_operand(0, r); a.keys = conv_operand(H * r, r); a.values = conv_operand(2 * H * r, V);
+            a.log_decay = sd_operand{log_decay, T * H * r, H * r, r};
+            a.gamma = sd_operand{geometry, T * H, H, 1};
+            a.y = y; a.C_T = f32(C); a.S_T = f32(S);
+            a.saved = saved; a.saved_bytes = plan[i].saved; a.scratch = scratch; a.scratch_bytes = plan[i].scratch;
+            check(sd_forward_inference(&a, stream));
+            sd_norm_gate_args g{};
+            g.V = (int32_t)V; g.rows = R * H; g.eps = (float)l.out_eps;
+            g.x = y; g.gate = gate; g.weight = f32(l.copies.get(5, l.out_norm)); g.y = y_normed;
+            check(sd_norm_gate_forward(&g, stream));
+            linear(y_normed, H * V, l.out_weight, l.out_bias, mixed);
+            delta = mixed;
+            norm_rows(l.copies.get(6, l.mlp_norm), l.mlp_eps, normed);
+            const int64_t inner = l.up_weight.size(0) / 2;
+            char *up = base, *act = base + bf16_rows(2 * inner);
+            linear(normed, D, l.up_weight, Tensor(), up);
+            sd_swiglu_args w{};
+            w.I = (int32_t)inner; w.rows = R; w.gate_value = up; w.out = act;
+            check(sd_swiglu(&w, stream));
+            linear(act, inner, l.down_weight, Tensor(), mlp);
+            delta = mlp;
+            if (want_states) states.append(py::make_tuple(C, S, window));
+        }
+        Tensor out = bf16_like(x, x.sizes());
+        norm_rows(copies.get(0, norm), norm_eps, out.data_ptr());
+        return py::make_tuple(out, states);
+    }
 };
 
 }  // namespace
@@ -936,7 +1062,8 @@ void register_glue(py::module_& m) {
         .def("watch_absent", [](TokenStack& t, py::dict d, py::object k) { t.absent.emplace_back(d, k); })
         .def("watch_empty", [](TokenStack& t, py::dict d) { t.empty.push_back(d); })
         .def("unchanged", &TokenStack::unchanged)
-        .def("step", &TokenStack::step);
+        .def("step", &TokenStack::step)
+        .def("prompt", &TokenStack::prompt);
     m.def("conv4_silu", &conv4_silu);
     m.def("kda_decay_gate", &kda_decay_gate);
     m.def("rms_norm_gated", &rms_norm_gated);

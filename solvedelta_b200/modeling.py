@@ -321,6 +321,21 @@ class SolveDeltaModel(SolveDeltaPreTrainedModel):
             cache._seen_tokens += 1
         return token
 
+    def _prompt(self, hidden_states: torch.Tensor, cache: Optional[SolveDeltaCache]) -> Optional[torch.Tensor]:
+        """A prompt without gradients from empty states: all blocks and the final norm in one native call, which fills
+        ``cache`` when one is given.  None when that call does not apply; nothing has been touched then."""
+        if (hidden_states.ndim != 3 or hidden_states.shape[1] < 2 or torch.is_grad_enabled()
+                or (cache is not None and cache.states) or torch.is_autocast_enabled("cuda")):
+            return None
+        stack = token_stack(self, SolveDeltaBlock, SolveDeltaCacheAdapter, SolveDeltaMLP)
+        result = None if stack is None else stack.prompt(hidden_states, cache is not None)
+        if result is None:
+            return None
+        hidden_states, states = result
+        for layer, (predictor, memory, conv) in enumerate(states):
+            cache.update(layer, recurrent_state=(predictor, memory), conv_state=conv, offset=hidden_states.shape[1])
+        return hidden_states
+
     def forward(self, input_ids: Optional[torch.Tensor] = None, attention_mask: Optional[torch.Tensor] = None,
                 inputs_embeds: Optional[torch.Tensor] = None,
                 past_key_values: Union[SolveDeltaCache, Sequence[Dict[str, Any]], None] = None,
@@ -341,6 +356,10 @@ class SolveDeltaModel(SolveDeltaPreTrainedModel):
             token = self._cached_token(hidden_states, past_key_values)
             if token is not None:
                 return BaseModelOutputWithPast(last_hidden_state=token, past_key_values=past_key_values)
+        if attention_mask is None and not output_hidden_states and not kwargs:
+            prompt = self._prompt(hidden_states, past_key_values)
+            if prompt is not None:
+                return BaseModelOutputWithPast(last_hidden_state=prompt, past_key_values=past_key_values)
         cu_seqlens = kwargs.get("cu_seqlens")
         if cu_seqlens is not None and "solvedelta_reset_mask" not in kwargs:
             kwargs["solvedelta_reset_mask"] = segment_reset_mask(hidden_states, cu_seqlens)

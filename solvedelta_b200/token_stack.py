@@ -1,7 +1,7 @@
-"""One cached token through a model's blocks in one native call.
+"""One cached token, or a prompt, through a model's blocks in one native call.
 
 A single-token step of a generation loop is a chain of short launches, so per-layer module
-calls cost more than the kernels behind them.  :func:`token_stack` gives the native stack of a
+calls cost more than the kernels behind them; so does a prompt of up to a few thousand tokens.  :func:`token_stack` gives the native stack of a
 ``SolveDeltaModel`` (csrc/sd_host_glue.cpp): it holds the model's own parameter tensors and is
 rebuilt when a module, a parameter object or an epsilon has been replaced; a hook or a replaced
 ``forward`` anywhere in the blocks turns it off, so that the module path, which calls them, runs.
@@ -14,11 +14,12 @@ from typing import Optional
 from torch import nn
 from torch.nn.modules import module as module_globals
 
-from . import _lib
+from . import _lib, model as mixer_module
 from .model import RMSNormGated, SolveDelta
 
 _STACKS: "weakref.WeakKeyDictionary" = weakref.WeakKeyDictionary()
 _FUSED_DECODE_APPLIES = SolveDelta._fused_decode_applies
+_OPERATOR = mixer_module.solvedelta_native
 
 
 def _eps(norm: nn.RMSNorm) -> float:
@@ -69,7 +70,7 @@ def _build(model, block_type, adapter_type, mlp_type):
 
 def token_stack(model, block_type, adapter_type, mlp_type) -> Optional[object]:
     """The native stack of ``model`` in its present form, or None when the module path has to run."""
-    if SolveDelta._fused_decode_applies is not _FUSED_DECODE_APPLIES:
+    if SolveDelta._fused_decode_applies is not _FUSED_DECODE_APPLIES or mixer_module.solvedelta_native is not _OPERATOR:
         return None
     entry = _STACKS.get(model)
     if entry is not None and entry[0] == len(model.layers) and (entry[1] is None or entry[1].unchanged()):

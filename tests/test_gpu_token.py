@@ -58,3 +58,25 @@ def test_token_stack_equals_the_module_path(B):
             handle.remove()
     for got, want in zip(*seen):
         assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
+
+
+@pytest.mark.parametrize("B,T", [(1, 33), (3, 70), (2, 129)])
+def test_prompt_through_the_stack_equals_the_module_path(B, T):
+    torch.manual_seed(6)
+    model = SolveDeltaForCausalLM(SolveDeltaConfig(hidden_size=256, num_heads=4, head_k_dim=64, head_v_dim=64,
+                                                   num_hidden_layers=2, vocab_size=320)).prepare("cuda").eval()
+    ids = torch.randint(0, 320, (B, T), device="cuda")
+    seen = []
+    for hooked in (False, True):
+        handle = model.model.layers[1].mlp.register_forward_hook(lambda *a: None) if hooked else None
+        with torch.no_grad():
+            bare = model(input_ids=ids, use_cache=False).logits
+            out = model(input_ids=ids, use_cache=True)
+        assert torch.equal(out.logits, bare)
+        cache = out.past_key_values
+        assert cache.get_seq_length() == T and len(cache) == 2
+        seen.append((out.logits, *cache[1]["recurrent_state"], cache[1]["conv_state"]))
+        if handle is not None:
+            handle.remove()
+    for got, want in zip(*seen):
+        assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
