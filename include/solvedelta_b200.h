@@ -297,6 +297,10 @@ size_t sd_backward_scratch_bytes(const sd_shape *shape);
 /* `stream` is a cudaStream_t passed as void* (NULL = legacy default stream). */
 int sd_forward(const sd_forward_args *args, void *stream);
 int sd_backward(const sd_backward_args *args, void *stream);
+/* The same with the BF16 gradients written into wider rows: tokens of dq, dkeys and dvalues are qkv_pitch elements
+ * apart, tokens of du, dh, derase_raw and dwrite_raw row_pitch (batch rows T times that).  r, V and both pitches
+ * multiples of 8, pointers 16-byte aligned, else SD_ERR_UNSUPPORTED_SHAPE. */
+int sd_backward_pitched(const sd_backward_args *args, int64_t qkv_pitch, int64_t row_pitch, void *stream);
 /* sd_forward for a call that no reverse pass follows: the panels only sd_backward reads are not stored, `saved` is a
  * workspace of sd_inference_bytes. */
 size_t sd_inference_bytes(const sd_shape *shape);
@@ -460,6 +464,8 @@ typedef struct {
 size_t sd_conv4_backward_scratch_bytes(int32_t B, int32_t T, int32_t D);
 int sd_conv4_silu_forward(const sd_conv4_forward_args *args, void *stream);
 int sd_conv4_silu_backward(const sd_conv4_backward_args *args, void *stream);
+/* The same with dx inside wider rows: tokens dx_pitch >= D elements apart. */
+int sd_conv4_silu_backward_pitched(const sd_conv4_backward_args *args, int64_t dx_pitch, void *stream);
 
 typedef struct {
     int64_t rows;                  /* B*T */

@@ -275,7 +275,8 @@ class NormGateArgs(ctypes.Structure):
 
 EXPORTS = (
     "sd_saved_bytes", "sd_forward_scratch_bytes", "sd_backward_scratch_bytes",
-    "sd_forward", "sd_forward_inference", "sd_inference_bytes", "sd_backward", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
+    "sd_forward", "sd_forward_inference", "sd_inference_bytes", "sd_backward", "sd_backward_pitched",
+    "sd_conv4_silu_backward_pitched", "sd_decode_step", "sd_decode_step_from", "sd_forward_launches",
     "sd_backward_launches", "sd_panel_info", "sd_status_string", "sd_version",
     "sd_chunk_tokens", "sd_forward_static", "sd_panel_kind", "sd_device_fault", "sd_device_fault_clear",
     "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step",

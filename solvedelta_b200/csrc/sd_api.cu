@@ -628,12 +628,22 @@ struct PredictorOnly {
     const void *d_action, *d_update, *action_in;  // reverse inputs, same layout (the cotangents may be null)
 };
 int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po, bool keep = true);
-int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly* po);
+int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly* po, int64_t qkv_pitch = 0, int64_t row_pitch = 0);
 }  // namespace
 
 int sd_forward(const sd_forward_args* a, void* stream_) { return forward_impl(a, stream_, nullptr); }
 int sd_forward_inference(const sd_forward_args* a, void* stream_) { return forward_impl(a, stream_, nullptr, false); }
 int sd_backward(const sd_backward_args* a, void* stream_) { return backward_impl(a, stream_, nullptr); }
+int sd_backward_pitched(const sd_backward_args* a, int64_t qkv_pitch, int64_t row_pitch, void* stream_) {
+    if (!a) return SD_ERR_INVALID_ARGUMENT;
+    // the 16-byte stores need every row on such a boundary
+    uintptr_t bits = 0;
+    for (const void* q : {a->du, a->dh, a->dq, a->dkeys, a->dvalues, a->derase_raw, a->dwrite_raw}) bits |= reinterpret_cast<uintptr_t>(q);
+    if ((bits & 15) != 0 || a->shape.r % 8 != 0 || a->shape.V % 8 != 0 || qkv_pitch % 8 != 0 || row_pitch % 8 != 0) return SD_ERR_UNSUPPORTED_SHAPE;
+    const int64_t widest = (int64_t)a->shape.H * (a->shape.r > a->shape.V ? a->shape.r : a->shape.V);
+    if (qkv_pitch < widest || row_pitch < widest) return SD_ERR_INVALID_ARGUMENT;
+    return backward_impl(a, stream_, nullptr, qkv_pitch, row_pitch);
+}
 
 namespace {
 int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* po, bool keep) {
@@ -742,7 +752,7 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     return launch_status();
 }
 
-int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly* po) {
+int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly* po, int64_t qkv_pitch, int64_t row_pitch) {
     if (!a || !shape_ok(&a->shape)) return SD_ERR_INVALID_ARGUMENT;
     if (!shape_supported(&a->shape)) return SD_ERR_UNSUPPORTED_SHAPE;
     const sd_operand ops[] = {a->u,         a->h,         a->q,         a->keys,  a->values,
@@ -802,6 +812,10 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
 #undef SD_BB
 #undef SD_BP
     p.du = a->du; p.dh = a->dh; p.dq = a->dq; p.dk = a->dkeys; p.dv = a->dvalues;
+    p.pitch_q = qkv_pitch ? qkv_pitch : (int64_t)s->H * s->r;
+    p.pitch_v = qkv_pitch ? qkv_pitch : (int64_t)s->H * s->V;
+    p.pitch_u = row_pitch ? row_pitch : (int64_t)s->H * s->r;
+    p.pitch_w = row_pitch ? row_pitch : (int64_t)s->H * s->V;
     p.der = a->derase_raw; p.dwr = a->dwrite_raw; p.dld = a->dlog_decay; p.dgam = a->dgamma;
 
     const int chunks = (int)total_chunks(s);
@@ -1016,7 +1030,7 @@ size_t sd_conv4_backward_scratch_bytes(int32_t B, int32_t T, int32_t D) {
 // channel pairs can move as 4-byte accesses: even widths and strides, 4-byte aligned bases
 static bool conv_pairs_ok(const ConvParams& p) {
     auto al = [](const void* q) { return q == nullptr || (reinterpret_cast<uintptr_t>(q) & 3) == 0; };
-    return (p.D & 1) == 0 && (p.sb & 1) == 0 && (p.st & 1) == 0 && al(p.x) && al(p.y) && al(p.dy) && al(p.dx);
+    return (p.D & 1) == 0 && (p.sb & 1) == 0 && (p.st & 1) == 0 && (p.dxt & 1) == 0 && al(p.x) && al(p.y) && al(p.dy) && al(p.dx);
 }
 
 int sd_conv4_silu_forward(const sd_conv4_forward_args* a, void* stream_) {
@@ -1044,7 +1058,10 @@ int sd_conv4_silu_forward(const sd_conv4_forward_args* a, void* stream_) {
 }
 
 int sd_conv4_silu_backward(const sd_conv4_backward_args* a, void* stream_) {
-    if (!a || a->B <= 0 || a->T <= 0 || a->D <= 0 || !a->x || !a->weight || !a->dy || !a->dx || !a->dweight ||
+    return a ? sd_conv4_silu_backward_pitched(a, a->D, stream_) : SD_ERR_INVALID_ARGUMENT;
+}
+int sd_conv4_silu_backward_pitched(const sd_conv4_backward_args* a, int64_t dx_pitch, void* stream_) {
+    if (!a || dx_pitch < a->D || a->B <= 0 || a->T <= 0 || a->D <= 0 || !a->x || !a->weight || !a->dy || !a->dx || !a->dweight ||
         !a->scratch)
         return SD_ERR_INVALID_ARGUMENT;
     if (a->scratch_bytes < sd_conv4_backward_scratch_bytes(a->B, a->T, a->D)) return SD_ERR_BUFFER_TOO_SMALL;
@@ -1057,6 +1074,7 @@ int sd_conv4_silu_backward(const sd_conv4_backward_args* a, void* stream_) {
     p.init = reinterpret_cast<const __nv_bfloat16*>(a->initial_state);
     p.dy = reinterpret_cast<const __nv_bfloat16*>(a->dy);
     p.dx = reinterpret_cast<__nv_bfloat16*>(a->dx);
+    p.dxt = dx_pitch;
     p.dinit = reinterpret_cast<__nv_bfloat16*>(a->dinitial_state);
     p.dw_part = reinterpret_cast<float*>(a->scratch);
     p.valid = a->valid_mask; p.reset = a->reset_mask;

@@ -35,6 +35,7 @@ struct BwdParams {
     float *SdS;
     // outputs
     void *du, *dh, *dq, *dk, *dv, *der, *dwr;
+    long long pitch_q, pitch_v, pitch_u, pitch_w;   // elements between tokens of dq and dk; dv; du, dh and der; dwr
     float *dld, *dgam;
 };
 
@@ -253,8 +254,8 @@ __device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& c
         }
         float dq[8];
         norm_vjp8(dqh, qh, rstd_q, dq);
-        store8_bf16<FAST>(p.dq, p.g, ch, i, c0, r, dq);
-        store8_bf16<FAST>(p.der, p.g, ch, i, c0, r, der);
+        store8_bf16<FAST>(p.dq, p.pitch_q, p.g, ch, i, c0, r, dq);
+        store8_bf16<FAST>(p.der, p.pitch_u, p.g, ch, i, c0, r, der);
         store8_bpanel(bpanel_ptr(p.duPart, ch.gi), i, c0, duh);
         store8_bpanel(bpanel_ptr(p.dkPart, ch.gi), i, c0, dkp);
         store8_bpanel(bpanel_ptr(p.dDelta, ch.gi), i, c0, ddl);
@@ -273,8 +274,8 @@ __device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& c
             dv[e] = sw * dr[e];
             dwr[e] = dr[e] * v[e] * sw * (1.f - sw);
         }
-        store8_bf16<FAST>(p.dv, p.g, ch, i, c0, V, dv);
-        store8_bf16<FAST>(p.dwr, p.g, ch, i, c0, V, dwr);
+        store8_bf16<FAST>(p.dv, p.pitch_v, p.g, ch, i, c0, V, dv);
+        store8_bf16<FAST>(p.dwr, p.pitch_w, p.g, ch, i, c0, V, dwr);
     }
 }
 
@@ -730,8 +731,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
         dota = (s_dot[ia * 4] + s_dot[ia * 4 + 1]) + (s_dot[ia * 4 + 2] + s_dot[ia * 4 + 3]);
         dotb = (s_dot[ib * 4] + s_dot[ib * 4 + 1]) + (s_dot[ib * 4 + 2] + s_dot[ib * 4 + 3]);
         __nv_bfloat16* dk = reinterpret_cast<__nv_bfloat16*>(p.dk);
-        __nv_bfloat16* rowa = dk + (((long long)ch.b * p.g.T + ch.t0 + ia) * p.g.H + ch.hh) * (long long)r;
-        __nv_bfloat16* rowb = dk + (((long long)ch.b * p.g.T + ch.t0 + ib) * p.g.H + ch.hh) * (long long)r;
+        __nv_bfloat16* rowa = dk + ((long long)ch.b * p.g.T + ch.t0 + ia) * p.pitch_q + ch.hh * r;
+        __nv_bfloat16* rowb = dk + ((long long)ch.b * p.g.T + ch.t0 + ib) * p.pitch_q + ch.hh * r;
 #pragma unroll
         for (int nt = 0; nt < NT128; ++nt) {
             const int j = n0 + nt * 8 + 2 * t;
@@ -1067,8 +1068,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
             const float gm = s_gam[i];
 #pragma unroll
             for (int e = 0; e < 8; ++e) dh[e] = gm * drr[e];
-            store8_bf16<FAST>(p.du, p.g, ch, i, c0, r, du);
-            store8_bf16<FAST>(p.dh, p.g, ch, i, c0, r, dh);
+            store8_bf16<FAST>(p.du, p.pitch_u, p.g, ch, i, c0, r, du);
+            store8_bf16<FAST>(p.dh, p.pitch_u, p.g, ch, i, c0, r, dh);
         }
     }
     __syncthreads();

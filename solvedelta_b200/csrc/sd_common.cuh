@@ -250,13 +250,13 @@ __device__ __forceinline__ void load8_f32(const float* row, int c0, int width, i
     }
 }
 
-// Contiguous outputs [B,T,H,width]: eight channels of one row.
+// Outputs [B,T,H,width], tokens `pitch` elements apart: eight channels of one row.
 template <bool FAST, class CH>
-__device__ __forceinline__ void store8_bf16(void* base, const Geometry& g, const CH& ch, int i, int c0,
+__device__ __forceinline__ void store8_bf16(void* base, long long pitch, const Geometry& g, const CH& ch, int i, int c0,
                                             int width, const float (&x)[8]) {
     if (FAST) {
         __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(base) +
-                             (((long long)ch.b * g.T + ch.t0 + i) * g.H + ch.hh) * (long long)width;
+                             ((long long)ch.b * g.T + ch.t0 + i) * pitch + ch.hh * width;
         uint4 raw;
         __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&raw);
 #pragma unroll
@@ -271,11 +271,11 @@ __device__ __forceinline__ void store8_bf16(void* base, const Geometry& g, const
         for (int e = 0; e < 8; ++e)
             if (c0 + e < width)
                 (reinterpret_cast<__nv_bfloat16*>(base) +
-                 (((long long)ch.b * g.T + ch.t0 + i) * g.H + ch.hh) * (long long)width)[c0 + e] = __float2bfloat16_rn(0.f);
+                 ((long long)ch.b * g.T + ch.t0 + i) * pitch + ch.hh * width)[c0 + e] = __float2bfloat16_rn(0.f);
         return;
     }
     __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(base) +
-                         (((long long)ch.b * g.T + ch.t0 + i) * g.H + ch.hh) * (long long)width;
+                         ((long long)ch.b * g.T + ch.t0 + i) * pitch + ch.hh * width;
     if ((width & 7) == 0) {
         uint4 raw;
         __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&raw);

@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
             float a[8], dl[8];
             load8_smem(s_kh, i, c0, a);
             load8_panel(gDelta, i, c0, dl);
-            store8_bf16<FAST>(p.action, p.g, ch, i, c0, r, a);
-            store8_bf16<FAST>(p.update, p.g, ch, i, c0, r, dl);
+            store8_bf16<FAST>(p.action, (long long)p.g.H * r, p.g, ch, i, c0, r, a);
+            store8_bf16<FAST>(p.update, (long long)p.g.H * r, p.g, ch, i, c0, r, dl);
         }
         return;
     }

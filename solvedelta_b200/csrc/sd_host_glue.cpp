@@ -598,6 +598,203 @@ py::tuple mixer_front(const Tensor& x, int64_t heads, int64_t width, int64_t val
                           fin.defined() ? py::cast(fin) : py::none());
 }
 
+// Where the slices of the projection row stand, and the operator's operands on that row and on the conv's output.
+struct RowPlan {
+    int64_t B, T, H, r, V, P;   // P: columns of the row
+    int64_t conv() const { return 2 * H * r + H * V; }           // q | k | v, then u, h, erase, write
+    int64_t geometry() const { return conv() + 3 * H * r + H * V; }
+    int64_t decay_hidden() const { return geometry() + H; }
+    int64_t gate_hidden() const { return decay_hidden() + V; }
+    int64_t used() const { return gate_hidden() + V; }
+    sd_shape shape() const { return sd_shape{(int32_t)B, (int32_t)T, (int32_t)H, (int32_t)r, (int32_t)V}; }
+    template <class Args>
+    void fill(Args& a, const void* row, const void* qkv, const void* log_decay, const void* rate) const {
+        a.shape = shape();
+        const auto on_row = [&](int64_t col, int64_t w) { return sd_operand{static_cast<const char*>(row) + 2 * col, T * P, P, w}; };
+        const int64_t D = conv();
+        const auto on_conv = [&](int64_t col, int64_t w) { return sd_operand{static_cast<const char*>(qkv) + 2 * col, T * D, D, w}; };
+        a.u = on_row(D, r); a.h = on_row(D + H * r, r);
+        a.erase_raw = on_row(D + 2 * H * r, r); a.write_raw = on_row(D + 3 * H * r, V);
+        a.q = on_conv(0, r); a.keys = on_conv(H * r, r); a.values = on_conv(2 * H * r, V);
+        a.log_decay = sd_operand{log_decay, T * H * r, H * r, r};
+        a.gamma = sd_operand{rate, T * H, H, 1};
+    }
+};
+
+// The whole layer as one autograd node: what its separate nodes do, on the same kernels.  One node because the separate
+// ones cost the host 1.2 ms a training call, more than the device needs below some four thousand tokens, and because
+// the reverse pass knows where every gradient belongs: the operator's kernels write dq, dk, dv straight into the conv's
+// cotangent rows and du, dh, d erase, d write into the projection row's gradient, the conv and the two small products
+// write their columns of it, and no kernel gathers them (130 us of 3250 at 8 x 2048 tokens of width 1024).
+struct MixerFunction : torch::autograd::Function<MixerFunction> {
+    static RowPlan plan(const Tensor& x, int64_t H, int64_t r, int64_t V, const Tensor& in_weight) {
+        return RowPlan{x.size(0), x.size(1), H, r, V, in_weight.size(0)};
+    }
+
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& in_weight, const OptTensor& in_bias,
+                          const Tensor& conv_weight, const Tensor& decay_weight, const Tensor& gate_weight, const OptTensor& gate_bias,
+                          const Tensor& log_rate, const Tensor& decay_bias, const Tensor& geometry_bias, const Tensor& norm_weight,
+                          const Tensor& out_weight, const OptTensor& out_bias, const OptTensor& valid, const OptTensor& reset,
+                          int64_t heads, int64_t width, int64_t value_width, double eps) {
+        const c10::cuda::CUDAGuard guard(x.device());
+        const RowPlan m = plan(x, heads, width, value_width, in_weight);
+        const int64_t H = m.H, r = m.r, V = m.V, P = m.P, R = m.B * m.T, Dc = m.conv();
+        void* stream = stream_of(x);
+        const Tensor x2 = x.view({R, x.size(2)});
+        const auto product = [](const Tensor& a, const Tensor& w, const OptTensor& b) {
+            return b.has_value() ? at::addmm(*b, a, w.t()) : at::mm(a, w.t());
+        };
+        const Tensor row = product(x2, in_weight, in_bias);
+        const Tensor w32 = f32_contiguous(conv_weight), A32 = f32_contiguous(log_rate), b32 = f32_contiguous(decay_bias);
+        const Tensor n32 = f32_contiguous(norm_weight);
+        const Tensor qkv = bf16_like(x, {R, Dc});
+        sd_conv4_forward_args c{};
+        c.B = (int32_t)m.B; c.T = (int32_t)m.T; c.D = (int32_t)Dc;
+        c.x = row.data_ptr(); c.x_stride_b = m.T * P; c.x_stride_t = P;
+        c.weight = f32(w32); c.y = qkv.data_ptr();
+        c.valid_mask = bytes(given(valid)); c.reset_mask = bytes(given(reset));
+        check(sd_conv4_silu_forward(&c, stream));
+        const Tensor decay_raw = product(row.narrow(1, m.decay_hidden(), V), decay_weight, std::nullopt);
+        const Tensor gate = product(row.narrow(1, m.gate_hidden(), V), gate_weight, gate_bias).view({R * H, V});
+        const Tensor log_decay = gate_forward(decay_raw.view({R, H, r}), A32, b32);
+        const Tensor rate = at::add(row.narrow(1, m.geometry(), H), geometry_bias.to(at::kFloat)).sigmoid_();
+        const sd_shape sh = m.shape();
+        const Tensor y = bf16_like(x, {R * H, V}), saved = workspace(x, sd_saved_bytes(&sh));
+        {
+            const Tensor scratch = workspace(x, sd_forward_scratch_bytes(&sh));
+            sd_forward_args a{};
+            m.fill(a, row.data_ptr(), qkv.data_ptr(), log_decay.data_ptr(), rate.data_ptr());
+            a.y = y.data_ptr();
+            a.saved = saved.data_ptr(); a.saved_bytes = (size_t)saved.numel();
+            a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+            a.valid_mask = c.valid_mask; a.reset_mask = c.reset_mask;
+            check(sd_forward(&a, stream));
+        }
+        const Tensor out = product(norm_gate_forward(y, gate, n32, eps).view({R, H * V}), out_weight, out_bias);
+        ctx->set_materialize_grads(false);
+        ctx->save_for_backward({x, in_weight, decay_weight, gate_weight, out_weight, row, qkv, decay_raw, gate, log_decay, rate, y, saved,
+                                w32, A32, b32, n32, given(valid), given(reset)});
+        auto& data = ctx->saved_data;
+        data["heads"] = heads; data["width"] = width; data["value_width"] = value_width; data["eps"] = eps;
+        data["in_bias"] = in_bias.has_value(); data["gate_bias"] = gate_bias.has_value(); data["out_bias"] = out_bias.has_value();
+        data["x"] = x.requires_grad();
+        const auto remember = [&](const char* name, const Tensor& t) { data[name] = (int64_t)t.scalar_type(); };
+        remember("conv", conv_weight); remember("rate", log_rate); remember("decay", decay_bias);
+        remember("geometry", geometry_bias); remember("norm", norm_weight);
+        data["rate_shape"] = log_rate.sizes().vec(); data["decay_shape"] = decay_bias.sizes().vec();
+        return out.view({m.B, m.T, out_weight.size(0)});
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list result(19);
+        if (!grads[0].defined()) return result;
+        const variable_list sv = ctx->get_saved_variables();
+        auto& data = ctx->saved_data;
+        const Tensor &x = sv[0], &in_weight = sv[1], &decay_weight = sv[2], &gate_weight = sv[3], &out_weight = sv[4], &row = sv[5];
+        const Tensor &qkv = sv[6], &decay_raw = sv[7], &gate = sv[8], &log_decay = sv[9], &rate = sv[10], &y = sv[11], &saved = sv[12];
+        const Tensor &w32 = sv[13], &A32 = sv[14], &b32 = sv[15], &n32 = sv[16], &valid = sv[17], &reset = sv[18];
+        const c10::cuda::CUDAGuard guard(x.device());
+        const double eps = data["eps"].toDouble();
+        const RowPlan m = plan(x, data["heads"].toInt(), data["width"].toInt(), data["value_width"].toInt(), in_weight);
+        const int64_t H = m.H, r = m.r, V = m.V, P = m.P, R = m.B * m.T, Dc = m.conv();
+        void* stream = stream_of(x);
+        const auto as = [&](const char* name, const Tensor& t) { return t.to((at::ScalarType)data[name].toInt()); };
+        // output projection and gated norm
+        const Tensor dout = grads[0].to(at::kBFloat16).reshape({R, out_weight.size(0)});
+        result[11] = at::mm(dout.t(), norm_gate_forward(y, gate, n32, eps).view({R, H * V}));   // the norm is produced again
+        if (data["out_bias"].toBool()) result[12] = dout.to(at::kFloat).sum(0).to(at::kBFloat16);
+        const auto [dy, dgate3, dnorm] = norm_gate_backward(y, gate, n32, eps, at::mm(dout, out_weight).view({R * H, V}));
+        result[10] = as("norm", dnorm);
+        // the projection row's gradient, written piece by piece
+        Tensor drow = bf16_like(x, {R, P});
+        const Tensor dqkv = bf16_like(x, {R, Dc});
+        const auto at_col = [&](const Tensor& t, int64_t col) { return static_cast<char*>(t.data_ptr()) + 2 * col; };
+        const Tensor dgate = dgate3.view({R, H * V});
+        Tensor piece = drow.narrow(1, m.gate_hidden(), V);
+        at::mm_out(piece, dgate, gate_weight);
+        result[5] = at::mm(dgate.t(), row.narrow(1, m.gate_hidden(), V));
+        if (data["gate_bias"].toBool()) result[6] = dgate.sum(0);
+        Tensor dld = f32_like(x, {R, H * r}), drate = f32_like(x, {R, H});
+        const sd_shape sh = m.shape();
+        {
+            const Tensor scratch = workspace(x, sd_backward_scratch_bytes(&sh));
+            sd_backward_args a{};
+            m.fill(a, row.data_ptr(), qkv.data_ptr(), log_decay.data_ptr(), rate.data_ptr());
+            a.dy = sd_operand{dy.data_ptr(), m.T * H * V, H * V, V};
+            a.saved = saved.data_ptr(); a.saved_bytes = (size_t)saved.numel();
+            a.scratch = scratch.data_ptr(); a.scratch_bytes = (size_t)scratch.numel();
+            a.dq = at_col(dqkv, 0); a.dkeys = at_col(dqkv, H * r); a.dvalues = at_col(dqkv, 2 * H * r);
+            a.du = at_col(drow, Dc); a.dh = at_col(drow, Dc + H * r);
+            a.derase_raw = at_col(drow, Dc + 2 * H * r); a.dwrite_raw = at_col(drow, Dc + 3 * H * r);
+            a.dlog_decay = f32(dld); a.dgamma = f32(drate);
+            a.valid_mask = bytes(valid); a.reset_mask = bytes(reset);
+            check(sd_backward_pitched(&a, Dc, P, stream));
+        }
+        {   // decay gate and its small product
+            Tensor draw = at::empty_like(decay_raw), dA = f32_like(x, {H}), db = f32_like(x, {H * r});
+            const Tensor scratch = workspace(x, sd_kda_gate_backward_scratch_bytes(R, (int32_t)H, (int32_t)r));
+            sd_kda_gate_args k{};
+            k.rows = R; k.H = (int32_t)H; k.r = (int32_t)r;
+            k.raw = decay_raw.data_ptr(); k.log_rate = f32(A32); k.bias = f32(b32); k.dlog_decay = f32(dld);
+            k.draw = draw.data_ptr(); k.dlog_rate = f32(dA); k.dbias = f32(db);
+            k.scratch = scratch.data_ptr(); k.scratch_bytes = (size_t)scratch.numel();
+            check(sd_kda_gate_backward(&k, stream));
+            result[7] = as("rate", dA).view(data["rate_shape"].toIntVector());
+            result[8] = as("decay", db).view(data["decay_shape"].toIntVector());
+            piece = drow.narrow(1, m.decay_hidden(), V);
+            at::mm_out(piece, draw, decay_weight);
+            result[4] = at::mm(draw.t(), row.narrow(1, m.decay_hidden(), V));
+        }
+        const Tensor dgeometry = at::sigmoid_backward(drate, rate);
+        drow.narrow(1, m.geometry(), H).copy_(dgeometry);
+        result[9] = as("geometry", dgeometry.sum(0));
+        if (m.used() < P) drow.narrow(1, m.used(), P - m.used()).zero_();
+        {   // conv
+            const Tensor dw = f32_like(x, {Dc, 4});
+            const Tensor scratch = workspace(x, sd_conv4_backward_scratch_bytes((int32_t)m.B, (int32_t)m.T, (int32_t)Dc));
+            sd_conv4_backward_args c{};
+            c.B = (int32_t)m.B; c.T = (int32_t)m.T; c.D = (int32_t)Dc;
+            c.x = row.data_ptr(); c.x_stride_b = m.T * P; c.x_stride_t = P;
+            c.weight = f32(w32); c.dy = dqkv.data_ptr(); c.dx = drow.data_ptr(); c.dweight = f32(dw);
+            c.scratch = scratch.data_ptr(); c.scratch_bytes = (size_t)scratch.numel();
+            c.valid_mask = bytes(valid); c.reset_mask = bytes(reset);
+            check(sd_conv4_silu_backward_pitched(&c, P, stream));
+            result[3] = as("conv", dw);
+        }
+        // input projection
+        result[1] = at::mm(drow.t(), x.view({R, x.size(2)}));
+        if (data["in_bias"].toBool()) result[2] = drow.sum(0);
+        if (data["x"].toBool()) result[0] = at::mm(drow, in_weight).view(x.sizes());
+        return result;
+    }
+};
+
+// The layer on [B,T,D] with gradients recorded, from empty states, or None when this is not a call the node takes.
+OptTensor mixer_train(const Tensor& x, int64_t heads, int64_t width, int64_t value_width, const Tensor& in_weight, const OptTensor& in_bias,
+                      const Tensor& conv_weight, const Tensor& decay_weight, const Tensor& gate_weight, const OptTensor& gate_bias,
+                      const Tensor& log_rate, const Tensor& decay_bias, const Tensor& geometry_bias, const Tensor& norm_weight, double eps,
+                      const Tensor& out_weight, const OptTensor& out_bias, const OptTensor& valid, const OptTensor& reset) {
+    if (!at::GradMode::is_enabled() || !x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 3 || !x.is_contiguous() || x.numel() == 0)
+        return std::nullopt;
+    const RowPlan m{x.size(0), x.size(1), heads, width, value_width, in_weight.size(0)};
+    const auto dense = [&](const Tensor& t) { return t.is_contiguous() && t.scalar_type() == at::kBFloat16 && t.device() == x.device() && t.requires_grad(); };
+    for (const Tensor* t : {&in_weight, &decay_weight, &gate_weight, &out_weight})
+        if (!dense(*t) || !aligned16(*t)) return std::nullopt;
+    for (const OptTensor* t : {&in_bias, &gate_bias, &out_bias})
+        if (t->has_value() && !dense(**t)) return std::nullopt;
+    for (const Tensor* t : {&conv_weight, &log_rate, &decay_bias, &geometry_bias, &norm_weight})
+        if (t->device() != x.device() || !t->requires_grad()) return std::nullopt;
+    const int64_t H = heads, r = width, V = value_width;
+    if (r % 8 != 0 || V % 8 != 0 || r > 128 || V > 128 || m.P % 8 != 0 || m.P < m.used() || in_weight.size(1) != x.size(2) ||
+        !is_shape(decay_weight, {H * r, V}) || !is_shape(gate_weight, {H * V, V}) || out_weight.dim() != 2 || out_weight.size(1) != H * V ||
+        !is_shape(conv_weight, {m.conv(), 4}) || log_rate.numel() != H || decay_bias.numel() != H * r || geometry_bias.numel() != H ||
+        !is_shape(norm_weight, {V}))
+        return std::nullopt;
+    const OptTensor v = conv_mask("valid_mask", valid, x), z = conv_mask("reset_mask", reset, x);
+    return MixerFunction::apply(x, in_weight, in_bias, conv_weight, decay_weight, gate_weight, gate_bias, log_rate, decay_bias,
+                                geometry_bias, norm_weight, out_weight, out_bias, v, z, heads, width, value_width, eps);
+}
+
 // One cached token between the fused projection row and the output projection, in one launch; argument meanings as in
 // mixer_decode_step (mixer_ops.py).
 struct DecodeToken {
@@ -926,7 +1123,7 @@ struct TokenStack {
             return py::none();
         const int64_t B = x.size(0), T = x.size(1), D = x.size(2), R = B * T;
         if (R <= SD_TOKEN_MAX_ROWS || !addnorm_reverse_ok(D) || !aligned16(x)) return py::none();
-        struct Plan { sd_shape shape; size_t saved, scratch; };
+        struct Plan { size_t saved, scratch; };
         std::vector<Plan> plan;
         const auto up256 = [](size_t n) { return (n + 255) & ~size_t(255); };
         const auto bf16_rows = [&](int64_t width) { return up256((size_t)R * (size_t)width * 2); };
@@ -936,7 +1133,7 @@ struct TokenStack {
             if (!weights_ok(l, x)) return py::none();
             const int64_t H = l.heads, r = l.width, V = l.value_width;
             const sd_shape sh{(int32_t)B, (int32_t)T, (int32_t)H, (int32_t)r, (int32_t)V};
-            const Plan pl{sh, up256(sd_inference_bytes(&sh)), up256(sd_forward_scratch_bytes(&sh))};
+            const Plan pl{up256(sd_inference_bytes(&sh)), up256(sd_forward_scratch_bytes(&sh))};
             const size_t mixer = bf16_rows(l.in_weight.size(0)) + bf16_rows(2 * H * r + H * V) + 3 * bf16_rows(H * r) + bf16_rows(2 * H) +
                                  3 * bf16_rows(H * V) + pl.saved + pl.scratch;
             area = std::max({area, mixer, bf16_rows(l.up_weight.size(0)) + bf16_rows(l.up_weight.size(0) / 2)});
@@ -976,6 +1173,7 @@ struct TokenStack {
         for (size_t i = 0; i < layers.size(); ++i) {
             TokenLayer& l = layers[i];
             const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0), Dc = 2 * H * r + H * V;
+            const RowPlan rows{B, T, H, r, V, P};
             char* at = base;
             const auto take = [&](size_t bytes) { char* p = at; at += bytes; return p; };
             char *row = take(bf16_rows(P)), *qkv = take(bf16_rows(Dc)), *decay_raw = take(bf16_rows(H * r));
@@ -995,26 +1193,18 @@ struct TokenStack {
             c.weight = f32(l.copies.get(1, l.conv_weight)); c.y = qkv; c.final_state = raw(window);
             check(sd_conv4_silu_forward(&c, stream));
             const auto at_col = [&](int64_t col) { return row + 2 * col; };
-            const int64_t geom = Dc + 3 * H * r + H * V;
-            linear(at_col(geom + H), P, l.decay_weight, Tensor(), decay_raw);
-            linear(at_col(geom + H + V), P, l.gate_weight, l.gate_bias, gate);
+            linear(at_col(rows.decay_hidden()), P, l.decay_weight, Tensor(), decay_raw);
+            linear(at_col(rows.gate_hidden()), P, l.gate_weight, l.gate_bias, gate);
             sd_kda_gate_args k{};
             k.rows = R; k.H = (int32_t)H; k.r = (int32_t)r;
             k.raw = decay_raw; k.log_rate = f32(l.copies.get(2, l.log_rate)); k.bias = f32(l.copies.get(3, l.decay_bias));
             k.log_decay = reinterpret_cast<float*>(log_decay);
             check(sd_kda_gate_forward(&k, stream));
             Tensor rate = at::from_blob(geometry, {R, H}, fp32);
-            at::add_out(rate, matrix(at_col(geom), H, P), l.copies.get(4, l.geometry_bias));
+            at::add_out(rate, matrix(at_col(rows.geometry()), H, P), l.copies.get(4, l.geometry_bias));
             at::sigmoid_(rate);
             sd_forward_args a{};
-            a.shape = plan[i].shape;
-            const auto row_operand = [&](int64_t col, int64_t w) { return sd_operand{at_col(col), T * P, P, w}; };
-            const auto conv_operand = [&](int64_t col, int64_t w) { return sd_operand{qkv + 2 * col, T * Dc, Dc, w}; };
-            a.u = row_operand(Dc, r); a.h = row_operand(Dc + H * r, r);
-            a.erase_raw = row_operand(Dc + 2 * H * r, r); a.write_raw = row_operand(Dc + 3 * H * r, V);
-            a.q = conv_operand(0, r); a.keys = conv_operand(H * r, r); a.values = conv_operand(2 * H * r, V);
-            a.log_decay = sd_operand{log_decay, T * H * r, H * r, r};
-            a.gamma = sd_operand{geometry, T * H, H, 1};
+            rows.fill(a, row, qkv, log_decay, geometry);
             a.y = y; a.C_T = f32(C); a.S_T = f32(S);
             a.saved = saved; a.saved_bytes = plan[i].saved; a.scratch = scratch; a.scratch_bytes = plan[i].scratch;
             check(sd_forward_inference(&a, stream));
@@ -1076,6 +1266,7 @@ void register_glue(py::module_& m) {
     m.def("gated_mlp", &gated_mlp);
     m.def("pack_rows", &pack_rows);
     m.def("mixer_front", &mixer_front);
+    m.def("mixer_train", &mixer_train);
     m.def("mixer_decode_step", &mixer_decode_step);
     m.def("mixer_decode", &mixer_decode);
 }

@@ -25,7 +25,8 @@ struct ConvParams {
     __nv_bfloat16* fin;          // [B][D][3] or null
     // backward
     const __nv_bfloat16* dy;     // [B,T,D] contiguous
-    __nv_bfloat16* dx;           // [B,T,D] contiguous
+    __nv_bfloat16* dx;           // [B,T,D], tokens dxt elements apart
+    long long dxt;
     __nv_bfloat16* dinit;        // [B][D][3] or null
     float* dw_part;              // [B * tiles][D][4]
     // masks, one byte per (batch, token), either may be null (all valid / no reset)
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv4_silu_bwd(ConvParams p) {
     const int t_last = min(t_end + 3, p.T);   // tokens past the tile still feed its last three gradients
     const __nv_bfloat16* xin = p.x + b * p.sb + d;
     const __nv_bfloat16* gin = p.dy + (long long)b * p.T * p.D + d;
-    __nv_bfloat16* dxout = p.dx + (long long)b * p.T * p.D + d;
+    __nv_bfloat16* dxout = p.dx + (long long)b * p.T * p.dxt + d;
     if (PAIR) {
         __shared__ unsigned ring_x[CONV_RING][CONV_THREADS], ring_g[CONV_RING][CONV_THREADS];
         auto issue = [&](int t) {
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv4_silu_bwd(ConvParams p) {
             const float da = wa[0] * g3.x + wa[1] * g2.x + wa[2] * g1.x + wa[3] * g0.x;
             const float db = wb[0] * g3.y + wb[1] * g2.y + wb[2] * g1.y + wb[3] * g0.y;
             if (INNER || (tq >= t0 && tq < t_end)) {
-                store_pair<PAIR>(dxout + (long long)tq * p.D, two, da, db);
+                store_pair<PAIR>(dxout + (long long)tq * p.dxt, two, da, db);
             } else if (tq < 0 && t0 == 0 && p.dinit != nullptr) {
                 __nv_bfloat16* sd = p.dinit + ((long long)b * p.D + d) * 3 + (tq + 3);
                 sd[0] = __float2bfloat16_rn(da);
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv4_silu_bwd(ConvParams p) {
                 const float da = wa[0] * g3.x + wa[1] * g2.x + wa[2] * g1.x + wa[3] * g0.x;
                 const float db = wb[0] * g3.y + wb[1] * g2.y + wb[2] * g1.y + wb[3] * g0.y;
                 if (tq >= t0 && tq < t_end) {
-                    store_pair<PAIR>(dxout + (long long)tq * p.D, two, da, db);
+                    store_pair<PAIR>(dxout + (long long)tq * p.dxt, two, da, db);
                 } else if (tq < 0 && t0 == 0 && p.dinit != nullptr) {
                     __nv_bfloat16* s = p.dinit + ((long long)b * p.D + d) * 3 + (tq + 3);
                     s[0] = __float2bfloat16_rn(da);
@@ -374,12 +375,12 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv4_silu_bwd_masked(ConvPara
     const int t_end = min(t0 + CONV_TT, p.T);
     const __nv_bfloat16* xin = p.x + b * p.sb + d;
     const __nv_bfloat16* gin = p.dy + (long long)b * p.T * p.D + d;
-    __nv_bfloat16* dxout = p.dx + (long long)b * p.T * p.D + d;
+    __nv_bfloat16* dxout = p.dx + (long long)b * p.T * p.dxt + d;
     auto own = [&](int t) { return (t >= t0 && t < t_end) || (t < 0 && t >= -3 && t0 == 0 && p.dinit != nullptr); };
     auto emit = [&](int t, float2 a) {
         if (!own(t)) return;
         if (t >= 0) {
-            store_pair<PAIR>(dxout + (long long)t * p.D, two, a.x, a.y);
+            store_pair<PAIR>(dxout + (long long)t * p.dxt, two, a.x, a.y);
         } else {
             __nv_bfloat16* s = p.dinit + ((long long)b * p.D + d) * 3 + (t + 3);
             s[0] = __float2bfloat16_rn(a.x);
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(CONV_THREADS) k_conv4_silu_bwd_masked(ConvPara
     for (int t = t0; t < p.T; ++t) {
         if (t >= t_end && !own(i0) && !own(i1) && !own(i2)) break;
         if (!conv_valid(p, b, t)) {
-            if (t < t_end) store_pair<PAIR>(dxout + (long long)t * p.D, two, 0.f, 0.f);
+            if (t < t_end) store_pair<PAIR>(dxout + (long long)t * p.dxt, two, 0.f, 0.f);
             continue;
         }
         if (conv_reset(p, b, t)) {

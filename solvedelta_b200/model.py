@@ -28,6 +28,9 @@ from .mixer_ops import rms_norm_gated
 from .ops import SolveDeltaState, solvedelta_masked_native, solvedelta_native
 
 
+_OPERATOR = (solvedelta_native, solvedelta_masked_native)
+
+
 class SolveDeltaLayerState(NamedTuple):
     operator: SolveDeltaState
     conv: Optional[torch.Tensor]
@@ -101,6 +104,13 @@ class SolveDelta(nn.Module):
         return (conv.dtype == torch.bfloat16 and conv.is_contiguous() and C.dtype == torch.float32
                 and S.dtype == torch.float32 and C.is_contiguous() and S.is_contiguous())
 
+    def _one_node_applies(self, initial_state, return_final_state, geometry_enabled, associative_decay_enabled) -> bool:
+        """Training from empty states: the layer is one autograd node of the host extension.  Not when the operator's
+        call site below has been replaced, nor under autocast, which would cast the separate products."""
+        return (initial_state is None and not return_final_state and self.config.use_short_conv and geometry_enabled
+                and associative_decay_enabled and torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")
+                and (solvedelta_native, solvedelta_masked_native) == _OPERATOR)
+
     def forward(self, hidden_states: torch.Tensor, *, initial_state: Optional[SolveDeltaLayerState] = None,
                 valid_mask: Optional[torch.Tensor] = None, reset_mask: Optional[torch.Tensor] = None,
                 geometry_enabled: bool = True, associative_decay_enabled: bool = True,
@@ -140,6 +150,15 @@ class SolveDelta(nn.Module):
                 operator.predictor, operator.S, output_norm.weight, output_norm.eps, output_proj.weight,
                 output_proj.bias)
             return result, SolveDeltaLayerState(SolveDeltaState(operator.predictor, operator.S), initial_state.conv)
+        if self._one_node_applies(initial_state, return_final_state, geometry_enabled, associative_decay_enabled):
+            output_norm, output_proj = self.output_norm, self.output_proj
+            result = host.mixer_train(
+                hidden_states, heads, width, value_width, in_proj.weight, in_proj.bias, self.conv_weight,
+                decay_proj.weight, gate_proj.weight, gate_proj.bias, self.associative_log_rate,
+                self.associative_decay_bias, self.geometry_write_bias, output_norm.weight, output_norm.eps,
+                output_proj.weight, output_proj.bias, valid_mask, reset_mask)
+            if result is not None:
+                return result
         conv_state = initial_state.conv if initial_state is not None else None
         (u, h, q, keys, values, log_decay, erase_raw, write_raw, geometry_write, output_gate,
          final_conv) = host.mixer_front(
