@@ -148,6 +148,8 @@ typedef struct {
 } sd_swiglu_args;
 
 int sd_add_rmsnorm(const sd_add_rmsnorm_args *args, void *stream);
+/* The same between chained launches (sd_token_linear): it may start under the launch before it. */
+int sd_add_rmsnorm_chained(const sd_add_rmsnorm_args *args, void *stream);
 size_t sd_add_rmsnorm_backward_scratch_bytes(int64_t rows, int32_t D);
 int sd_add_rmsnorm_backward(const sd_add_rmsnorm_backward_args *args, void *stream);
 int sd_swiglu(const sd_swiglu_args *args, void *stream);
@@ -194,7 +196,7 @@ int sd_gemv(const sd_gemv_args *args, void *stream);
 
 /*
  * The same projection for up to SD_TOKEN_MAX_ROWS rows, with the block's residual add and RMSNorm in front of it:
- * when norm_weight is given (M <= 8, K <= 2048) the rows of the product are RMSNorm(x + delta) * norm_weight, rounded
+ * when norm_weight is given (M <= 16, K <= 2048) the rows of the product are RMSNorm(x + delta) * norm_weight, rounded
  * as sd_add_rmsnorm rounds them, and sum receives x + delta (with delta == NULL: RMSNorm(x), sum unused).
  * chained != 0: the launch may start while the kernel before it in the stream still runs and reads its weights
  * meanwhile; x, delta and what that kernel wrote are read after it has finished.  The weights, and the states of

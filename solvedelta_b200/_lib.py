@@ -280,7 +280,7 @@ EXPORTS = (
     "sd_backward_launches", "sd_panel_info", "sd_status_string", "sd_version",
     "sd_chunk_tokens", "sd_forward_static", "sd_panel_kind", "sd_device_fault", "sd_device_fault_clear",
     "sd_predictor_forward", "sd_predictor_backward", "sd_mixer_decode_step",
-    "sd_mixer_decode_step_chained", "sd_token_linear", "sd_add_rmsnorm", "sd_swiglu",
+    "sd_mixer_decode_step_chained", "sd_token_linear", "sd_add_rmsnorm", "sd_add_rmsnorm_chained", "sd_swiglu",
     "sd_add_rmsnorm_backward_scratch_bytes", "sd_add_rmsnorm_backward", "sd_swiglu_backward", "sd_pack_rows",
     "sd_cross_entropy_forward", "sd_cross_entropy_backward", "sd_gemv",
     "sd_conv4_backward_scratch_bytes", "sd_conv4_silu_forward", "sd_conv4_silu_backward",

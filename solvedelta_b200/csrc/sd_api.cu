@@ -405,6 +405,10 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_decode_step<false, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_decode_step<true, 1, 8, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_decode_step<true, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 1, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 2, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_token_linear<2, 2, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 2, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<1, 1, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
@@ -500,8 +504,10 @@ cudaError_t launch_token_linear(const TokenLinearParams& p, bool chained, cudaSt
 }
 template <int CG>
 cudaError_t dispatch_token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) {
-    if (p.norm_w != nullptr)
+    if (p.norm_w != nullptr && p.M <= 8)
         return p.K <= 1024 ? launch_token_linear<1, CG, 4>(p, chained, stream) : launch_token_linear<1, CG, 8>(p, chained, stream);
+    if (p.norm_w != nullptr)
+        return p.K <= 1024 ? launch_token_linear<2, CG, 4>(p, chained, stream) : launch_token_linear<2, CG, 8>(p, chained, stream);
     if (p.M <= 8) return launch_token_linear<1, CG, 0>(p, chained, stream);
     if (p.M <= 16) return launch_token_linear<2, CG, 0>(p, chained, stream);
     return launch_token_linear<4, CG, 0>(p, chained, stream);
@@ -533,6 +539,35 @@ cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int st
     cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS, FULL>, p, m);
 }
+int add_rmsnorm(const sd_add_rmsnorm_args* a, bool chained, void* stream_) {
+    if (!a || a->rows <= 0 || a->D <= 0 || !a->x || !a->weight || !a->normed || (a->delta && !a->sum))
+        return SD_ERR_INVALID_ARGUMENT;
+    if (a->rows > 0x7fffffffLL) return SD_ERR_UNSUPPORTED_SHAPE;
+    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+    AddNormParams p{};
+    p.N = a->rows; p.D = a->D; p.eps = a->eps;
+    p.x = reinterpret_cast<const __nv_bfloat16*>(a->x);
+    p.delta = reinterpret_cast<const __nv_bfloat16*>(a->delta);
+    p.w = a->weight;
+    p.sum = reinterpret_cast<__nv_bfloat16*>(a->sum);
+    p.normed = reinterpret_cast<__nv_bfloat16*>(a->normed);
+    // few rows (single-token steps): a whole CTA per row finishes sooner than one warp per row
+    if (addnorm_rows_ok(a->D) && (a->rows >= 1024 || !a->delta)) {
+        dispatch_addnorm_rows(p, false, stream);
+    } else {
+        if (!a->delta) return SD_ERR_UNSUPPORTED_SHAPE;   // the norm alone is only built for the row kernels
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)a->rows);
+        cfg.blockDim = dim3(256);
+        cfg.stream = stream;
+        cudaLaunchAttribute at = chained_launch();
+        cfg.attrs = &at;
+        cfg.numAttrs = chained ? 1 : 0;
+        if (cudaLaunchKernelEx(&cfg, k_add_rmsnorm, p) != cudaSuccess) return SD_ERR_LAUNCH_FAILED;
+    }
+    return launch_status();
+}
+
 template <bool MIXER>
 int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
     if (configure_kernels() != cudaSuccess) return SD_ERR_NO_DEVICE;
@@ -1205,27 +1240,8 @@ int sd_norm_gate_backward(const sd_norm_gate_args* a, void* stream_) {
     return launch_status();
 }
 
-int sd_add_rmsnorm(const sd_add_rmsnorm_args* a, void* stream_) {
-    if (!a || a->rows <= 0 || a->D <= 0 || !a->x || !a->weight || !a->normed || (a->delta && !a->sum))
-        return SD_ERR_INVALID_ARGUMENT;
-    if (a->rows > 0x7fffffffLL) return SD_ERR_UNSUPPORTED_SHAPE;
-    cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    AddNormParams p{};
-    p.N = a->rows; p.D = a->D; p.eps = a->eps;
-    p.x = reinterpret_cast<const __nv_bfloat16*>(a->x);
-    p.delta = reinterpret_cast<const __nv_bfloat16*>(a->delta);
-    p.w = a->weight;
-    p.sum = reinterpret_cast<__nv_bfloat16*>(a->sum);
-    p.normed = reinterpret_cast<__nv_bfloat16*>(a->normed);
-    // few rows (single-token steps): a whole CTA per row finishes sooner than one warp per row
-    if (addnorm_rows_ok(a->D) && (a->rows >= 1024 || !a->delta)) {
-        dispatch_addnorm_rows(p, false, stream);
-    } else {
-        if (!a->delta) return SD_ERR_UNSUPPORTED_SHAPE;   // the norm alone is only built for the row kernels
-        k_add_rmsnorm<<<(unsigned)a->rows, 256, 0, stream>>>(p);
-    }
-    return launch_status();
-}
+int sd_add_rmsnorm(const sd_add_rmsnorm_args* a, void* stream_) { return add_rmsnorm(a, false, stream_); }
+int sd_add_rmsnorm_chained(const sd_add_rmsnorm_args* a, void* stream_) { return add_rmsnorm(a, true, stream_); }
 
 size_t sd_add_rmsnorm_backward_scratch_bytes(int64_t rows, int32_t D) {
     if (rows <= 0 || D <= 0) return 0;

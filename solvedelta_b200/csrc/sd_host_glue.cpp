@@ -914,7 +914,7 @@ Tensor mixer_decode(Fp32Copies& copies, const Tensor& x, int64_t heads, int64_t 
 
 // ---- a cached token through the whole stack ------------------------------------------------------------------
 // The blocks and the final norm of a model for one cached token without gradients, as one call: five chained launches a
-// layer on pointers into one workspace (seven past eight rows, where the norms are launches of their own).  The
+// layer on pointers into one workspace (seven past sixteen rows, where the norms are launches of their own).  The
 // parameters are held as the module's own tensors; what is watched says when the module has changed under it (see
 // token_stack.py).
 struct TokenLayer {
@@ -1022,7 +1022,7 @@ struct TokenStack {
         const void* residual = x.data_ptr();
         const void* delta = nullptr;
         bool chained = false;   // nothing of this call is in flight: the first launch follows the stream in full
-        const bool fuse_norm = B <= 8;
+        const bool fuse_norm = B <= 16;
         const auto linear = [&](const void* in, int64_t K, const Tensor& weight, const void* bias, void* out, bool with_swiglu,
                                 const float* norm_w, double eps) {
             if (B > 16 && !with_swiglu && weight.size(0) >= 16 * 148) {
@@ -1059,8 +1059,9 @@ struct TokenStack {
             sd_add_rmsnorm_args a{};
             a.rows = B; a.D = (int32_t)D; a.eps = (float)eps;
             a.x = residual; a.delta = delta; a.weight = norm_w; a.sum = delta != nullptr ? sums[next] : nullptr; a.normed = out;
-            check(sd_add_rmsnorm(&a, stream));
-            chained = false;   // a plain launch: the next one follows it in full
+            // without delta: the first launch, in the kernel for many rows, which follows the stream in full
+            check(chained && delta != nullptr ? sd_add_rmsnorm_chained(&a, stream) : sd_add_rmsnorm(&a, stream));
+            chained = delta != nullptr;
             advance();
         };
         // projection of the normalised residual stream

@@ -793,6 +793,8 @@ struct AddNormParams {
 };
 
 __global__ void __launch_bounds__(256) k_add_rmsnorm(AddNormParams p) {
+    chain_wait();
+    chain_release();
     __shared__ float red[8];
     const long long row = blockIdx.x;
     const __nv_bfloat16* x = p.x + row * p.D;

@@ -27,7 +27,7 @@ __device__ __forceinline__ uint4 load16_live(const __nv_bfloat16* p) {
 }
 
 constexpr int TOKEN_MAX_ROWS = 32;
-constexpr int TOKEN_NORM_MAX_ROWS = 8;   // the fused norm: one row per warp
+constexpr int TOKEN_NORM_MAX_ROWS = 16;  // the fused norm: up to two rows per warp
 constexpr int TOKEN_NORM_MAX_K = 2048;   // ... whose pieces sit in registers
 constexpr size_t TOKEN_SMEM_MAX = 200 * 1024;   // of one CTA, beside the static part
 constexpr int TOKEN_BATCH = 8;           // weight pieces per lane and step
@@ -58,7 +58,7 @@ template <int RG, int CG, int NORM>
 __global__ void __launch_bounds__(256, RG <= 2 ? 2 : 1) k_token_linear(TokenLinearParams p) {
     constexpr int KS = 8 / CG;          // K slices
     constexpr int MT = (RG + 1) / 2;    // 16-row tiles
-    static_assert(NORM == 0 || RG == 1, "the fused norm takes one row per warp");
+    static_assert(NORM == 0 || RG <= 2, "the fused norm takes up to two rows per warp");
     extern __shared__ __align__(16) unsigned char tok_smem[];
     const int pitch = token_pitch(p.K);
     __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(tok_smem);
@@ -95,11 +95,11 @@ __global__ void __launch_bounds__(256, RG <= 2 ? 2 : 1) k_token_linear(TokenLine
     chain_release();
 
     if constexpr (NORM > 0) {
-        // one warp per row: sum, its mean square, the normalised row (the sum is rounded to BF16 first, as the separate
+        // a warp takes every eighth row: sum, its mean square, the normalised row (the sum is rounded to BF16 first, as the separate
         // add stores it)
         __syncthreads();   // norm weights
-        const int m = warp;
-        if (m < p.M) {
+#pragma unroll 1
+        for (int m = warp; m < p.M; m += 8) {
             const __nv_bfloat16* x = p.x + m * p.x_stride;
             const __nv_bfloat16* d = p.delta != nullptr ? p.delta + m * p.x_stride : nullptr;
             uint4 xv[NORM], dv[NORM];

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,norm,delta,swiglu", [
     (1, 24, 8, False, False, False), (7, 2376, 264, True, True, False), (8, 2368, 2048, True, False, False),
     (9, 40, 2816, False, False, False), (16, 2384, 1000, False, False, False), (17, 8, 72, False, False, True),
-    (32, 112, 1024, False, False, True), (3, 48, 1024, True, True, True)])
+    (32, 112, 1024, False, False, True), (3, 48, 1024, True, True, True),
+    (9, 2376, 1024, True, True, False), (16, 48, 2048, True, False, True)])
 def test_token_linear(M, N, K, norm, delta, swiglu):
     gen = torch.Generator().manual_seed(M * N + K)
     bf = lambda *s: torch.randn(*s, generator=gen).to(torch.bfloat16).cuda()
