@@ -1203,7 +1203,8 @@ int sd_norm_gate_forward(const sd_norm_gate_args* a, void* stream_) {
     p.w = a->weight;
     p.out = reinterpret_cast<__nv_bfloat16*>(a->y);
     long long blocks = (a->rows + 15) / 16;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    const long long wave = resident_ctas(k_norm_gate_fwd, 256, 0);   // one wave: a CTA carries its next rows
+    if (blocks > wave) blocks = wave;
     k_norm_gate_fwd<<<(unsigned)blocks, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(p);
     return launch_status();
 }
