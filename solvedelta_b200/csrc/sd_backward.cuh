@@ -197,7 +197,7 @@ __device__ __forceinline__ void sources_bwd_rows(const BwdParams& p, const CH& c
             load8_bsm(sdDt, i, c0, ddt);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float ep = __expf(G[e]), et = __expf(GL[e] - G[e]);
+                const float ep = exp_ftz(G[e]), et = exp_ftz(GL[e] - G[e]);
                 dd[e] = py[e] + et * ddt[e];
                 xext[e] = ddt[e] * d[e] * et;
                 dg_[e] = dd[e] * ep;
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
         const float2 G = *reinterpret_cast<const float2*>(s_G + i * LDP + j);
         float2 Gp = make_float2(0.f, 0.f);
         if (ref >= 0) Gp = *reinterpret_cast<const float2*>(s_G + ref * LDP + j);
-        return make_float2(__expf(G.x - Gp.x), __expf(G.y - Gp.y));
+        return make_float2(exp_ftz(G.x - Gp.x), exp_ftz(G.y - Gp.y));
     };
     // exp(G_ref - G_j) for rows of block J = I of the anti-causal result
     auto col_factor = [&](int i, int j) {
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
         const float2 G = *reinterpret_cast<const float2*>(s_G + i * LDP + j);
         float2 Ge = make_float2(0.f, 0.f);
         if (ref >= 0) Ge = *reinterpret_cast<const float2*>(s_G + ref * LDP + j);
-        return make_float2(__expf(Ge.x - G.x), __expf(Ge.y - G.y));
+        return make_float2(exp_ftz(Ge.x - G.x), exp_ftz(Ge.y - G.y));
     };
     {
         float a1[NT128][4], a2[NT128][4];
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(NTHREADS) k_predictor_seed_bwd(BwdParams p, Op
         load8_panel(gG, i, c0, G);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            dg[e] = dd[e] * __expf(G[e]);
+            dg[e] = dd[e] * exp_ftz(G[e]);
             dgp[e] = dd[e] * a[e];
         }
         store8_bpanel(bpanel_ptr(p.DG, ch.gi), i, c0, dg);
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
     {   // BF16 copy of 1 / beta for the fast diagonal pair blocks (0 where the block is not fast)
         const int J = threadIdx.x >> 7, c = threadIdx.x & (DP - 1);
         const float d = fG(BT * J + BT - 1, c) - (J ? fG(BT * J - 1, c) : 0.f);
-        s_ibeta_b[threadIdx.x] = __float2bfloat16_rn(d >= -FAST_BLOCK_NATS ? __expf(-d) : 0.f);
+        s_ibeta_b[threadIdx.x] = __float2bfloat16_rn(d >= -FAST_BLOCK_NATS ? exp_ftz(-d) : 0.f);
     }
     pair_block_scales_bf16(s_Mb, fG);
     {
@@ -610,10 +610,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
             float uc[8], ub[8], rn[8], ddr[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                uc[e] = uh[e] * __expf(Ge[e] - G[e]);
-                ub[e] = uh[e] * __expf(GL[e] - G[e]);
-                rn[e] = -gm * uh[e] * __expf(E[e]);
-                ddr[e] = dd[e] * __expf(G[e] - Gp[e]);
+                uc[e] = uh[e] * exp_ftz(Ge[e] - G[e]);
+                ub[e] = uh[e] * exp_ftz(GL[e] - G[e]);
+                rn[e] = -gm * uh[e] * exp_ftz(E[e]);
+                ddr[e] = dd[e] * exp_ftz(G[e] - Gp[e]);
             }
             store8_bsm(b_uc, i, c0, uc);
             store8_bsm(b_ur, i, c0, uh);
@@ -685,7 +685,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
             const float2 G = *reinterpret_cast<const float2*>(gG + i * DP + j);
             float2 Ge = make_float2(0.f, 0.f);
             if (ref >= 0) Ge = *reinterpret_cast<const float2*>(gG + ref * DP + j);
-            return make_float2(__expf(Ge.x - G.x), __expf(Ge.y - G.y));
+            return make_float2(exp_ftz(Ge.x - G.x), exp_ftz(Ge.y - G.y));
         });
     }
     cp_wait<0>();
@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
     block_decay_tables(s_beta, nullptr, s_fastw, fG);
     for (int idx = threadIdx.x; idx < 3 * DP; idx += NTHREADS) {
         const int m = idx >> 7, c = idx & (DP - 1);
-        s_pref[idx] = __float2bfloat16_rn(__expf(gG[((m + 1) * BT - 1) * DP + c]));
+        s_pref[idx] = __float2bfloat16_rn(exp_ftz(gG[((m + 1) * BT - 1) * DP + c]));
     }
     {
         const int lr = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
@@ -867,8 +867,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
             float uc[8], ur[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                uc[e] = uh[e] * __expf(Ge[e] - G[e]);
-                ur[e] = uh[e] * __expf(E[e] - Gp[e]);
+                uc[e] = uh[e] * exp_ftz(Ge[e] - G[e]);
+                ur[e] = uh[e] * exp_ftz(E[e] - Gp[e]);
             }
             store8_bsm(b_uc, i, c0, uc);
             store8_bsm(b_ur, i, c0, ur);
@@ -986,14 +986,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
             E.x -= ch.eoff(i);
             E.y -= ch.eoff(i);
             if (ref >= 0) Gp = *reinterpret_cast<const float2*>(gG + ref * DP + j);
-            return make_float2(__expf(E.x - Gp.x), __expf(E.y - Gp.y));
+            return make_float2(exp_ftz(E.x - Gp.x), exp_ftz(E.y - Gp.y));
         });
         epi_scale_store_bsm<NT128>(atj, r0, n0, b_tj, [&](int i, int j) {   // exp(G_ref - G_j)
             const int ref = fast ? r0 - 1 : r0 + BT - 1;
             const float2 G = *reinterpret_cast<const float2*>(gG + i * DP + j);
             float2 Ge = make_float2(0.f, 0.f);
             if (ref >= 0) Ge = *reinterpret_cast<const float2*>(gG + ref * DP + j);
-            return make_float2(__expf(Ge.x - G.x), __expf(Ge.y - G.y));
+            return make_float2(exp_ftz(Ge.x - G.x), exp_ftz(Ge.y - G.y));
         });
     }
     if (threadIdx.x < CL && threadIdx.x < ch.nvalid) {
@@ -1048,7 +1048,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
             float duh[8], dE[8], dG[8], X[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float eE = __expf(E[e]), et = __expf(GL[e] - G[e]);
+                const float eE = exp_ftz(E[e]), et = exp_ftz(GL[e] - G[e]);
                 const float tu = tpre[e], t_i = ti[e], t_j = tj[e];
                 duh[e] = dup[e] + tu + dub[e] * et + dut[e] * eE + t_i + t_j;
                 dE[e] = dut[e] * (uh[e] * eE) + uh[e] * t_i;
@@ -1090,7 +1090,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
         s_tot[(4 + seg) * DP + c] = tx;
         __syncthreads();
         if (c < r) {
-            float run = __expf(gG[(CL - 1) * DP + c]) * (p.SdS[ch.gi * DP + c] + s_cdc[c]) +
+            float run = exp_ftz(gG[(CL - 1) * DP + c]) * (p.SdS[ch.gi * DP + c] + s_cdc[c]) +
                         ((s_tot[4 * DP + c] + s_tot[5 * DP + c]) + (s_tot[6 * DP + c] + s_tot[7 * DP + c]));
             for (int s2 = seg + 1; s2 < 4; ++s2) run += s_tot[s2 * DP + c];
             // a masked token has no gradient; nor does the decay of a reset token, which multiplies the zero state

@@ -144,7 +144,20 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // 1 / (1 + exp(-x)) with the fast reciprocal (2 ulp): exp(-x) = inf gives exactly 0.
-__device__ __forceinline__ float sigmoidf_(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
+// exp and 1/x on the hardware's base-2 exponential and reciprocal, subnormals flushed: two instructions and one, where
+// the forms that keep subnormals scale their argument and result (about five each).  Arguments here are sums of a one
+// and an exponential, or factors that multiply numbers of order one: below 1e-38 nothing of them is left in a result.
+__device__ __forceinline__ float exp_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float sigmoidf_(float x) { return rcp_ftz(1.0f + exp_ftz(-x)); }
 
 // ---- half-warp (16 lanes = one token row) reductions ---------------------
 __device__ __forceinline__ float row_sum16(float v) {

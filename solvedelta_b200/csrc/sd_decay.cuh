@@ -49,8 +49,8 @@ __device__ __forceinline__ void block_decay_tables(float* s_beta, float* s_ibeta
     const int J = threadIdx.x >> 7, c = threadIdx.x & (DP - 1);
     const float d = fg(BT * J + BT - 1, c) - (J ? fg(BT * J - 1, c) : 0.f);
     const bool ok = d >= -FAST_BLOCK_NATS;
-    if (s_beta != nullptr) s_beta[threadIdx.x] = __expf(d);
-    if (s_ibeta != nullptr) s_ibeta[threadIdx.x] = ok ? __expf(-d) : 0.f;
+    if (s_beta != nullptr) s_beta[threadIdx.x] = exp_ftz(d);
+    if (s_ibeta != nullptr) s_ibeta[threadIdx.x] = ok ? exp_ftz(-d) : 0.f;
     const int all = __all_sync(0xffffffffu, ok);
     if ((threadIdx.x & 31) == 0) s_fastw[threadIdx.x >> 5] = all;
 }
@@ -67,7 +67,7 @@ __device__ __forceinline__ void pair_block_scales(float* s_M, FG fg) {
     for (int idx = threadIdx.x; idx < 3 * DP; idx += NTHREADS) {
         const int m = idx >> 7, c = idx & (DP - 1);
         const float e0 = fg(BT - 1, c), e1 = fg(2 * BT - 1, c), e2 = fg(3 * BT - 1, c);
-        s_M[idx] = __expf(m == 0 ? e1 - e0 : (m == 1 ? e2 - e1 : e2 - e0));
+        s_M[idx] = exp_ftz(m == 0 ? e1 - e0 : (m == 1 ? e2 - e1 : e2 - e0));
     }
 }
 __device__ __forceinline__ int pair_scale_index(int I, int J) {  // -1: adjacent blocks, no scale
@@ -127,7 +127,7 @@ __device__ __forceinline__ void pair_block_scales_bf16(bf16* s_Mb, FG fg) {
     for (int idx = threadIdx.x; idx < 3 * DP; idx += NTHREADS) {
         const int m = idx >> 7, c = idx & (DP - 1);
         const float e0 = fg(BT - 1, c), e1 = fg(2 * BT - 1, c), e2 = fg(3 * BT - 1, c);
-        s_Mb[idx] = __float2bfloat16_rn(__expf(m == 0 ? e1 - e0 : (m == 1 ? e2 - e1 : e2 - e0)));
+        s_Mb[idx] = __float2bfloat16_rn(exp_ftz(m == 0 ? e1 - e0 : (m == 1 ? e2 - e1 : e2 - e0)));
     }
 }
 
@@ -260,7 +260,7 @@ __device__ __forceinline__ void block_alphas(float (&al)[BT], FG fG) {
 #pragma unroll
     for (int k = 0; k < BT; ++k) {
         const float g = fG(i0 + k, c);
-        al[k] = __expf(g - prev);
+        al[k] = exp_ftz(g - prev);
         prev = g;
     }
 }

@@ -307,30 +307,30 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(
             const float graw = warp_sum_rows<RW>(gg);
             if (FULL || my_row < r) {
                 const float z = __bfloat162float(__float2bfloat16_rn(draw)) + mix.decay_bias[hh * r + my_row];
-                own_alpha = __expf(-__expf(mix.log_rate[hh]) * softplus_fast(z));
+                own_alpha = exp_ftz(-exp_ftz(mix.log_rate[hh]) * softplus_fast(z));
             }
             if (lane % LPR == 0) {
                 const float bias = my_row < V && mix.gate_b != nullptr ? __bfloat162float(mix.gate_b[hh * V + my_row]) : 0.f;
                 s_own[2][my_row - rank * ROWS] = __bfloat162float(__float2bfloat16_rn(graw + bias));
             }
         } else {
-            const float rate = __expf(mix.log_rate[hh]);
+            const float rate = exp_ftz(mix.log_rate[hh]);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 if (c0 + e < r) {
                     const int hc = hh * r + c0 + e;
                     const float z = __bfloat162float(mix.decay_raw[(long long)b * mix.decay_sb + hc]) + mix.decay_bias[hc];
-                    al[e] = __expf(-rate * softplus_fast(z));
+                    al[e] = exp_ftz(-rate * softplus_fast(z));
                 }
         }
         const float graw = __bfloat162float(mix.geom_raw[(long long)b * mix.geom_sb + hh]) + mix.geom_bias[hh];
-        gamma = 1.f / (1.f + __expf(-graw));
+        gamma = 1.f / (1.f + exp_ftz(-graw));
     } else {
         dec_bf4(row_bf16(p.k, ch, 0), c0, r, FULL || (p.k.vec && v4r), k);
         dec_bf4(row_bf16(p.q, ch, 0), c0, r, FULL || (p.q.vec && v4r), q);
         dec_bf4(row_bf16(p.v, ch, 0), c0, V, FULL || (p.v.vec && v4v), vv);
         const float4 l4 = dec_load4(row_f32(p.ld, ch, 0), c0, r, FULL || (p.ld.vec && v4r));
-        al[0] = __expf(l4.x); al[1] = __expf(l4.y); al[2] = __expf(l4.z); al[3] = __expf(l4.w);
+        al[0] = exp_ftz(l4.x); al[1] = exp_ftz(l4.y); al[2] = exp_ftz(l4.z); al[3] = exp_ftz(l4.w);
         gamma = *row_f32(p.gam, ch, 0);
     }
     dec_bf4(row_bf16(p.u, ch, 0), c0, r, FULL || (p.u.vec && v4r), u);

@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
             float E = i ? s_A[(i - 1) * LDP + c] : 0.f;
             if (any_reset) E -= ch.eoff(i);   // block-uniform branch
             const float uh = s_B[i * LDP + c];
-            ut[k] = uh * __expf(E - s_gp[I * DP + c]);
-            un[k] = uh * __expf(s_ge[I * DP + c] - G);
+            ut[k] = uh * exp_ftz(E - s_gp[I * DP + c]);
+            un[k] = uh * exp_ftz(s_ge[I * DP + c] - G);
         }
         __syncthreads();
 #pragma unroll
@@ -232,8 +232,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
             const float4 ge = *reinterpret_cast<const float4*>(s_ge + I * DP + c4);
             const float4 gl = *reinterpret_cast<const float4*>(GL + c4);
             *reinterpret_cast<float4*>(gUbar + i * DP + c4) =
-                make_float4(round_tf32(un.x * __expf(gl.x - ge.x)), round_tf32(un.y * __expf(gl.y - ge.y)),
-                            round_tf32(un.z * __expf(gl.z - ge.z)), round_tf32(un.w * __expf(gl.w - ge.w)));
+                make_float4(round_tf32(un.x * exp_ftz(gl.x - ge.x)), round_tf32(un.y * exp_ftz(gl.y - ge.y)),
+                            round_tf32(un.z * exp_ftz(gl.z - ge.z)), round_tf32(un.w * exp_ftz(gl.w - ge.w)));
         }
     }
     __syncthreads();
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 h[e] *= gm;
-                ut[e] *= gm * __expf(gp[e]);
+                ut[e] *= gm * exp_ftz(gp[e]);
             }
             store8_smem(s_B, i, c0, h);
             store8_smem(s_A, i, c0, ut);
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
         *reinterpret_cast<float4*>(gQc + i * DP + c4) =
             make_float4(round_tf32(-w.x), round_tf32(-w.y), round_tf32(-w.z), round_tf32(-w.w));
     }
-    if (threadIdx.x < DP) p.Lam[ch.gi * DP + threadIdx.x] = __expf(s_ge[(NBLK - 1) * DP + threadIdx.x]);
+    if (threadIdx.x < DP) p.Lam[ch.gi * DP + threadIdx.x] = exp_ftz(s_ge[(NBLK - 1) * DP + threadIdx.x]);
     SD_PHASE(p.g, ph);
 }
 
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
         const int c = threadIdx.x & (DP - 1), i0 = (threadIdx.x >> 7) * BT;
         const float Gend = s_G[(i0 + BT - 1) * LDP + c];
 #pragma unroll
-        for (int k = 0; k < BT; ++k) s_un[(i0 + k) * LDP + c] *= __expf(Gend - s_G[(i0 + k) * LDP + c]);
+        for (int k = 0; k < BT; ++k) s_un[(i0 + k) * LDP + c] *= exp_ftz(Gend - s_G[(i0 + k) * LDP + c]);
     }
     cp_wait<0>();
     __syncthreads();
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
         float2 Gp = make_float2(0.f, 0.f), dg = make_float2(0.f, 0.f);
         if (ref >= 0) Gp = *reinterpret_cast<const float2*>(s_G + ref * LDP + j);
         if (!fast) dg = *reinterpret_cast<const float2*>(s_dl + i * LDP + j);
-        const float2 act = make_float2(__expf(G.x - Gp.x) * v0 + dg.x, __expf(G.y - Gp.y) * v1 + dg.y);
+        const float2 act = make_float2(exp_ftz(G.x - Gp.x) * v0 + dg.x, exp_ftz(G.y - Gp.y) * v1 + dg.y);
         const float2 d = make_float2(kh.x + act.x, kh.y + act.y);
         if (keep) *reinterpret_cast<float2*>(gd + i * DP + j) = d;
         *reinterpret_cast<float2*>(s_kh + i * LDP + j) = PRED ? act : d;
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
                 load8_smem(s_G, i, c0, Gi);
                 load8_smem(s_G, i0 + BT - 1, c0, Ge);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) uh[e] *= __expf(Gi[e] - Ge[e]);
+                for (int e = 0; e < 8; ++e) uh[e] *= exp_ftz(Gi[e] - Ge[e]);
                 load8_smem(s_dl, i, c0, dl);
             } else {
                 load8_norm<FAST>(p.u, ch, i, c0, r, uh);
@@ -485,12 +485,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
             float a[2][8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const float ep = __expf(G[e]), rw = __expf(G[e] - Gp[e]);
+                const float ep = exp_ftz(G[e]), rw = exp_ftz(G[e] - Gp[e]);
                 xg[e] = src.chi[e] * ep;
                 ag[e] = -src.e[e] * ep;
                 xr[e] = src.chi[e] * rw;
                 ern[e] = -src.e[e] * rw;
-                dt[e] = d[e] * __expf(GL[e] - G[e]);
+                dt[e] = d[e] * exp_ftz(GL[e] - G[e]);
                 z[e] = sigmoidf_(wr[e]) * v[e];
                 a[0][e] = src.chi[e];
                 a[1][e] = -src.e[e];
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
                 float Ge[8], dc[8];
                 load8_smem(s_G, i0 + BT - 1, c0, Ge);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) dc[e] = d[e] * __expf(Ge[e] - G[e]);
+                for (int e = 0; e < 8; ++e) dc[e] = d[e] * exp_ftz(Ge[e] - G[e]);
                 store8_smem(s_d, i, c0, dc);
                 if (keep) store8_bpanel(bpanel_ptr(p.Dcol, ch.gi), i, c0, dc);
             } else if (keep) {
@@ -543,8 +543,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
             float4 d = *reinterpret_cast<const float4*>(s_d + j * LDP + c4);
             const float4 G = *reinterpret_cast<const float4*>(s_G + j * LDP + c4);
             const float4 Ge = *reinterpret_cast<const float4*>(s_G + (j | (BT - 1)) * LDP + c4);
-            d.x *= __expf(Ge.x - G.x); d.y *= __expf(Ge.y - G.y);
-            d.z *= __expf(Ge.z - G.z); d.w *= __expf(Ge.w - G.w);
+            d.x *= exp_ftz(Ge.x - G.x); d.y *= exp_ftz(Ge.y - G.y);
+            d.z *= exp_ftz(Ge.z - G.z); d.w *= exp_ftz(Ge.w - G.w);
             *reinterpret_cast<float4*>(s_d + j * LDP + c4) = d;
             if (keep) {
                 bf16* gDc = bpanel_ptr(p.Dcol, ch.gi) + j * DP + c4;

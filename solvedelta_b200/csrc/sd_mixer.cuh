@@ -34,10 +34,10 @@ struct ConvParams {
     const unsigned char* reset;
 };
 
-// the fast reciprocal (2 ulp) instead of an IEEE division: these kernels are bound by instruction issue
-__device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+// the hardware reciprocal instead of an IEEE division: these kernels are bound by instruction issue
+__device__ __forceinline__ float silu_f(float z) { return z * rcp_ftz(1.f + exp_ftz(-z)); }
 __device__ __forceinline__ float silu_grad_f(float z) {
-    const float s = __fdividef(1.f, 1.f + __expf(-z));
+    const float s = rcp_ftz(1.f + exp_ftz(-z));
     return s * (1.f + z * (1.f - s));
 }
 
@@ -488,15 +488,15 @@ struct GateParams {
 // logarithm lies in (1, 2], where its absolute error (about 4e-7) is below half an ulp of the BF16 input's own
 // spacing by four orders of magnitude; below exp(-|z|) = 1e-3 two series terms replace it (relative error 3e-7).
 __device__ __forceinline__ float softplus_fast(float z) {
-    const float en = __expf(-fabsf(z));
+    const float en = exp_ftz(-fabsf(z));
     return fmaxf(z, 0.f) + (en < 1e-3f ? en * (1.f - 0.5f * en) : __logf(1.f + en));
 }
 // sigmoid(z) and softplus(z) from one exponential, en = exp(-|z|) in (0, 1]:
 // softplus = max(z, 0) + log1p(en) (two series terms below 1e-3, where log(1 + en) would lose its digits).
 // The reverse kernels use it: softplus only enters the sum for the rate gradient there.
 __device__ __forceinline__ void sigmoid_softplus(float z, float& sig, float& sp) {
-    const float en = __expf(-fabsf(z));
-    const float inv = __fdividef(1.f, 1.f + en);
+    const float en = exp_ftz(-fabsf(z));
+    const float inv = rcp_ftz(1.f + en);
     sig = z >= 0.f ? inv : en * inv;
     sp = fmaxf(z, 0.f) + (en < 1e-3f ? en * (1.f - 0.5f * en) : __logf(1.f + en));
 }
@@ -508,7 +508,7 @@ __global__ void k_kda_gate_fwd(GateParams p) {
         const int hc = (int)(i % (p.H * p.r));
         const int h = hc / p.r;
         const float z = __bfloat162float(p.raw[i]) + p.bias[hc];
-        p.out[i] = -__expf(p.A[h]) * softplus_fast(z);
+        p.out[i] = -exp_ftz(p.A[h]) * softplus_fast(z);
     }
 }
 
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(256) k_kda_gate_fwd_v8(GateParams p) {
          i8 += (long long)gridDim.x * blockDim.x) {
         const long long i = i8 * 8;
         const int hc = (int)(i % HR);
-        const float rate = -__expf(p.A[hc / p.r]);   // r % 8 == 0: the eight share a head
+        const float rate = -exp_ftz(p.A[hc / p.r]);   // r % 8 == 0: the eight share a head
         const uint4 raw = *reinterpret_cast<const uint4*>(p.raw + i);
         const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
         const float4 b0 = *reinterpret_cast<const float4*>(p.bias + hc);
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(256) k_kda_gate_bwd(GateParams p) {
     const int hc = blockIdx.y * 256 + threadIdx.x, HR = p.H * p.r;
     if (hc >= HR) return;
     const int h = hc / p.r;
-    const float rate = -__expf(p.A[h]), bias = p.bias[hc];
+    const float rate = -exp_ftz(p.A[h]), bias = p.bias[hc];
     const long long n0 = (long long)blockIdx.x * p.rows_per_block;
     const long long n1 = (n0 + p.rows_per_block < p.N) ? n0 + p.rows_per_block : p.N;
     float sum_b = 0.f, sum_a = 0.f;
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(256) k_kda_gate_bwd_v8(GateParams p, int cgb) 
 #pragma unroll
     for (int e = 0; e < 8; ++e) sb[e] = sa[e] = 0.f;
     if (live) {
-        const float rate = -__expf(p.A[hc / p.r]);
+        const float rate = -exp_ftz(p.A[hc / p.r]);
         const float4 b0 = *reinterpret_cast<const float4*>(p.bias + hc);
         const float4 b1 = *reinterpret_cast<const float4*>(p.bias + hc + 4);
         const float bias[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
@@ -1178,12 +1178,12 @@ __global__ void __launch_bounds__(256) k_cross_entropy_fwd(CrossEntropyParams p)
         float add = 0.f;
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            if (c0 + e < p.V) add += __expf(v[e] - gm);
-        sum = sum * __expf(mx - gm) + add;   // exp(-inf - finite) = 0 on the first group
+            if (c0 + e < p.V) add += exp_ftz(v[e] - gm);
+        sum = sum * exp_ftz(mx - gm) + add;   // exp(-inf - finite) = 0 on the first group
         mx = gm;
     }
     const float top = ce_block_reduce(mx, true, red);
-    const float total = ce_block_reduce(mx == -INFINITY ? 0.f : sum * __expf(mx - top), false, red);
+    const float total = ce_block_reduce(mx == -INFINITY ? 0.f : sum * exp_ftz(mx - top), false, red);
     if (threadIdx.x == 0) {
         const float lse = top + __logf(total);
         p.lse[row] = lse;
@@ -1203,7 +1203,7 @@ __global__ void __launch_bounds__(256) k_cross_entropy_bwd(CrossEntropyParams p)
         float v[8], g[8];
         norm_load8(x, c0, p.V, true, v);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) g[e] = live ? (__expf(v[e] - lse) - (c0 + e == label ? 1.f : 0.f)) * coef : 0.f;
+        for (int e = 0; e < 8; ++e) g[e] = live ? (exp_ftz(v[e] - lse) - (c0 + e == label ? 1.f : 0.f)) * coef : 0.f;
         norm_store8(d, c0, p.V, true, g);
     }
 }
