@@ -1052,7 +1052,14 @@ int sd_forward_static(const sd_forward_args* a, void* stream_) {
 // Mixer glue
 namespace {
 int conv_tiles(int T) { return (T + CONV_TT - 1) / CONV_TT; }
-constexpr int GATE_ROWS_PER_BLOCK = 64;
+// Rows of a CTA of the gate's reverse kernel.  A thread walks its rows one load latency after the other, so they are
+// halved while the CTAs do not reach every SM (1024 x 1024: 34 to 9 us).  More CTAs than that only add partial sums: at
+// 16384 rows the kernel took 42 instead of 44 us and the sums 4 us more.
+int gate_rows_per_block(int64_t rows) {
+    int n = 64;
+    while (n > 8 && rows / n < 148) n /= 2;
+    return n;
+}
 constexpr int NORM_ROWS_PER_BLOCK = 256;
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 }  // namespace
@@ -1130,7 +1137,8 @@ int sd_conv4_silu_backward_pitched(const sd_conv4_backward_args* a, int64_t dx_p
 
 size_t sd_kda_gate_backward_scratch_bytes(int64_t rows, int32_t H, int32_t r) {
     if (rows <= 0 || H <= 0 || r <= 0) return 0;
-    const size_t blocks = size_t((rows + GATE_ROWS_PER_BLOCK - 1) / GATE_ROWS_PER_BLOCK);
+    const int per_block = gate_rows_per_block(rows);
+    const size_t blocks = size_t((rows + per_block - 1) / per_block);
     return align256((2 * blocks + 1) * size_t(H) * r * sizeof(float));
 }
 
@@ -1160,7 +1168,7 @@ int sd_kda_gate_backward(const sd_kda_gate_args* a, void* stream_) {
     const int HR = a->H * a->r;
     if (a->scratch_bytes < sd_kda_gate_backward_scratch_bytes(a->rows, a->H, a->r)) return SD_ERR_BUFFER_TOO_SMALL;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    const int blocks = (int)((a->rows + GATE_ROWS_PER_BLOCK - 1) / GATE_ROWS_PER_BLOCK);
+    const int per_block = gate_rows_per_block(a->rows), blocks = (int)((a->rows + per_block - 1) / per_block);
     GateParams p{};
     p.N = a->rows; p.H = a->H; p.r = a->r;
     p.raw = reinterpret_cast<const __nv_bfloat16*>(a->raw);
@@ -1169,7 +1177,7 @@ int sd_kda_gate_backward(const sd_kda_gate_args* a, void* stream_) {
     p.dbias_part = reinterpret_cast<float*>(a->scratch);
     p.dA_part = p.dbias_part + (size_t)blocks * HR;
     float* dA_cols = p.dA_part + (size_t)blocks * HR;
-    p.rows_per_block = GATE_ROWS_PER_BLOCK;
+    p.rows_per_block = per_block;
     const bool vec = (a->r & 7) == 0 &&
                      ((reinterpret_cast<uintptr_t>(a->raw) | reinterpret_cast<uintptr_t>(a->bias) |
                        reinterpret_cast<uintptr_t>(a->dlog_decay) | reinterpret_cast<uintptr_t>(a->draw)) & 15) == 0;
@@ -1187,9 +1195,15 @@ int sd_kda_gate_backward(const sd_kda_gate_args* a, void* stream_) {
     return launch_status();
 }
 
+// rows of a CTA when they make less than one wave of three CTAs an SM: whole steps of 16, at least two
+static int64_t norm_rows_few(int64_t rows) {
+    const int64_t n = (rows + 148 * 3 - 1) / (148 * 3);
+    return n > NORM_ROWS_PER_BLOCK ? NORM_ROWS_PER_BLOCK : n < 32 ? 32 : (n + 15) / 16 * 16;
+}
 size_t sd_norm_gate_backward_scratch_bytes(int64_t rows, int32_t V) {
     if (rows <= 0 || V <= 0) return 0;
-    const size_t blocks = size_t((rows + NORM_ROWS_PER_BLOCK - 1) / NORM_ROWS_PER_BLOCK);
+    const size_t blocks = std::max(size_t((rows + NORM_ROWS_PER_BLOCK - 1) / NORM_ROWS_PER_BLOCK),
+                                   size_t((rows + norm_rows_few(rows) - 1) / norm_rows_few(rows)));
     return align256(blocks * size_t(V) * sizeof(float));
 }
 
@@ -1216,14 +1230,15 @@ int sd_norm_gate_backward(const sd_norm_gate_args* a, void* stream_) {
     if (a->V > DP) return SD_ERR_UNSUPPORTED_SHAPE;
     if (a->scratch_bytes < sd_norm_gate_backward_scratch_bytes(a->rows, a->V)) return SD_ERR_BUFFER_TOO_SMALL;
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-    // rows per CTA: at least NORM_ROWS_PER_BLOCK (the scratch is sized for that), stretched so that the grid is a
-    // whole number of waves of resident CTAs
+    // rows per CTA: NORM_ROWS_PER_BLOCK or more, stretched so that the grid is a whole number of waves of resident CTAs;
+    // fewer when they would not fill one wave (the scratch is sized for both)
     long long rpb = NORM_ROWS_PER_BLOCK;
     {
         const long long wave = resident_ctas(k_norm_gate_bwd, 256, 0);
         const long long waves = a->rows / (wave * NORM_ROWS_PER_BLOCK);
         if (waves >= 1) rpb = ((a->rows + wave * waves - 1) / (wave * waves) + 15) / 16 * 16;
         if (rpb < NORM_ROWS_PER_BLOCK) rpb = NORM_ROWS_PER_BLOCK;
+        if (waves < 1) rpb = norm_rows_few(a->rows);
     }
     const int blocks = (int)((a->rows + rpb - 1) / rpb);
     NormParams p{};
