@@ -18,7 +18,7 @@ _SRC = os.path.join(_PKG, "csrc")
 _BUILD = os.path.join(_PKG, "_build")
 LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200.so")
 # the profiling build: same sources with -DSD_DIAGNOSTICS (phase clock stamps, per-launch events);
-# only bench.py's per-kernel breakdown loads it
+# loaded by bench.py's per-kernel breakdown and the tests of the elementary functions
 DIAG_LIB_PATH = os.path.join(_BUILD, "libsolvedelta_b200_diag.so")
 # the host side of the entry points (checks, tensors, autograd node) as a Python extension over the C ABI
 HOST_PATH = os.path.join(_BUILD, "sd_host.so")
@@ -306,6 +306,9 @@ def load_diagnostics() -> ctypes.CDLL:
         _diag.sd_profile_step.argtypes = [ctypes.POINTER(ForwardArgs), ctypes.POINTER(BackwardArgs),
                                           ctypes.c_void_p, ctypes.POINTER(ctypes.c_float), ctypes.c_int,
                                           ctypes.POINTER(ctypes.c_int)]
+        _diag.sd_debug_elementwise.restype = ctypes.c_int
+        _diag.sd_debug_elementwise.argtypes = [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong,
+                                               ctypes.c_void_p]
         _diag.sd_launch_name.restype = ctypes.c_char_p
         _diag.sd_launch_name.argtypes = [ctypes.c_int]
     return _diag

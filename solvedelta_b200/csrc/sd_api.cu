@@ -964,6 +964,15 @@ int sd_predictor_backward(const sd_predictor_backward_args* a, void* stream_) {
 #ifdef SD_DIAGNOSTICS
 void sd_debug_timeline(void* device_buffer) { g_dbg = reinterpret_cast<long long*>(device_buffer); }
 
+static __global__ void k_debug_elementwise(int function, const float* x, float* y, long long count) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
+        y[i] = function == 0 ? exp_ftz(x[i]) : rcp_ftz(x[i]);
+}
+int sd_debug_elementwise(int function, const float* x, float* y, long long count, void* stream_) {
+    if (function < 0 || function > 1 || !x || !y || count < 1) return SD_ERR_INVALID_ARGUMENT;
+    k_debug_elementwise<<<256, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(function, x, y, count);
+    return launch_status();
+}
 #endif
 
 int sd_device_fault(void) {

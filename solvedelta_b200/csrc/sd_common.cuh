@@ -143,10 +143,12 @@ __device__ __forceinline__ const float* state_ptr(const float* base, long long g
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// 1 / (1 + exp(-x)) with the fast reciprocal (2 ulp): exp(-x) = inf gives exactly 0.
-// exp and 1/x on the hardware's base-2 exponential and reciprocal, subnormals flushed: two instructions and one, where
-// the forms that keep subnormals scale their argument and result (about five each).  Arguments here are sums of a one
-// and an exponential, or factors that multiply numbers of order one: below 1e-38 nothing of them is left in a result.
+// exp(x) = 2^(x log2 e), and 1/x, on PTX's ex2.approx.ftz and rcp.approx.ftz; subnormal arguments and results are zero.
+// Arguments here are sums of a one and an exponential, or factors that multiply numbers of order one: below 1e-38
+// nothing of them is left in a result.  Relative errors, held by test_gpu_elementwise.py: the rounded product and its
+// rounded constant give exp 1.5 |x| 2^-24 beside the 2^-22 of the instruction; the reciprocal has 2^-23.
+// The chunk and conv kernels are short of issue slots: forward + reverse at 8 x 4096 tokens 3740 -> 3690 us against
+// CUDA's intrinsics, conv forward 103 -> 97 us.
 __device__ __forceinline__ float exp_ftz(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
@@ -157,6 +159,7 @@ __device__ __forceinline__ float rcp_ftz(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// 1 / (1 + exp(-x)): exp(-x) = inf gives exactly 0
 __device__ __forceinline__ float sigmoidf_(float x) { return rcp_ftz(1.0f + exp_ftz(-x)); }
 
 // ---- half-warp (16 lanes = one token row) reductions ---------------------

@@ -27,6 +27,11 @@ const char *sd_launch_name(int index);
  * NULL switches the recording off.  Process-wide, not thread safe.
  */
 void sd_debug_timeline(void *device_buffer);
+/*
+ * y[i] = f(x[i]) for the elementary functions that the kernels are built from, on `count`
+ * device floats: 0 exp_ftz, 1 rcp_ftz.  For tests of their error bounds.
+ */
+int sd_debug_elementwise(int function, const float *x, float *y, long long count, void *stream);
 
 #ifdef __cplusplus
 }
