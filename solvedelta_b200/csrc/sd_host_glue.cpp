@@ -1010,8 +1010,20 @@ struct TokenStack {
             y_max = std::max(y_max, (size_t)(H * V));
             act_max = std::max(act_max, (size_t)(l.up_weight.size(0) / 2));
         }
+        const bool fuse_norm = B <= 16;
+        if (!fuse_norm && (D % 256 != 0)) return std::nullopt;   // the norm alone takes whole groups of 256 channels
         const c10::cuda::CUDAGuard guard(x.device());
         void* stream = stream_of(x);
+        // All FP32 copies are taken here, ahead of the first launch: one that is missing or out of date is a conversion
+        // kernel, and a chained launch reads its parameters while the kernel directly before it still runs.
+        struct Parameters { const float *mixer_norm, *conv, *log_rate, *decay_bias, *geometry_bias, *out_norm, *mlp_norm; };
+        std::vector<Parameters> fp32;
+        fp32.reserve(layers.size());
+        for (TokenLayer& l : layers)   // braces: in this order
+            fp32.push_back(Parameters{f32(l.copies.get(0, l.mixer_norm)), f32(l.copies.get(1, l.conv_weight)), f32(l.copies.get(2, l.log_rate)),
+                                      f32(l.copies.get(3, l.decay_bias)), f32(l.copies.get(4, l.geometry_bias)),
+                                      f32(l.copies.get(5, l.out_norm)), f32(l.copies.get(6, l.mlp_norm))});
+        const float* const last_norm = f32(copies.get(0, norm));
         const auto piece = [&](size_t width) { return (width * (size_t)B * 2 + 255) & ~size_t(255); };
         const size_t row_b = piece(row_max), y_b = piece(y_max), act_b = piece(act_max), d_b = piece((size_t)D);
         const Tensor work = workspace(x, row_b + y_b + act_b + 5 * d_b);
@@ -1022,7 +1034,6 @@ struct TokenStack {
         const void* residual = x.data_ptr();
         const void* delta = nullptr;
         bool chained = false;   // nothing of this call is in flight: the first launch follows the stream in full
-        const bool fuse_norm = B <= 16;
         const auto linear = [&](const void* in, int64_t K, const Tensor& weight, const void* bias, void* out, bool with_swiglu,
                                 const float* norm_w, double eps) {
             if (B > 16 && !with_swiglu && weight.size(0) >= 16 * 148) {
@@ -1074,12 +1085,12 @@ struct TokenStack {
                 linear(normed, D, weight, bias, out, with_swiglu, nullptr, 0);
             }
         };
-        if (!fuse_norm && (D % 256 != 0)) return std::nullopt;   // the norm alone takes whole groups of 256 channels
         for (size_t i = 0; i < layers.size(); ++i) {
-            TokenLayer& l = layers[i];
+            const TokenLayer& l = layers[i];
+            const Parameters& w = fp32[i];
             State& st = state[i];
             const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0);
-            norm_linear(f32(l.copies.get(0, l.mixer_norm)), l.mixer_eps, l.in_weight, raw(l.in_bias), row, false);
+            norm_linear(w.mixer_norm, l.mixer_eps, l.in_weight, raw(l.in_bias), row, false);
             sd_mixer_decode_args a{};
             a.shape = sd_shape{(int32_t)B, 1, (int32_t)H, (int32_t)r, (int32_t)V};
             const auto at_col = [&](int64_t c) { return row + 2 * c; };
@@ -1089,11 +1100,11 @@ struct TokenStack {
             a.erase_raw = sd_operand{at_col(qkv + 2 * H * r), P, P, r};
             a.write_raw = sd_operand{at_col(qkv + 3 * H * r), P, P, V};
             a.qkv = row; a.qkv_stride_b = P;
-            a.conv_weight = f32(l.copies.get(1, l.conv_weight)); a.conv_state = st.conv.data_ptr();
-            a.log_rate = f32(l.copies.get(2, l.log_rate)); a.decay_bias = f32(l.copies.get(3, l.decay_bias));
-            a.geometry_raw = at_col(geom); a.geometry_stride_b = P; a.geometry_bias = f32(l.copies.get(4, l.geometry_bias));
+            a.conv_weight = w.conv; a.conv_state = st.conv.data_ptr();
+            a.log_rate = w.log_rate; a.decay_bias = w.decay_bias;
+            a.geometry_raw = at_col(geom); a.geometry_stride_b = P; a.geometry_bias = w.geometry_bias;
             a.C = f32(st.C); a.S = f32(st.S); a.y = y;
-            a.norm_weight = f32(l.copies.get(5, l.out_norm)); a.norm_eps = (float)l.out_eps;
+            a.norm_weight = w.out_norm; a.norm_eps = (float)l.out_eps;
             a.gate_rank = (int32_t)V;
             a.decay_hidden = at_col(geom + H); a.decay_hidden_stride_b = P;
             a.gate_hidden = at_col(geom + H + V); a.gate_hidden_stride_b = P;
@@ -1102,16 +1113,15 @@ struct TokenStack {
             check(sd_mixer_decode_step_chained(&a, stream));
             linear(y, H * V, l.out_weight, raw(l.out_bias), mixed, false, nullptr, 0);
             delta = mixed;
-            norm_linear(f32(l.copies.get(6, l.mlp_norm)), l.mlp_eps, l.up_weight, nullptr, act, true);
+            norm_linear(w.mlp_norm, l.mlp_eps, l.up_weight, nullptr, act, true);
             linear(act, l.up_weight.size(0) / 2, l.down_weight, nullptr, mlp, false, nullptr, 0);
             delta = mlp;
         }
-        const Tensor norm_w = copies.get(0, norm);
         Tensor out = bf16_like(x, {B, 1, head.has_value() ? head->size(0) : D});
         if (head.has_value())
-            norm_linear(f32(norm_w), norm_eps, *head, nullptr, out.data_ptr(), false);
+            norm_linear(last_norm, norm_eps, *head, nullptr, out.data_ptr(), false);
         else
-            norm_rows(f32(norm_w), norm_eps, out.data_ptr());
+            norm_rows(last_norm, norm_eps, out.data_ptr());
         return out;
     }
 

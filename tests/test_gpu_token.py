@@ -1,9 +1,11 @@
 """The projections of a cached token at the edges of their tiles, and the native token stack against the module path."""
+import copy
 import ctypes
 
 import pytest
 import torch
 import torch.nn.functional as F
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from solvedelta_b200 import SolveDeltaConfig, SolveDeltaForCausalLM, _lib
 from tests.helpers import rel_l2
@@ -81,3 +83,41 @@ def test_prompt_through_the_stack_equals_the_module_path(B, T):
             handle.remove()
     for got, want in zip(*seen):
         assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
+
+
+class _Dispatched(TorchDispatchMode):
+    """The torch calls made below the Python layer, in order: name and result type."""
+
+    def __init__(self):
+        super().__init__()
+        self.calls = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        out = func(*args, **(kwargs or {}))
+        self.calls.append((func.overloadpacket.__name__, getattr(out, "dtype", None)))
+        return out
+
+
+@pytest.mark.parametrize("B", [1, 20])
+def test_parameter_copies_precede_the_launches(B):
+    """A chained launch reads its FP32 parameters while the kernel before it runs, so the copies that a parameter update
+    has put out of date are all made ahead of the first launch (and with it of the workspace); the step then sees the
+    new values."""
+    torch.manual_seed(6)
+    model = SolveDeltaForCausalLM(SolveDeltaConfig(hidden_size=256, num_heads=4, head_k_dim=64, head_v_dim=64,
+                                                   num_hidden_layers=2, vocab_size=320)).prepare("cuda").eval()
+    ids = torch.randint(0, 320, (B, 41), device="cuda")
+    with torch.no_grad():
+        cache = model(input_ids=ids[:, :40], use_cache=True).past_key_values
+        same = copy.deepcopy(cache)
+        for name, p in model.named_parameters():
+            if "norm" in name or "conv_weight" in name:
+                p.add_(0.25 * torch.randn_like(p))
+        with _Dispatched() as log:
+            got = model(input_ids=ids[:, 40:], past_key_values=cache, use_cache=True).logits
+        model.model.layers[1].mlp.register_forward_hook(lambda *a: None)   # the module path
+        want = model(input_ids=ids[:, 40:], past_key_values=same, use_cache=True).logits
+    copies = [i for i, call in enumerate(log.calls) if call == ("_to_copy", torch.float32)]
+    workspace = [i for i, call in enumerate(log.calls) if call == ("empty", torch.uint8)]
+    assert len(copies) == 4 * 2 + 1 and len(workspace) == 1 and max(copies) < workspace[0]
+    assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
