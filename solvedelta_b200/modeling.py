@@ -17,6 +17,7 @@ from typing import Any, Dict, List, Optional, Sequence, Tuple, Union
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.nn.modules import module as module_globals
 from transformers import PreTrainedModel
 from transformers.generation import GenerationMixin
 from transformers.modeling_outputs import BaseModelOutputWithPast, CausalLMOutputWithPast
@@ -24,7 +25,7 @@ from transformers.modeling_outputs import BaseModelOutputWithPast, CausalLMOutpu
 from . import _lib
 from .config import SolveDeltaConfig
 from .ops import SolveDeltaState
-from .mixer_ops import add_rmsnorm, add_rmsnorm_reverse_supported, gated_mlp
+from .mixer_ops import add_rmsnorm, add_rmsnorm_reverse_supported, gated_mlp, swiglu
 from .model import SolveDelta, SolveDeltaLayerState
 from .token_stack import token_stack
 
@@ -107,6 +108,14 @@ def segment_reset_mask(hidden_states: torch.Tensor, cu_seqlens: torch.Tensor) ->
     return mask.unsqueeze(0)
 
 
+def _bare_linear(layer: nn.Module) -> bool:
+    """A plain ``nn.Linear`` whose call does nothing beside its product: no hook, adapter, parametrisation or replaced
+    ``forward``, so that its weight may be used in its place."""
+    return (type(layer) is nn.Linear and "forward" not in layer.__dict__
+            and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks
+                     or layer._backward_pre_hooks or module_globals._has_any_global_hook()))
+
+
 class SolveDeltaMLP(nn.Module):
     """Gated MLP with one common-input gate/up projection (modeling_solvedelta.py:31-101)."""
 
@@ -130,10 +139,14 @@ class SolveDeltaMLP(nn.Module):
         self.down_proj = nn.Linear(intermediate_size, hidden_size, bias=False)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if self.hidden_act == "swish" and x.is_cuda and x.dtype == torch.bfloat16:
-            up, down = self.gate_up_proj, self.down_proj
+        up, down = self.gate_up_proj, self.down_proj
+        kernels = self.hidden_act == "swish" and x.is_cuda and x.dtype == torch.bfloat16
+        if kernels and _bare_linear(up) and _bare_linear(down):
             return gated_mlp(x, up.weight, up.bias, down.weight, down.bias)
-        gate, value = self.gate_up_proj(x).chunk(2, dim=-1)
+        gate_value = up(x)
+        if kernels and gate_value.dtype == torch.bfloat16:
+            return down(swiglu(gate_value))   # activation and product in one kernel
+        gate, value = gate_value.chunk(2, dim=-1)
         if self.hidden_act == "swish":
             activated = F.silu(gate)
         else:
@@ -142,7 +155,7 @@ class SolveDeltaMLP(nn.Module):
             safe = torch.where(positive, gate, torch.ones_like(gate))
             exponent = self.powglu_power / (torch.sqrt(safe) + 1.0)
             activated = torch.where(positive, torch.exp(exponent * torch.log(safe)) * sigmoid, gate * sigmoid)
-        return self.down_proj(activated * value)
+        return down(activated * value)
 
 
 class SolveDeltaCacheAdapter(nn.Module):

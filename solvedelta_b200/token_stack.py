@@ -1,10 +1,12 @@
 """One cached token, or a prompt, through a model's blocks in one native call.
 
 A single-token step of a generation loop is a chain of short launches, so per-layer module
-calls cost more than the kernels behind them; so does a prompt of up to a few thousand tokens.  :func:`token_stack` gives the native stack of a
-``SolveDeltaModel`` (csrc/sd_host_glue.cpp): it holds the model's own parameter tensors and is
-rebuilt when a module, a parameter object or an epsilon has been replaced; a hook or a replaced
-``forward`` anywhere in the blocks turns it off, so that the module path, which calls them, runs.
+calls cost more than the kernels behind them; so does a prompt of up to a few thousand tokens.
+:func:`token_stack` gives the native stack of a ``SolveDeltaModel`` (csrc/sd_host_glue.cpp): it
+holds the model's own parameter tensors and is rebuilt when a module, a parameter object or an
+epsilon has been replaced; a hook or a replaced ``forward`` anywhere in the blocks turns it off,
+and the module path runs.  That path calls the blocks, the mixers, the MLPs and an MLP's two
+projections as modules; the norms and a mixer's own projections it uses through their weights.
 """
 from __future__ import annotations
 
