@@ -688,6 +688,9 @@ struct MixerFunction : torch::autograd::Function<MixerFunction> {
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         variable_list result(19);
         if (!grads[0].defined()) return result;
+        // first-order gradients only, also under create_graph=True: the kernels have no second derivative, and products
+        // into columns of a tensor are refused while gradients are recorded
+        const at::NoGradGuard no_grad;
         const variable_list sv = ctx->get_saved_variables();
         auto& data = ctx->saved_data;
         const Tensor &x = sv[0], &in_weight = sv[1], &decay_weight = sv[2], &gate_weight = sv[3], &out_weight = sv[4], &row = sv[5];
