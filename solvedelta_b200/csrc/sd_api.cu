@@ -966,10 +966,10 @@ void sd_debug_timeline(void* device_buffer) { g_dbg = reinterpret_cast<long long
 
 static __global__ void k_debug_elementwise(int function, const float* x, float* y, long long count) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
-        y[i] = function == 0 ? exp_ftz(x[i]) : rcp_ftz(x[i]);
+        y[i] = function == 0 ? exp_ftz(x[i]) : function == 1 ? rcp_ftz(x[i]) : __uint_as_float(mma_tf32_bits(x[i]) & 0xffffe000u);
 }
 int sd_debug_elementwise(int function, const float* x, float* y, long long count, void* stream_) {
-    if (function < 0 || function > 1 || !x || !y || count < 1) return SD_ERR_INVALID_ARGUMENT;
+    if (function < 0 || function > 2 || !x || !y || count < 1) return SD_ERR_INVALID_ARGUMENT;
     k_debug_elementwise<<<256, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(function, x, y, count);
     return launch_status();
 }

@@ -29,7 +29,8 @@ const char *sd_launch_name(int index);
 void sd_debug_timeline(void *device_buffer);
 /*
  * y[i] = f(x[i]) for the elementary functions that the kernels are built from, on `count`
- * device floats: 0 exp_ftz, 1 rcp_ftz.  For tests of their error bounds.
+ * device floats: 0 exp_ftz, 1 rcp_ftz, 2 the TF32 number that mma.sync
+ * makes of mma_tf32_bits.  For tests of their error bounds.
  */
 int sd_debug_elementwise(int function, const float *x, float *y, long long count, void *stream);
 

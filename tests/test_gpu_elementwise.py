@@ -39,3 +39,19 @@ def test_reciprocal():
     assert ((_apply(1, x).double() - want).abs() <= want.abs() * 2.0 ** -23).all()
     edges = _apply(1, torch.tensor([INF, -INF, 0.0, TINY / 2, 2.0 ** 127, NAN]))
     assert edges[:2].tolist() == [0.0, 0.0] and edges[2:4].tolist() == [INF, INF] and edges[4] == 0.0 and edges[5].isnan()
+
+
+def test_tf32_operand_rounding():
+    """To the nearest of ten fraction bits, ties away from zero, as the conversion instruction does it; infinities and the
+    NaN that arithmetic returns (0x7fffffff) stay what they are."""
+    gen = torch.Generator().manual_seed(3)
+    bits = torch.cat([torch.randint(0, 0x7f800000, (400000,), generator=gen), torch.arange(0x3f800000, 0x3f804000)])
+    bits = bits.to(torch.int32)
+    x = torch.cat([bits, bits | torch.tensor(-2 ** 31, dtype=torch.int32)]).view(torch.float32)
+    fraction = torch.frexp(x.double())
+    want = torch.ldexp(torch.sign(x.double()) * (fraction.mantissa.abs() * 2048 + 0.5).floor(), fraction.exponent - 11)
+    normal = x.abs() >= TINY   # below it the spacing is fixed, not ten bits
+    assert torch.equal(_apply(2, x).double()[normal], want.float().double()[normal])
+    assert _apply(2, torch.tensor([INF, -INF])).tolist() == [INF, -INF]
+    nans = torch.tensor([0x7fffffff, 0x7fc00000, -0x400000, 0x7fbfffff, 0x7f802000], dtype=torch.int32).view(torch.float32)
+    assert _apply(2, nans).isnan().all()
