@@ -4,6 +4,9 @@
 // seven launches of a cached token, several times the device time of short sequences.
 #include "sd_host.h"
 
+#include <c10/core/Event.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+
 namespace {
 
 Tensor bf16_contiguous(const Tensor& t) { return t.to(at::kBFloat16).contiguous(); }
@@ -21,22 +24,44 @@ bool records_gradients(std::initializer_list<const Tensor*> tensors) {
     return false;
 }
 
-// FP32 copies of parameters that the inference kernels read in FP32, made again when a parameter has changed.
+// FP32 copies of parameters that the inference kernels read in FP32, made again when a parameter has changed.  A copy is
+// made on the stream of the call that misses it: a call on another stream waits for it and keeps its memory from being
+// used again too early.  While a graph is captured nothing is kept (a conversion then belongs to the graph) and nothing
+// is waited for (a capture begins behind a synchronisation).
 struct Fp32Copies {
     struct Entry {
         const void* ptr = nullptr;
         int64_t version = -1;
         Tensor copy;
+        std::optional<c10::Stream> stream;
+        std::shared_ptr<c10::Event> made;
     };
     std::vector<Entry> entries;
+    static bool capturing() {
+        return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    }
     Tensor get(size_t slot, const Tensor& t) {
         if (t.scalar_type() == at::kFloat && t.is_contiguous()) return t.detach();
         if (entries.size() <= slot) entries.resize(slot + 1);
         Entry& e = entries[slot];
+        const bool cuda = t.is_cuda();
         if (e.ptr != t.data_ptr() || e.version != (int64_t)t._version()) {
+            if (cuda && capturing()) return f32_contiguous(t);
             e.copy = f32_contiguous(t);
             e.ptr = t.data_ptr();
             e.version = (int64_t)t._version();
+            e.stream.reset();
+            if (cuda) {
+                e.stream = c10::cuda::getCurrentCUDAStream(t.device().index());
+                e.made = std::make_shared<c10::Event>(c10::DeviceType::CUDA);
+                e.made->record(*e.stream);
+            }
+        } else if (cuda && e.stream.has_value()) {
+            const c10::Stream now = c10::cuda::getCurrentCUDAStream(t.device().index());
+            if (now != *e.stream && !capturing()) {
+                e.made->block(now);
+                e.copy.record_stream(now);
+            }
         }
         return e.copy;
     }
@@ -958,6 +983,17 @@ struct TokenStack {
                                     up_weight, down_weight, mixer_eps, mlp_eps, out_eps, heads, width, value_width, {}});
     }
 
+    struct LayerFp32 { Tensor mixer_norm, conv, log_rate, decay_bias, geometry_bias, out_norm, mlp_norm; };
+    std::vector<LayerFp32> layer_copies() {
+        std::vector<LayerFp32> out;
+        out.reserve(layers.size());
+        for (TokenLayer& l : layers)
+            out.push_back(LayerFp32{l.copies.get(0, l.mixer_norm), l.copies.get(1, l.conv_weight), l.copies.get(2, l.log_rate),
+                                    l.copies.get(3, l.decay_bias), l.copies.get(4, l.geometry_bias), l.copies.get(5, l.out_norm),
+                                    l.copies.get(6, l.mlp_norm)});
+        return out;
+    }
+
     static bool bf16_dense(const Tensor& t, const Tensor& like) {
         return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && t.device() == like.device() && aligned16(t);
     }
@@ -1019,14 +1055,8 @@ struct TokenStack {
         void* stream = stream_of(x);
         // All FP32 copies are taken here, ahead of the first launch: one that is missing or out of date is a conversion
         // kernel, and a chained launch reads its parameters while the kernel directly before it still runs.
-        struct Parameters { const float *mixer_norm, *conv, *log_rate, *decay_bias, *geometry_bias, *out_norm, *mlp_norm; };
-        std::vector<Parameters> fp32;
-        fp32.reserve(layers.size());
-        for (TokenLayer& l : layers)   // braces: in this order
-            fp32.push_back(Parameters{f32(l.copies.get(0, l.mixer_norm)), f32(l.copies.get(1, l.conv_weight)), f32(l.copies.get(2, l.log_rate)),
-                                      f32(l.copies.get(3, l.decay_bias)), f32(l.copies.get(4, l.geometry_bias)),
-                                      f32(l.copies.get(5, l.out_norm)), f32(l.copies.get(6, l.mlp_norm))});
-        const float* const last_norm = f32(copies.get(0, norm));
+        const std::vector<LayerFp32> params = layer_copies();
+        const Tensor last_norm = copies.get(0, norm);
         const auto piece = [&](size_t width) { return (width * (size_t)B * 2 + 255) & ~size_t(255); };
         const size_t row_b = piece(row_max), y_b = piece(y_max), act_b = piece(act_max), d_b = piece((size_t)D);
         const Tensor work = workspace(x, row_b + y_b + act_b + 5 * d_b);
@@ -1090,10 +1120,10 @@ struct TokenStack {
         };
         for (size_t i = 0; i < layers.size(); ++i) {
             const TokenLayer& l = layers[i];
-            const Parameters& w = fp32[i];
+            const LayerFp32& w = params[i];
             State& st = state[i];
             const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0);
-            norm_linear(w.mixer_norm, l.mixer_eps, l.in_weight, raw(l.in_bias), row, false);
+            norm_linear(f32(w.mixer_norm), l.mixer_eps, l.in_weight, raw(l.in_bias), row, false);
             sd_mixer_decode_args a{};
             a.shape = sd_shape{(int32_t)B, 1, (int32_t)H, (int32_t)r, (int32_t)V};
             const auto at_col = [&](int64_t c) { return row + 2 * c; };
@@ -1103,11 +1133,11 @@ struct TokenStack {
             a.erase_raw = sd_operand{at_col(qkv + 2 * H * r), P, P, r};
             a.write_raw = sd_operand{at_col(qkv + 3 * H * r), P, P, V};
             a.qkv = row; a.qkv_stride_b = P;
-            a.conv_weight = w.conv; a.conv_state = st.conv.data_ptr();
-            a.log_rate = w.log_rate; a.decay_bias = w.decay_bias;
-            a.geometry_raw = at_col(geom); a.geometry_stride_b = P; a.geometry_bias = w.geometry_bias;
+            a.conv_weight = f32(w.conv); a.conv_state = st.conv.data_ptr();
+            a.log_rate = f32(w.log_rate); a.decay_bias = f32(w.decay_bias);
+            a.geometry_raw = at_col(geom); a.geometry_stride_b = P; a.geometry_bias = f32(w.geometry_bias);
             a.C = f32(st.C); a.S = f32(st.S); a.y = y;
-            a.norm_weight = w.out_norm; a.norm_eps = (float)l.out_eps;
+            a.norm_weight = f32(w.out_norm); a.norm_eps = (float)l.out_eps;
             a.gate_rank = (int32_t)V;
             a.decay_hidden = at_col(geom + H); a.decay_hidden_stride_b = P;
             a.gate_hidden = at_col(geom + H + V); a.gate_hidden_stride_b = P;
@@ -1116,15 +1146,15 @@ struct TokenStack {
             check(sd_mixer_decode_step_chained(&a, stream));
             linear(y, H * V, l.out_weight, raw(l.out_bias), mixed, false, nullptr, 0);
             delta = mixed;
-            norm_linear(w.mlp_norm, l.mlp_eps, l.up_weight, nullptr, act, true);
+            norm_linear(f32(w.mlp_norm), l.mlp_eps, l.up_weight, nullptr, act, true);
             linear(act, l.up_weight.size(0) / 2, l.down_weight, nullptr, mlp, false, nullptr, 0);
             delta = mlp;
         }
         Tensor out = bf16_like(x, {B, 1, head.has_value() ? head->size(0) : D});
         if (head.has_value())
-            norm_linear(last_norm, norm_eps, *head, nullptr, out.data_ptr(), false);
+            norm_linear(f32(last_norm), norm_eps, *head, nullptr, out.data_ptr(), false);
         else
-            norm_rows(last_norm, norm_eps, out.data_ptr());
+            norm_rows(f32(last_norm), norm_eps, out.data_ptr());
         return out;
     }
 
@@ -1155,6 +1185,7 @@ struct TokenStack {
         }
         const c10::cuda::CUDAGuard guard(x.device());
         void* stream = stream_of(x);
+        const std::vector<LayerFp32> params = layer_copies();
         const size_t d_b = bf16_rows(D);
         const Tensor work = workspace(x, area + 5 * d_b);
         char* const base = static_cast<char*>(work.data_ptr());
@@ -1185,7 +1216,8 @@ struct TokenStack {
         };
         py::list states;
         for (size_t i = 0; i < layers.size(); ++i) {
-            TokenLayer& l = layers[i];
+            const TokenLayer& l = layers[i];
+            const LayerFp32& w32 = params[i];
             const int64_t H = l.heads, r = l.width, V = l.value_width, P = l.in_weight.size(0), Dc = 2 * H * r + H * V;
             const RowPlan rows{B, T, H, r, V, P};
             char* at = base;
@@ -1193,7 +1225,7 @@ struct TokenStack {
             char *row = take(bf16_rows(P)), *qkv = take(bf16_rows(Dc)), *decay_raw = take(bf16_rows(H * r));
             char *log_decay = take(2 * bf16_rows(H * r)), *geometry = take(bf16_rows(2 * H)), *gate = take(bf16_rows(H * V));
             char *y = take(bf16_rows(H * V)), *y_normed = take(bf16_rows(H * V)), *saved = take(plan[i].saved), *scratch = take(plan[i].scratch);
-            norm_rows(l.copies.get(0, l.mixer_norm), l.mixer_eps, normed);
+            norm_rows(w32.mixer_norm, l.mixer_eps, normed);
             linear(normed, D, l.in_weight, l.in_bias, row);
             Tensor C, S, window;
             if (want_states) {
@@ -1204,18 +1236,18 @@ struct TokenStack {
             sd_conv4_forward_args c{};
             c.B = (int32_t)B; c.T = (int32_t)T; c.D = (int32_t)Dc;
             c.x = row; c.x_stride_b = T * P; c.x_stride_t = P;
-            c.weight = f32(l.copies.get(1, l.conv_weight)); c.y = qkv; c.final_state = raw(window);
+            c.weight = f32(w32.conv); c.y = qkv; c.final_state = raw(window);
             check(sd_conv4_silu_forward(&c, stream));
             const auto at_col = [&](int64_t col) { return row + 2 * col; };
             linear(at_col(rows.decay_hidden()), P, l.decay_weight, Tensor(), decay_raw);
             linear(at_col(rows.gate_hidden()), P, l.gate_weight, l.gate_bias, gate);
             sd_kda_gate_args k{};
             k.rows = R; k.H = (int32_t)H; k.r = (int32_t)r;
-            k.raw = decay_raw; k.log_rate = f32(l.copies.get(2, l.log_rate)); k.bias = f32(l.copies.get(3, l.decay_bias));
+            k.raw = decay_raw; k.log_rate = f32(w32.log_rate); k.bias = f32(w32.decay_bias);
             k.log_decay = reinterpret_cast<float*>(log_decay);
             check(sd_kda_gate_forward(&k, stream));
             Tensor rate = at::from_blob(geometry, {R, H}, fp32);
-            at::add_out(rate, matrix(at_col(rows.geometry()), H, P), l.copies.get(4, l.geometry_bias));
+            at::add_out(rate, matrix(at_col(rows.geometry()), H, P), w32.geometry_bias);
             at::sigmoid_(rate);
             sd_forward_args a{};
             rows.fill(a, row, qkv, log_decay, geometry);
@@ -1224,11 +1256,11 @@ struct TokenStack {
             check(sd_forward_inference(&a, stream));
             sd_norm_gate_args g{};
             g.V = (int32_t)V; g.rows = R * H; g.eps = (float)l.out_eps;
-            g.x = y; g.gate = gate; g.weight = f32(l.copies.get(5, l.out_norm)); g.y = y_normed;
+            g.x = y; g.gate = gate; g.weight = f32(w32.out_norm); g.y = y_normed;
             check(sd_norm_gate_forward(&g, stream));
             linear(y_normed, H * V, l.out_weight, l.out_bias, mixed);
             delta = mixed;
-            norm_rows(l.copies.get(6, l.mlp_norm), l.mlp_eps, normed);
+            norm_rows(w32.mlp_norm, l.mlp_eps, normed);
             const int64_t inner = l.up_weight.size(0) / 2;
             char *up = base, *act = base + bf16_rows(2 * inner);
             linear(normed, D, l.up_weight, Tensor(), up);

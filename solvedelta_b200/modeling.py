@@ -528,7 +528,9 @@ class GraphedDecoder:
     A decode step is a few hundred small launches (24 layers of projections, glue kernels and the
     one-token operator kernel), so its cost at small batch is launch and host time.  The step is captured
     once on static buffers (token ids in, logits out, the cache updated in place inside the graph) and
-    replayed per token.  Build it from the cache a prefill returned; ``cache`` stays valid and current."""
+    replayed per token.  Build it from the cache a prefill returned; ``cache`` stays valid and current.
+    The graph holds the FP32 copies of norm weights and conv taps as they were: build a new decoder after
+    an update of the parameters."""
 
     def __init__(self, model: "SolveDeltaForCausalLM", cache: SolveDeltaCache, batch: int) -> None:
         self.model = model

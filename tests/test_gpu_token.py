@@ -121,3 +121,28 @@ def test_parameter_copies_precede_the_launches(B):
     workspace = [i for i, call in enumerate(log.calls) if call == ("empty", torch.uint8)]
     assert len(copies) == 4 * 2 + 1 and len(workspace) == 1 and max(copies) < workspace[0]
     assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 1e-2
+
+
+def test_parameter_copies_made_on_another_stream():
+    """The copies that one stream is still making (behind a long kernel) are waited for on the other."""
+    torch.manual_seed(7)
+    model = SolveDeltaForCausalLM(SolveDeltaConfig(hidden_size=256, num_heads=4, head_k_dim=64, head_v_dim=64,
+                                                   num_hidden_layers=2, vocab_size=320)).prepare("cuda").eval()
+    ids = torch.randint(0, 320, (2, 41), device="cuda")
+    step = lambda cache: model(input_ids=ids[:, 40:], past_key_values=cache, use_cache=True).logits
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.no_grad():
+        cache = model(input_ids=ids[:, :40], use_cache=True).past_key_values
+        caches = [copy.deepcopy(cache) for _ in range(3)]
+        for name, p in model.named_parameters():
+            if "norm" in name or "conv_weight" in name:
+                p.add_(0.25 * torch.randn_like(p))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            torch.cuda._sleep(200_000_000)
+            first = step(caches[0])
+        with torch.cuda.stream(two):
+            second = step(caches[1])
+        torch.cuda.synchronize()
+        want = step(caches[2])
+    assert torch.equal(first, want) and torch.equal(second, want)
