@@ -1,8 +1,11 @@
-"""The layer as one autograd node against its separate nodes: ragged lengths, unequal widths, biases, masks."""
+"""The layer as one autograd node against its separate nodes and the checker: ragged lengths, unequal widths, biases, masks."""
+import numpy as np
 import pytest
 import torch
 
+from oracle import mixer_oracle as mo
 from solvedelta_b200 import SolveDelta, SolveDeltaConfig
+from tests.helpers import max_rel, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +56,49 @@ def test_first_order_gradients_with_create_graph(one, monkeypatch):
     recorded = torch.autograd.grad(layer(x), leaves, dy, create_graph=True)
     for got, want in zip(recorded, plain):
         assert torch.equal(got.detach(), want)
+
+
+@pytest.mark.parametrize("B,T,hidden,heads,r,V,bias,masked", [
+    (2, 128, 256, 4, 64, 64, False, False), (2, 150, 128, 3, 24, 40, True, True)])
+def test_one_node_matches_checker(B, T, hidden, heads, r, V, bias, masked):
+    """What a training step runs (BF16 weights, one autograd node) against the FP64 checker, output and every gradient
+    end to end."""
+    torch.manual_seed(6)
+    layer = SolveDelta(SolveDeltaConfig(hidden_size=hidden, num_heads=heads, head_k_dim=r, head_v_dim=V, bias=bias)).cuda()
+    for name, p in layer.named_parameters():
+        if name not in ("geometry_write_bias", "associative_log_rate", "associative_decay_bias"):
+            p.data = p.data.to(torch.bfloat16)
+    gen = torch.Generator().manual_seed(7)
+    x = torch.randn(B, T, hidden, generator=gen).to(torch.bfloat16)
+    dy = torch.randn(B, T, hidden, generator=gen).to(torch.bfloat16)
+    masks = {}
+    if masked:
+        valid = torch.rand(B, T, generator=gen) < 0.9
+        masks = dict(valid_mask=valid, reset_mask=(torch.rand(B, T, generator=gen) < 0.05) & valid)
+    named = dict(layer.named_parameters())
+    xg = x.cuda().requires_grad_()
+    out = layer(xg, **{k: m.cuda() for k, m in masks.items()})
+    assert "MixerFunction" in out.grad_fn.name()
+    grads = dict(zip(["x", *named], torch.autograd.grad(out, [xg, *named.values()], dy.cuda())))
+    f = lambda t: t.detach().double().cpu().numpy()
+    checker = mo.MixerOracle({n: f(p) for n, p in named.items()}, hidden_size=hidden, num_heads=heads, head_k_dim=r,
+                             head_v_dim=V, use_short_conv=True, norm_eps=layer.output_norm.eps,
+                             activation_rounding=lambda z: torch.as_tensor(z).to(torch.bfloat16).double().numpy())
+    want_out, _, _ = checker.forward(f(x), **{k: m.numpy() for k, m in masks.items()})
+    assert max_rel(f(out), want_out) <= 2e-2
+    dx, want, _, _ = checker.backward(f(dy))
+    want["x"] = dx
+    # The operator's gradients are good to 2e-2 of their largest value at each token.  The three gate families are sums
+    # of them over the tokens, times a factor each, that may cancel: 2e-2 of the largest times the factors' sum.
+    c, og = checker.cache, checker.operator_grads
+    rate = np.exp(f(named["associative_log_rate"]))[None, None, :, None]
+    bound = {"geometry_write_bias": np.abs(og["geometry_write"]).max() * (c["gamma"] * (1 - c["gamma"])).sum((0, 1)),
+             "associative_log_rate": np.abs(og["log_decay"]).max() * np.abs(c["log_decay"]).sum((0, 1, 3)),
+             "associative_decay_bias": np.abs(og["log_decay"]).max() * (rate * (1 - np.exp(c["log_decay"] / rate))).sum((0, 1))}
+    for name, got in grads.items():
+        got = f(got).reshape(want[name].shape)
+        if name in bound:
+            assert (np.abs(got - want[name]) <= 2e-2 * bound[name].reshape(got.shape)).all(), name
+        else:
+            # the decay projection's gradient cancels over the tokens too
+            assert rel_l2(got, want[name]) <= (5e-2 if name == "decay_proj.weight" else 2e-2), name
