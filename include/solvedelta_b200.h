@@ -177,7 +177,7 @@ int sd_pack_rows(const sd_pack_rows_args *args, void *stream);
 
 /*
  * A projection of a cached single-token step: y [M][N] = x [M][K] weight^T (+ bias) for M <= 4 rows
- * (nn.Linear layout, BF16, FP32 accumulation), one warp per output column.  With swiglu != 0 the output is
+ * (nn.Linear layout, BF16, FP32 accumulation): sd_token_linear for few rows.  With swiglu != 0 the output is
  * [M][N/2] = silu(y[:, :N/2]) * y[:, N/2:] (the gated MLP's first projection and activation,
  * causallsso/modeling_solvedelta.py:68-101).  K and x_stride multiples of 8, x and weight 16-byte aligned,
  * else SD_ERR_UNSUPPORTED_SHAPE (the caller then runs its library GEMM).

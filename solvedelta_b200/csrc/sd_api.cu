@@ -401,10 +401,10 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<true>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<false, 1, 8, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<false, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<true, 1, 8, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_decode_step<true, 1, 8, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<false, 1, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<false, 1, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<true, 1, false>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_decode_step<true, 1, true>, DECODE_STATE_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<2, 1, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<2, 1, 8>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
     if ((e = allow_smem(k_token_linear<2, 2, 4>, TOKEN_SMEM_MAX)) != cudaSuccess) return e;
@@ -519,11 +519,11 @@ int token_linear(const TokenLinearParams& p, bool chained, cudaStream_t stream) 
     return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }
 
-template <bool MIXER, int NS, int WARPS, bool FULL>
+template <bool MIXER, int NS, bool FULL>
 cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int streams, bool chained, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(streams * NS));
-    cfg.blockDim = dim3(WARPS * 32);
+    cfg.blockDim = dim3(DECODE_WARPS * 32);
     cfg.dynamicSmemBytes = NS == 1 ? DECODE_STATE_BYTES : 0;
     cfg.stream = stream;
     cudaLaunchAttribute at[2];
@@ -537,7 +537,7 @@ cudaError_t launch_decode_ns(const DecodeParams& p, const MixerDecode& m, int st
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, WARPS, FULL>, p, m);
+    return cudaLaunchKernelEx(&cfg, k_decode_step<MIXER, NS, FULL>, p, m);
 }
 int add_rmsnorm(const sd_add_rmsnorm_args* a, bool chained, void* stream_) {
     if (!a || a->rows <= 0 || a->D <= 0 || !a->x || !a->weight || !a->normed || (a->delta && !a->sum))
@@ -578,10 +578,10 @@ int launch_decode(const DecodeParams& p, const MixerDecode& m, int streams, bool
     const bool full = p.g.r == DP && p.g.V == DP && p.Cin != nullptr && p.Sin != nullptr && (states & 15) == 0 &&
                       p.u.vec && p.er.vec && p.wr.vec && (MIXER || (p.q.vec && p.k.vec && p.v.vec && p.ld.vec));
     const bool split = decode_split(streams) == 4;
-    const cudaError_t e = full ? (split ? launch_decode_ns<MIXER, 4, 8, true>(p, m, streams, chained, stream)
-                                        : launch_decode_ns<MIXER, 1, 8, true>(p, m, streams, chained, stream))
-                               : (split ? launch_decode_ns<MIXER, 4, 8, false>(p, m, streams, chained, stream)
-                                        : launch_decode_ns<MIXER, 1, 8, false>(p, m, streams, chained, stream));
+    const cudaError_t e = full ? (split ? launch_decode_ns<MIXER, 4, true>(p, m, streams, chained, stream)
+                                        : launch_decode_ns<MIXER, 1, true>(p, m, streams, chained, stream))
+                               : (split ? launch_decode_ns<MIXER, 4, false>(p, m, streams, chained, stream)
+                                        : launch_decode_ns<MIXER, 1, false>(p, m, streams, chained, stream));
     mark(stream);
     return e == cudaSuccess ? launch_status() : SD_ERR_LAUNCH_FAILED;
 }

@@ -178,12 +178,14 @@ __device__ __forceinline__ float2 dec_ld_remote2(unsigned a) {
     return v;
 }
 
+constexpr int DECODE_WARPS = 8;
+
 // FULL: r = V = 128, every row aligned for the wide accesses, both states given.  Bounds and strides are then constants:
 // the row loops are loads at immediate offsets, without a predicate or an address each, which is a third of the step
 // (one CTA per stream: 55 -> 41 us at 768 streams; clusters of four: 6.6 -> 4.4 us at 8 streams).
-template <bool MIXER, int NS, int WARPS, bool FULL>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) k_decode_step(DecodeParams p, MixerDecode mix) {
-    constexpr int THREADS = WARPS * 32;
+template <bool MIXER, int NS, bool FULL>
+__global__ void __launch_bounds__(DECODE_WARPS * 32, 2) k_decode_step(DecodeParams p, MixerDecode mix) {
+    constexpr int WARPS = DECODE_WARPS, THREADS = WARPS * 32;
     constexpr int ROWS = DP / NS;            // state rows of this CTA
     constexpr int RW = ROWS / WARPS;         // ... of a warp
     constexpr int LPR = 32 / RW;             // lanes that hold a row's scalars after warp_sum_rows

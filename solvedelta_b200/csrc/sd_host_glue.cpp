@@ -451,8 +451,7 @@ Tensor swiglu(const Tensor& gate_value) {
 constexpr int64_t GEMV_MAX_ROWS = 4;
 bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 
-// The projection of a cached single-token step in the one-warp-per-column kernel, or undefined when the call is not one
-// it takes.
+// The projection of a cached single-token step in k_token_linear, or undefined when the call is not one it takes.
 Tensor small_projection(const Tensor& x, const Tensor& weight, const Tensor& bias, bool with_swiglu) {
     if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || weight.scalar_type() != at::kBFloat16 || weight.dim() != 2) return {};
     const int64_t K = x.size(-1), N = weight.size(0);
@@ -823,8 +822,9 @@ OptTensor mixer_train(const Tensor& x, int64_t heads, int64_t width, int64_t val
                                 geometry_bias, norm_weight, out_weight, out_bias, v, z, heads, width, value_width, eps);
 }
 
-// One cached token between the fused projection row and the output projection, in one launch; argument meanings as in
-// mixer_decode_step (mixer_ops.py).
+// One cached token between the fused projection row and the output projection, in one launch: conv4 + SiLU of the
+// q | k | v slice against the conv window [B,D,3] (advanced in place), decay gate, geometry rate, the recurrent step on
+// the FP32 states (updated in place), gated norm.  The rows are views of the projection row; parameters are FP32.
 struct DecodeToken {
     Tensor u, h, erase, write, qkv, conv_weight, conv_state, decay_raw, log_rate, decay_bias, geometry_raw, geometry_bias;
     Tensor predictor, memory, output_gate, norm_weight;
@@ -890,19 +890,6 @@ Tensor decode_launch(const DecodeToken& t) {
     }
     check(sd_mixer_decode_step(&a, stream_of(t.u)));
     return y;
-}
-
-Tensor mixer_decode_step(const Tensor& u, const Tensor& h, const Tensor& erase, const Tensor& write, const Tensor& qkv,
-                         const Tensor& conv_weight, const Tensor& conv_state, const OptTensor& decay_raw, const Tensor& log_rate,
-                         const Tensor& decay_bias, const Tensor& geometry_raw, const Tensor& geometry_bias, const Tensor& predictor,
-                         const Tensor& memory, const OptTensor& output_gate, const OptTensor& norm_weight, double eps,
-                         const OptTensor& decay_hidden, const OptTensor& decay_weight, const OptTensor& gate_hidden,
-                         const OptTensor& gate_weight, const OptTensor& gate_bias) {
-    const at::NoGradGuard no_grad;
-    return decode_launch(DecodeToken{u, h, erase, write, qkv, conv_weight, conv_state, given(decay_raw), log_rate, decay_bias,
-                                     geometry_raw, geometry_bias, predictor, memory, given(output_gate), given(norm_weight),
-                                     given(decay_hidden), given(decay_weight), given(gate_hidden), given(gate_weight),
-                                     given(gate_bias), eps});
 }
 
 // The whole mixer for one cached token without gradients: fused projection, decode launch (conv window and operator
@@ -1313,6 +1300,5 @@ void register_glue(py::module_& m) {
     m.def("pack_rows", &pack_rows);
     m.def("mixer_front", &mixer_front);
     m.def("mixer_train", &mixer_train);
-    m.def("mixer_decode_step", &mixer_decode_step);
     m.def("mixer_decode", &mixer_decode);
 }

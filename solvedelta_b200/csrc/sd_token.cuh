@@ -11,7 +11,7 @@
 // * the product runs on mma.sync m16n8k16 with the rows of x as the M side: the contraction index is permuted so that a
 //   lane's 16-byte piece of a weight row is its B fragment of two instructions (k = 8 t + {0,1,2,3} and {4,5,6,7}), and
 //   x, in shared memory, is read with the same permutation; an FMA per weight and row would bound it from 8 rows on;
-// * up to eight rows the norm is taken by every CTA for itself on the way into shared memory, which removes a launch.
+// * up to sixteen rows the norm is taken by every CTA for itself on the way into shared memory, which removes a launch.
 #pragma once
 #include "sd_bf16.cuh"
 #include "sd_common.cuh"

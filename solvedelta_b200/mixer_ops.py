@@ -41,29 +41,6 @@ def conv4_silu_segmented(x: torch.Tensor, weight: torch.Tensor, plan, initial_st
     return conv4_silu(x, weight, initial_state, return_final_state, plan.valid_mask, plan.reset_mask)
 
 
-def mixer_decode_step(u: torch.Tensor, h: torch.Tensor, erase_raw: torch.Tensor, write_raw: torch.Tensor,
-                      qkv: torch.Tensor, conv_weight: torch.Tensor, conv_state: torch.Tensor,
-                      decay_raw: torch.Tensor, log_rate: torch.Tensor, decay_bias: torch.Tensor,
-                      geometry_raw: torch.Tensor, geometry_bias: torch.Tensor,
-                      predictor: torch.Tensor, memory: torch.Tensor, *, output_gate: Optional[torch.Tensor] = None,
-                      norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 1e-6,
-                      gate_projections: Optional[tuple] = None) -> torch.Tensor:
-    """One cached token of the mixer between its projections, in ONE launch: conv4 + SiLU of the q | k | v slice
-    against ``conv_state`` (advanced in place), the decay gate, the geometry rate and the recurrent step on
-    ``predictor`` / ``memory`` (updated in place).  ``u, h`` are ``[B,1,H,r]`` and ``erase_raw, write_raw``
-    ``[B,1,H,r|V]`` views of the projection row, ``qkv`` ``[B,1,D]``, ``decay_raw`` ``[B,1,H,r]``, ``geometry_raw``
-    ``[B,1,H]``; FP32 ``conv_weight [D,4]``, ``log_rate [H]``, ``decay_bias [H*r]``, ``geometry_bias [H]``.
-    Returns the output row ``[B,1,H,V]`` (BF16).  Same arithmetic as ``conv4_silu`` + ``kda_decay_gate`` +
-    ``sigmoid`` + the T = 1 branch of ``solvedelta_native``; with ``output_gate`` ``[B,1,H,V]`` and FP32
-    ``norm_weight [V]`` the row also passes through ``rms_norm_gated``.  ``gate_projections`` =
-    ``(decay_hidden [B,1,G], decay_proj.weight [H*r,G], gate_hidden [B,1,G], output_gate_proj.weight [H*V,G],
-    output_gate_proj.bias [H*V] | None)``, all BF16, moves the two small projections in front of the gates into the
-    kernel as well (``decay_raw`` and ``output_gate`` may then be None; needs ``norm_weight``)."""
-    return _lib.host().mixer_decode_step(u, h, erase_raw, write_raw, qkv, conv_weight, conv_state, decay_raw, log_rate,
-                                         decay_bias, geometry_raw, geometry_bias, predictor, memory, output_gate,
-                                         norm_weight, norm_eps, *(gate_projections or (None,) * 5))
-
-
 def add_rmsnorm_reverse_supported(width: int) -> bool:
     """Row widths the reverse pass of :func:`add_rmsnorm` is built for (whole groups of 256 channels, up to 2048)."""
     return width % 256 == 0 and 0 < width <= 2048
@@ -84,8 +61,8 @@ def swiglu(gate_value: torch.Tensor) -> torch.Tensor:
 
 def small_linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, *,
                  swiglu: bool = False) -> Optional[torch.Tensor]:
-    """``F.linear(x, weight, bias)`` for the one to four rows of a cached single-token step (inference only), one warp
-    per output column; with ``swiglu`` the result is ``silu(y[..., :N/2]) * y[..., N/2:]``.  Returns ``None`` when the
+    """``F.linear(x, weight, bias)`` for the one to four rows of a cached single-token step (inference only) in the
+    tensor-core kernel of the cached step (csrc/sd_token.cuh); with ``swiglu`` the result is ``silu(y[..., :N/2]) * y[..., N/2:]``.  Returns ``None`` when the
     call is not one the kernel takes (gradients recorded, more rows, not BF16 CUDA, unaligned), and the caller runs
     its library projection."""
     return _lib.host().small_linear(x, weight, bias, swiglu)
@@ -147,6 +124,5 @@ def rms_norm_gated(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, ep
     return _lib.host().rms_norm_gated(x, gate, weight, eps)
 
 
-__all__ = ["add_rmsnorm", "conv4_silu", "conv4_silu_segmented", "kda_decay_gate", "mixer_decode_step", "rms_norm_gated",
-           "swiglu",
-           "gated_mlp", "rms_norm_gated_linear"]
+__all__ = ["add_rmsnorm", "conv4_silu", "conv4_silu_segmented", "gated_mlp", "kda_decay_gate", "rms_norm_gated",
+           "rms_norm_gated_linear", "swiglu"]
