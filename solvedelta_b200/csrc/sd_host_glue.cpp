@@ -4,6 +4,8 @@
 // seven launches of a cached token, several times the device time of short sequences.
 #include "sd_host.h"
 
+#include <algorithm>
+
 #include <c10/core/Event.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 
@@ -25,15 +27,15 @@ bool records_gradients(std::initializer_list<const Tensor*> tensors) {
 }
 
 // FP32 copies of parameters that the inference kernels read in FP32, made again when a parameter has changed.  A copy is
-// made on the stream of the call that misses it: a call on another stream waits for it and keeps its memory from being
-// used again too early.  While a graph is captured nothing is kept (a conversion then belongs to the graph) and nothing
+// made on the stream of the call that misses it: the first call on another stream waits for it there and keeps its
+// memory from being used again too early.  While a graph is captured nothing is kept (a conversion then belongs to the graph) and nothing
 // is waited for (a capture begins behind a synchronisation).
 struct Fp32Copies {
     struct Entry {
         const void* ptr = nullptr;
         int64_t version = -1;
         Tensor copy;
-        std::optional<c10::Stream> stream;
+        std::vector<c10::Stream> ordered;   // streams whose work follows the conversion
         std::shared_ptr<c10::Event> made;
     };
     std::vector<Entry> entries;
@@ -50,17 +52,18 @@ struct Fp32Copies {
             e.copy = f32_contiguous(t);
             e.ptr = t.data_ptr();
             e.version = (int64_t)t._version();
-            e.stream.reset();
+            e.ordered.clear();
             if (cuda) {
-                e.stream = c10::cuda::getCurrentCUDAStream(t.device().index());
+                e.ordered.push_back(c10::cuda::getCurrentCUDAStream(t.device().index()));
                 e.made = std::make_shared<c10::Event>(c10::DeviceType::CUDA);
-                e.made->record(*e.stream);
+                e.made->record(e.ordered.front());
             }
-        } else if (cuda && e.stream.has_value()) {
+        } else if (cuda) {
             const c10::Stream now = c10::cuda::getCurrentCUDAStream(t.device().index());
-            if (now != *e.stream && !capturing()) {
+            if (std::find(e.ordered.begin(), e.ordered.end(), now) == e.ordered.end() && !capturing()) {
                 e.made->block(now);
                 e.copy.record_stream(now);
+                if (e.ordered.size() < 16) e.ordered.push_back(now);   // past that a call waits each time
             }
         }
         return e.copy;

@@ -146,3 +146,29 @@ def test_parameter_copies_made_on_another_stream():
         torch.cuda.synchronize()
         want = step(caches[2])
     assert torch.equal(first, want) and torch.equal(second, want)
+
+
+def test_copies_missing_during_a_capture_belong_to_the_graph():
+    """A step captured with its parameter copies out of date converts them inside the graph, and leaves nothing behind that
+    only a replay would fill."""
+    torch.manual_seed(8)
+    model = SolveDeltaForCausalLM(SolveDeltaConfig(hidden_size=256, num_heads=4, head_k_dim=64, head_v_dim=64,
+                                                   num_hidden_layers=2, vocab_size=320)).prepare("cuda").eval()
+    ids = torch.randint(0, 320, (2, 41), device="cuda")
+    token = ids[:, 40:].contiguous()
+    step = lambda cache: model(input_ids=token, past_key_values=cache, use_cache=True).logits
+    with torch.no_grad():
+        cache = model(input_ids=ids[:, :40], use_cache=True).past_key_values
+        caches = [copy.deepcopy(cache) for _ in range(3)]
+        step(copy.deepcopy(cache))   # lazy initialisation
+        for name, p in model.named_parameters():
+            if "norm" in name or "conv_weight" in name:
+                p.add_(0.25 * torch.randn_like(p))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = step(caches[0])
+        want = step(caches[1])
+        graph.replay()
+        assert torch.equal(captured, want)
+        del graph
+        assert torch.equal(step(caches[2]), want)
