@@ -344,8 +344,8 @@ __device__ __forceinline__ uint32_t f2tf32(float x) {
 // The same rounding for an operand of mma.sync alone, which reads the upper 19 bits: half a unit added, nothing masked
 // (one integer instruction; the conversion has a quarter of its rate, and operands are rounded at every use: solve of the
 // fused forward kernel 6.0 -> 4.0 us).  The maximum with the number's own bits keeps the NaN that arithmetic returns,
-// 0x7fffffff, whose sum would leave the signed range and read as minus zero; it is part of the same instruction (3703 us
-// forward + reverse at 8 x 4096 tokens with it, 3703 without).  Not kept are NaNs that only memory can hold: a negative
+// 0x7fffffff, whose sum would leave the signed range and read as minus zero; it is part of the same instruction (forward
+// + reverse at 8 x 4096 tokens 3703 us with it and without, at 5 x 1531 with masks 1070 against 1068).  Not kept are NaNs that only memory can hold: a negative
 // one with all ones (0xfffff000 and up) counts as zero, one whose fraction lies in the bits cut off (0x7f800001 to
 // 0x7f800fff) as an infinity.
 __device__ __forceinline__ uint32_t mma_tf32_bits(float x) {
