@@ -345,9 +345,10 @@ __device__ __forceinline__ uint32_t f2tf32(float x) {
 // (one integer instruction; the conversion has a quarter of its rate, and operands are rounded at every use: solve of the
 // fused forward kernel 6.0 -> 4.0 us).  The maximum with the number's own bits keeps the NaN that arithmetic returns,
 // 0x7fffffff, whose sum would leave the signed range and read as minus zero; it is part of the same instruction (forward
-// + reverse at 8 x 4096 tokens 3703 us with it and without, at 5 x 1531 with masks 1070 against 1068).  Not kept are NaNs that only memory can hold: a negative
-// one with all ones (0xfffff000 and up) counts as zero, one whose fraction lies in the bits cut off (0x7f800001 to
-// 0x7f800fff) as an infinity.
+// + reverse at 8 x 4096 tokens 3703 us with it and without, at 5 x 1531 with masks 1070 against 1068).  NaNs that only
+// memory can hold are not kept here, a negative one with all ones (0xfffff000 and up) and one whose fraction lies in the
+// bits cut off (0x7f800001 to 0x7f800fff); the FP32 operands reach a contraction through arithmetic or beside a path that
+// keeps them (test_gpu_nonfinite.py).
 __device__ __forceinline__ uint32_t mma_tf32_bits(float x) {
     const int b = __float_as_int(x);
     return (uint32_t)__viaddmax_s32(b, 0x1000, b);

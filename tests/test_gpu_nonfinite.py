@@ -24,15 +24,22 @@ def _run(dev, dy):
     return f(y), f(fin.predictor), f(fin.S), [f(g) for g in grads]
 
 
+QUIET, ALL_ONES, SIGNALLING = 0x7fc00000, -1, 0x7f800001   # FP32 patterns; only memory can hold the last two
+
+
 @pytest.mark.parametrize("r,V", [(32, 48), (20, 12)])   # aligned rows, and the general row accesses
-@pytest.mark.parametrize("name", OPERANDS + ("C0", "S0"))
-def test_nan_reaches_what_it_reaches_in_the_checker(name, r, V):
+@pytest.mark.parametrize("name,bits", [(n, QUIET) for n in OPERANDS + ("C0", "S0")] + [
+    (n, b) for n in ("log_decay", "geometry_write", "C0", "S0") for b in (ALL_ONES, SIGNALLING)])
+def test_nan_reaches_what_it_reaches_in_the_checker(name, bits, r, V):
     cpu, dev = make_inputs(B, T, H, r, V, seed=11)
     dy = torch.randn(B, T, H, V, generator=torch.Generator().manual_seed(12)).to(torch.bfloat16)
     clean = _run(dev, dy.cuda())
     where = (0, HEAD, 1, 3) if name in ("C0", "S0") else (0, AT, HEAD) + ((0,) if cpu[name].ndim == 5 else ()) + (
         () if cpu[name].ndim == 3 else (3,))
-    cpu[name][where] = float("nan")
+    if bits == QUIET:
+        cpu[name][where] = float("nan")
+    else:
+        cpu[name].view(torch.int32)[where] = bits
     dev[name] = cpu[name].cuda()
     y, C, S, grads = _run(dev, dy.cuda())
     with np.errstate(invalid="ignore"):
