@@ -9,6 +9,7 @@
 #include "sd_common.cuh"
 #include "sd_decode.cuh"
 #include "sd_forward.cuh"
+#include "sd_forward_tc.cuh"
 #include "sd_mixer.cuh"
 #include "sd_scan_tc.cuh"
 #include "sd_output_tc.cuh"
@@ -25,12 +26,12 @@ struct PanelDesc {
     int kind;
 };
 
-const PanelDesc kSaved[] = {{"Lam", 3}, {"G", 0}, {"Delta", 0}, {"Dprim", 0}, {"Zt", 4}, {"CtCk", 2}, {"CtCkB", 6}, {"SCk", 6},
+const PanelDesc kSaved[] = {{"Lam", 3}, {"Flags", 3}, {"G", 0}, {"Delta", 0}, {"Dprim", 0}, {"Zt", 4}, {"CtCk", 2}, {"CtCkB", 6}, {"SCk", 6},
                             {"N", 1}, {"Aed", 1}, {"Aqd", 5},
                             // BF16 source panels of the exterior, written once by the forward pass
                             {"Xg", 4}, {"Ag", 4}, {"Xr", 4}, {"Er", 4}, {"Dcol", 4}, {"DtB", 4}, {"Chi", 4}, {"Ee", 4}};
 // what a call without gradients keeps of it: the panels that later forward kernels read
-const PanelDesc kInfer[] = {{"Lam", 3}, {"G", 0}, {"Delta", 0}, {"Zt", 4}, {"CtCk", 2}, {"SCk", 6}, {"Aqd", 5}, {"Xg", 4}};
+const PanelDesc kInfer[] = {{"Lam", 3}, {"Flags", 3}, {"G", 0}, {"Delta", 0}, {"Zt", 4}, {"CtCk", 2}, {"SCk", 6}, {"Aqd", 5}, {"Xg", 4}};
 const PanelDesc kFwd[] = {{"Upd", 0}, {"Qc", 0}, {"Ubar", 0}, {"Wd", 0}, {"Ud", 0}, {"Dt", 0}};
 const PanelDesc kBwd[] = {{"Pp", 4},     {"Qp", 4},     {"Dyf", 4},    {"dR", 4},     {"dSeCk", 6},
                           {"SdS", 3},    {"duPart", 4}, {"dkPart", 4}, {"dGPart", 4}, {"dDelta", 4}, {"DG", 4},
@@ -397,6 +398,10 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_primal_exterior_fwd<true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<true, false>, CTA_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<false, false>, CTA_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<true, true>, CTA_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<false, true>, CTA_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_state_scan_tc<false>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
@@ -479,6 +484,31 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_
         else if (fast) launch(kernel<true, true>, chunks, NTHREADS, smem, chained, stream, p);          \
         else if (!masked) launch(kernel<false, false>, chunks, NTHREADS, smem, chained, stream, p);     \
         else launch(kernel<false, true>, chunks, NTHREADS, smem, chained, stream, p);                   \
+    } while (0)
+
+// ... a pair of them (sd_chunk_tc.cuh): the slow chunks with one CTA to an SM, and the fast ones with two
+// Up to 148 chunks the fast ones ask for an SM each: their CTAs arrive while the slow kernel's leave, and would double up
+// on the SMs that are free first (128 chunks: 29 us in the CTA against 21).
+size_t fast_smem(int chunks) { return chunks <= 148 ? CTA_SMEM : FAST_SMEM; }
+// A masked call has slow chunks wherever a sequence starts: one chunk per CTA, so that the SMs without a slow one take more.
+int chunk_grid(int chunks, int resident) { return chunks < 148 * resident ? chunks : 148 * resident; }
+#define SD_LAUNCH_PAIR(fast_kernel, kernel, smem)                                                            \
+    do {                                                                                                     \
+        const int g1 = chunk_grid(chunks, 1), g2 = masked ? chunks : chunk_grid(chunks, 2);                  \
+        const size_t fsm = fast_smem(chunks);                                                                \
+        if (fast && !masked) {                                                                               \
+            launch(kernel<true, false>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
+            launch(fast_kernel<true, false>, g2, NTHREADS, fsm, true, stream, p, chunks);              \
+        } else if (fast) {                                                                                   \
+            launch(kernel<true, true>, g1, NTHREADS, smem, true, stream, p, chunks);                         \
+            launch(fast_kernel<true, true>, g2, NTHREADS, fsm, true, stream, p, chunks);               \
+        } else if (!masked) {                                                                                \
+            launch(kernel<false, false>, g1, NTHREADS, smem, true, stream, p, chunks);                       \
+            launch(fast_kernel<false, false>, g2, NTHREADS, fsm, true, stream, p, chunks);             \
+        } else {                                                                                             \
+            launch(kernel<false, true>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
+            launch(fast_kernel<false, true>, g2, NTHREADS, fsm, true, stream, p, chunks);              \
+        }                                                                                                    \
     } while (0)
 
 bool operands_ok(const sd_operand* ops, int n) {
@@ -631,7 +661,7 @@ int sd_panel_kind(const sd_shape* shape, int which, const char* name) {
 // a scan that is cut into segments is three launches
 int sd_forward_launches(const sd_shape* shape) {
     if (!shape_ok(shape)) return 0;
-    return 5 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, FWD_STEP_US, FWD_TRANSFER_US) > 1 ? 4 : 0);
+    return 6 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, FWD_STEP_US, FWD_TRANSFER_US) > 1 ? 4 : 0);
 }
 int sd_backward_launches(const sd_shape* shape) {
     if (!shape_ok(shape)) return 0;
@@ -724,6 +754,9 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     p.Npair = fp32("N"); p.Aed = fp32("Aed"); p.Dprim = fp32("Dprim");
     p.Lam = fp32("Lam"); p.Gp = fp32("G"); p.Delta = fp32("Delta"); p.CtCk = fp32("CtCk");
     p.Zt = half("Zt"); p.SCk = half("SCk");
+    p.Flags = reinterpret_cast<unsigned char*>(fp32("Flags"));
+    p.fault = scan_fault_ptr();
+    if (p.fault == nullptr) return SD_ERR_LAUNCH_FAILED;
     p.y = a->y;
     p.action = po ? po->action : nullptr;
     p.update = po ? po->update : nullptr;
@@ -756,10 +789,10 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     }
     set_dbg(p.g, 2, chunks);
     if (po) {
-        k_primal_exterior_fwd<false, true, true><<<chunks, NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p);
+        k_primal_exterior_fwd<false, true, true><<<chunk_grid(chunks, 1), NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p, chunks);
         return launch_status();   // the kernel stops after its primal half
     }
-    SD_LAUNCH_CHUNK(k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM, true);
+    SD_LAUNCH_PAIR(k_primal_exterior_fast, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
     mark(stream);
     {
         ScanParams sp{};

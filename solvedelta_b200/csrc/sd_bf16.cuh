@@ -218,53 +218,56 @@ struct PanelBF16 {
     }
 };
 
+// D <- (I + sgn T)^-1 - I in place for a strictly triangular 16 x 16 block of pitch LDA, by substitution; one warp, one lane
+// per column of the inverse.
+template <bool UPPER>
+__device__ __forceinline__ void invert_diagonal_block(float* D, float sgn) {
+    const int lane = threadIdx.x & 31, j = lane & 15;   // both half-warps compute the same block
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = (i == j) ? 1.f : 0.f;
+    if (!UPPER) {
+#pragma unroll
+        for (int i = 1; i < 16; ++i) {
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+            for (int k4 = 0; k4 < i; k4 += 4) {
+                const float4 m = *reinterpret_cast<const float4*>(D + i * LDA + k4);
+                a0 = fmaf(m.x, x[k4], a0);
+                a1 = fmaf(m.y, x[k4 + 1], a1);
+                a0 = fmaf(m.z, x[k4 + 2], a0);
+                a1 = fmaf(m.w, x[k4 + 3], a1);
+            }
+            x[i] = (i > j) ? -sgn * (a0 + a1) : x[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 14; i >= 0; --i) {
+            float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+            for (int k4 = ((i + 1) & ~3); k4 < 16; k4 += 4) {
+                const float4 m = *reinterpret_cast<const float4*>(D + i * LDA + k4);
+                a0 = fmaf(m.x, x[k4], a0);
+                a1 = fmaf(m.y, x[k4 + 1], a1);
+                a0 = fmaf(m.z, x[k4 + 2], a0);
+                a1 = fmaf(m.w, x[k4 + 3], a1);
+            }
+            x[i] = (i < j) ? -sgn * (a0 + a1) : x[i];
+        }
+    }
+    __syncwarp();   // every lane has read the block before anyone overwrites it
+    if (lane < 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) D[i * LDA + j] = (i == j) ? 0.f : x[i];
+    }
+}
+
 template <bool UPPER, class Panel>
 __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) {
     static_assert(NTHREADS == 2 * DP * 2, "16 warps of 16 right-hand-side columns each");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     constexpr int NB = CL / 16;
-    // ---- the four diagonal blocks: D_I <- (I + sgn T_II)^-1 - I, in place -------------
-    if (warp < NB) {
-        float* D = Mr + (16 * warp) * LDA + 16 * warp;
-        const int j = lane & 15;   // column of the inverse (both half-warps compute the same block)
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = (i == j) ? 1.f : 0.f;
-        if (!UPPER) {
-#pragma unroll
-            for (int i = 1; i < 16; ++i) {
-                float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-                for (int k4 = 0; k4 < i; k4 += 4) {
-                    const float4 m = *reinterpret_cast<const float4*>(D + i * LDA + k4);
-                    a0 = fmaf(m.x, x[k4], a0);
-                    a1 = fmaf(m.y, x[k4 + 1], a1);
-                    a0 = fmaf(m.z, x[k4 + 2], a0);
-                    a1 = fmaf(m.w, x[k4 + 3], a1);
-                }
-                x[i] = (i > j) ? -sgn * (a0 + a1) : x[i];
-            }
-        } else {
-#pragma unroll
-            for (int i = 14; i >= 0; --i) {
-                float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-                for (int k4 = ((i + 1) & ~3); k4 < 16; k4 += 4) {
-                    const float4 m = *reinterpret_cast<const float4*>(D + i * LDA + k4);
-                    a0 = fmaf(m.x, x[k4], a0);
-                    a1 = fmaf(m.y, x[k4 + 1], a1);
-                    a0 = fmaf(m.z, x[k4 + 2], a0);
-                    a1 = fmaf(m.w, x[k4 + 3], a1);
-                }
-                x[i] = (i < j) ? -sgn * (a0 + a1) : x[i];
-            }
-        }
-        __syncwarp();   // every lane has read the block before anyone overwrites it
-        if (lane < 16) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) D[i * LDA + j] = (i == j) ? 0.f : x[i];
-        }
-    }
+    if (warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * warp) * LDA + 16 * warp, sgn);
     __syncthreads();
     // ---- warp-local sweep over this warp's 16 columns ---------------------------------
     const int n0 = 16 * warp;

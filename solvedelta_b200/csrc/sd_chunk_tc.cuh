@@ -1,0 +1,356 @@
+// What the fast chunk kernels share: chunks whose contractions run on the fifth-generation tensor cores.
+//
+// Fast chunks.  A chunk that forgets at most FAST_CHUNK_NATS in every channel needs no block centring: with G the
+// inclusive prefix of the log decay, every decay-weighted term exp(x_i - G_j) is the product of a row factor exp(x_i) <= 1
+// and a column factor exp(-G_j) <= e^60, both far inside the range of FP32, TF32 and BF16 (which share their exponent),
+// so a pair matrix is ONE contraction over all channels and a causal or anti-causal sum ONE contraction over all tokens,
+// masked by a select.  Such chunks take tcgen05 in the kernels named *_fast; a chunk that forgets more, or holds a reset,
+// takes the block-centred kernels (sd_decay.cuh), which walk over the slow chunks of a launch with one CTA per SM.  The
+// choice is made per chunk by k_prep_fwd, which stores it in the chunk's flag word: from what the chunk itself holds, so it
+// does not depend on what else is in the call.
+//
+// A chunk is a chain of loads, contractions, row passes and a solve, each of which leaves most of an SM idle: what counts
+// is the length of that chain and how many chains share the SM.  The fast kernels are persistent, two CTAs of 16 warps to
+// an SM (64 registers a thread, half of the shared and of the tensor memory each); with accumulators and the operands
+// between two contractions in tensor memory the FP32 panels of a chunk fit a CTA's 113 KB.
+#pragma once
+#include "sd_decay.cuh"
+#include "sd_scan_tc.cuh"
+
+namespace sd {
+
+constexpr float FAST_CHUNK_NATS = 60.f;
+constexpr int FLAG_SLOW = 1;              // some channel's prefix leaves [-FAST_CHUNK_NATS, FAST_CHUNK_NATS]
+constexpr int FAST_PASSES = CL / 16;      // row-wise passes: a warp takes a row, a lane four channels
+constexpr int FAST_BARS = 8;
+constexpr unsigned FAST_TMEM = 256;       // tensor-memory columns of a CTA
+constexpr size_t FAST_SMEM = 113 * 1024, CTA_SMEM = 227 * 1024;   // two CTAs per SM, one
+constexpr size_t FAST_BAR_OFF = FAST_SMEM - (FAST_BARS + 1) * 8;
+constexpr unsigned F32_TILE = CL * 128;   // [64 rows][32 channels] FP32, or [64 rows][64 channels] BF16: 128-byte rows
+
+struct FastCta {
+    int tid, warp, lane, quarter, part;   // quarter: the tensor-memory lanes of this warp, part: its quarter of the columns
+    unsigned char* sm;
+    unsigned tmem, bars, parity;
+    bool alive;
+    int* fault;
+    __device__ __forceinline__ unsigned bar(int i) const { return bars + 8 * i; }
+    // every barrier is used once per task; a wait that runs out raises the fault word and ends all later ones
+    __device__ __forceinline__ void wait(int i, int code) {
+        bool done = alive && tc_wait(bar(i), parity);
+        done = __all_sync(0xffffffffu, done);
+        if (alive && !done && lane == 0) atomicExch(fault, code);
+        alive = done;
+        tc_fence_after();
+    }
+    __device__ __forceinline__ unsigned lanes() const { return tmem + ((unsigned)(quarter * 32) << 16); }
+    // tensor-memory and shared-memory accesses of all threads are ordered before the contractions issued after this
+    __device__ __forceinline__ void publish() const {
+        tc_fence_before();
+        tc_fence_async_smem();
+        __syncthreads();
+    }
+};
+
+// The slow chunks' kernel of a pair is launched first and lets the fast one start as soon as its own predecessor is
+// complete: what the fast kernel reads is older than the slow one, they write different chunks, and its CTAs fill the SMs
+// that have no slow chunk to work on.  It waits for the slow one at its end, for the kernels that follow both.
+//
+// Tensor memory is allocated before the launch lets its successor start, so that a kernel that starts early can never hold
+// what this one still waits for.  These kernels have no static shared memory: the dynamic part starts on the 1024-byte
+// boundary that the swizzled tiles need (behind the 1 KB the system keeps), which is checked.
+__device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, int* fault) {
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + FAST_BAR_OFF);
+    unsigned* s_tmem = reinterpret_cast<unsigned*>(bars + FAST_BARS);
+    cta.tid = threadIdx.x;
+    cta.warp = cta.tid >> 5;
+    cta.lane = cta.tid & 31;
+    cta.quarter = cta.warp & 3;
+    cta.part = cta.warp >> 2;
+    if (cta.tid == 0) {
+        for (int i = 0; i < FAST_BARS; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&bars[i])));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (cta.warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(s_tmem)), "r"(FAST_TMEM));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    cta.sm = smem;
+    cta.tmem = *s_tmem;
+    cta.bars = tc_smem(bars);
+    cta.parity = 0;
+    cta.alive = (tc_smem(smem) & 1023u) == 0;   // else nothing here can be right: no waits, and the fault word says so
+    cta.fault = fault;
+    if (!cta.alive && cta.tid == 0) atomicExch(fault, 20);
+    chain_release();
+}
+__device__ __forceinline__ void fast_teardown(const FastCta& cta) {
+    tc_fence_before();
+    __syncthreads();
+    chain_wait();
+    if (cta.warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cta.tmem), "r"(FAST_TMEM));
+}
+__device__ __forceinline__ int chunk_flags(const unsigned char* flags, long long gi) { return __ldg(flags + gi); }
+
+// The tasks of a persistent CTA: f(task) for its fast chunks, the next flag word on its way meanwhile.
+template <class F>
+__device__ __forceinline__ void for_fast_chunks(FastCta& cta, const unsigned char* flags, int tasks, F f) {
+    int t = blockIdx.x, word = chunk_flags(flags, t);
+    while (t < tasks) {
+        const int next = t + gridDim.x, next_word = next < tasks ? chunk_flags(flags, next) : 0;
+        if (!(word & FLAG_SLOW)) {
+            f(t);
+            cta.parity ^= 1;
+        }
+        t = next;
+        word = next_word;
+    }
+}
+
+// The slow chunks of a launch (all of them without flags), shared out over the CTAs by their rank, so that a CTA's share
+// does not depend on where they lie.
+template <class F>
+__device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int tasks, F f) {
+    if (flags == nullptr) {
+        for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
+            f(t);
+            __syncthreads();   // the next chunk's loads overwrite what this one reads
+        }
+        return;
+    }
+    int rank = 0;
+    constexpr int WINDOW = NTHREADS * 16;   // one 16-byte load per thread tells whether there is a slow chunk at all
+    for (int base = 0; base < tasks; base += WINDOW) {
+        const int t0 = base + threadIdx.x * 16;
+        unsigned any = 0;
+        if (t0 < tasks) {   // the flag panel has room past the last chunk
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + t0));
+            const unsigned words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & FLAG_SLOW;
+        }
+        if (__syncthreads_or(any) == 0) continue;
+        for (int b = base; b < tasks && b < base + WINDOW; b += 32) {
+            const int t = b + (threadIdx.x & 31);
+            unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & FLAG_SLOW));
+            while (slow != 0) {
+                if (rank++ % gridDim.x == blockIdx.x) {
+                    f(b + __ffs(slow) - 1);
+                    __syncthreads();
+                }
+                slow &= slow - 1;
+            }
+        }
+    }
+}
+
+// Profiling build: thread 0 of the CTA that works on the chosen chunk records the SM clock (see SD_PHASE).
+#ifdef SD_DIAGNOSTICS
+#define SD_PHASE_T(g, ch, ph)                                                                                 \
+    do {                                                                                                      \
+        if ((g).dbg != nullptr && (int)(ch).gi == (g).dbg_block && threadIdx.x == 0 && (ph) < 16)             \
+            (g).dbg[(ph)] = clock64();                                                                        \
+        ++(ph);                                                                                               \
+    } while (0)
+#else
+#define SD_PHASE_T(g, ch, ph) do { (void)(ph); } while (0)
+#endif
+
+// ---- operand tiles -----------------------------------------------------------
+// K-major FP32 operand, 128-byte swizzle: tiles of 32 channels (TS bytes apart), 128-byte rows, 16-byte piece j of row i at
+// piece j ^ (i mod 8).  The same tiles serve as plain panels: row-wise, lane-per-row and column accesses are all free of
+// bank conflicts.
+template <unsigned TS>
+__device__ __forceinline__ unsigned f32_off(int i, int c) {
+    return (c >> 5) * TS + i * 128 + ((((c >> 2) & 7) ^ (i & 7)) << 4) + ((c & 3) << 2);
+}
+// MN-major FP32 operand (the row is the contraction index): 128-byte swizzle of 32-byte atoms, atom j of row i at j ^ (i mod 4)
+__device__ __forceinline__ unsigned f32_mn_off(int i, int c) {
+    return (c >> 5) * F32_TILE + i * 128 + ((((c >> 3) & 3) ^ (i & 3)) << 5) + ((c & 7) << 2);
+}
+__device__ __forceinline__ float4 tf32_bits4(const float4& v) {   // rounded for a contraction, which cuts the low bits off
+    return make_float4(__uint_as_float(mma_tf32_bits(v.x)), __uint_as_float(mma_tf32_bits(v.y)),
+                       __uint_as_float(mma_tf32_bits(v.z)), __uint_as_float(mma_tf32_bits(v.w)));
+}
+__device__ __forceinline__ float4 pack4(const float (&x)[4]) { return make_float4(x[0], x[1], x[2], x[3]); }
+__device__ __forceinline__ void unpack4(const float4& v, float (&x)[4]) { x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w; }
+__device__ __forceinline__ void unpack4(const uint2& raw, float (&x)[4]) {
+    x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xffff0000u);
+    x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xffff0000u);
+}
+__device__ __forceinline__ uint2 pack4_bf16(const float (&x)[4]) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(x[0], x[1]), b = __floats2bfloat162_rn(x[2], x[3]);
+    return make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+// Four channels of a BF16 row as they lie, zeros past the width and where the row is not `valid`
+template <bool FAST>
+__device__ __forceinline__ uint2 load4_raw(const bf16* row, int c0, int width, int vec, bool valid) {
+    uint2 raw = make_uint2(0u, 0u);
+    if (!valid || c0 >= width) return raw;
+    if (FAST || (vec && c0 + 4 <= width)) return *reinterpret_cast<const uint2*>(row + c0);
+    const unsigned short* src = reinterpret_cast<const unsigned short*>(row) + c0;
+    raw.x = src[0];
+    if (c0 + 1 < width) raw.x |= (unsigned)src[1] << 16;
+    if (c0 + 2 < width) raw.y = src[2];
+    if (c0 + 3 < width) raw.y |= (unsigned)src[3] << 16;
+    return raw;
+}
+// Sums over the 32 lanes of a row.  Three exchanges leave each lane with one of eight sums over a quarter of the lanes, two
+// more complete it, and the sums are then fetched by lane: 9 shuffles and 8 fetches, where butterflies take 40.
+__device__ __forceinline__ void row_sums32(float (&v)[8]) {
+    const int lane = threadIdx.x & 31;
+    float a[4], b[2];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        const bool up = lane & 16;
+        a[n] = (up ? v[n + 4] : v[n]) + __shfl_xor_sync(0xffffffffu, up ? v[n] : v[n + 4], 16);
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        const bool up = lane & 8;
+        b[n] = (up ? a[n + 2] : a[n]) + __shfl_xor_sync(0xffffffffu, up ? a[n] : a[n + 2], 8);
+    }
+    const bool up = lane & 4;
+    float c = (up ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+#pragma unroll
+    for (int n = 0; n < 8; ++n) v[n] = __shfl_sync(0xffffffffu, c, 4 * n);   // lanes 4 n .. hold sum n
+}
+__device__ __forceinline__ void row_sums32(float (&v)[4]) {
+    const int lane = threadIdx.x & 31;
+    float a[2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        const bool up = lane & 16;
+        a[n] = (up ? v[n + 2] : v[n]) + __shfl_xor_sync(0xffffffffu, up ? v[n] : v[n + 2], 16);
+    }
+    const bool up = lane & 8;
+    float c = (up ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[1], 8);
+    c += __shfl_xor_sync(0xffffffffu, c, 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) v[n] = __shfl_sync(0xffffffffu, c, 8 * n);
+}
+// prefetch_rows for the rows of a whole CTA, up to four lines each
+template <class CH>
+__device__ __forceinline__ void prefetch_fast_rows(const Operand& op, const CH& ch, int row_bytes) {
+    const int i = threadIdx.x >> 3, l = threadIdx.x & 7;
+    if (l * 128 < row_bytes && ch.ok(i)) prefetch_l2(reinterpret_cast<const char*>(row_bf16(op, ch, i)) + l * 128);
+}
+
+// ---- contractions (one thread issues) -------------------------------------------
+__device__ __forceinline__ void tc_mma_ss(unsigned d_tmem, unsigned long long da, unsigned long long db, unsigned idesc,
+                                          unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ unsigned long long f32_desc(unsigned addr) { return tc_desc(addr, 16, 1024) | (2ull << 61); }
+__device__ __forceinline__ unsigned long long f32_mn_desc(unsigned addr) {
+    return tc_desc(addr, F32_TILE, TC_R_SBO) | (1ull << 61);
+}
+// D[128][N] (+)= A[128][128] B[N][128]^T over K-major FP32 tiles; a descriptor counts addresses in 16-byte units
+template <unsigned TSA, unsigned TSB>
+__device__ __forceinline__ void mma_tf32_kk(unsigned d_tmem, unsigned a, unsigned b, int n, unsigned accumulate) {
+    const unsigned id = tc_idesc(n);
+    const unsigned long long da = f32_desc(a), db = f32_desc(b);
+#pragma unroll
+    for (int k = 0; k < DP / 8; ++k)
+        tc_mma_ss(d_tmem, da + ((k / 4) * TSA + (k % 4) * 32) / 16, db + ((k / 4) * TSB + (k % 4) * 32) / 16, id,
+                  k > 0 ? 1u : accumulate);
+}
+
+// ---- tensor memory, four columns at a time ---------------------------------------
+__device__ __forceinline__ void tc_st4(unsigned taddr, const float (&r)[4]) {
+    const unsigned* u = reinterpret_cast<const unsigned*>(r);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%4], {%0,%1,%2,%3};" ::"r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]),
+                 "r"(taddr)
+                 : "memory");
+}
+
+// ---- unit-triangular solve ----------------------------------------------------------
+// trisolve_blocked (sd_bf16.cuh) on FP32 tiles: after the four diagonal blocks are inverted, each of the sixteen warps
+// owns 16 of the 256 right-hand-side columns, half of a tile, and never waits for another warp.
+template <bool UPPER>
+__device__ __forceinline__ void trisolve_tiles(const FastCta& cta, float* Mr, float sgn, unsigned char* tile) {
+    const int g = cta.lane >> 2, t = cta.lane & 3, h4 = (cta.warp & 1) * 4;   // first 16-byte piece of this warp's half
+    constexpr int NB = CL / 16, NT = 2;
+    if (cta.warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * cta.warp) * LDA + 16 * cta.warp, sgn);
+    __syncthreads();
+    auto at2 = [&](int i, int nt) {   // i mod 8 = g
+        return reinterpret_cast<float2*>(tile + i * 128 + (((h4 + nt * 2 + (t >> 1)) ^ g) << 4) + ((t & 1) << 3));
+    };
+    auto get = [&](int kk, int odd, int nt) {   // row kk + 2 t + odd, column 8 nt + g
+        return *reinterpret_cast<const float*>(tile + (kk + 2 * t + odd) * 128 + (((h4 + nt * 2 + (g >> 2)) ^ (2 * t + odd)) << 4) + ((g & 3) << 2));
+    };
+    auto contract = [&](float (&acc)[NT][4], int r0, int kbeg, int kend) {
+#pragma unroll
+        for (int kk = kbeg; kk < kend; kk += 8) {   // permuted contraction index, as in warp_mma_pairs
+            const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
+            const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
+            const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+                mma_tf32(acc[nt], a0, a1, a2, a3, mma_tf32_bits(get(kk, 0, nt)), mma_tf32_bits(get(kk, 1, nt)));
+        }
+    };
+#pragma unroll
+    for (int step = 0; step < NB; ++step) {
+        const int I = UPPER ? (NB - 1 - step) : step, r0 = 16 * I;
+        float rr[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const float2 a = *at2(r0 + g, nt), b = *at2(r0 + g + 8, nt);
+            rr[nt][0] = a.x; rr[nt][1] = a.y; rr[nt][2] = b.x; rr[nt][3] = b.y;
+        }
+        if (step > 0) {
+            float acc[NT][4];
+            acc_zero<NT>(acc);
+            contract(acc, r0, UPPER ? r0 + 16 : 0, UPPER ? CL : r0);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) rr[nt][e] = fmaf(-sgn, acc[nt][e], rr[nt][e]);
+                *at2(r0 + g, nt) = make_float2(rr[nt][0], rr[nt][1]);
+                *at2(r0 + g + 8, nt) = make_float2(rr[nt][2], rr[nt][3]);
+            }
+            __syncwarp();
+        }
+        float acc[NT][4];
+        acc_zero<NT>(acc);
+        contract(acc, r0, r0, r0 + 16);
+        __syncwarp();   // every lane has read the block's right-hand sides
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            *at2(r0 + g, nt) = make_float2(rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
+            *at2(r0 + g + 8, nt) = make_float2(rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
+        }
+        __syncwarp();
+    }
+}
+// The warp's solved half tile to its 16 columns of a dense global panel.
+template <bool TF32>
+__device__ __forceinline__ void store_half_tile(const FastCta& cta, float* g, const unsigned char* tile) {
+    const int j = (cta.warp & 1) * 4 + (cta.lane & 3);
+#pragma unroll
+    for (int it = 0; it < CL / 8; ++it) {
+        const int i = it * 8 + (cta.lane >> 2);
+        float4 v = *reinterpret_cast<const float4*>(tile + i * 128 + ((j ^ (i & 7)) << 4));
+        if (TF32) v = make_float4(round_tf32(v.x), round_tf32(v.y), round_tf32(v.z), round_tf32(v.w));
+        *reinterpret_cast<float4*>(g + i * DP + 4 * j) = v;
+    }
+}
+
+}  // namespace sd

@@ -1,9 +1,10 @@
 // Chunk-parallel forward kernels: one CTA per (stream, chunk).
 //
-// Pipeline: k_prep_fwd -> scan(C) -> k_primal_exterior_fwd -> scan(S) -> k_output_fwd_tc.
+// Pipeline: k_prep_fwd -> scan(C) -> k_primal_exterior_fwd / _fast -> scan(S) -> k_output_fwd_tc.
 #pragma once
 #include "sd_bf16.cuh"
 #include "sd_common.cuh"
+#include "sd_chunk_tc.cuh"
 #include "sd_decay.cuh"
 
 namespace sd {
@@ -25,6 +26,8 @@ struct FwdParams {
     float *Dprim;
     float *Npair, *Aed;  // pair matrices N = Lm / gamma and Aed, [CL][CL]
     bf16 *Zt, *SCk;  // only BF16 contractions read these
+    unsigned char* Flags;   // [chunks], see sd_chunk_tc.cuh (the panel has room for a vector a chunk)
+    int* fault;      // device fault word of the bounded waits
     void* y;
     // predictor-only entry (null otherwise): BF16 [B,T,H,r] outputs frame action d - k^ and update Delta;
     // k_primal_exterior_fwd then stops after its primal half
@@ -155,17 +158,20 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
     auto fG = [&](int i, int c) { return s_A[i * LDP + c]; };
     pair_block_scales(s_M, fG);
     block_decay_tables(nullptr, s_ibeta, s_fastw, fG);
+    bool in_range;
     {
         const int J = threadIdx.x >> 7, c = threadIdx.x & (DP - 1);
         s_gp[threadIdx.x] = J ? fG(BT * J - 1, c) : 0.f;
         s_ge[threadIdx.x] = fG(BT * J + BT - 1, c);
+        in_range = fabsf(s_ge[threadIdx.x]) <= FAST_CHUNK_NATS;   // false for a NaN
     }
     float* gG = panel_ptr(p.Gp, ch.gi);
     for (int idx = threadIdx.x; idx < CL * (DP / 4); idx += NTHREADS) {
         const int i = idx >> 5, c4 = (idx & 31) << 2;
         *reinterpret_cast<float4*>(gG + i * DP + c4) = *reinterpret_cast<const float4*>(s_A + i * LDP + c4);
     }
-    __syncthreads();
+    const bool fast_chunk = __syncthreads_and(in_range) != 0;
+    if (threadIdx.x == 0) p.Flags[ch.gi] = fast_chunk ? 0 : FLAG_SLOW;
     // Lm = gamma stril(N), N[i][j] = sum_c u^_ic u^_jc exp(E_ic - G_jc); N itself is kept for backward.
     // Diagonal blocks that are not fast: direct evaluation, while u^ and G are still in the slots.
     float* gN = p.Npair != nullptr ? mat_ptr(p.Npair, ch.gi) : nullptr;
@@ -277,7 +283,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
 }
 
 // ---------------------------------------------------------------------------
-// Primal address and exterior preparation in one CTA per chunk task.
+// Primal address and exterior preparation of one chunk, block-centred.
 // First half: d = k^ + C_t^T k^ for every token of the chunk,
 //   d_i = k^_i + exp(G_i) (K^ Ct^T)_i + sum_{j<=i} (k^_i . Delta_j) u^_j exp(G_i - G_j),
 // the decay-weighted sum in block-centred form (Horner over blocks, direct diagonal).
@@ -303,13 +309,10 @@ __device__ __forceinline__ void async_state_cols_f32(float* sm, const float* st,
     }
 }
 
-template <bool FAST, bool MASKED, bool PRED = false>
-__global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p) {
-    chain_wait();
-    chain_release();
+template <bool FAST, bool MASKED, bool PRED>
+__device__ __forceinline__ void primal_exterior_blocks(const FwdParams& p, const ChunkT<MASKED> ch, float* smem) {
     int ph = 0;
     SD_PHASE(p.g, ph);
-    extern __shared__ __align__(16) float smem[];
     float* s_kh = smem;
     float* s_un = s_kh + PANEL_FLOATS;
     float* s_G = s_un + PANEL_FLOATS;
@@ -321,9 +324,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     float* s_M = s_beta + NBLK * DP;
     float* s_ibeta = s_M + 3 * DP;
     int* s_fastw = reinterpret_cast<int*>(s_ibeta + NBLK * DP);
-    const int V = p.g.V;
-    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
-    const int r = p.g.r;
+    const int V = p.g.V, r = p.g.r;
     const float* ct = state_ptr(p.CtCk, ch.gi);
 
     // everything that is already FP32 in HBM streams in while the BF16 operands are normalised
@@ -574,6 +575,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p
     s2g_panel_tf32(panel_ptr(p.Wd, ch.gi), s_ag);   // a contraction operand of the state scan
     s2g_panel(panel_ptr(p.Ud, ch.gi), s_z);
     SD_PHASE(p.g, ph);
+}
+
+// The slow chunks of a launch, one CTA per SM that walks over them (every chunk for the predictor-only entry).
+template <bool FAST, bool MASKED, bool PRED = false>
+__global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p, int tasks) {
+    extern __shared__ __align__(16) float smem[];
+    chain_wait();
+    chain_release();
+    for_slow_chunks(PRED ? nullptr : p.Flags, tasks, [&](int t) {
+        primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem);
+    });
 }
 
 // The output rows y = Xg S_c + tril(Aqd) Z~ are k_output_fwd_tc (sd_output_tc.cuh).

@@ -382,7 +382,7 @@ if (identity) {
                 if (p.ck != nullptr) {
                     float* ck = state_ptr(p.ck, gi) + p0 * DP + c;
 #pragma unroll
-                    for (int j = 0; j < TC_SCOLS; ++j) __stcs(ck + j * DP, st[j]);
+                    for (int j = 0; j < TC_SCOLS; ++j) __stcs(ck + j * DP, tc_round(st[j]));   // only read as an operand
                 }
                 if (p.ckb != nullptr) tc_store_pairs<TC_SCOLS>(p.ckb + gi * (long long)(DP * DP) + p0 * DP, c, lane, st);
             }

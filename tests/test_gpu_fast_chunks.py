@@ -1,0 +1,73 @@
+"""The two kinds of chunk kernels against the checker where a call changes from one to the other: a chunk is fast while
+every channel's prefix stays within 60 nats.  Decays just inside, just outside and mixed over heads and chunks; chunks of
+one token, full ones and ragged ends; widths that need the padded and the unaligned accesses; masked tokens."""
+import numpy as np
+import pytest
+import torch
+
+from solvedelta_b200 import SolveDeltaState, solvedelta_native
+from tests.gpu_harness import RawRun, make_inputs
+from tests.test_gpu_parity import _check_forward, _check_vjp, _masked_case, _native
+
+pytestmark = pytest.mark.gpu
+
+NATS = 60.0
+
+
+def _with_decay(cpu, dev, per_token):
+    """Channel 1 of head h and chunk c forgets per_token[h][c] nats a token, which alone decides the chunk's kind; the
+    others keep about 0.02.  (With every channel near a nat a token the log-decay gradient is the difference of BF16 terms
+    ten times its size, 2^-9 of which is 2e-2 to 3e-2 of it in either kind of kernel: at the oracle's bound, no test of it.)"""
+    for t in range(cpu["log_decay"].shape[1]):
+        for h in range(cpu["log_decay"].shape[2]):
+            cpu["log_decay"][:, t, h, 1] = -per_token[h][t // 64]
+    dev["log_decay"] = cpu["log_decay"].cuda()
+
+
+# the oracle's tolerances of tests/test_gpu_parity.py: 2e-2 on BF16 results, 1e-3 on the FP32 states
+@pytest.mark.parametrize("T,r,V", [(64, 128, 128), (65, 64, 96), (130, 20, 12), (191, 128, 64)])
+@pytest.mark.parametrize("kind", ["inside", "outside", "mixed"])
+def test_chunks_at_the_limit_match_checker(T, r, V, kind):
+    cpu, dev = make_inputs(1, T, 2, r, V, seed=41)
+    low, high = 0.995 * NATS / 64, 1.005 * NATS / 64
+    rows = {"inside": [[low] * 3, [0.02] * 3], "outside": [[high] * 3, [2.5] * 3],
+            "mixed": [[0.02, high, 0.02], [high, 0.3, 4.0]]}[kind]
+    _with_decay(cpu, dev, rows)
+    full = [(h, c) for h in range(2) for c in range((T + 63) // 64) if rows[h][c] * min(64, T - 64 * c) > NATS]
+    flags, _ = RawRun(dev).panel(0, "Flags")
+    flags = flags.contiguous().flatten().numpy().view(np.uint8)[:2 * ((T + 63) // 64)].reshape(2, -1)
+    assert sorted(map(tuple, np.argwhere(flags & 1))) == full
+    leaves, state, y, fin = _native(dev, grad=True)
+    _check_forward(cpu, y, fin)
+    _check_vjp(cpu, leaves, state, y, fin)
+
+
+def test_more_chunks_than_resident_ctas_with_slow_ones_between():
+    """Every CTA walks over several chunks, slow ones among them: the bits of each stream on its own."""
+    B, T, H, r, V = 5, 64 * 24 + 7, 4, 32, 32   # 500 chunks, more than two CTAs on each of 148 SMs
+    cpu, dev = make_inputs(B, T, H, r, V, seed=43)
+    for b in range(B):
+        cpu["log_decay"][b, 64 * (3 + b):64 * (3 + b) + 90, b % H] -= 1.5
+    dev["log_decay"] = cpu["log_decay"].cuda()
+    names = ("u", "h", "q", "keys", "values", "log_decay", "erase_raw", "write_raw", "geometry_write")
+    dy = torch.randn(B, T, H, V, generator=torch.Generator().manual_seed(44)).to(torch.bfloat16).cuda()
+
+    def run(cut):
+        leaves = [cut(dev[n]).contiguous().requires_grad_() for n in names]
+        y, fin = solvedelta_native(*leaves, initial_state=SolveDeltaState(cut(dev["C0"]), cut(dev["S0"])),
+                                   return_final_state=True)
+        return [y, *fin, *torch.autograd.grad(y, leaves, cut(dy))]
+
+    whole = run(lambda t: t)
+    for b in (0, 4):
+        for one, all_ in zip(run(lambda t: t[b:b + 1]), whole):
+            assert torch.equal(one[0], all_[b])
+
+
+@pytest.mark.parametrize("r,V", [(128, 128), (20, 12)])
+def test_masked_tokens_without_resets_in_fast_chunks(r, V):
+    cpu, dev = make_inputs(2, 150, 2, r, V, seed=47)
+    valid = torch.ones(2, 150, dtype=torch.bool)
+    valid[0, :70] = False      # a whole chunk and the head of the next
+    valid[1, 100:103] = False
+    _masked_case(cpu, dev, valid, torch.zeros_like(valid))
