@@ -6,6 +6,7 @@
 #include "../../include/solvedelta_b200.h"
 #include "sd_diagnostics.h"
 #include "sd_backward.cuh"
+#include "sd_backward_tc.cuh"
 #include "sd_common.cuh"
 #include "sd_decode.cuh"
 #include "sd_forward.cuh"
@@ -398,10 +399,14 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_primal_exterior_fwd<true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<true, false>, CTA_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<false, false>, CTA_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<true, true>, CTA_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<false, true>, CTA_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<true, false>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<false, false>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<true, true>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_primal_exterior_fast<false, true>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_exterior_pair_fast<true, false>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_exterior_pair_fast<false, false>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_exterior_pair_fast<true, true>, FAST_SMEM)) != cudaSuccess) return e;
+    if ((e = allow_smem(k_exterior_pair_fast<false, true>, FAST_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_state_scan_tc<false>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
@@ -487,27 +492,24 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_
     } while (0)
 
 // ... a pair of them (sd_chunk_tc.cuh): the slow chunks with one CTA to an SM, and the fast ones with two
-// Up to 148 chunks the fast ones ask for an SM each: their CTAs arrive while the slow kernel's leave, and would double up
-// on the SMs that are free first (128 chunks: 29 us in the CTA against 21).
-size_t fast_smem(int chunks) { return chunks <= 148 ? CTA_SMEM : FAST_SMEM; }
-// A masked call has slow chunks wherever a sequence starts: one chunk per CTA, so that the SMs without a slow one take more.
-int chunk_grid(int chunks, int resident) { return chunks < 148 * resident ? chunks : 148 * resident; }
+// Masked calls have slow chunks wherever a sequence starts: those go first, and the fast chunks fill the SMs around them
+// (5 x 1531 tokens with masks 1088 -> 1072 us).  Without masks slow chunks are the exception: they go last, and
+// the fast kernel starts while its predecessor ends (128 chunks: 20 us in the CTA against 28 behind an empty launch).
 #define SD_LAUNCH_PAIR(fast_kernel, kernel, smem)                                                            \
     do {                                                                                                     \
-        const int g1 = chunk_grid(chunks, 1), g2 = masked ? chunks : chunk_grid(chunks, 2);                  \
-        const size_t fsm = fast_smem(chunks);                                                                \
+        const int g1 = chunks < 148 ? chunks : 148;                                                          \
         if (fast && !masked) {                                                                               \
+            launch(fast_kernel<true, false>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
             launch(kernel<true, false>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
-            launch(fast_kernel<true, false>, g2, NTHREADS, fsm, true, stream, p, chunks);              \
         } else if (fast) {                                                                                   \
             launch(kernel<true, true>, g1, NTHREADS, smem, true, stream, p, chunks);                         \
-            launch(fast_kernel<true, true>, g2, NTHREADS, fsm, true, stream, p, chunks);               \
+            launch(fast_kernel<true, true>, chunks, NTHREADS, FAST_SMEM, true, stream, p);            \
         } else if (!masked) {                                                                                \
+            launch(fast_kernel<false, false>, chunks, NTHREADS, FAST_SMEM, true, stream, p);              \
             launch(kernel<false, false>, g1, NTHREADS, smem, true, stream, p, chunks);                       \
-            launch(fast_kernel<false, false>, g2, NTHREADS, fsm, true, stream, p, chunks);             \
         } else {                                                                                             \
             launch(kernel<false, true>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
-            launch(fast_kernel<false, true>, g2, NTHREADS, fsm, true, stream, p, chunks);              \
+            launch(fast_kernel<false, true>, chunks, NTHREADS, FAST_SMEM, true, stream, p);           \
         }                                                                                                    \
     } while (0)
 
@@ -665,7 +667,7 @@ int sd_forward_launches(const sd_shape* shape) {
 }
 int sd_backward_launches(const sd_shape* shape) {
     if (!shape_ok(shape)) return 0;
-    return 6 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, BWD_STEP_US, BWD_TRANSFER_US) > 1 ? 4 : 0);
+    return 7 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, BWD_STEP_US, BWD_TRANSFER_US) > 1 ? 4 : 0);
 }
 int sd_chunk_tokens(void) { return CL; }
 int sd_version(void) { return 1; }
@@ -789,7 +791,7 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
     }
     set_dbg(p.g, 2, chunks);
     if (po) {
-        k_primal_exterior_fwd<false, true, true><<<chunk_grid(chunks, 1), NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p, chunks);
+        k_primal_exterior_fwd<false, true, true><<<chunks, NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p, chunks);
         return launch_status();   // the kernel stops after its primal half
     }
     SD_LAUNCH_PAIR(k_primal_exterior_fast, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
@@ -852,6 +854,9 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     p.gam = make_operand(a->gamma, 4);
     p.dy = make_operand(a->dy, 2);
     void* sv = const_cast<void*>(a->saved);
+    p.Flags = reinterpret_cast<const unsigned char*>(panel_at(kSaved, s, sv, "Flags"));
+    p.fault = scan_fault_ptr();
+    if (p.fault == nullptr) return SD_ERR_LAUNCH_FAILED;
     p.Lam = panel_at(kSaved, s, sv, "Lam");
     p.Gp = panel_at(kSaved, s, sv, "G");
     p.Delta = panel_at(kSaved, s, sv, "Delta");
@@ -925,7 +930,7 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     mark(stream);
     }
     set_dbg(p.g, 7, chunks);
-    SD_LAUNCH_CHUNK(k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM, true);
+    SD_LAUNCH_PAIR(k_exterior_pair_fast, k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM);
     mark(stream);
     }
     set_dbg(p.g, 8, chunks);

@@ -18,6 +18,8 @@ namespace sd {
 struct BwdParams {
     Geometry g;
     Operand u, h, q, k, v, er, wr, ld, gam, dy;
+    const unsigned char* Flags;   // [chunks], see sd_chunk_tc.cuh
+    int* fault;                   // device fault word of the bounded waits
     // kept by forward (FP32)
     const float *Lam, *Gp, *Delta, *Dprim, *CtCk;
     const float *Npair, *Aed;   // pair matrices N and Aed of the forward pass, [CL][CL]
@@ -304,12 +306,9 @@ __device__ __forceinline__ void epi_scale_store_bsm(float (&acc)[NTW][4], int r0
 }
 
 template <bool FAST, bool MASKED>
-__global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) {
-    chain_wait();
-    chain_release();
+__device__ __forceinline__ void exterior_pair_blocks(const BwdParams& p, const ChunkT<MASKED> ch, unsigned char* smem_raw) {
     int ph = 0;
     SD_PHASE(p.g, ph);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* b_dy = reinterpret_cast<bf16*>(smem_raw);   // dy      -> d chi
     bf16* b_zt = b_dy + BSLOT_ELEMS;
     bf16* b_dr = b_zt + BSLOT_ELEMS;
@@ -323,7 +322,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     float* s_beta = reinterpret_cast<float*>(b_daed + BMAT_ELEMS);
     int* s_fastw = reinterpret_cast<int*>(s_beta + NBLK * DP);
     float* s_G = reinterpret_cast<float*>(s_fastw + 16);   // [CL][LDP] prefix: every epilogue and the row pass use it
-    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const float* gG = panel_ptr(p.Gp, ch.gi);
     auto fG = [&](int i, int c) { return gG[i * DP + c]; };
 
@@ -477,6 +475,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p) 
     SD_PHASE(p.g, ph);
     sources_bwd_rows<FAST>(p, ch, s_G, b_dy, b_dc, b_xr, b_er, b_dr);
     SD_PHASE(p.g, ph);
+}
+// The slow chunks of a launch, one CTA per SM that walks over them.
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p, int tasks) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    for_slow_chunks(p.Flags, tasks, [&](int t) { exterior_pair_blocks<FAST, MASKED>(p, chunk_of<MASKED>(p.g, t), smem_raw); });
 }
 
 // ---------------------------------------------------------------------------

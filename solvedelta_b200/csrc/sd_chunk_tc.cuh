@@ -10,9 +10,10 @@
 // does not depend on what else is in the call.
 //
 // A chunk is a chain of loads, contractions, row passes and a solve, each of which leaves most of an SM idle: what counts
-// is the length of that chain and how many chains share the SM.  The fast kernels are persistent, two CTAs of 16 warps to
-// an SM (64 registers a thread, half of the shared and of the tensor memory each); with accumulators and the operands
-// between two contractions in tensor memory the FP32 panels of a chunk fit a CTA's 113 KB.
+// is the length of that chain and how many chains share the SM.  The fast kernels run one chunk a CTA of 16 warps, two CTAs
+// to an SM (64 registers a thread, half of the shared and of the tensor memory each); with accumulators and the operands
+// between two contractions in tensor memory the FP32 panels of a chunk fit a CTA's 113 KB.  Persistent CTAs were slower (the
+// primal kernel 557 against 500 us at 4096 chunks: their row passes met more often).
 #pragma once
 #include "sd_decay.cuh"
 #include "sd_scan_tc.cuh"
@@ -24,20 +25,22 @@ constexpr int FLAG_SLOW = 1;              // some channel's prefix leaves [-FAST
 constexpr int FAST_PASSES = CL / 16;      // row-wise passes: a warp takes a row, a lane four channels
 constexpr int FAST_BARS = 8;
 constexpr unsigned FAST_TMEM = 256;       // tensor-memory columns of a CTA
-constexpr size_t FAST_SMEM = 113 * 1024, CTA_SMEM = 227 * 1024;   // two CTAs per SM, one
+constexpr size_t FAST_SMEM = 113 * 1024;  // two CTAs per SM
 constexpr size_t FAST_BAR_OFF = FAST_SMEM - (FAST_BARS + 1) * 8;
 constexpr unsigned F32_TILE = CL * 128;   // [64 rows][32 channels] FP32, or [64 rows][64 channels] BF16: 128-byte rows
+
+__device__ __forceinline__ int chunk_flags(const unsigned char* flags, long long gi) { return __ldg(flags + gi); }
 
 struct FastCta {
     int tid, warp, lane, quarter, part;   // quarter: the tensor-memory lanes of this warp, part: its quarter of the columns
     unsigned char* sm;
-    unsigned tmem, bars, parity;
+    unsigned tmem, bars;
     bool alive;
     int* fault;
     __device__ __forceinline__ unsigned bar(int i) const { return bars + 8 * i; }
-    // every barrier is used once per task; a wait that runs out raises the fault word and ends all later ones
+    // every barrier is used once; a wait that runs out raises the fault word and ends all later ones
     __device__ __forceinline__ void wait(int i, int code) {
-        bool done = alive && tc_wait(bar(i), parity);
+        bool done = alive && tc_wait(bar(i), 0);
         done = __all_sync(0xffffffffu, done);
         if (alive && !done && lane == 0) atomicExch(fault, code);
         alive = done;
@@ -52,13 +55,15 @@ struct FastCta {
     }
 };
 
-// The slow chunks' kernel of a pair is launched first and lets the fast one start as soon as its own predecessor is
-// complete: what the fast kernel reads is older than the slow one, they write different chunks, and its CTAs fill the SMs
-// that have no slow chunk to work on.  It waits for the slow one at its end, for the kernels that follow both.
+// WAIT: the launch begins once its predecessor is complete.  Without it (masked calls) the slow chunks' kernel has been
+// launched just before and let this one start as soon as its own predecessor was complete: what is read here is older than
+// the slow kernel, the two write different chunks, and the CTAs here fill the SMs that have no slow chunk to work on.  The
+// wait for the slow kernel is then at the end, for the kernels that follow both.
 //
 // Tensor memory is allocated before the launch lets its successor start, so that a kernel that starts early can never hold
 // what this one still waits for.  These kernels have no static shared memory: the dynamic part starts on the 1024-byte
 // boundary that the swizzled tiles need (behind the 1 KB the system keeps), which is checked.
+template <bool WAIT>
 __device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, int* fault) {
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + FAST_BAR_OFF);
     unsigned* s_tmem = reinterpret_cast<unsigned*>(bars + FAST_BARS);
@@ -82,11 +87,19 @@ __device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, in
     cta.sm = smem;
     cta.tmem = *s_tmem;
     cta.bars = tc_smem(bars);
-    cta.parity = 0;
     cta.alive = (tc_smem(smem) & 1023u) == 0;   // else nothing here can be right: no waits, and the fault word says so
     cta.fault = fault;
     if (!cta.alive && cta.tid == 0) atomicExch(fault, 20);
+    if (WAIT) chain_wait();
     chain_release();
+}
+// True for a slow chunk, which another kernel does: the CTA only keeps its place in the chain of launches.  (The flags are
+// older than the launch before.)
+__device__ __forceinline__ bool leave_to_slow_kernel(const unsigned char* flags) {
+    if (!(chunk_flags(flags, blockIdx.x) & FLAG_SLOW)) return false;
+    chain_wait();
+    chain_release();
+    return true;
 }
 __device__ __forceinline__ void fast_teardown(const FastCta& cta) {
     tc_fence_before();
@@ -95,59 +108,36 @@ __device__ __forceinline__ void fast_teardown(const FastCta& cta) {
     if (cta.warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cta.tmem), "r"(FAST_TMEM));
 }
-__device__ __forceinline__ int chunk_flags(const unsigned char* flags, long long gi) { return __ldg(flags + gi); }
 
-// The tasks of a persistent CTA: f(task) for its fast chunks, the next flag word on its way meanwhile.
-template <class F>
-__device__ __forceinline__ void for_fast_chunks(FastCta& cta, const unsigned char* flags, int tasks, F f) {
-    int t = blockIdx.x, word = chunk_flags(flags, t);
-    while (t < tasks) {
-        const int next = t + gridDim.x, next_word = next < tasks ? chunk_flags(flags, next) : 0;
-        if (!(word & FLAG_SLOW)) {
-            f(t);
-            cta.parity ^= 1;
-        }
-        t = next;
-        word = next_word;
-    }
-}
-
-// The slow chunks of a launch (all of them without flags), shared out over the CTAs by their rank, so that a CTA's share
-// does not depend on where they lie.
+// The slow chunks of a launch, shared out over the CTAs by their rank, so that a CTA's share does not depend on where they
+// lie.  The flags are older than the launch before: they are looked through while that one still runs, 16 a thread, so that
+// a launch without slow chunks ends as soon as its predecessor does.
 template <class F>
 __device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int tasks, F f) {
-    if (flags == nullptr) {
-        for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
-            f(t);
-            __syncthreads();   // the next chunk's loads overwrite what this one reads
-        }
-        return;
+    unsigned any = 0;
+    for (int t0 = threadIdx.x * 16; t0 < tasks; t0 += NTHREADS * 16) {   // the flag panel has room past the last chunk
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + t0));
+        const unsigned words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & FLAG_SLOW;
     }
+    any = __syncthreads_or(any);
+    chain_wait();
+    chain_release();
+    if (any == 0) return;
     int rank = 0;
-    constexpr int WINDOW = NTHREADS * 16;   // one 16-byte load per thread tells whether there is a slow chunk at all
-    for (int base = 0; base < tasks; base += WINDOW) {
-        const int t0 = base + threadIdx.x * 16;
-        unsigned any = 0;
-        if (t0 < tasks) {   // the flag panel has room past the last chunk
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + t0));
-            const unsigned words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & FLAG_SLOW;
-        }
-        if (__syncthreads_or(any) == 0) continue;
-        for (int b = base; b < tasks && b < base + WINDOW; b += 32) {
-            const int t = b + (threadIdx.x & 31);
-            unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & FLAG_SLOW));
-            while (slow != 0) {
-                if (rank++ % gridDim.x == blockIdx.x) {
-                    f(b + __ffs(slow) - 1);
-                    __syncthreads();
-                }
-                slow &= slow - 1;
+    for (int b = 0; b < tasks; b += 32) {
+        const int t = b + (threadIdx.x & 31);
+        unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & FLAG_SLOW));
+        while (slow != 0) {
+            if (rank++ % gridDim.x == blockIdx.x) {
+                f(b + __ffs(slow) - 1);
+                __syncthreads();   // the next chunk's loads overwrite what this one reads
             }
+            slow &= slow - 1;
         }
     }
 }
@@ -190,12 +180,28 @@ __device__ __forceinline__ uint2 pack4_bf16(const float (&x)[4]) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(x[0], x[1]), b = __floats2bfloat162_rn(x[2], x[3]);
     return make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
 }
+// Loads that stay where they are written: a row pass requests all its rows before it uses one.  (Left to itself the compiler
+// moves each load to its first use, which makes several memory latencies of one.)
+__device__ __forceinline__ uint2 ld_pinned8(const void* p, bool ok) {   // zeros unless ok
+    uint2 v;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t@p ld.global.v2.b32 {%0, %1}, [%2];\n\t}"
+        : "=r"(v.x), "=r"(v.y)
+        : "l"(p), "r"((unsigned)ok));
+    return v;
+}
+__device__ __forceinline__ float4 ld_pinned16(const float* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 // Four channels of a BF16 row as they lie, zeros past the width and where the row is not `valid`
 template <bool FAST>
 __device__ __forceinline__ uint2 load4_raw(const bf16* row, int c0, int width, int vec, bool valid) {
+    if (FAST) return ld_pinned8(row + c0, valid && c0 < width);
     uint2 raw = make_uint2(0u, 0u);
     if (!valid || c0 >= width) return raw;
-    if (FAST || (vec && c0 + 4 <= width)) return *reinterpret_cast<const uint2*>(row + c0);
+    if (vec && c0 + 4 <= width) return *reinterpret_cast<const uint2*>(row + c0);
     const unsigned short* src = reinterpret_cast<const unsigned short*>(row) + c0;
     raw.x = src[0];
     if (c0 + 1 < width) raw.x |= (unsigned)src[1] << 16;

@@ -581,11 +581,16 @@ __device__ __forceinline__ void primal_exterior_blocks(const FwdParams& p, const
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p, int tasks) {
     extern __shared__ __align__(16) float smem[];
-    chain_wait();
-    chain_release();
-    for_slow_chunks(PRED ? nullptr : p.Flags, tasks, [&](int t) {
-        primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem);
-    });
+    if constexpr (PRED) {
+        chain_wait();
+        chain_release();
+        for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
+            primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem);
+            __syncthreads();
+        }
+    } else {
+        for_slow_chunks(p.Flags, tasks, [&](int t) { primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem); });
+    }
 }
 
 // The output rows y = Xg S_c + tril(Aqd) Z~ are k_output_fwd_tc (sd_output_tc.cuh).

@@ -9,8 +9,8 @@
 // operand [chi exp(G); -e exp(G)] (128 rows: one contraction gives both pair matrices) and S2 d exp(-G) in place of d;
 // then S0 z, S1 Aed and S2 -e exp(G), whose FP32 values wait in tensor memory meanwhile, for the solve.
 //
-// What bounds it: the latency of a chunk's chain (21 us alone on an SM) and, with two on an SM, shared-memory and
-// global accesses (64 % of the load/store pipe's wavefronts; DRAM 3.4 TB/s).  At 8 x 4096 tokens of 8 heads 530 us against
+// What bounds it: the latency of a chunk's chain (19 us alone on an SM) and, with two on an SM, shared-memory and
+// global accesses (60 % of the load/store pipe's wavefronts; DRAM 3.4 TB/s).  At 8 x 4096 tokens of 8 heads 492 us against
 // 838 us of the block-centred kernel; two chunks of 256 threads with 128 registers to an SM took 583 us, a next row kept in
 // registers 600 us (spills), and prefetching the next task's panels into L2 40 us more.
 // Tensor memory (256 columns): 0 D2, later the FP32 -e exp(G); 128 K^ Delta^T, later the pair matrices; 192 tril(K^ Delta^T).
@@ -189,7 +189,7 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
         unpack4(*reinterpret_cast<const float4*>(s_lam + c0), lam);
 #pragma unroll 1
         for (int it = 0; it < FAST_PASSES; ++it) {
-            const int i = cta.warp + 16 * it, i0 = i & ~(BT - 1);
+            const int i = cta.warp + 16 * it;
             SourceRow row;
             {
                 const bool ok = ch.ok(i);
@@ -197,8 +197,8 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
                 row.q = load4_raw<FAST>(row_bf16(p.q, ch, i), c0, r, p.q.vec, ok);
                 row.u = load4_raw<FAST>(row_bf16(p.u, ch, i), c0, r, p.u.vec, ok);
                 row.er = load4_raw<FAST>(row_bf16(p.er, ch, i), c0, r, p.er.vec, ok);
-                row.dl = *reinterpret_cast<const float4*>(gDelta + i * DP + c0);
-                row.g = *reinterpret_cast<const float4*>(gG + i * DP + c0);
+                row.dl = ld_pinned16(gDelta + i * DP + c0);
+                row.g = ld_pinned16(gG + i * DP + c0);
             }
             float k[4], q[4], dl[4], bk[4], sums[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             unpack4(row.k, k);
@@ -252,20 +252,7 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
             *reinterpret_cast<uint2*>(p.Xg + at) = pack4_bf16(xg);
             if (keep) {
                 *reinterpret_cast<uint2*>(p.Ag + at) = pack4_bf16(ag);
-                // block-centred operands of the reverse kernels
-                float Gp[4], Ge[4];
-                unpack4(*reinterpret_cast<const float4*>(gG + (i0 ? i0 - 1 : 0) * DP + c0), Gp);
-                unpack4(*reinterpret_cast<const float4*>(gG + (i0 + BT - 1) * DP + c0), Ge);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float f = i0 ? exp_ftz(-Gp[e]) : 1.f;
-                    xg[e] *= f;
-                    ag[e] *= f;
-                    Ge[e] = d[e] * exp_ftz(Ge[e]);
-                }
-                *reinterpret_cast<uint2*>(p.Xr + at) = pack4_bf16(xg);
-                *reinterpret_cast<uint2*>(p.Er + at) = pack4_bf16(ag);
-                *reinterpret_cast<uint2*>(p.Dcol + at) = pack4_bf16(Ge);
+                *reinterpret_cast<uint2*>(p.Dcol + at) = pack4_bf16(d);
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) d[e] *= lam[e];
@@ -350,16 +337,16 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
         store_half_tile<true>(cta, panel_ptr(p.Wd, ch.gi) + 32 * pt, tile);   // a contraction operand of the state scan
     else
         store_half_tile<false>(cta, panel_ptr(p.Ud, ch.gi) + 32 * pt, tile);
-    __syncthreads();   // the next task's loads overwrite the slots
     SD_PHASE_T(p.g, ch, ph);
 }
 
 template <bool FAST, bool MASKED>
-__global__ void __launch_bounds__(NTHREADS, 2) k_primal_exterior_fast(FwdParams p, int tasks) {
+__global__ void __launch_bounds__(NTHREADS, 2) k_primal_exterior_fast(FwdParams p) {
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (leave_to_slow_kernel(p.Flags)) return;
     FastCta cta;
-    fast_setup(cta, fsm_raw, p.fault);
-    for_fast_chunks(cta, p.Flags, tasks, [&](int t) { primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, t), cta); });
+    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
 
