@@ -399,14 +399,20 @@ cudaError_t configure_kernels() {
     if ((e = allow_smem(k_primal_exterior_fwd<true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
     if ((e = allow_smem(k_primal_exterior_fwd<false, true, true>, PRIMAL_EXT_FWD_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<true, false>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<false, false>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<true, true>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_primal_exterior_fast<false, true>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_exterior_pair_fast<true, false>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_exterior_pair_fast<false, false>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_exterior_pair_fast<true, true>, FAST_SMEM)) != cudaSuccess) return e;
-    if ((e = allow_smem(k_exterior_pair_fast<false, true>, FAST_SMEM)) != cudaSuccess) return e;
+#define SD_ALLOW_KINDS_OF(name, smem, F, M)                                                 \
+    if ((e = allow_smem(name##_fast<F, M>, FAST_SMEM)) != cudaSuccess) return e;           \
+    if ((e = allow_smem(name##_one<F, M>, smem)) != cudaSuccess) return e
+#define SD_ALLOW_KINDS(name, smem)               \
+    SD_ALLOW_KINDS_OF(name, smem, true, false);  \
+    SD_ALLOW_KINDS_OF(name, smem, false, false); \
+    SD_ALLOW_KINDS_OF(name, smem, true, true);   \
+    SD_ALLOW_KINDS_OF(name, smem, false, true)
+    SD_ALLOW_KINDS(k_primal_exterior, PRIMAL_EXT_FWD_SMEM);
+    SD_ALLOW_KINDS(k_exterior_pair, EXT_PAIR_BWD_SMEM);
+    SD_ALLOW_KINDS(k_primal, PRIMAL_BWD_SMEM);
+    SD_ALLOW_KINDS(k_predictor_close, PRED_CLOSE_BWD_SMEM);
+#undef SD_ALLOW_KINDS
+#undef SD_ALLOW_KINDS_OF
     if ((e = allow_smem(k_state_scan_tc<false>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_state_scan_tc<true>, SCAN_TC_SMEM_BYTES)) != cudaSuccess) return e;
     if ((e = allow_smem(k_output_fwd_tc<false>, OUTPUT_TC_SMEM)) != cudaSuccess) return e;
@@ -491,27 +497,35 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_
         else launch(kernel<false, true>, chunks, NTHREADS, smem, chained, stream, p);                   \
     } while (0)
 
-// ... a pair of them (sd_chunk_tc.cuh): the slow chunks with one CTA to an SM, and the fast ones with two
-// Masked calls have slow chunks wherever a sequence starts: those go first, and the fast chunks fill the SMs around them
-// (5 x 1531 tokens with masks 1088 -> 1072 us).  Without masks slow chunks are the exception: they go last, and
-// the fast kernel starts while its predecessor ends (128 chunks: 20 us in the CTA against 28 behind an empty launch).
-#define SD_LAUNCH_PAIR(fast_kernel, kernel, smem)                                                            \
-    do {                                                                                                     \
-        const int g1 = chunks < 148 ? chunks : 148;                                                          \
-        if (fast && !masked) {                                                                               \
-            launch(fast_kernel<true, false>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
-            launch(kernel<true, false>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
-        } else if (fast) {                                                                                   \
-            launch(kernel<true, true>, g1, NTHREADS, smem, true, stream, p, chunks);                         \
-            launch(fast_kernel<true, true>, chunks, NTHREADS, FAST_SMEM, true, stream, p);            \
-        } else if (!masked) {                                                                                \
-            launch(fast_kernel<false, false>, chunks, NTHREADS, FAST_SMEM, true, stream, p);              \
-            launch(kernel<false, false>, g1, NTHREADS, smem, true, stream, p, chunks);                       \
-        } else {                                                                                             \
-            launch(kernel<false, true>, g1, NTHREADS, smem, true, stream, p, chunks);                        \
-            launch(fast_kernel<false, true>, chunks, NTHREADS, FAST_SMEM, true, stream, p);           \
-        }                                                                                                    \
+// The chunk kernels that come in two kinds (sd_chunk_tc.cuh).  Up to 32 chunks both kinds are in one launch, NAME_one: such a
+// call takes the host longer to issue (165 us forward and reverse) than the GPU to run, and four launches more cost it 9 us.
+// From 64 chunks on the GPU is what is waited for and the larger kernels are slower (64 chunks 247 us of kernels against 229,
+// 128 chunks 331 against 305, the same 195 at 32).  Beyond 32, slow chunks run with one CTA to an SM and fast ones with two.
+// Masked calls have slow chunks wherever a sequence starts: those go first, and the fast chunks fill the SMs around them (5 x
+// 1531 tokens with masks 1088 -> 1072 us).  Without masks slow chunks are the exception: they go last, and the fast kernel
+// starts while its predecessor ends.
+constexpr int ONE_LAUNCH_CHUNKS = 32;
+#define SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, F, M)                                          \
+    do {                                                                                           \
+        if (chunks <= ONE_LAUNCH_CHUNKS) {                                                                 \
+            launch(name##_one<F, M>, chunks, NTHREADS, smem, true, stream, p);                     \
+        } else if (M) {                                                                            \
+            launch(slow_kernel<F, M>, chunks < 148 ? chunks : 148, NTHREADS, smem, true, stream, p, chunks); \
+            launch(name##_fast<F, M>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
+        } else {                                                                                   \
+            launch(name##_fast<F, M>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
+            launch(slow_kernel<F, M>, chunks < 148 ? chunks : 148, NTHREADS, smem, true, stream, p, chunks); \
+        }                                                                                          \
     } while (0)
+#define SD_LAUNCH_KINDS(name, slow_kernel, smem)                                                   \
+    do {                                                                                           \
+        if (fast && !masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, true, false);             \
+        else if (fast) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, true, true);                    \
+        else if (!masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, false, false);               \
+        else SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, false, true);                             \
+    } while (0)
+constexpr int KINDS_FORWARD = 1, KINDS_BACKWARD = 3;
+int kind_launches(const sd_shape* s, int kinds) { return total_chunks(s) <= ONE_LAUNCH_CHUNKS ? 0 : kinds; }
 
 bool operands_ok(const sd_operand* ops, int n) {
     for (int i = 0; i < n; ++i)
@@ -663,11 +677,11 @@ int sd_panel_kind(const sd_shape* shape, int which, const char* name) {
 // a scan that is cut into segments is three launches
 int sd_forward_launches(const sd_shape* shape) {
     if (!shape_ok(shape)) return 0;
-    return 6 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, FWD_STEP_US, FWD_TRANSFER_US) > 1 ? 4 : 0);
+    return 5 + kind_launches(shape, KINDS_FORWARD) + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, FWD_STEP_US, FWD_TRANSFER_US) > 1 ? 4 : 0);
 }
 int sd_backward_launches(const sd_shape* shape) {
     if (!shape_ok(shape)) return 0;
-    return 7 + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, BWD_STEP_US, BWD_TRANSFER_US) > 1 ? 4 : 0);
+    return 6 + kind_launches(shape, KINDS_BACKWARD) + (scan_segments(shape->B * shape->H, (shape->T + CL - 1) / CL, BWD_STEP_US, BWD_TRANSFER_US) > 1 ? 4 : 0);
 }
 int sd_chunk_tokens(void) { return CL; }
 int sd_version(void) { return 1; }
@@ -794,7 +808,7 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         k_primal_exterior_fwd<false, true, true><<<chunks, NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p, chunks);
         return launch_status();   // the kernel stops after its primal half
     }
-    SD_LAUNCH_PAIR(k_primal_exterior_fast, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
+    SD_LAUNCH_KINDS(k_primal_exterior, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
     mark(stream);
     {
         ScanParams sp{};
@@ -930,14 +944,14 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     mark(stream);
     }
     set_dbg(p.g, 7, chunks);
-    SD_LAUNCH_PAIR(k_exterior_pair_fast, k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM);
+    SD_LAUNCH_KINDS(k_exterior_pair, k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM);
     mark(stream);
     }
     set_dbg(p.g, 8, chunks);
     if (po)
-        k_primal_bwd<false, true, true><<<chunks, NTHREADS, PRIMAL_BWD_SMEM, stream>>>(p);
+        k_primal_bwd<false, true, true><<<chunks, NTHREADS, PRIMAL_BWD_SMEM, stream>>>(p, chunks);
     else
-        SD_LAUNCH_CHUNK(k_primal_bwd, PRIMAL_BWD_SMEM, true);
+        SD_LAUNCH_KINDS(k_primal, k_primal_bwd, PRIMAL_BWD_SMEM);
     mark(stream);
     {
         ScanParamsB sp{};
@@ -950,9 +964,9 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     }
     set_dbg(p.g, 10, chunks);
     if (po)
-        k_predictor_close_bwd<false, true, true><<<chunks, NTHREADS, PRED_CLOSE_BWD_SMEM, stream>>>(p);
+        k_predictor_close_bwd<false, true, true><<<chunks, NTHREADS, PRED_CLOSE_BWD_SMEM, stream>>>(p, chunks);
     else
-        SD_LAUNCH_CHUNK(k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM, true);
+        SD_LAUNCH_KINDS(k_predictor_close, k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM);
     mark(stream);
     return launch_status();
 }

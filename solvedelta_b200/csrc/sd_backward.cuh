@@ -480,7 +480,7 @@ __device__ __forceinline__ void exterior_pair_blocks(const BwdParams& p, const C
 template <bool FAST, bool MASKED>
 __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_bwd(BwdParams p, int tasks) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    for_slow_chunks(p.Flags, tasks, [&](int t) { exterior_pair_blocks<FAST, MASKED>(p, chunk_of<MASKED>(p.g, t), smem_raw); });
+    for_slow_chunks<FLAG_SLOW>(p.Flags, tasks, [&](int t) { exterior_pair_blocks<FAST, MASKED>(p, chunk_of<MASKED>(p.g, t), smem_raw); });
 }
 
 // ---------------------------------------------------------------------------
@@ -537,13 +537,10 @@ constexpr size_t PRIMAL_BWD_SMEM = 7 * BSLOT_BYTES + BSTATE_BYTES + 2 * BMAT_BYT
                                    (3 * CL + 4 * CL + NBLK * DP + 16) * sizeof(float) +
                                    (3 + NBLK) * DP * sizeof(bf16);
 
-template <bool FAST, bool MASKED, bool PRED = false>
-__global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
-    chain_wait();
-    chain_release();
+template <bool FAST, bool MASKED, bool PRED>
+__device__ __forceinline__ void primal_blocks(const BwdParams& p, const ChunkT<MASKED> ch, unsigned char* smem_raw) {
     int ph = 0;
     SD_PHASE(p.g, ph);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* b_uc = reinterpret_cast<bf16*>(smem_raw);   // u^ col
     bf16* b_ur = b_uc + BSLOT_ELEMS;   // u^ itself (diagonal blocks), then t_u off the diagonal blocks
     bf16* b_ub = b_ur + BSLOT_ELEMS;   // Ubar, then Q''
@@ -565,7 +562,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
     int* s_fastw = reinterpret_cast<int*>(s_beta + NBLK * DP);
     bf16* s_Mb = reinterpret_cast<bf16*>(s_fastw + 16);
     bf16* s_ibeta_b = s_Mb + 3 * DP;
-    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const int r = p.g.r;
     const float* gG = panel_ptr(p.Gp, ch.gi);
     const bf16* gDd = bpanel_ptr(p.Dd, ch.gi);
@@ -789,6 +785,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p) {
     SD_PHASE(p.g, ph);
 }
 
+// The slow chunks of a launch, one CTA per SM that walks over them (every chunk, one a CTA, for the predictor-only entry).
+template <bool FAST, bool MASKED, bool PRED = false>
+__global__ void __launch_bounds__(NTHREADS, 1) k_primal_bwd(BwdParams p, int tasks) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if constexpr (PRED) {
+        chain_wait();
+        chain_release();
+        primal_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, blockIdx.x), smem_raw);
+    } else {
+        for_slow_chunks<FLAG_SLOW>(p.Flags, tasks, [&](int t) {
+            primal_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem_raw);
+        });
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Last kernel of the reverse pass: the contractions that need the scanned
 // dRr / dC, then the gate closure, in one CTA.
@@ -807,13 +818,10 @@ constexpr size_t PRED_CLOSE_BWD_SMEM = 5 * BSLOT_BYTES + 2 * BMAT_BYTES + 3 * si
                                        6 * DP * sizeof(bf16);
 static_assert(3 * size_t(CL) * LDP * 4 >= 2 * BSTATE_BYTES, "closure panels overlay both BF16 states");
 
-template <bool FAST, bool MASKED, bool PRED = false>
-__global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p) {
-    chain_wait();
-    chain_release();
+template <bool FAST, bool MASKED, bool PRED>
+__device__ __forceinline__ void predictor_close_blocks(const BwdParams& p, const ChunkT<MASKED> ch, unsigned char* smem_raw) {
     int ph = 0;
     SD_PHASE(p.g, ph);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* b_ur = reinterpret_cast<bf16*>(smem_raw);   // u^ rowE -> dUbar
     bf16* b_uc = b_ur + BSLOT_ELEMS;                   // u^ col  -> dUt
     bf16* b_dl = b_uc + BSLOT_ELEMS;                   // Delta   -> t_i
@@ -835,7 +843,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
     int* s_fastw = reinterpret_cast<int*>(s_beta + NBLK * DP);
     bf16* s_Mb = reinterpret_cast<bf16*>(s_fastw + 16);
     bf16* s_pref = s_Mb + 3 * DP;   // exp(Gprev_I) for I = 1..3: U~ = (u^ rowE) .* pref along channels
-    const ChunkT<MASKED> ch = chunk_of<MASKED>(p.g, blockIdx.x);
     const int r = p.g.r;
     const float* gG = panel_ptr(p.Gp, ch.gi);
     auto fG = [&](int i, int c) { return gG[i * DP + c]; };
@@ -1109,6 +1116,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p
         }
     }
     SD_PHASE(p.g, ph);
+}
+
+// The slow chunks of a launch, one CTA per SM that walks over them (every chunk, one a CTA, for the predictor-only entry).
+template <bool FAST, bool MASKED, bool PRED = false>
+__global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_bwd(BwdParams p, int tasks) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if constexpr (PRED) {
+        chain_wait();
+        chain_release();
+        predictor_close_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, blockIdx.x), smem_raw);
+    } else {
+        for_slow_chunks<FLAG_SLOW | FLAG_GAMMA>(p.Flags, tasks, [&](int t) {
+            predictor_close_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem_raw);
+        });
+    }
 }
 
 }  // namespace sd

@@ -341,10 +341,626 @@ __device__ __forceinline__ void exterior_pair_fast(const BwdParams& p, const Chu
 template <bool FAST, bool MASKED>
 __global__ void __launch_bounds__(NTHREADS, 2) k_exterior_pair_fast(BwdParams p) {
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
-    if (leave_to_slow_kernel(p.Flags)) return;
+    if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
     FastCta cta;
     fast_setup<!MASKED>(cta, fsm_raw, p.fault);
     exterior_pair_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+// Both kinds of chunk in one launch, for calls that leave SMs empty anyway.
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_one(BwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (chunk_flags(p.Flags, blockIdx.x) & (FLAG_SLOW)) {
+        chain_wait();
+        chain_release();
+        exterior_pair_blocks<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), fsm_raw);
+        return;
+    }
+    FastCta cta;
+    fast_setup<true>(cta, fsm_raw, p.fault);
+    exterior_pair_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+
+// ---------------------------------------------------------------------------
+// FP32 accumulator columns 32 part .. of this warp's lanes (rows i) as pieces of an FP32 tiled panel
+__device__ __forceinline__ void acc32_to_f32_tiles(const FastCta& cta, unsigned taddr, unsigned char* sm, int i) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int col = 32 * cta.part + 16 * h;
+        float a[16];
+        tc_ld16(taddr + col, a);
+        tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+            *reinterpret_cast<float4*>(sm + f32_off<F32_TILE>(i, col + j)) = make_float4(a[j], a[j + 1], a[j + 2], a[j + 3]);
+    }
+}
+
+// trisolve_blocked (sd_bf16.cuh) on two BF16 panels of tiles: each of the sixteen warps owns 16 of the 256 columns, pieces
+// piece0 and piece0 + 1 of `tile`.
+template <bool UPPER>
+__device__ __forceinline__ void trisolve_bf16_tiles(const FastCta& cta, float* Mr, float sgn, unsigned char* tile, int piece0) {
+    const int g = cta.lane >> 2, t = cta.lane & 3;
+    constexpr int NB = CL / 16, NT = 2;
+    if (cta.warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * cta.warp) * LDA + 16 * cta.warp, sgn);
+    __syncthreads();
+    auto at2 = [&](int i, int nt) {   // i mod 8 = g; columns 8 nt + 2 t, + 1
+        return reinterpret_cast<__nv_bfloat162*>(tile + i * 128 + (((piece0 + nt) ^ g) << 4) + (t << 2));
+    };
+    auto get = [&](int kk, int odd, int nt) {   // row kk + 2 t + odd, column 8 nt + g
+        return __bfloat162float(*reinterpret_cast<const bf16*>(tile + (kk + 2 * t + odd) * 128 + (((piece0 + nt) ^ (2 * t + odd)) << 4) + (g << 1)));
+    };
+    auto contract = [&](float (&acc)[NT][4], int r0, int kbeg, int kend) {
+#pragma unroll
+        for (int kk = kbeg; kk < kend; kk += 8) {   // permuted contraction index, as in warp_mma_pairs
+            const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
+            const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
+            const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)   // a BF16 number is a TF32 number
+                mma_tf32(acc[nt], a0, a1, a2, a3, __float_as_uint(get(kk, 0, nt)), __float_as_uint(get(kk, 1, nt)));
+        }
+    };
+#pragma unroll
+    for (int step = 0; step < NB; ++step) {
+        const int I = UPPER ? (NB - 1 - step) : step, r0 = 16 * I;
+        float rr[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const float2 a = __bfloat1622float2(*at2(r0 + g, nt)), b = __bfloat1622float2(*at2(r0 + g + 8, nt));
+            rr[nt][0] = a.x; rr[nt][1] = a.y; rr[nt][2] = b.x; rr[nt][3] = b.y;
+        }
+        if (step > 0) {
+            float acc[NT][4];
+            acc_zero<NT>(acc);
+            contract(acc, r0, UPPER ? r0 + 16 : 0, UPPER ? CL : r0);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) rr[nt][e] = fmaf(-sgn, acc[nt][e], rr[nt][e]);
+                *at2(r0 + g, nt) = __floats2bfloat162_rn(rr[nt][0], rr[nt][1]);
+                *at2(r0 + g + 8, nt) = __floats2bfloat162_rn(rr[nt][2], rr[nt][3]);
+            }
+            __syncwarp();
+        }
+        float acc[NT][4];
+        acc_zero<NT>(acc);
+        contract(acc, r0, r0, r0 + 16);
+        __syncwarp();   // every lane has read the block's right-hand sides
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            *at2(r0 + g, nt) = __floats2bfloat162_rn(rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
+            *at2(r0 + g + 8, nt) = __floats2bfloat162_rn(rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
+        }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// k_primal_fast: reverse of the primal address and preparation of the dC scan (k_primal_bwd).  With DG = dd exp(G), Ucol =
+// u^ exp(-G) and the stack [K^; DG]:
+//     Aqk = tril(K^ Delta^T), dAqk = tril(DG Ucol^T)        t_u = exp(-G) (Aqk^T DG)
+//     dk^ = dkPart + DG Ct + dAqk Delta                     dDelta_loc = dDelta + dAqk^T K^
+//     P'' = (I+Lm)^-T dDelta_loc,  Q'' = (I+Lm)^-T Ubar,  Rneg = -gamma u^ exp(E)
+// Shared memory (112 KB): the stack 32, Delta 16, the stacked pair matrices 16, Ucol then Ubar 16, Ct 32; the three results
+// that leave FP32 take the stack, Delta with the pair matrices, and Ct; then the solve has its matrix in the stack's place
+// and dDelta_loc in Ct's.  At 8 x 4096 tokens of 8 heads 391 us against 559 us of the block-centred kernel; bound like the
+// kernel before (the head, seven loads a row deep, is a third of the chain).  Tensor memory: 0 and 64 the pair matrices, then t_u; 128 dk^, then dDelta.
+constexpr unsigned PB_A = 0, PB_DL = 32 * 1024, PB_PP = 48 * 1024, PB_UC = 64 * 1024, PB_CT = 80 * 1024, PB_GAM = 112 * 1024;
+constexpr unsigned PB_DK = PB_CT, PB_TU = PB_DL, PB_DD = PB_A, PB_RHS = PB_CT, PB_LM = PB_A;
+static_assert(PB_GAM + CL * 4 <= FAST_BAR_OFF, "tiles and table fit");
+
+template <bool FAST, bool MASKED>
+__device__ __forceinline__ void primal_fast(const BwdParams& p, const ChunkT<MASKED>& ch, FastCta& cta) {
+    unsigned char* sm = cta.sm;
+    const unsigned smem = tc_smem(sm);
+    float* s_gam = reinterpret_cast<float*>(sm + PB_GAM);
+    const int r = p.g.r, c0 = cta.lane * 4;
+    int ph = 0;
+    SD_PHASE_T(p.g, ch, ph);
+    async_tiles<CL, 2 * BF_TILE>(sm + PB_A + BF_TILE, bpanel_ptr(p.DG, ch.gi));
+    cp_commit();
+    async_tiles<DP, 2 * BF_TILE>(sm + PB_CT, bstate_ptr(p.CtCkB, ch.gi));
+    cp_commit();
+    load_gamma(p.gam, ch, s_gam);
+    __syncthreads();
+    uint2 ubar[FAST_PASSES];
+    const long long at0 = ch.gi * (CL * DP) + (4 * cta.warp) * DP + c0;   // rows 4 warp .. of every panel
+    {
+        uint2 ku[2 * FAST_PASSES];
+        float4 G[FAST_PASSES + 1];
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            const int i = 4 * cta.warp + it;
+            ku[it] = load4_raw<FAST>(row_bf16(p.k, ch, i), c0, r, p.k.vec, ch.ok(i));
+            ku[FAST_PASSES + it] = load4_raw<FAST>(row_bf16(p.u, ch, i), c0, r, p.u.vec, ch.ok(i));
+            G[it + 1] = ld_pinned16(p.Gp + at0 + it * DP);
+        }
+        G[0] = cta.warp > 0 ? ld_pinned16(p.Gp + at0 - DP) : make_float4(0.f, 0.f, 0.f, 0.f);   // E of a row is G of the one before
+        float lam[4], ss[8];
+        unpack4(*reinterpret_cast<const float4*>(p.Lam + ch.gi * DP + c0), lam);
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            float x[4];
+            unpack4(ku[n], x);
+            ss[n] = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+        }
+        row_sums32(ss);
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            const int i = 4 * cta.warp + it;
+            float x[4], g[4], E[4], o[4];
+            unpack4(ku[it], x);
+            const float rk = rsqrtf(ss[it] + 1e-24f), ru = rsqrtf(ss[FAST_PASSES + it] + 1e-24f), gm = s_gam[i];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] *= rk;
+            const uint2 kh = pack4_bf16(x);
+            *reinterpret_cast<uint2*>(sm + PB_A + bf_off4<2 * BF_TILE>(i, cta.lane)) = kh;
+            *reinterpret_cast<uint2*>(p.Khat + at0 + it * DP) = kh;
+            unpack4(ku[FAST_PASSES + it], x);
+            unpack4(G[it + 1], g);
+            unpack4(G[it], E);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                x[e] *= ru;
+                g[e] = x[e] * exp_ftz(-g[e]);
+                o[e] = -gm * x[e] * exp_ftz(E[e]);
+            }
+            *reinterpret_cast<uint2*>(p.Rneg + at0 + it * DP) = pack4_bf16(o);
+            *reinterpret_cast<uint2*>(sm + PB_UC + bf_off4<BF_TILE>(i, cta.lane)) = pack4_bf16(g);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) g[e] *= lam[e];
+            ubar[it] = pack4_bf16(g);
+            unpack4(ld_pinned16(p.Delta + at0 + it * DP), x);
+            *reinterpret_cast<uint2*>(sm + PB_DL + bf_off4<BF_TILE>(i, cta.lane)) = pack4_bf16(x);
+        }
+    }
+    cp_wait<1>();
+    cta.publish();
+    SD_PHASE_T(p.g, ch, ph);
+    if (cta.tid == 0) {
+        tc_fence_after();
+        mma_bf<DP, 2 * BF_TILE, false, BF_TILE, false>(cta.tmem, smem + PB_A, smem + PB_DL, CL, 0u);
+        mma_bf<DP, 2 * BF_TILE, false, BF_TILE, false>(cta.tmem + CL, smem + PB_A, smem + PB_UC, CL, 0u);
+        tc_commit(cta.bar(0));
+    }
+    __syncwarp();
+    cp_wait<0>();
+    cta.publish();
+    if (cta.tid == 32) {
+        tc_fence_after();
+        mma_bf<DP, 2 * BF_TILE, false, 2 * BF_TILE, true>(cta.tmem + 128, smem + PB_A, smem + PB_CT, DP, 0u);   // lanes 64 ..: DG Ct
+    }
+    __syncwarp();
+    cta.wait(0, 11);
+    const int row = 32 * cta.quarter + cta.lane;
+    {   // lanes 0 .. 63: Aqk, lanes 64 .. 127: dAqk
+        float a[16];
+        tc_ld16(cta.lanes() + (cta.quarter < 2 ? 0 : CL) + 16 * cta.part, a);
+        tc_wait_ld();
+        const int i = row & (CL - 1), j0 = 16 * cta.part;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = j0 + 8 * h + e <= i ? a[8 * h + e] : 0.f;
+            *reinterpret_cast<uint4*>(sm + PB_PP + bf_off<BF_TILE>(row, 2 * cta.part + h)) = pack8_bf16(w);
+        }
+    }
+#pragma unroll
+    for (int it = 0; it < FAST_PASSES; ++it)   // Ucol is free
+        *reinterpret_cast<uint2*>(sm + PB_UC + bf_off4<BF_TILE>(4 * cta.warp + it, cta.lane)) = ubar[it];
+    cta.publish();
+    if (cta.tid == 32) {   // the thread that issued DG Ct: the sum goes on in order
+        tc_fence_after();
+        mma_bf<CL, BF_TILE, false, BF_TILE, true>(cta.tmem + 128, smem + PB_PP, smem + PB_DL, DP, 1u);   // + dAqk Delta
+        tc_commit(cta.bar(2));
+        mma_bf<CL, BF_TILE, true, 2 * BF_TILE, true>(cta.tmem, smem + PB_PP, smem + PB_A + BF_TILE, DP, 0u);   // Aqk^T DG
+        tc_commit(cta.bar(3));
+    }
+    __syncwarp();
+    SD_PHASE_T(p.g, ch, ph);
+    cta.wait(2, 12);
+    if (cta.quarter >= 2) acc32_to_f32_tiles(cta, cta.lanes() + 128, sm + PB_DK, row - CL);
+    tc_fence_before();
+    __syncthreads();
+    if (cta.tid == 96) {
+        tc_fence_after();
+        mma_bf<CL, BF_TILE, true, 2 * BF_TILE, true>(cta.tmem + 128, smem + PB_PP + BF_TILE, smem + PB_A, DP, 0u);   // dAqk^T K^
+        tc_commit(cta.bar(4));
+    }
+    __syncwarp();
+    cta.wait(3, 13);
+    cta.wait(4, 14);   // the operands are free: t_u takes the place of Delta and the pair matrices, dDelta that of the stack
+    if (cta.quarter < 2) {
+        acc32_to_f32_tiles(cta, cta.lanes(), sm + PB_TU, row);
+        acc32_to_f32_tiles(cta, cta.lanes() + 128, sm + PB_DD, row);
+    }
+    __syncthreads();
+    SD_PHASE_T(p.g, ch, ph);
+    uint2 rhs[FAST_PASSES];
+#pragma unroll
+    for (int it = 0; it < FAST_PASSES; ++it) {
+        const int i = 4 * cta.warp + it;
+        const auto piece = [&](unsigned base) {
+            return reinterpret_cast<const float4*>(sm + base + (cta.lane >> 3) * F32_TILE + i * 128 + (((cta.lane & 7) ^ (i & 7)) << 4));
+        };
+        const uint2 rk_ = load4_raw<FAST>(row_bf16(p.k, ch, i), c0, r, p.k.vec, ch.ok(i));
+        const float4 rg_ = ld_pinned16(p.Gp + at0 + it * DP);
+        const uint2 rd_ = ld_pinned8(p.dDelta + at0 + it * DP, true), rp_ = ld_pinned8(p.dkPart + at0 + it * DP, true);
+        float x[4], y[4];
+        unpack4(rg_, x);
+        unpack4(*piece(PB_TU), y);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] *= exp_ftz(-x[e]);
+        *reinterpret_cast<uint2*>(p.Tu + at0 + it * DP) = pack4_bf16(y);
+        unpack4(rd_, x);
+        unpack4(*piece(PB_DD), y);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] += x[e];
+        rhs[it] = pack4_bf16(y);
+        // dk^ and its norm reverse
+        unpack4(rp_, x);
+        unpack4(*piece(PB_DK), y);
+        float k[4], ss[2] = {0.f, 0.f};
+        unpack4(rk_, k);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            y[e] += x[e];
+            ss[0] = fmaf(k[e], k[e], ss[0]);
+            ss[1] = fmaf(k[e], y[e], ss[1]);
+        }
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], m);
+            ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], m);
+        }
+        const float rk = rsqrtf(ss[0] + 1e-24f), dot = ss[1] * rk * rk;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = (y[e] - dot * k[e]) * rk;
+        store4_bf16<FAST>(p.dk, p.pitch_q, p.g, ch, i, c0, r, y);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < FAST_PASSES; ++it)
+        *reinterpret_cast<uint2*>(sm + PB_RHS + bf_off4<BF_TILE>(4 * cta.warp + it, cta.lane)) = rhs[it];
+    float* s_lm = reinterpret_cast<float*>(sm + PB_LM);
+    g2s_mat_transposed(s_lm, mat_ptr(p.Npair, ch.gi), [&](int i) { return s_gam[i]; });
+    __syncthreads();
+    SD_PHASE_T(p.g, ch, ph);
+    const int panel = cta.warp >> 3, cw = cta.warp & 7;
+    unsigned char* tile = sm + (panel == 0 ? PB_RHS : PB_UC) + (cw >> 2) * BF_TILE;
+    const int piece0 = (cw & 3) * 2;
+    trisolve_bf16_tiles<true>(cta, s_lm, 1.f, tile, piece0);
+    SD_PHASE_T(p.g, ch, ph);
+    bf16* out = (panel == 0 ? bpanel_ptr(p.Ppp, ch.gi) : bpanel_ptr(p.Qpp, ch.gi)) + 16 * cw;
+#pragma unroll
+    for (int it = 0; it < CL / 16; ++it) {   // 32 bytes of a row per lane pair
+        const int i = it * 16 + (cta.lane >> 1), h = cta.lane & 1;
+        *reinterpret_cast<uint4*>(out + i * DP + 8 * h) = *reinterpret_cast<const uint4*>(tile + i * 128 + (((piece0 + h) ^ (i & 7)) << 4));
+    }
+    SD_PHASE_T(p.g, ch, ph);
+}
+
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 2) k_primal_fast(BwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
+    FastCta cta;
+    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    primal_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+// Both kinds of chunk in one launch, for calls that leave SMs empty anyway.
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 1) k_primal_one(BwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (chunk_flags(p.Flags, blockIdx.x) & (FLAG_SLOW)) {
+        chain_wait();
+        chain_release();
+        primal_blocks<FAST, MASKED, false>(p, chunk_of<MASKED>(p.g, blockIdx.x), fsm_raw);
+        return;
+    }
+    FastCta cta;
+    fast_setup<true>(cta, fsm_raw, p.fault);
+    primal_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+
+// ---------------------------------------------------------------------------
+// k_predictor_close_fast: the end of the reverse pass (k_predictor_close_bwd).  With P = stril(dR Delta^T), Ucol = u^ exp(-G)
+// and Rneg = -gamma u^ exp(E):
+//     dUbar = Delta dC_end^T,   W = -gamma (dR Ct^T + P Ucol)  (= dU~ + t_i exp(-E)),   t_j = exp(-G) (P^T Rneg)
+//     dgamma = (dR . Delta) / gamma   since Delta = gamma (h - U~ Ct - stril(N) Delta): no contraction, and neither h nor N
+// (a chunk with a vanishing gamma takes the slow kernel, which evaluates the residual).  A warp takes four token rows in a
+// row, last first, so that the suffix sums of d log_decay need one exchange between the warps.
+// Shared memory (112 KB): Delta, then P, 16; dR 16; Ct 32, then W and t_j; dC 32, then Rneg and dUbar; Ucol 16, then the
+// warps' sums.  At 8 x 4096 tokens of 8 heads 325 us against 635 us of the block-centred kernel, which evaluates the residual
+// and three FP32 panels for the sums.  Tensor memory: 0 P, then W; 128 dUbar, then t_j; 0 again keeps what the row pass leaves for the end.
+constexpr unsigned PC_DL = 0, PC_DR = 16 * 1024, PC_CT = 32 * 1024, PC_DC = 64 * 1024, PC_UC = 96 * 1024, PC_GAM = 112 * 1024;
+constexpr unsigned PC_P = PC_DL, PC_W = PC_CT, PC_TJ = PC_CT + 16 * 1024, PC_RN = PC_DC, PC_DUB = PC_DC + 16 * 1024, PC_TOT = PC_UC;
+constexpr unsigned PC_CDC = PC_GAM + CL * 4;
+static_assert(PC_CDC + DP * 4 <= FAST_BAR_OFF, "tiles and tables fit");
+
+template <bool FAST, bool MASKED>
+__device__ __forceinline__ void predictor_close_fast(const BwdParams& p, const ChunkT<MASKED>& ch, FastCta& cta) {
+    unsigned char* sm = cta.sm;
+    const unsigned smem = tc_smem(sm);
+    float *s_gam = reinterpret_cast<float*>(sm + PC_GAM), *s_cdc = reinterpret_cast<float*>(sm + PC_CDC);
+    const int r = p.g.r, c0 = cta.lane * 4;
+    int ph = 0;
+    SD_PHASE_T(p.g, ch, ph);
+    async_tiles<CL, BF_TILE>(sm + PC_DR, bpanel_ptr(p.dRr, ch.gi));
+    cp_commit();
+    async_tiles<DP, 2 * BF_TILE>(sm + PC_DC, bstate_ptr(p.dCeCk, ch.gi));
+    async_tiles<DP, 2 * BF_TILE>(sm + PC_CT, bstate_ptr(p.CtCkB, ch.gi));
+    cp_commit();
+    load_gamma(p.gam, ch, s_gam);
+    const long long at0 = ch.gi * (CL * DP) + (4 * cta.warp) * DP + c0;   // rows 4 warp .. of every panel
+    {
+        uint2 u[FAST_PASSES];
+        float4 G[FAST_PASSES], dl[FAST_PASSES];
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            const int i = 4 * cta.warp + it;
+            dl[it] = ld_pinned16(p.Delta + at0 + it * DP);
+            u[it] = load4_raw<FAST>(row_bf16(p.u, ch, i), c0, r, p.u.vec, ch.ok(i));
+            G[it] = ld_pinned16(p.Gp + at0 + it * DP);
+        }
+        float ss[4];
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            float x[4];
+            unpack4(dl[it], x);
+            *reinterpret_cast<uint2*>(sm + PC_DL + bf_off4<BF_TILE>(4 * cta.warp + it, cta.lane)) = pack4_bf16(x);
+            unpack4(u[it], x);
+            ss[it] = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+        }
+        row_sums32(ss);
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            float x[4], g[4];
+            unpack4(u[it], x);
+            unpack4(G[it], g);
+            const float ru = rsqrtf(ss[it] + 1e-24f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] *= ru * exp_ftz(-g[e]);
+            *reinterpret_cast<uint2*>(sm + PC_UC + bf_off4<BF_TILE>(4 * cta.warp + it, cta.lane)) = pack4_bf16(x);
+        }
+        cp_wait<1>();
+        cta.publish();
+        if (cta.tid == 0) {
+            tc_fence_after();
+            mma_bf<DP, BF_TILE, false, BF_TILE, false>(cta.tmem, smem + PC_DR, smem + PC_DL, CL, 0u);
+            tc_commit(cta.bar(0));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {   // dgamma
+            float x[4], y[4];
+            unpack4(dl[it], x);
+            unpack4(tile4(sm + PC_DR, 4 * cta.warp + it, cta.lane), y);
+            ss[it] = fmaf(x[0], y[0], fmaf(x[1], y[1], fmaf(x[2], y[2], x[3] * y[3])));
+        }
+        row_sums32(ss);
+        if (cta.lane < FAST_PASSES) {
+            const int i = 4 * cta.warp + cta.lane;
+            const float s = cta.lane == 0 ? ss[0] : cta.lane == 1 ? ss[1] : cta.lane == 2 ? ss[2] : ss[3];
+            if (i < ch.nvalid)
+                p.dgam[((long long)ch.b * p.g.T + ch.t0 + i) * p.g.H + ch.hh] = ch.ok(i) ? s / s_gam[i] : 0.f;
+        }
+    }
+    SD_PHASE_T(p.g, ch, ph);
+    cp_wait<0>();
+    cta.publish();
+    if (cta.tid == 32) {
+        tc_fence_after();
+        mma_bf<DP, BF_TILE, false, 2 * BF_TILE, false>(cta.tmem + 128, smem + PC_DL, smem + PC_DC, DP, 0u);
+        tc_commit(cta.bar(1));
+    }
+    __syncwarp();
+    {   // CdC[c] = sum_a Ct[c][a] dCt_end[c][a], as SdS in exterior_pair_fast
+        const int c = cta.tid >> 2, qt = cta.tid & 3;
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned off = bf_off<2 * BF_TILE>(c, 4 * (k ^ (c & 1)) + qt);
+            float a[8], b[8];
+            unpack8_bf16(*reinterpret_cast<const uint4*>(sm + PC_CT + off), a);
+            unpack8_bf16(*reinterpret_cast<const uint4*>(sm + PC_DC + off), b);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc = fmaf(a[e], b[e], acc);
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        if (qt == 0) s_cdc[c] = p.Lam[ch.gi * DP + c] * (p.SdS[ch.gi * DP + c] + acc);
+    }
+    cta.wait(0, 11);
+    const int row = 32 * cta.quarter + cta.lane;
+    uint4 pair[2];
+    if (cta.quarter < 2) {   // P, strictly lower
+        float a[16];
+        tc_ld16(cta.lanes() + 16 * cta.part, a);
+        tc_wait_ld();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = 16 * cta.part + 8 * h + e < row ? a[8 * h + e] : 0.f;
+            pair[h] = pack8_bf16(w);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();   // P is read, CdC is done
+    if (cta.tid == 64) {
+        tc_fence_after();
+        mma_bf<DP, BF_TILE, false, 2 * BF_TILE, false>(cta.tmem, smem + PC_DR, smem + PC_CT, DP, 0u);
+    }
+    __syncwarp();
+    cta.wait(1, 12);   // Delta and dC are free
+    async_tiles<CL, BF_TILE>(sm + PC_RN, bpanel_ptr(p.Rneg, ch.gi));
+    cp_commit();
+    if (cta.quarter < 2) {
+        *reinterpret_cast<uint4*>(sm + PC_P + bf_off<BF_TILE>(row, 2 * cta.part)) = pair[0];
+        *reinterpret_cast<uint4*>(sm + PC_P + bf_off<BF_TILE>(row, 2 * cta.part + 1)) = pair[1];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)   // dUbar
+            acc16_to_tiles(cta.lanes() + 128 + 32 * cta.part + 16 * h, sm + PC_DUB, row, 4 * cta.part + 2 * h);
+    }
+    cp_wait<0>();
+    cta.publish();
+    if (cta.tid == 64) {   // the thread that issued dR Ct^T: the sum goes on in order
+        tc_fence_after();
+        mma_bf<CL, BF_TILE, false, BF_TILE, true>(cta.tmem, smem + PC_P, smem + PC_UC, DP, 1u);
+        tc_commit(cta.bar(2));
+        mma_bf<CL, BF_TILE, true, BF_TILE, true>(cta.tmem + 128, smem + PC_P, smem + PC_RN, DP, 0u);
+        tc_commit(cta.bar(3));
+    }
+    __syncwarp();
+    SD_PHASE_T(p.g, ch, ph);
+    cta.wait(2, 13);
+    if (cta.quarter < 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            acc16_to_tiles(cta.lanes() + 32 * cta.part + 16 * h, sm + PC_W, row, 4 * cta.part + 2 * h);
+    }
+    cta.wait(3, 14);
+    if (cta.quarter < 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            acc16_to_tiles(cta.lanes() + 128 + 32 * cta.part + 16 * h, sm + PC_TJ, row, 4 * cta.part + 2 * h);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    SD_PHASE_T(p.g, ch, ph);
+    float* s_tot = reinterpret_cast<float*>(sm + PC_TOT);   // [16 warps][DP] sums of dG
+    float* s_x = s_tot + 16 * DP;                            // ... of X
+    {
+        float lam[4], run[4] = {0.f, 0.f, 0.f, 0.f}, X[4] = {0.f, 0.f, 0.f, 0.f};
+        unpack4(*reinterpret_cast<const float4*>(p.Lam + ch.gi * DP + c0), lam);
+#pragma unroll 1
+        for (int it = FAST_PASSES - 1; it >= 0; --it) {
+            const int i = 4 * cta.warp + it;
+            const long long at = at0 + it * DP;
+            const uint2 ru_ = load4_raw<FAST>(row_bf16(p.u, ch, i), c0, r, p.u.vec, ch.ok(i));
+            const float4 rg_ = ld_pinned16(p.Gp + at), re_ = ld_pinned16(p.Gp + (i > 0 ? at - DP : at));
+            const uint2 r1_ = ld_pinned8(p.duPart + at, true), r2_ = ld_pinned8(p.Tu + at, true);
+            const uint2 r3_ = ld_pinned8(p.dGPart + at, true), r4_ = ld_pinned8(p.Xext + at, true);
+            float u[4], ie[4], eE[4], duh[4], w[4], tj[4], dub[4], tu[4];
+            unpack4(ru_, u);
+            unpack4(rg_, ie);
+            unpack4(re_, eE);
+            unpack4(r1_, duh);
+            unpack4(r2_, tu);
+            unpack4(tile4(sm + PC_W, i, cta.lane), w);
+            unpack4(tile4(sm + PC_TJ, i, cta.lane), tj);
+            unpack4(tile4(sm + PC_DUB, i, cta.lane), dub);
+            const float gm = s_gam[i];
+            float ss[2] = {0.f, 0.f};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                ie[e] = exp_ftz(-ie[e]);
+                w[e] *= -gm * (i > 0 ? exp_ftz(eE[e]) : 1.f);   // (dU~ + t_i exp(-E)) exp(E)
+                tj[e] *= ie[e];
+                dub[e] *= lam[e] * ie[e];
+                duh[e] += tu[e] + dub[e] + w[e] + tj[e];
+                ss[0] = fmaf(u[e], u[e], ss[0]);
+                ss[1] = fmaf(u[e], duh[e], ss[1]);
+            }
+#pragma unroll
+            for (int m = 16; m > 0; m >>= 1) {
+                ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], m);
+                ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], m);
+            }
+            const float rs = rsqrtf(ss[0] + 1e-24f), dot = ss[1] * rs * rs;
+            float o[4], dgp[4], xe[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = (duh[e] - dot * u[e]) * rs;
+            store4_bf16<FAST>(p.du, p.pitch_u, p.g, ch, i, c0, r, o);
+            unpack4(tile4(sm + PC_DR, i, cta.lane), o);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] *= gm;
+            store4_bf16<FAST>(p.dh, p.pitch_u, p.g, ch, i, c0, r, o);
+            unpack4(r3_, dgp);
+            unpack4(r4_, xe);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                u[e] *= rs;
+                const float dE = u[e] * w[e], x = xe[e] + dub[e] * u[e];
+                X[e] += x;
+                run[e] += dgp[e] - u[e] * tu[e] - x - u[e] * tj[e] + dE;   // dG, summed from the warp's last row on
+                o[e] = run[e] - dE;
+            }
+            tc_st4(cta.lanes() + 16 * cta.part + 4 * it, o);
+        }
+        *reinterpret_cast<float4*>(s_tot + cta.warp * DP + c0) = pack4(run);
+        *reinterpret_cast<float4*>(s_x + cta.warp * DP + c0) = pack4(X);
+        tc_wait_st();
+    }
+    __syncthreads();
+    SD_PHASE_T(p.g, ch, ph);
+    if (cta.tid < DP) {   // end-of-chunk terms, then the sums of later warps
+        float run = s_cdc[cta.tid];
+#pragma unroll
+        for (int w = 0; w < 16; ++w) run += s_x[w * DP + cta.tid];
+#pragma unroll
+        for (int w = 15; w >= 0; --w) {
+            const float own = s_tot[w * DP + cta.tid];
+            s_tot[w * DP + cta.tid] = run;
+            run += own;
+        }
+    }
+    __syncthreads();
+    {
+        float v[16], base[4];
+        tc_ld16(cta.lanes() + 16 * cta.part, v);
+        tc_wait_ld();
+        unpack4(*reinterpret_cast<const float4*>(s_tot + cta.warp * DP + c0), base);
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            const int i = 4 * cta.warp + it;
+            if (i >= ch.nvalid) break;
+            float* out = p.dld + (((long long)ch.b * p.g.T + ch.t0 + i) * p.g.H + ch.hh) * (long long)r + c0;
+            const float z = ch.ok(i) ? 1.f : 0.f;
+            if (FAST && (reinterpret_cast<uintptr_t>(p.dld) & 15) == 0) {
+                if (c0 < r)
+                    *reinterpret_cast<float4*>(out) = z != 0.f ? make_float4(v[4 * it] + base[0], v[4 * it + 1] + base[1], v[4 * it + 2] + base[2], v[4 * it + 3] + base[3])
+                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (c0 + e < r) out[e] = z != 0.f ? v[4 * it + e] + base[e] : 0.f;
+            }
+        }
+    }
+    SD_PHASE_T(p.g, ch, ph);
+}
+
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 2) k_predictor_close_fast(BwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (leave_to_slow_kernel(p.Flags, FLAG_SLOW | FLAG_GAMMA)) return;
+    FastCta cta;
+    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    predictor_close_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+// Both kinds of chunk in one launch, for calls that leave SMs empty anyway.
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_one(BwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (chunk_flags(p.Flags, blockIdx.x) & (FLAG_SLOW | FLAG_GAMMA)) {
+        chain_wait();
+        chain_release();
+        predictor_close_blocks<FAST, MASKED, false>(p, chunk_of<MASKED>(p.g, blockIdx.x), fsm_raw);
+        return;
+    }
+    FastCta cta;
+    fast_setup<true>(cta, fsm_raw, p.fault);
+    predictor_close_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
 

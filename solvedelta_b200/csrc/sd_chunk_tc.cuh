@@ -22,6 +22,8 @@ namespace sd {
 
 constexpr float FAST_CHUNK_NATS = 60.f;
 constexpr int FLAG_SLOW = 1;              // some channel's prefix leaves [-FAST_CHUNK_NATS, FAST_CHUNK_NATS]
+constexpr int FLAG_GAMMA = 2;             // some valid token's geometry rate is below MIN_GAMMA
+constexpr float MIN_GAMMA = 1e-20f;
 constexpr int FAST_PASSES = CL / 16;      // row-wise passes: a warp takes a row, a lane four channels
 constexpr int FAST_BARS = 8;
 constexpr unsigned FAST_TMEM = 256;       // tensor-memory columns of a CTA
@@ -95,8 +97,8 @@ __device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, in
 }
 // True for a slow chunk, which another kernel does: the CTA only keeps its place in the chain of launches.  (The flags are
 // older than the launch before.)
-__device__ __forceinline__ bool leave_to_slow_kernel(const unsigned char* flags) {
-    if (!(chunk_flags(flags, blockIdx.x) & FLAG_SLOW)) return false;
+__device__ __forceinline__ bool leave_to_slow_kernel(const unsigned char* flags, int mask) {
+    if (!(chunk_flags(flags, blockIdx.x) & mask)) return false;
     chain_wait();
     chain_release();
     return true;
@@ -112,7 +114,7 @@ __device__ __forceinline__ void fast_teardown(const FastCta& cta) {
 // The slow chunks of a launch, shared out over the CTAs by their rank, so that a CTA's share does not depend on where they
 // lie.  The flags are older than the launch before: they are looked through while that one still runs, 16 a thread, so that
 // a launch without slow chunks ends as soon as its predecessor does.
-template <class F>
+template <int MASK, class F>
 __device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int tasks, F f) {
     unsigned any = 0;
     for (int t0 = threadIdx.x * 16; t0 < tasks; t0 += NTHREADS * 16) {   // the flag panel has room past the last chunk
@@ -122,7 +124,7 @@ __device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int 
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & FLAG_SLOW;
+                if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & MASK;
     }
     any = __syncthreads_or(any);
     chain_wait();
@@ -131,7 +133,7 @@ __device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int 
     int rank = 0;
     for (int b = 0; b < tasks; b += 32) {
         const int t = b + (threadIdx.x & 31);
-        unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & FLAG_SLOW));
+        unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & MASK));
         while (slow != 0) {
             if (rank++ % gridDim.x == blockIdx.x) {
                 f(b + __ffs(slow) - 1);

@@ -171,7 +171,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
         *reinterpret_cast<float4*>(gG + i * DP + c4) = *reinterpret_cast<const float4*>(s_A + i * LDP + c4);
     }
     const bool fast_chunk = __syncthreads_and(in_range) != 0;
-    if (threadIdx.x == 0) p.Flags[ch.gi] = fast_chunk ? 0 : FLAG_SLOW;
+    if (threadIdx.x < 32) {
+        bool live = true;   // false for a NaN
+        for (int i = threadIdx.x; i < CL; i += 32)
+            if (ch.ok(i)) live = live && s_gam[i] >= MIN_GAMMA;
+        live = __all_sync(0xffffffffu, live);
+        if (threadIdx.x == 0) p.Flags[ch.gi] = (unsigned char)((fast_chunk ? 0 : FLAG_SLOW) | (live ? 0 : FLAG_GAMMA));
+    }
     // Lm = gamma stril(N), N[i][j] = sum_c u^_ic u^_jc exp(E_ic - G_jc); N itself is kept for backward.
     // Diagonal blocks that are not fast: direct evaluation, while u^ and G are still in the slots.
     float* gN = p.Npair != nullptr ? mat_ptr(p.Npair, ch.gi) : nullptr;
@@ -577,19 +583,16 @@ __device__ __forceinline__ void primal_exterior_blocks(const FwdParams& p, const
     SD_PHASE(p.g, ph);
 }
 
-// The slow chunks of a launch, one CTA per SM that walks over them (every chunk for the predictor-only entry).
+// The slow chunks of a launch, one CTA per SM that walks over them (every chunk, one a CTA, for the predictor-only entry).
 template <bool FAST, bool MASKED, bool PRED = false>
 __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_fwd(FwdParams p, int tasks) {
     extern __shared__ __align__(16) float smem[];
     if constexpr (PRED) {
         chain_wait();
         chain_release();
-        for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
-            primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem);
-            __syncthreads();
-        }
+        primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, blockIdx.x), smem);
     } else {
-        for_slow_chunks(p.Flags, tasks, [&](int t) { primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem); });
+        for_slow_chunks<FLAG_SLOW>(p.Flags, tasks, [&](int t) { primal_exterior_blocks<FAST, MASKED, PRED>(p, chunk_of<MASKED>(p.g, t), smem); });
     }
 }
 

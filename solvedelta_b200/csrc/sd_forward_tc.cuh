@@ -343,9 +343,24 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
 template <bool FAST, bool MASKED>
 __global__ void __launch_bounds__(NTHREADS, 2) k_primal_exterior_fast(FwdParams p) {
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
-    if (leave_to_slow_kernel(p.Flags)) return;
+    if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
     FastCta cta;
     fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
+    fast_teardown(cta);
+}
+// Both kinds of chunk in one launch, for calls that leave SMs empty anyway.
+template <bool FAST, bool MASKED>
+__global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_one(FwdParams p) {
+    extern __shared__ __align__(1024) unsigned char fsm_raw[];
+    if (chunk_flags(p.Flags, blockIdx.x) & (FLAG_SLOW)) {
+        chain_wait();
+        chain_release();
+        primal_exterior_blocks<FAST, MASKED, false>(p, chunk_of<MASKED>(p.g, blockIdx.x), reinterpret_cast<float*>(fsm_raw));
+        return;
+    }
+    FastCta cta;
+    fast_setup<true>(cta, fsm_raw, p.fault);
     primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
