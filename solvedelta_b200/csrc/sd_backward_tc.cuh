@@ -446,8 +446,8 @@ __device__ __forceinline__ void trisolve_bf16_tiles(const FastCta& cta, float* M
 //     P'' = (I+Lm)^-T dDelta_loc,  Q'' = (I+Lm)^-T Ubar,  Rneg = -gamma u^ exp(E)
 // Shared memory (112 KB): the stack 32, Delta 16, the stacked pair matrices 16, Ucol then Ubar 16, Ct 32; the three results
 // that leave FP32 take the stack, Delta with the pair matrices, and Ct; then the solve has its matrix in the stack's place
-// and dDelta_loc in Ct's.  At 8 x 4096 tokens of 8 heads 391 us against 559 us of the block-centred kernel; bound like the
-// kernel before (the head, seven loads a row deep, is a third of the chain).  Tensor memory: 0 and 64 the pair matrices, then t_u; 128 dk^, then dDelta.
+// and dDelta_loc in Ct's.  A warp takes four token rows in a row and requests all four before it uses one (391 -> 353 us
+// against row by row).  At 8 x 4096 tokens of 8 heads 353 us against 559 us of the block-centred kernel.  Tensor memory: 0 and 64 the pair matrices, then t_u; 128 dk^, then dDelta.
 constexpr unsigned PB_A = 0, PB_DL = 32 * 1024, PB_PP = 48 * 1024, PB_UC = 64 * 1024, PB_CT = 80 * 1024, PB_GAM = 112 * 1024;
 constexpr unsigned PB_DK = PB_CT, PB_TU = PB_DL, PB_DD = PB_A, PB_RHS = PB_CT, PB_LM = PB_A;
 static_assert(PB_GAM + CL * 4 <= FAST_BAR_OFF, "tiles and table fit");
@@ -466,42 +466,66 @@ __device__ __forceinline__ void primal_fast(const BwdParams& p, const ChunkT<MAS
     cp_commit();
     load_gamma(p.gam, ch, s_gam);
     __syncthreads();
-    uint2 ubar[FAST_PASSES];
+    uint2 ubar[FAST_PASSES], k_raw[FAST_PASSES];
+    float rk[FAST_PASSES];
     const long long at0 = ch.gi * (CL * DP) + (4 * cta.warp) * DP + c0;   // rows 4 warp .. of every panel
-    {
-        uint2 ku[2 * FAST_PASSES];
-        float4 G[FAST_PASSES + 1];
+    {   // k^ and Delta
+        float4 dl[FAST_PASSES];
+        const bf16* row = row_bf16(p.k, ch, 4 * cta.warp);
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            k_raw[it] = load4_raw<FAST>(row + it * p.k.st, c0, r, p.k.vec, ch.ok(4 * cta.warp + it));
+            dl[it] = ld_pinned16(p.Delta + at0 + it * DP);
+        }
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            float x[4];
+            unpack4(k_raw[it], x);
+            rk[it] = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+        }
+        row_sums32(rk);
 #pragma unroll
         for (int it = 0; it < FAST_PASSES; ++it) {
             const int i = 4 * cta.warp + it;
-            ku[it] = load4_raw<FAST>(row_bf16(p.k, ch, i), c0, r, p.k.vec, ch.ok(i));
-            ku[FAST_PASSES + it] = load4_raw<FAST>(row_bf16(p.u, ch, i), c0, r, p.u.vec, ch.ok(i));
+            float x[4];
+            unpack4(dl[it], x);
+            *reinterpret_cast<uint2*>(sm + PB_DL + bf_off4<BF_TILE>(i, cta.lane)) = pack4_bf16(x);
+            rk[it] = rsqrtf(rk[it] + 1e-24f);
+            unpack4(k_raw[it], x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] *= rk[it];
+            const uint2 kh = pack4_bf16(x);
+            *reinterpret_cast<uint2*>(sm + PB_A + bf_off4<2 * BF_TILE>(i, cta.lane)) = kh;
+            *reinterpret_cast<uint2*>(p.Khat + at0 + it * DP) = kh;
+        }
+    }
+    {   // u^: Ucol, Ubar, Rneg
+        uint2 u[FAST_PASSES];
+        float4 G[FAST_PASSES + 1];
+        const bf16* row = row_bf16(p.u, ch, 4 * cta.warp);
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            u[it] = load4_raw<FAST>(row + it * p.u.st, c0, r, p.u.vec, ch.ok(4 * cta.warp + it));
             G[it + 1] = ld_pinned16(p.Gp + at0 + it * DP);
         }
         G[0] = cta.warp > 0 ? ld_pinned16(p.Gp + at0 - DP) : make_float4(0.f, 0.f, 0.f, 0.f);   // E of a row is G of the one before
-        float lam[4], ss[8];
+        float lam[4], ss[4];
         unpack4(*reinterpret_cast<const float4*>(p.Lam + ch.gi * DP + c0), lam);
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
+        for (int it = 0; it < FAST_PASSES; ++it) {
             float x[4];
-            unpack4(ku[n], x);
-            ss[n] = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+            unpack4(u[it], x);
+            ss[it] = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
         }
         row_sums32(ss);
 #pragma unroll
         for (int it = 0; it < FAST_PASSES; ++it) {
             const int i = 4 * cta.warp + it;
             float x[4], g[4], E[4], o[4];
-            unpack4(ku[it], x);
-            const float rk = rsqrtf(ss[it] + 1e-24f), ru = rsqrtf(ss[FAST_PASSES + it] + 1e-24f), gm = s_gam[i];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) x[e] *= rk;
-            const uint2 kh = pack4_bf16(x);
-            *reinterpret_cast<uint2*>(sm + PB_A + bf_off4<2 * BF_TILE>(i, cta.lane)) = kh;
-            *reinterpret_cast<uint2*>(p.Khat + at0 + it * DP) = kh;
-            unpack4(ku[FAST_PASSES + it], x);
+            unpack4(u[it], x);
             unpack4(G[it + 1], g);
             unpack4(G[it], E);
+            const float ru = rsqrtf(ss[it] + 1e-24f), gm = s_gam[i];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 x[e] *= ru;
@@ -513,8 +537,6 @@ __device__ __forceinline__ void primal_fast(const BwdParams& p, const ChunkT<MAS
 #pragma unroll
             for (int e = 0; e < 4; ++e) g[e] *= lam[e];
             ubar[it] = pack4_bf16(g);
-            unpack4(ld_pinned16(p.Delta + at0 + it * DP), x);
-            *reinterpret_cast<uint2*>(sm + PB_DL + bf_off4<BF_TILE>(i, cta.lane)) = pack4_bf16(x);
         }
     }
     cp_wait<1>();
@@ -580,54 +602,78 @@ __device__ __forceinline__ void primal_fast(const BwdParams& p, const ChunkT<MAS
     }
     __syncthreads();
     SD_PHASE_T(p.g, ch, ph);
+    const auto piece = [&](unsigned base, int i) {
+        return reinterpret_cast<const float4*>(sm + base + (cta.lane >> 3) * F32_TILE + i * 128 + (((cta.lane & 7) ^ (i & 7)) << 4));
+    };
     uint2 rhs[FAST_PASSES];
+    {   // dk^ and its norm reverse; a row of the solve's right-hand sides is only packed here, its place is still in use
+        uint2 dkp[FAST_PASSES];
+        float dot[FAST_PASSES];
 #pragma unroll
-    for (int it = 0; it < FAST_PASSES; ++it) {
-        const int i = 4 * cta.warp + it;
-        const auto piece = [&](unsigned base) {
-            return reinterpret_cast<const float4*>(sm + base + (cta.lane >> 3) * F32_TILE + i * 128 + (((cta.lane & 7) ^ (i & 7)) << 4));
-        };
-        const uint2 rk_ = load4_raw<FAST>(row_bf16(p.k, ch, i), c0, r, p.k.vec, ch.ok(i));
-        const float4 rg_ = ld_pinned16(p.Gp + at0 + it * DP);
-        const uint2 rd_ = ld_pinned8(p.dDelta + at0 + it * DP, true), rp_ = ld_pinned8(p.dkPart + at0 + it * DP, true);
-        float x[4], y[4];
-        unpack4(rg_, x);
-        unpack4(*piece(PB_TU), y);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] *= exp_ftz(-x[e]);
-        *reinterpret_cast<uint2*>(p.Tu + at0 + it * DP) = pack4_bf16(y);
-        unpack4(rd_, x);
-        unpack4(*piece(PB_DD), y);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] += x[e];
-        rhs[it] = pack4_bf16(y);
-        // dk^ and its norm reverse
-        unpack4(rp_, x);
-        unpack4(*piece(PB_DK), y);
-        float k[4], ss[2] = {0.f, 0.f};
-        unpack4(rk_, k);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            y[e] += x[e];
-            ss[0] = fmaf(k[e], k[e], ss[0]);
-            ss[1] = fmaf(k[e], y[e], ss[1]);
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            dkp[it] = ld_pinned8(p.dkPart + at0 + it * DP, true);
+            rhs[it] = ld_pinned8(p.dDelta + at0 + it * DP, true);
         }
 #pragma unroll
-        for (int m = 16; m > 0; m >>= 1) {
-            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], m);
-            ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], m);
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            float x[4], y[4], k[4];
+            unpack4(dkp[it], x);
+            unpack4(*piece(PB_DK, 4 * cta.warp + it), y);
+            unpack4(k_raw[it], k);
+            dot[it] = fmaf(k[0], y[0] + x[0], fmaf(k[1], y[1] + x[1], fmaf(k[2], y[2] + x[2], k[3] * (y[3] + x[3]))));
         }
-        const float rk = rsqrtf(ss[0] + 1e-24f), dot = ss[1] * rk * rk;
+        row_sums32(dot);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] = (y[e] - dot * k[e]) * rk;
-        store4_bf16<FAST>(p.dk, p.pitch_q, p.g, ch, i, c0, r, y);
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            const int i = 4 * cta.warp + it;
+            float x[4], y[4], k[4];
+            unpack4(dkp[it], x);
+            unpack4(*piece(PB_DK, i), y);
+            unpack4(k_raw[it], k);
+            const float along = dot[it] * rk[it] * rk[it];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = (y[e] + x[e] - along * k[e]) * rk[it];
+            store4_bf16<FAST>(p.dk, p.pitch_q, p.g, ch, i, c0, r, y);
+            unpack4(rhs[it], x);
+            unpack4(*piece(PB_DD, i), y);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] += x[e];
+            rhs[it] = pack4_bf16(y);
+        }
+    }
+    float4 N[2];   // (gamma N)^T, the matrix of the solve: two pieces a thread, as g2s_mat_transposed takes them
+    {
+        float4 G[FAST_PASSES];
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) G[it] = ld_pinned16(p.Gp + at0 + it * DP);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int idx = cta.tid + NTHREADS * k;
+            N[k] = ld_pinned16(mat_ptr(p.Npair, ch.gi) + (idx & (CL - 1)) * CL + ((idx >> 6) << 2));
+        }
+#pragma unroll
+        for (int it = 0; it < FAST_PASSES; ++it) {
+            float x[4], y[4];
+            unpack4(G[it], x);
+            unpack4(*piece(PB_TU, 4 * cta.warp + it), y);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] *= exp_ftz(-x[e]);
+            *reinterpret_cast<uint2*>(p.Tu + at0 + it * DP) = pack4_bf16(y);
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < FAST_PASSES; ++it)
         *reinterpret_cast<uint2*>(sm + PB_RHS + bf_off4<BF_TILE>(4 * cta.warp + it, cta.lane)) = rhs[it];
     float* s_lm = reinterpret_cast<float*>(sm + PB_LM);
-    g2s_mat_transposed(s_lm, mat_ptr(p.Npair, ch.gi), [&](int i) { return s_gam[i]; });
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int idx = cta.tid + NTHREADS * k, i = idx & (CL - 1);
+        float x[4];
+        unpack4(N[k], x);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s_lm[(((idx >> 6) << 2) + e) * LDA + i] = s_gam[i] * x[e];
+    }
     __syncthreads();
     SD_PHASE_T(p.g, ch, ph);
     const int panel = cta.warp >> 3, cw = cta.warp & 7;
