@@ -288,20 +288,20 @@ _F, _B, _S, _T, _M, _P = 32 * KIB, 16 * KIB, 64 * KIB, 32 * KIB, 8 * KIB, 16 * K
 KERNEL_BYTES_PER_CHUNK = {
     "k_prep_fwd": 2 * _B + _F + 4 * _F + _P,                    # u,h,g -> Upd,Qc,Ubar,G,N
     "k_state_scan[C]": 4 * _F + _S + _T,                        # P,Q,R -> X, FP32 + BF16 ckpt
-    # u,k,q,er,wr,v,G,Delta,Ct -> d, Wd,Ud,Dt, Aqd,Aed, 7 BF16 source panels
-    "k_primal_exterior_fwd": 6 * _B + 2 * _F + _S + _F + 3 * _F + _M + _P + 7 * _B,
+    # u,k,q,er,wr,v,G,Delta,Ubar,Ct -> d, Wd,Ud,Dt, Aqd,Aed, Xg,Ag,Dcol,DtB (fast chunks, like the three below)
+    "k_primal_exterior_fwd": 6 * _B + 3 * _F + _S + _F + 3 * _F + _M + _P + 4 * _B,
     "k_state_scan[S]": 3 * _F + _B + _T,                        # P,Q,R -> Z~ (BF16), BF16 ckpt
     "k_output_fwd_tc": _B + _M + _B + _T + _B,                  # Xg,Aqd,Zt,S -> y
     # dy,DtB,Aqd,Aed -> Dyf,Pp,Qp
     "k_exterior_prep_bwd": 2 * _B + _M + _P + 3 * _B,
     "k_state_scan_b[dS]": 6 * _B + _T,
-    # Dyf,dR,Zt,Dcol,Xr,Er,Chi,Ee,S,dSe + u,k,q,er,wr,v,G,Delta,d -> 5 partial panels, DG,Dd, dq,der,dv,dwr
-    "k_exterior_pair_bwd": 8 * _B + 2 * _T + 6 * _B + 3 * _F + 7 * _B + 4 * _B,
-    # u,k,G,Delta,DG,Dd,Ct(bf16),N,dkPart,dDelta -> Khat,Rneg,Tu,dk,Ppp,Qpp
-    "k_primal_bwd": 2 * _B + 2 * _F + 2 * _B + _T + _P + 2 * _B + 6 * _B,
+    # Dyf,dR,Zt,Dcol,Xg,Ag,S,dSe + u,k,q,er,wr,v,G,Delta,d -> 5 partial panels, DG,Dd, dq,der,dv,dwr
+    "k_exterior_pair_bwd": 6 * _B + 2 * _T + 6 * _B + 3 * _F + 7 * _B + 4 * _B,
+    # u,k,G,Delta,DG,Ct(bf16),N,dkPart,dDelta -> Khat,Rneg,Tu,dk,Ppp,Qpp
+    "k_primal_bwd": 2 * _B + 2 * _F + _B + _T + _P + 2 * _B + 6 * _B,
     "k_state_scan_b[dC]": 6 * _B + _T,
-    # u,h,G,Delta,dRr,Ct,dCe,N,duPart,Tu,dGPart,Xext -> du,dh,dlog_decay
-    "k_predictor_close_bwd": 2 * _B + 2 * _F + _B + _T + _T + _P + 4 * _B + 2 * _B + _F,
+    # u,G,Delta,dRr,Ct,dCe,Rneg,duPart,Tu,dGPart,Xext -> du,dh,dlog_decay
+    "k_predictor_close_bwd": _B + 2 * _F + _B + _T + _T + 5 * _B + 2 * _B + _F,
 }
 
 
@@ -347,19 +347,23 @@ def summarize_ncu(csv_path, tasks):
     def short(full):
         return full.split("(")[0].replace("void ", "").split("<")[0].replace("sd::", "")
 
-    # the last complete step of the capture: k_prep_fwd ... k_predictor_close_bwd, 11 launches
-    names = [short(per_launch[k]["name"]) for k in order]
+    # the last complete step of the capture: k_prep_fwd ... k_predictor_close_bwd.  Of the kernels that come in two kinds
+    # the fast chunks' one is the line's (this case has no slow chunks).
+    kinds = {"k_primal_exterior_fast": "k_primal_exterior_fwd", "k_exterior_pair_fast": "k_exterior_pair_bwd",
+             "k_primal_fast": "k_primal_bwd", "k_predictor_close_fast": "k_predictor_close_bwd"}
+    order = [k for k in order if short(per_launch[k]["name"]) not in kinds.values()]
+    names = [kinds.get(n, n) for n in (short(per_launch[k]["name"]) for k in order)]
     starts = [i for i, n in enumerate(names) if n == "k_prep_fwd" and i + 11 <= len(names)
               and names[i + 10] == "k_predictor_close_bwd"]
     if not starts:
-        raise SystemExit("no complete fwd+bwd step (11 launches) in the capture")
+        raise SystemExit("no complete fwd+bwd step in the capture")
     order = order[starts[-1]:starts[-1] + 11]
     scans = iter(("k_state_scan[C]", "k_state_scan[S]"))
     scans_b = iter(("k_state_scan_b[dS]", "k_state_scan_b[dC]"))
     print("# kernel  KiB-per-chunk-task (DRAM read + write, ncu)  time-us")
     for key in order:
         m = per_launch[key]
-        name = short(m["name"])
+        name = kinds.get(short(m["name"]), short(m["name"]))
         if name == "k_state_scan_tc":
             name = next(scans)
         elif name == "k_state_scan_b":
