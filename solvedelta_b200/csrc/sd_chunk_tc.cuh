@@ -249,13 +249,6 @@ __device__ __forceinline__ void row_sums32(float (&v)[4]) {
 #pragma unroll
     for (int n = 0; n < 4; ++n) v[n] = __shfl_sync(0xffffffffu, c, 8 * n);
 }
-// prefetch_rows for the rows of a whole CTA, up to four lines each
-template <class CH>
-__device__ __forceinline__ void prefetch_fast_rows(const Operand& op, const CH& ch, int row_bytes) {
-    const int i = threadIdx.x >> 3, l = threadIdx.x & 7;
-    if (l * 128 < row_bytes && ch.ok(i)) prefetch_l2(reinterpret_cast<const char*>(row_bf16(op, ch, i)) + l * 128);
-}
-
 // ---- contractions (one thread issues) -------------------------------------------
 __device__ __forceinline__ void tc_mma_ss(unsigned d_tmem, unsigned long long da, unsigned long long db, unsigned idesc,
                                           unsigned accumulate) {

@@ -71,3 +71,15 @@ def test_masked_tokens_without_resets_in_fast_chunks(r, V):
     valid[0, :70] = False      # a whole chunk and the head of the next
     valid[1, 100:103] = False
     _masked_case(cpu, dev, valid, torch.zeros_like(valid))
+
+
+@pytest.mark.parametrize("rate", [0.0, 1e-30, -0.01])
+def test_vanishing_geometry_rates_between_others(rate):
+    """The closure divides by the rate in fast chunks: a chunk with one below 1e-20 evaluates the residual instead."""
+    cpu, dev = make_inputs(1, 200, 2, 64, 96, seed=53)
+    cpu["geometry_write"][0, 70, 0] = rate    # second chunk of head 0
+    cpu["geometry_write"][0, 199, 1] = rate   # the ragged end of head 1
+    dev["geometry_write"] = cpu["geometry_write"].cuda()
+    leaves, state, y, fin = _native(dev, grad=True)
+    _check_forward(cpu, y, fin)
+    _check_vjp(cpu, leaves, state, y, fin)
