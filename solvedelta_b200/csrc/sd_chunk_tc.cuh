@@ -31,6 +31,9 @@ constexpr size_t FAST_SMEM = 113 * 1024;  // two CTAs per SM
 constexpr size_t FAST_BAR_OFF = FAST_SMEM - (FAST_BARS + 1) * 8;
 constexpr unsigned F32_TILE = CL * 128;   // [64 rows][32 channels] FP32, or [64 rows][64 channels] BF16: 128-byte rows
 
+// The flags are read before a launch waits for the one before it.  They are two launches older or more: every launch of the
+// sequence waits for its predecessor before it lets its successor begin, so k_prep_fwd has completed, with its writes performed,
+// before any launch that reads flags begins; such a launch reads them once and holds no older copy.
 __device__ __forceinline__ int chunk_flags(const unsigned char* flags, long long gi) { return __ldg(flags + gi); }
 
 struct FastCta {
@@ -112,35 +115,70 @@ __device__ __forceinline__ void fast_teardown(const FastCta& cta) {
 }
 
 // The slow chunks of a launch, shared out over the CTAs by their rank, so that a CTA's share does not depend on where they
-// lie.  The flags are older than the launch before: they are looked through while that one still runs, 16 a thread, so that
-// a launch without slow chunks ends as soon as its predecessor does.
+// lie.  A pass ranks 8192 flags, 16 a thread, and each CTA lists the chunks whose rank is its own (a few us; stepping through
+// all slow chunks to find them took 0.12 us for each, 0.5 ms of a kernel with 4096).  Whether there are any is looked up while
+// the launch before still runs (see chunk_flags): what stands between a wait and the end of a launch without slow chunks is
+// waited for by all that follow (looked up behind the wait: 1024 tokens of 8 heads 267 -> 278 us forward and reverse).
+// With every chunk slow, 8 x 4096 tokens of 8 heads take 3.84 ms forward and reverse, 3.72 in kernels of one CTA for each
+// chunk; the CTAs of the fast kernels that skip are the difference.
+constexpr int SLOW_PASS = NTHREADS * 16;
+constexpr int SLOW_LIST = SLOW_PASS / 148 + 1;   // a share of a pass; grids of fewer CTAs have no more chunks than CTAs
 template <int MASK, class F>
 __device__ __forceinline__ void for_slow_chunks(const unsigned char* flags, int tasks, F f) {
-    unsigned any = 0;
-    for (int t0 = threadIdx.x * 16; t0 < tasks; t0 += NTHREADS * 16) {   // the flag panel has room past the last chunk
+    __shared__ unsigned short s_list[SLOW_LIST];
+    __shared__ unsigned short s_count[NTHREADS / 32];
+    unsigned any = 0;   // the flags are followed by zeros
+#pragma unroll 1
+    for (int t0 = 16 * threadIdx.x; t0 < tasks; t0 += SLOW_PASS) {
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + t0));
-        const unsigned words[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (t0 + 4 * i + k < tasks) any |= (words[i] >> (8 * k)) & MASK;
+        any |= w.x | w.y | w.z | w.w;
     }
-    any = __syncthreads_or(any);
+    any = __syncthreads_or(any & (MASK * 0x01010101u));
     chain_wait();
     chain_release();
     if (any == 0) return;
-    int rank = 0;
-    for (int b = 0; b < tasks; b += 32) {
-        const int t = b + (threadIdx.x & 31);
-        unsigned slow = __ballot_sync(0xffffffffu, t < tasks && (chunk_flags(flags, t) & MASK));
-        while (slow != 0) {
-            if (rank++ % gridDim.x == blockIdx.x) {
-                f(b + __ffs(slow) - 1);
-                __syncthreads();   // the next chunk's loads overwrite what this one reads
-            }
-            slow &= slow - 1;
+    unsigned turn = blockIdx.x;   // this CTA's first rank among the slow chunks of the pass
+#pragma unroll 1
+    for (int base = 0; base < tasks; base += SLOW_PASS) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t0 = base + 16 * (int)threadIdx.x;
+        unsigned slow = 0;   // bit i: flag t0 + i
+        if (t0 < tasks) {
+            const uint4 w = __ldg(reinterpret_cast<const uint4*>(flags + t0));
+            const unsigned words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if ((words[i >> 2] >> (8 * (i & 3))) & MASK) slow |= 1u << i;
         }
+        const unsigned own = __popc(slow);
+        unsigned upto = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned below = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += below;
+        }
+        if (lane == 31) s_count[warp] = (unsigned short)upto;
+        __syncthreads();
+        unsigned rank = upto - own, total = 0;
+#pragma unroll
+        for (int w = 0; w < NTHREADS / 32; ++w) {
+            const unsigned n = s_count[w];
+            if (w < warp) rank += n;
+            total += n;
+        }
+        // of at most 16 consecutive ranks, at most one is this CTA's: grids of fewer CTAs are not launched
+        const unsigned k = rank > turn ? (rank - turn + gridDim.x - 1) / gridDim.x : 0, at = turn + k * gridDim.x - rank;
+        if (at < own) {
+            for (unsigned i = 0; i < at; ++i) slow &= slow - 1;
+            s_list[k] = (unsigned short)(16 * threadIdx.x + __ffs(slow) - 1);
+        }
+        __syncthreads();
+        const unsigned share = total > turn ? (total - turn - 1) / gridDim.x + 1 : 0;
+#pragma unroll 1
+        for (unsigned i = 0; i < share; ++i) {
+            f(base + s_list[i]);
+            __syncthreads();   // the next chunk's loads overwrite what this one reads
+        }
+        turn += share * gridDim.x - total;
     }
 }
 

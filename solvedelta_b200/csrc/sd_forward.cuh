@@ -177,6 +177,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
             if (ch.ok(i)) live = live && s_gam[i] >= MIN_GAMMA;
         live = __all_sync(0xffffffffu, live);
         if (threadIdx.x == 0) p.Flags[ch.gi] = (unsigned char)((fast_chunk ? 0 : FLAG_SLOW) | (live ? 0 : FLAG_GAMMA));
+        // the panel has room past the last chunk: zeros there let the flags be looked through 16 at a time
+        if (blockIdx.x == gridDim.x - 1 && threadIdx.x > 0 && threadIdx.x < 16) p.Flags[ch.gi + threadIdx.x] = 0;
     }
     // Lm = gamma stril(N), N[i][j] = sum_c u^_ic u^_jc exp(E_ic - G_jc); N itself is kept for backward.
     // Diagonal blocks that are not fast: direct evaluation, while u^ and G are still in the slots.

@@ -12,6 +12,7 @@ from tests.test_gpu_parity import _check_forward, _check_vjp, _masked_case, _nat
 pytestmark = pytest.mark.gpu
 
 NATS = 60.0
+NAMES = ("u", "h", "q", "keys", "values", "log_decay", "erase_raw", "write_raw", "geometry_write")
 
 
 def _with_decay(cpu, dev, per_token):
@@ -43,17 +44,16 @@ def test_chunks_at_the_limit_match_checker(T, r, V, kind):
 
 
 def test_more_chunks_than_resident_ctas_with_slow_ones_between():
-    """Every CTA walks over several chunks, slow ones among them: the bits of each stream on its own."""
+    """More CTAs than fit the device at once, slow chunks shared out over one CTA per SM: the bits of each stream on its own."""
     B, T, H, r, V = 5, 64 * 24 + 7, 4, 32, 32   # 500 chunks, more than two CTAs on each of 148 SMs
     cpu, dev = make_inputs(B, T, H, r, V, seed=43)
     for b in range(B):
         cpu["log_decay"][b, 64 * (3 + b):64 * (3 + b) + 90, b % H] -= 1.5
     dev["log_decay"] = cpu["log_decay"].cuda()
-    names = ("u", "h", "q", "keys", "values", "log_decay", "erase_raw", "write_raw", "geometry_write")
     dy = torch.randn(B, T, H, V, generator=torch.Generator().manual_seed(44)).to(torch.bfloat16).cuda()
 
     def run(cut):
-        leaves = [cut(dev[n]).contiguous().requires_grad_() for n in names]
+        leaves = [cut(dev[n]).contiguous().requires_grad_() for n in NAMES]
         y, fin = solvedelta_native(*leaves, initial_state=SolveDeltaState(cut(dev["C0"]), cut(dev["S0"])),
                                    return_final_state=True)
         return [y, *fin, *torch.autograd.grad(y, leaves, cut(dy))]
@@ -62,6 +62,60 @@ def test_more_chunks_than_resident_ctas_with_slow_ones_between():
     for b in (0, 4):
         for one, all_ in zip(run(lambda t: t[b:b + 1]), whole):
             assert torch.equal(one[0], all_[b])
+
+
+def _device_case(B, T, H, r, V, seed):
+    """Operands like those of make_inputs, drawn on the device, and the forward and reverse pass over some of the rows."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    bf = lambda t: t.to(torch.bfloat16)
+    unit = torch.nn.functional.normalize
+    x = dict(u=bf(rn(B, T, H, r)), h=bf(rn(B, T, H, r)), q=bf(unit(rn(B, T, H, r), dim=-1)),
+             keys=bf(unit(rn(B, T, H, 1, r), dim=-1)), values=bf(rn(B, T, H, 1, V)),
+             log_decay=torch.nn.functional.logsigmoid(rn(B, T, H, r) + 4.0), erase_raw=bf(0.5 * rn(B, T, H, 1, r)),
+             write_raw=bf(0.5 * rn(B, T, H, 1, V)), geometry_write=0.1 * torch.rand(B, T, H, generator=gen, device="cuda"))
+    dy = bf(rn(B, T, H, V))
+
+    def run(rows=slice(None)):
+        leaves = [x[n][rows].detach().requires_grad_() for n in NAMES]
+        y, fin = solvedelta_native(*leaves, return_final_state=True)
+        return [y.detach(), *(t.detach() for t in fin), *torch.autograd.grad(y, leaves, dy[rows])]
+
+    return x, run, gen
+
+
+def test_slow_chunks_beyond_one_pass_over_the_flags():
+    """8448 chunks, every third slow: the flags of a launch are ranked 8192 at a time.  The bits of one row on its own."""
+    B, T, H = 4, 64 * 66, 32
+    x, run, gen = _device_case(B, T, H, 16, 8, 59)
+    slow = torch.rand(B, T // 64, 1, H, 1, generator=gen, device="cuda") < 1 / 3
+    x["log_decay"].view(B, T // 64, 64, H, 16).sub_(1.5 * slow)
+    whole = run()
+    for b in (0, B - 1):
+        for one, all_ in zip(run(slice(b, b + 1)), whole):
+            assert torch.equal(one[0], all_[b])
+
+
+def test_slow_chunks_cost_their_own_work():
+    """4096 chunks, all slow, against the same number of fast ones: 1.4 times the time by the work of the two kinds of kernel.
+    With every CTA stepping through all slow chunks of a launch it was 2.2 times."""
+    x, run, _ = _device_case(8, 4096, 8, 128, 128, 61)
+
+    def milliseconds():
+        run()
+        times = []
+        for _ in range(5):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            run()
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return sorted(times)[2]
+
+    fast = milliseconds()
+    x["log_decay"] -= 1.3
+    assert milliseconds() < 1.8 * fast
 
 
 @pytest.mark.parametrize("r,V", [(128, 128), (20, 12)])
