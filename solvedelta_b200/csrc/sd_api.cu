@@ -501,17 +501,14 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_
 // call takes the host longer to issue (165 us forward and reverse) than the GPU to run, and four launches more cost it 9 us.
 // From 64 chunks on the GPU is what is waited for and the larger kernels are slower (64 chunks 247 us of kernels against 229,
 // 128 chunks 331 against 305, the same 195 at 32).  Beyond 32, slow chunks run with one CTA to an SM and fast ones with two.
-// Masked calls have slow chunks wherever a sequence starts: those go first, and the fast chunks fill the SMs around them (5 x
-// 1531 tokens with masks 1088 -> 1072 us).  Without masks slow chunks are the exception: they go last, and the fast kernel
-// starts while its predecessor ends.
+// The slow kernel goes last, with masks too: the fast kernel starts while its predecessor ends, and the slow one may have
+// nothing to do.  (Masked calls with the slow kernel first: 5 x 1531 tokens 893 us forward and reverse against 892; 881 if the
+// fast CTAs then start without waiting for a predecessor whose results they read, which nothing documented allows.)
 constexpr int ONE_LAUNCH_CHUNKS = 32;
 #define SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, F, M)                                          \
     do {                                                                                           \
         if (chunks <= ONE_LAUNCH_CHUNKS) {                                                                 \
             launch(name##_one<F, M>, chunks, NTHREADS, smem, true, stream, p);                     \
-        } else if (M) {                                                                            \
-            launch(slow_kernel<F, M>, chunks < 148 ? chunks : 148, NTHREADS, smem, true, stream, p, chunks); \
-            launch(name##_fast<F, M>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
         } else {                                                                                   \
             launch(name##_fast<F, M>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
             launch(slow_kernel<F, M>, chunks < 148 ? chunks : 148, NTHREADS, smem, true, stream, p, chunks); \

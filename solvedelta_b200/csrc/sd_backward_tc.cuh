@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_exterior_pair_fast(BwdParams p)
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
     if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
     FastCta cta;
-    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     exterior_pair_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_exterior_pair_one(BwdParams p) 
         return;
     }
     FastCta cta;
-    fast_setup<true>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     exterior_pair_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_primal_fast(BwdParams p) {
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
     if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
     FastCta cta;
-    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     primal_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_one(BwdParams p) {
         return;
     }
     FastCta cta;
-    fast_setup<true>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     primal_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -990,7 +990,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_predictor_close_fast(BwdParams 
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
     if (leave_to_slow_kernel(p.Flags, FLAG_SLOW | FLAG_GAMMA)) return;
     FastCta cta;
-    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     predictor_close_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_predictor_close_one(BwdParams p
         return;
     }
     FastCta cta;
-    fast_setup<true>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     predictor_close_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }

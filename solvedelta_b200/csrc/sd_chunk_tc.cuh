@@ -34,6 +34,7 @@ constexpr unsigned F32_TILE = CL * 128;   // [64 rows][32 channels] FP32, or [64
 // The flags are read before a launch waits for the one before it.  They are two launches older or more: every launch of the
 // sequence waits for its predecessor before it lets its successor begin, so k_prep_fwd has completed, with its writes performed,
 // before any launch that reads flags begins; such a launch reads them once and holds no older copy.
+// Nothing else is read before the wait.
 __device__ __forceinline__ int chunk_flags(const unsigned char* flags, long long gi) { return __ldg(flags + gi); }
 
 struct FastCta {
@@ -60,15 +61,9 @@ struct FastCta {
     }
 };
 
-// WAIT: the launch begins once its predecessor is complete.  Without it (masked calls) the slow chunks' kernel has been
-// launched just before and let this one start as soon as its own predecessor was complete: what is read here is older than
-// the slow kernel, the two write different chunks, and the CTAs here fill the SMs that have no slow chunk to work on.  The
-// wait for the slow kernel is then at the end, for the kernels that follow both.
-//
 // Tensor memory is allocated before the launch lets its successor start, so that a kernel that starts early can never hold
 // what this one still waits for.  These kernels have no static shared memory: the dynamic part starts on the 1024-byte
 // boundary that the swizzled tiles need (behind the 1 KB the system keeps), which is checked.
-template <bool WAIT>
 __device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, int* fault) {
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + FAST_BAR_OFF);
     unsigned* s_tmem = reinterpret_cast<unsigned*>(bars + FAST_BARS);
@@ -95,7 +90,7 @@ __device__ __forceinline__ void fast_setup(FastCta& cta, unsigned char* smem, in
     cta.alive = (tc_smem(smem) & 1023u) == 0;   // else nothing here can be right: no waits, and the fault word says so
     cta.fault = fault;
     if (!cta.alive && cta.tid == 0) atomicExch(fault, 20);
-    if (WAIT) chain_wait();
+    chain_wait();
     chain_release();
 }
 // True for a slow chunk, which another kernel does: the CTA only keeps its place in the chain of launches.  (The flags are
@@ -109,7 +104,6 @@ __device__ __forceinline__ bool leave_to_slow_kernel(const unsigned char* flags,
 __device__ __forceinline__ void fast_teardown(const FastCta& cta) {
     tc_fence_before();
     __syncthreads();
-    chain_wait();
     if (cta.warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cta.tmem), "r"(FAST_TMEM));
 }

@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_primal_exterior_fast(FwdParams 
     extern __shared__ __align__(1024) unsigned char fsm_raw[];
     if (leave_to_slow_kernel(p.Flags, FLAG_SLOW)) return;
     FastCta cta;
-    fast_setup<!MASKED>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_primal_exterior_one(FwdParams p
         return;
     }
     FastCta cta;
-    fast_setup<true>(cta, fsm_raw, p.fault);
+    fast_setup(cta, fsm_raw, p.fault);
     primal_exterior_fast<FAST, MASKED>(p, chunk_of<MASKED>(p.g, blockIdx.x), cta);
     fast_teardown(cta);
 }
