@@ -386,7 +386,8 @@ int sd_predictor_backward(const sd_predictor_backward_args *args, void *stream);
 #define SD_STATIC_WORKSPACE_BYTES (32u * 1024u * 1024u)
 int sd_forward_static(const sd_forward_args *args, void *stream);
 
-/* Number of kernels one call launches for this shape (for accounting). */
+/* Number of kernels one call launches for this shape (for accounting); sd_forward_inference launches one fewer than
+ * sd_forward for 33 to 148 chunks. */
 int sd_forward_launches(const sd_shape *shape);
 int sd_backward_launches(const sd_shape *shape);
 

@@ -497,32 +497,36 @@ int launch_status() { return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_
         else launch(kernel<false, true>, chunks, NTHREADS, smem, chained, stream, p);                   \
     } while (0)
 
-// The chunk kernels that come in two kinds (sd_chunk_tc.cuh).  Up to 32 chunks both kinds are in one launch, NAME_one: such a
-// call takes the host longer to issue (165 us forward and reverse) than the GPU to run, and four launches more cost it 9 us.
-// From 64 chunks on the GPU is what is waited for and the larger kernels are slower (64 chunks 247 us of kernels against 229,
-// 128 chunks 331 against 305, the same 195 at 32).  Beyond 32, slow chunks run with one CTA to an SM and fast ones with two.
-// The slow kernel goes last, with masks too: the fast kernel starts while its predecessor ends, and the slow one may have
+// The chunk kernels that come in two kinds (sd_chunk_tc.cuh).  Small calls have both kinds in one launch, NAME_one, with one CTA
+// to an SM; beyond, slow chunks run with one CTA to an SM and fast ones with two, in two launches.
+//   With gradients up to 32 chunks: such a call takes the host longer to issue (165 us forward and reverse) than the GPU to run,
+// and four launches more cost it 9 us.  From 64 chunks on the GPU is what is waited for and the larger kernels are slower (64
+// chunks 247 us of kernels against 229, 128 chunks 331 against 305, the same 195 at 32).
+//   Without gradients up to 148 chunks, one to an SM: one launch less is 1 to 2 us of the call, more where few scan steps follow
+// (two launches against one: 33 chunks 67 -> 65 us, 64 chunks 81 -> 70 and 95 -> 94, 128 chunks 108 -> 99 and 128 -> 127, 148
+// chunks 98 -> 96).  In calls with gradients the same launch makes 1 x 1024 tokens 264 -> 272 us.
+//   The slow kernel goes last, with masks too: the fast kernel starts while its predecessor ends, and the slow one may have
 // nothing to do.  (Masked calls with the slow kernel first: 5 x 1531 tokens 893 us forward and reverse against 892; 881 if the
 // fast CTAs then start without waiting for a predecessor whose results they read, which nothing documented allows.)
-constexpr int ONE_LAUNCH_CHUNKS = 32;
-#define SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, F, M)                                          \
+constexpr int ONE_LAUNCH_GRAD = 32, ONE_LAUNCH_NO_GRAD = 148;
+#define SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, limit, F, M)                                   \
     do {                                                                                           \
-        if (chunks <= ONE_LAUNCH_CHUNKS) {                                                                 \
+        if (chunks <= (limit)) {                                                                   \
             launch(name##_one<F, M>, chunks, NTHREADS, smem, true, stream, p);                     \
         } else {                                                                                   \
             launch(name##_fast<F, M>, chunks, NTHREADS, FAST_SMEM, true, stream, p);               \
             launch(slow_kernel<F, M>, chunks < 148 ? chunks : 148, NTHREADS, smem, true, stream, p, chunks); \
         }                                                                                          \
     } while (0)
-#define SD_LAUNCH_KINDS(name, slow_kernel, smem)                                                   \
+#define SD_LAUNCH_KINDS(name, slow_kernel, smem, limit)                                            \
     do {                                                                                           \
-        if (fast && !masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, true, false);             \
-        else if (fast) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, true, true);                    \
-        else if (!masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, false, false);               \
-        else SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, false, true);                             \
+        if (fast && !masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, limit, true, false);      \
+        else if (fast) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, limit, true, true);             \
+        else if (!masked) SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, limit, false, false);        \
+        else SD_LAUNCH_KINDS_OF(name, slow_kernel, smem, limit, false, true);                      \
     } while (0)
 constexpr int KINDS_FORWARD = 1, KINDS_BACKWARD = 3;
-int kind_launches(const sd_shape* s, int kinds) { return total_chunks(s) <= ONE_LAUNCH_CHUNKS ? 0 : kinds; }
+int kind_launches(const sd_shape* s, int kinds) { return total_chunks(s) <= ONE_LAUNCH_GRAD ? 0 : kinds; }
 
 bool operands_ok(const sd_operand* ops, int n) {
     for (int i = 0; i < n; ++i)
@@ -805,7 +809,7 @@ int forward_impl(const sd_forward_args* a, void* stream_, const PredictorOnly* p
         k_primal_exterior_fwd<false, true, true><<<chunks, NTHREADS, PRIMAL_EXT_FWD_SMEM, stream>>>(p, chunks);
         return launch_status();   // the kernel stops after its primal half
     }
-    SD_LAUNCH_KINDS(k_primal_exterior, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM);
+    SD_LAUNCH_KINDS(k_primal_exterior, k_primal_exterior_fwd, PRIMAL_EXT_FWD_SMEM, keep ? ONE_LAUNCH_GRAD : ONE_LAUNCH_NO_GRAD);
     mark(stream);
     {
         ScanParams sp{};
@@ -941,14 +945,14 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     mark(stream);
     }
     set_dbg(p.g, 7, chunks);
-    SD_LAUNCH_KINDS(k_exterior_pair, k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM);
+    SD_LAUNCH_KINDS(k_exterior_pair, k_exterior_pair_bwd, EXT_PAIR_BWD_SMEM, ONE_LAUNCH_GRAD);
     mark(stream);
     }
     set_dbg(p.g, 8, chunks);
     if (po)
         k_primal_bwd<false, true, true><<<chunks, NTHREADS, PRIMAL_BWD_SMEM, stream>>>(p, chunks);
     else
-        SD_LAUNCH_KINDS(k_primal, k_primal_bwd, PRIMAL_BWD_SMEM);
+        SD_LAUNCH_KINDS(k_primal, k_primal_bwd, PRIMAL_BWD_SMEM, ONE_LAUNCH_GRAD);
     mark(stream);
     {
         ScanParamsB sp{};
@@ -963,7 +967,7 @@ int backward_impl(const sd_backward_args* a, void* stream_, const PredictorOnly*
     if (po)
         k_predictor_close_bwd<false, true, true><<<chunks, NTHREADS, PRED_CLOSE_BWD_SMEM, stream>>>(p, chunks);
     else
-        SD_LAUNCH_KINDS(k_predictor_close, k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM);
+        SD_LAUNCH_KINDS(k_predictor_close, k_predictor_close_bwd, PRED_CLOSE_BWD_SMEM, ONE_LAUNCH_GRAD);
     mark(stream);
     return launch_status();
 }

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import solvedelta_oracle as orc
-from solvedelta_b200 import SolveDeltaState, solvedelta_native
+from solvedelta_b200 import SolveDeltaState, solvedelta_masked_native, solvedelta_native
 from tests.gpu_harness import RawRun, make_inputs, oracle_args, oracle_state, raw_gate_grads
 from tests.test_gpu_parity import _check_forward, _check_vjp, _masked_case, _native
 
@@ -149,6 +149,24 @@ def test_slow_chunks_cost_their_own_work():
     fast = milliseconds()
     x["log_decay"] -= 1.3
     assert milliseconds() < 1.8 * fast
+
+
+@pytest.mark.parametrize("B,T,H", [(11, 150, 1), (37, 200, 1), (1, 64 * 149, 1)])   # 33, 148 and 149 chunks
+@pytest.mark.parametrize("masked", [False, True])
+def test_calls_without_gradients_give_the_bits_of_those_with(B, T, H, masked):
+    """Both kinds of chunk in one launch up to 148 chunks without gradients, up to 32 with them: the same results."""
+    x, _, gen = _device_case(B, T, H, 32, 48, 71)
+    x["log_decay"] -= 1.5 * (torch.rand(B, T // 50 + 1, 1, H, 1, generator=gen, device="cuda") < 0.3).expand(
+        -1, -1, 50, -1, -1).reshape(B, -1, H, 1)[:, :T]
+    masks = dict(valid_mask=torch.rand(B, T, generator=gen, device="cuda") < 0.9,
+                 reset_mask=torch.rand(B, T, generator=gen, device="cuda") < 0.01) if masked else {}
+    masks = {n: m & masks["valid_mask"] for n, m in masks.items()}
+    call = solvedelta_masked_native if masked else solvedelta_native
+    leaves = [x[n].detach().requires_grad_() for n in NAMES]
+    y, fin = call(*leaves, **masks, return_final_state=True)
+    with torch.no_grad():
+        bare, end = call(*leaves, **masks, return_final_state=True)
+    assert torch.equal(bare, y) and all(torch.equal(a, b) for a, b in zip(end, fin))
 
 
 @pytest.mark.parametrize("r,V", [(128, 128), (20, 12)])
