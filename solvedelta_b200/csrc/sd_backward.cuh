@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_exterior_prep_bwd(BwdParams p) 
     __syncthreads();
     SD_PHASE(p.g, ph);
     trisolve_blocked<true>(f_aedT, -1.f, PanelBF16{b_dy, b_dt});
+    __syncthreads();
     SD_PHASE(p.g, ph);
     s2g_bpanel(bpanel_ptr(p.Pp, ch.gi), b_dy);
     s2g_bpanel(bpanel_ptr(p.Qp, ch.gi), b_dt);
@@ -779,6 +780,7 @@ __device__ __forceinline__ void primal_blocks(const BwdParams& p, const ChunkT<M
     __syncthreads();
     SD_PHASE(p.g, ph);
     trisolve_blocked<true>(f_lmT, 1.f, PanelBF16{b_dl, b_ub});
+    __syncthreads();
     SD_PHASE(p.g, ph);
     s2g_bpanel(bpanel_ptr(p.Ppp, ch.gi), b_dl);
     s2g_bpanel(bpanel_ptr(p.Qpp, ch.gi), b_ub);

@@ -378,66 +378,6 @@ __device__ __forceinline__ void acc32_to_f32_tiles(const FastCta& cta, unsigned 
     }
 }
 
-// trisolve_blocked (sd_bf16.cuh) on two BF16 panels of tiles: each of the sixteen warps owns 16 of the 256 columns, pieces
-// piece0 and piece0 + 1 of `tile`.
-template <bool UPPER>
-__device__ __forceinline__ void trisolve_bf16_tiles(const FastCta& cta, float* Mr, float sgn, unsigned char* tile, int piece0) {
-    const int g = cta.lane >> 2, t = cta.lane & 3;
-    constexpr int NB = CL / 16, NT = 2;
-    if (cta.warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * cta.warp) * LDA + 16 * cta.warp, sgn);
-    __syncthreads();
-    auto at2 = [&](int i, int nt) {   // i mod 8 = g; columns 8 nt + 2 t, + 1
-        return reinterpret_cast<__nv_bfloat162*>(tile + i * 128 + (((piece0 + nt) ^ g) << 4) + (t << 2));
-    };
-    auto get = [&](int kk, int odd, int nt) {   // row kk + 2 t + odd, column 8 nt + g
-        return __bfloat162float(*reinterpret_cast<const bf16*>(tile + (kk + 2 * t + odd) * 128 + (((piece0 + nt) ^ (2 * t + odd)) << 4) + (g << 1)));
-    };
-    auto contract = [&](float (&acc)[NT][4], int r0, int kbeg, int kend) {
-#pragma unroll
-        for (int kk = kbeg; kk < kend; kk += 8) {   // permuted contraction index, as in warp_mma_pairs
-            const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
-            const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
-            const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)   // a BF16 number is a TF32 number
-                mma_tf32(acc[nt], a0, a1, a2, a3, __float_as_uint(get(kk, 0, nt)), __float_as_uint(get(kk, 1, nt)));
-        }
-    };
-#pragma unroll
-    for (int step = 0; step < NB; ++step) {
-        const int I = UPPER ? (NB - 1 - step) : step, r0 = 16 * I;
-        float rr[NT][4];
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const float2 a = __bfloat1622float2(*at2(r0 + g, nt)), b = __bfloat1622float2(*at2(r0 + g + 8, nt));
-            rr[nt][0] = a.x; rr[nt][1] = a.y; rr[nt][2] = b.x; rr[nt][3] = b.y;
-        }
-        if (step > 0) {
-            float acc[NT][4];
-            acc_zero<NT>(acc);
-            contract(acc, r0, UPPER ? r0 + 16 : 0, UPPER ? CL : r0);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) rr[nt][e] = fmaf(-sgn, acc[nt][e], rr[nt][e]);
-                *at2(r0 + g, nt) = __floats2bfloat162_rn(rr[nt][0], rr[nt][1]);
-                *at2(r0 + g + 8, nt) = __floats2bfloat162_rn(rr[nt][2], rr[nt][3]);
-            }
-            __syncwarp();
-        }
-        float acc[NT][4];
-        acc_zero<NT>(acc);
-        contract(acc, r0, r0, r0 + 16);
-        __syncwarp();   // every lane has read the block's right-hand sides
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            *at2(r0 + g, nt) = __floats2bfloat162_rn(rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
-            *at2(r0 + g + 8, nt) = __floats2bfloat162_rn(rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
-        }
-        __syncwarp();
-    }
-}
-
 // ---------------------------------------------------------------------------
 // k_primal_fast: reverse of the primal address and preparation of the dC scan (k_primal_bwd).  With DG = dd exp(G), Ucol =
 // u^ exp(-G) and the stack [K^; DG]:
@@ -679,7 +619,7 @@ __device__ __forceinline__ void primal_fast(const BwdParams& p, const ChunkT<MAS
     const int panel = cta.warp >> 3, cw = cta.warp & 7;
     unsigned char* tile = sm + (panel == 0 ? PB_RHS : PB_UC) + (cw >> 2) * BF_TILE;
     const int piece0 = (cw & 3) * 2;
-    trisolve_bf16_tiles<true>(cta, s_lm, 1.f, tile, piece0);
+    trisolve_blocked<true>(s_lm, 1.f, TileBF16{tile, piece0});
     SD_PHASE_T(p.g, ch, ph);
     bf16* out = (panel == 0 ? bpanel_ptr(p.Ppp, ch.gi) : bpanel_ptr(p.Qpp, ch.gi)) + 16 * cw;
 #pragma unroll

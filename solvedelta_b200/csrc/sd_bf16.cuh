@@ -192,8 +192,8 @@ constexpr size_t BSTATE_BYTES = size_t(DP) * LDB * 2;  // a whole state in BF16
 struct PanelF32 {
     float* p0;
     float* p1;
-    __device__ __forceinline__ float get(int k, int n) const {
-        return (n < DP ? p0 : p1)[k * LDP + (n & (DP - 1))];
+    __device__ __forceinline__ uint32_t operand(int k, int n) const {
+        return mma_tf32_bits((n < DP ? p0 : p1)[k * LDP + (n & (DP - 1))]);
     }
     __device__ __forceinline__ float2 get2(int i, int n) const {
         return *reinterpret_cast<const float2*>((n < DP ? p0 : p1) + i * LDP + (n & (DP - 1)));
@@ -205,8 +205,8 @@ struct PanelF32 {
 struct PanelBF16 {
     bf16* p0;
     bf16* p1;
-    __device__ __forceinline__ float get(int k, int n) const {
-        return __bfloat162float((n < DP ? p0 : p1)[k * LDB + (n & (DP - 1))]);
+    __device__ __forceinline__ uint32_t operand(int k, int n) const {   // a BF16 number is a TF32 number
+        return __float_as_uint(__bfloat162float((n < DP ? p0 : p1)[k * LDB + (n & (DP - 1))]));
     }
     __device__ __forceinline__ float2 get2(int i, int n) const {
         return __bfloat1622float2(
@@ -266,77 +266,61 @@ template <bool UPPER, class Panel>
 __device__ __forceinline__ void trisolve_blocked(float* Mr, float sgn, Panel P) {
     static_assert(NTHREADS == 2 * DP * 2, "16 warps of 16 right-hand-side columns each");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    constexpr int NB = CL / 16;
+    constexpr int NB = CL / 16, NT = 2;
     if (warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * warp) * LDA + 16 * warp, sgn);
     __syncthreads();
-    // ---- warp-local sweep over this warp's 16 columns ---------------------------------
     const int n0 = 16 * warp;
+    // acc += Mr[r0 .. r0 + 15][kbeg .. kend - 1] X[kbeg .. kend - 1][the warp's columns]
+    auto contract = [&](float (&acc)[NT][4], int r0, int kbeg, int kend) {
+#pragma unroll
+        for (int kk = kbeg; kk < kend; kk += 8) {   // permuted contraction index, as in warp_mma_pairs
+            const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
+            const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
+            const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+                mma_tf32(acc[nt], a0, a1, a2, a3, P.operand(kk + 2 * t, n0 + nt * 8 + g), P.operand(kk + 2 * t + 1, n0 + nt * 8 + g));
+        }
+    };
     // fully unrolled: every bound below is a compile-time constant, so the operand loads of a block run ahead
     // of the contractions that use them
 #pragma unroll
     for (int step = 0; step < NB; ++step) {
-        const int I = UPPER ? (NB - 1 - step) : step;
-        const int r0 = 16 * I;
-        float rr[2][4];
+        const int I = UPPER ? (NB - 1 - step) : step, r0 = 16 * I;
+        float rr[NT][4];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
+        for (int nt = 0; nt < NT; ++nt) {
             const int j = n0 + nt * 8 + 2 * t;
             const float2 a = P.get2(r0 + g, j), b = P.get2(r0 + g + 8, j);
             rr[nt][0] = a.x; rr[nt][1] = a.y; rr[nt][2] = b.x; rr[nt][3] = b.y;
         }
-        if (step > 0) {
-            // r = RHS[I] - sgn * Mr[I rows][solved cols] * X[solved rows]
-            const int kbeg = UPPER ? 16 * (I + 1) : 0;
-            const int kend = UPPER ? CL : 16 * I;
-            float acc[2][4];
-            acc_zero<2>(acc);
+        if (step > 0) {   // r = RHS[I] - sgn * Mr[I rows][solved cols] * X[solved rows]
+            float acc[NT][4];
+            acc_zero<NT>(acc);
+            contract(acc, r0, UPPER ? r0 + 16 : 0, UPPER ? CL : r0);
 #pragma unroll
-            for (int kk = kbeg; kk < kend; kk += 8) {
-                // permuted contraction index, as in warp_mma_pairs
-                const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
-                const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
-                const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-                    mma_tf32(acc[nt], a0, a1, a2, a3, mma_tf32_bits(P.get(kk + 2 * t, n0 + nt * 8 + g)),
-                             mma_tf32_bits(P.get(kk + 2 * t + 1, n0 + nt * 8 + g)));
-            }
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
+            for (int nt = 0; nt < NT; ++nt) {
+                const int j = n0 + nt * 8 + 2 * t;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) rr[nt][e] = fmaf(-sgn, acc[nt][e], rr[nt][e]);
-                const int j = n0 + nt * 8 + 2 * t;
                 P.put2(r0 + g, j, rr[nt][0], rr[nt][1]);
                 P.put2(r0 + g + 8, j, rr[nt][2], rr[nt][3]);
             }
             __syncwarp();
         }
-        {
-            // X[I] = r + D_I r : the block's own rows, K = 16 (the identity part stays in FP32 registers)
-            float acc[2][4];
-            acc_zero<2>(acc);
+        // X[I] = r + D_I r : the block's own rows, K = 16 (the identity part stays in FP32 registers)
+        float acc[NT][4];
+        acc_zero<NT>(acc);
+        contract(acc, r0, r0, r0 + 16);
+        __syncwarp();   // every lane has read the block's right-hand sides
 #pragma unroll
-            for (int kk = 0; kk < 16; kk += 8) {
-                const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + r0 + kk + 2 * t);
-                const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + r0 + kk + 2 * t);
-                const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    const uint32_t b0 = mma_tf32_bits(P.get(r0 + kk + 2 * t, n0 + nt * 8 + g));
-                    const uint32_t b1 = mma_tf32_bits(P.get(r0 + kk + 2 * t + 1, n0 + nt * 8 + g));
-                    mma_tf32(acc[nt], a0, a1, a2, a3, b0, b1);
-                }
-            }
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                const int j = n0 + nt * 8 + 2 * t;
-                P.put2(r0 + g, j, rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
-                P.put2(r0 + g + 8, j, rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
-            }
-            __syncwarp();
+        for (int nt = 0; nt < NT; ++nt) {
+            const int j = n0 + nt * 8 + 2 * t;
+            P.put2(r0 + g, j, rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
+            P.put2(r0 + g + 8, j, rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
         }
+        __syncwarp();
     }
-    __syncthreads();
 }
 
 }  // namespace sd

@@ -313,66 +313,31 @@ __device__ __forceinline__ void tc_st4(unsigned taddr, const float (&r)[4]) {
                  : "memory");
 }
 
-// ---- unit-triangular solve ----------------------------------------------------------
-// trisolve_blocked (sd_bf16.cuh) on FP32 tiles: after the four diagonal blocks are inverted, each of the sixteen warps
-// owns 16 of the 256 right-hand-side columns, half of a tile, and never waits for another warp.
-template <bool UPPER>
-__device__ __forceinline__ void trisolve_tiles(const FastCta& cta, float* Mr, float sgn, unsigned char* tile) {
-    const int g = cta.lane >> 2, t = cta.lane & 3, h4 = (cta.warp & 1) * 4;   // first 16-byte piece of this warp's half
-    constexpr int NB = CL / 16, NT = 2;
-    if (cta.warp < NB) invert_diagonal_block<UPPER>(Mr + (16 * cta.warp) * LDA + 16 * cta.warp, sgn);
-    __syncthreads();
-    auto at2 = [&](int i, int nt) {   // i mod 8 = g
-        return reinterpret_cast<float2*>(tile + i * 128 + (((h4 + nt * 2 + (t >> 1)) ^ g) << 4) + ((t & 1) << 3));
-    };
-    auto get = [&](int kk, int odd, int nt) {   // row kk + 2 t + odd, column 8 nt + g
-        return *reinterpret_cast<const float*>(tile + (kk + 2 * t + odd) * 128 + (((h4 + nt * 2 + (g >> 2)) ^ (2 * t + odd)) << 4) + ((g & 3) << 2));
-    };
-    auto contract = [&](float (&acc)[NT][4], int r0, int kbeg, int kend) {
-#pragma unroll
-        for (int kk = kbeg; kk < kend; kk += 8) {   // permuted contraction index, as in warp_mma_pairs
-            const float2 lo = *reinterpret_cast<const float2*>(Mr + (r0 + g) * LDA + kk + 2 * t);
-            const float2 hi = *reinterpret_cast<const float2*>(Mr + (r0 + g + 8) * LDA + kk + 2 * t);
-            const uint32_t a0 = mma_tf32_bits(lo.x), a1 = mma_tf32_bits(hi.x), a2 = mma_tf32_bits(lo.y), a3 = mma_tf32_bits(hi.y);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-                mma_tf32(acc[nt], a0, a1, a2, a3, mma_tf32_bits(get(kk, 0, nt)), mma_tf32_bits(get(kk, 1, nt)));
-        }
-    };
-#pragma unroll
-    for (int step = 0; step < NB; ++step) {
-        const int I = UPPER ? (NB - 1 - step) : step, r0 = 16 * I;
-        float rr[NT][4];
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const float2 a = *at2(r0 + g, nt), b = *at2(r0 + g + 8, nt);
-            rr[nt][0] = a.x; rr[nt][1] = a.y; rr[nt][2] = b.x; rr[nt][3] = b.y;
-        }
-        if (step > 0) {
-            float acc[NT][4];
-            acc_zero<NT>(acc);
-            contract(acc, r0, UPPER ? r0 + 16 : 0, UPPER ? CL : r0);
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) rr[nt][e] = fmaf(-sgn, acc[nt][e], rr[nt][e]);
-                *at2(r0 + g, nt) = make_float2(rr[nt][0], rr[nt][1]);
-                *at2(r0 + g + 8, nt) = make_float2(rr[nt][2], rr[nt][3]);
-            }
-            __syncwarp();
-        }
-        float acc[NT][4];
-        acc_zero<NT>(acc);
-        contract(acc, r0, r0, r0 + 16);
-        __syncwarp();   // every lane has read the block's right-hand sides
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            *at2(r0 + g, nt) = make_float2(rr[nt][0] + acc[nt][0], rr[nt][1] + acc[nt][1]);
-            *at2(r0 + g + 8, nt) = make_float2(rr[nt][2] + acc[nt][2], rr[nt][3] + acc[nt][3]);
-        }
-        __syncwarp();
+// ---- unit-triangular solve (trisolve_blocked) --------------------------------------
+// A warp's 16 right-hand-side columns in an FP32 tile: half of it, from 16-byte piece h4 on.  Columns modulo 16.
+struct TileF32 {
+    unsigned char* tile;
+    int h4;
+    __device__ __forceinline__ float* at(int i, int n) const {
+        return reinterpret_cast<float*>(tile + i * 128 + (((h4 + ((n >> 2) & 3)) ^ (i & 7)) << 4) + ((n & 3) << 2));
     }
-}
+    __device__ __forceinline__ uint32_t operand(int k, int n) const { return mma_tf32_bits(*at(k, n)); }
+    __device__ __forceinline__ float2 get2(int i, int n) const { return *reinterpret_cast<const float2*>(at(i, n)); }
+    __device__ __forceinline__ void put2(int i, int n, float v0, float v1) const { *reinterpret_cast<float2*>(at(i, n)) = make_float2(v0, v1); }
+};
+// ... and in a BF16 tile: its pieces piece0 and piece0 + 1
+struct TileBF16 {
+    unsigned char* tile;
+    int piece0;
+    __device__ __forceinline__ bf16* at(int i, int n) const {
+        return reinterpret_cast<bf16*>(tile + i * 128 + (((piece0 + ((n >> 3) & 1)) ^ (i & 7)) << 4) + ((n & 7) << 1));
+    }
+    __device__ __forceinline__ uint32_t operand(int k, int n) const { return __float_as_uint(__bfloat162float(*at(k, n))); }
+    __device__ __forceinline__ float2 get2(int i, int n) const { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(at(i, n))); }
+    __device__ __forceinline__ void put2(int i, int n, float v0, float v1) const {
+        *reinterpret_cast<__nv_bfloat162*>(at(i, n)) = __floats2bfloat162_rn(v0, v1);
+    }
+};
 // The warp's solved half tile to its 16 columns of a dense global panel.
 template <bool TF32>
 __device__ __forceinline__ void store_half_tile(const FastCta& cta, float* g, const unsigned char* tile) {

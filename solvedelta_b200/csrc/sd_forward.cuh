@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_prep_fwd(FwdParams p) {
     __syncthreads();
     SD_PHASE(p.g, ph);
     trisolve_blocked<false>(s_lm, 1.f, PanelF32{s_B, s_A});
+    __syncthreads();
     SD_PHASE(p.g, ph);
     float* gUpd = panel_ptr(p.Upd, ch.gi);
     float* gQc = panel_ptr(p.Qc, ch.gi);
@@ -579,6 +580,7 @@ __device__ __forceinline__ void primal_exterior_blocks(const FwdParams& p, const
     __syncthreads();
     SD_PHASE(p.g, ph);
     trisolve_blocked<false>(s_aed, -1.f, PanelF32{s_ag, s_z});
+    __syncthreads();
     SD_PHASE(p.g, ph);
     s2g_panel_tf32(panel_ptr(p.Wd, ch.gi), s_ag);   // a contraction operand of the state scan
     s2g_panel(panel_ptr(p.Ud, ch.gi), s_z);

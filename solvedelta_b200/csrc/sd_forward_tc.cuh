@@ -331,7 +331,7 @@ __device__ __forceinline__ void primal_exterior_fast(const FwdParams& p, const C
     SD_PHASE_T(p.g, ch, ph);
     const int panel = cta.warp >> 3, pt = (cta.warp >> 1) & 3;
     unsigned char* tile = (panel == 0 ? S2 : S0) + pt * F32_TILE;
-    trisolve_tiles<false>(cta, s_aed, -1.f, tile);
+    trisolve_blocked<false>(s_aed, -1.f, TileF32{tile, (cta.warp & 1) * 4});
     SD_PHASE_T(p.g, ch, ph);
     if (panel == 0)
         store_half_tile<true>(cta, panel_ptr(p.Wd, ch.gi) + 32 * pt, tile);   // a contraction operand of the state scan
