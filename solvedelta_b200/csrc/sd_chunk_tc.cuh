@@ -5,9 +5,13 @@
 // and a column factor exp(-G_j) <= e^60, both far inside the range of FP32, TF32 and BF16 (which share their exponent),
 // so a pair matrix is ONE contraction over all channels and a causal or anti-causal sum ONE contraction over all tokens,
 // masked by a select.  Such chunks take tcgen05 in the kernels named *_fast; a chunk that forgets more, or holds a reset,
-// takes the block-centred kernels (sd_decay.cuh), which walk over the slow chunks of a launch with one CTA per SM.  The
+// takes the block-centred kernels (sd_decay.cuh), whose CTAs, one per SM, share the slow chunks of a launch.  The
 // choice is made per chunk by k_prep_fwd, which stores it in the chunk's flag word: from what the chunk itself holds, so it
 // does not depend on what else is in the call.
+//
+// A NaN or an infinity of one token reaches all tokens of its chunk, earlier ones too: in a causal sum over the chunk it meets
+// the zeros of the mask, and zero times NaN is NaN.  (In the block-centred kernels the primal address of its own 16 tokens; y
+// passes through such a sum, k_output_fwd_tc, after either.)  Nothing before its chunk is touched by it.
 //
 // A chunk is a chain of loads, contractions, row passes and a solve, each of which leaves most of an SM idle: what counts
 // is the length of that chain and how many chains share the SM.  The fast kernels run one chunk a CTA of 16 warps, two CTAs

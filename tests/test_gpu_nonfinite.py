@@ -59,3 +59,18 @@ def test_nan_reaches_what_it_reaches_in_the_checker(name, bits, r, V):
     assert np.array_equal(y[1], clean[0][1]) and np.array_equal(y[0, :, 1 - HEAD], clean[0][0, :, 1 - HEAD])
     if name not in ("C0", "S0"):
         assert np.array_equal(y[0, :64, HEAD], clean[0][0, :64, HEAD])
+
+
+@pytest.mark.parametrize("name", ["u", "h", "keys", "values", "log_decay", "erase_raw", "geometry_write"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_last_token_of_a_chunk_touches_nothing_before_the_chunk(name, bad):
+    """Sums over a chunk may carry a NaN to the chunk's earlier tokens (token 127 to 64 and on), but not further back."""
+    cpu, dev = make_inputs(B, T, H, 32, 48, seed=13)
+    args = lambda: [dev[n] for n in OPERANDS]
+    with torch.no_grad():
+        clean, _ = solvedelta_native(*args(), initial_state=SolveDeltaState(dev["C0"], dev["S0"]), return_final_state=True)
+        dev[name] = dev[name].clone()
+        dev[name][(0, 127, HEAD) + (0,) * (dev[name].ndim - 3)] = bad if name != "log_decay" else -abs(bad)
+        y, _ = solvedelta_native(*args(), initial_state=SolveDeltaState(dev["C0"], dev["S0"]), return_final_state=True)
+    assert torch.equal(y[0, :64, HEAD], clean[0, :64, HEAD])
+    assert torch.equal(y[1], clean[1]) and torch.equal(y[0, :, 1 - HEAD], clean[0, :, 1 - HEAD])
